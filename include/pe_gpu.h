@@ -134,10 +134,10 @@ int pe_gpu_set_contact_margin(pe_gpu_world* w, double margin);
  * the defaults are those below. */
 typedef struct pe_gpu_tuning {
     int sat_heavy_cost;       /* SAT pairs whose estimated work reaches this run on a block of warps (200000) */
-    int small_island_items;   /* islands up to this many items run on one thread each, 0..64 (8) */
-    int big_island_items;     /* islands above this many items are coloured and solved grid-wide (4096) */
-    int color_block;          /* threads per island block in coloured mode, 32..256, multiple of 32 (64) */
-    int level_block;          /* threads per island block in serial-order mode, 32..256, multiple of 32 (256) */
+    int small_island_items;   /* islands up to this many items count no colours, 0..64 (8) */
+    int big_island_items;     /* coloured mode: islands above this many items may run by first-fit colour (4096) */
+    int color_block;          /* accepted, 32..256, multiple of 32 (64); no kernel has island blocks any more */
+    int level_block;          /* as color_block (256) */
     int exact_levels_colored; /* coloured mode keeps a big island's exact levels up to this many, 0..1023 (512) */
     int scene_sort_max;       /* scenes up to this many bodies are sorted inside one block, 0..2048 (2048) */
     int side_streams;         /* streams for the narrowphase's per-class kernels, 1..4 (4) */

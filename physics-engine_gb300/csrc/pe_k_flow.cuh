@@ -1,0 +1,488 @@
+// Kernels of the rigid-body step, part 6: the solver's iterations, run as a flow of body velocities
+// between island items.
+//
+// An island's items (contact results, then joints) act on their two bodies' temporary velocities in
+// a fixed order.  Instead of running that order level by level with a barrier after every level, each
+// body's velocity is a token that its items hand on: an item runs once it holds the tokens of its
+// dynamic bodies, then passes each to the body's next item, the last one back to the first for the
+// next iteration.  Every body takes its updates in the same order as before, so the results are the
+// same bits, while different parts of an island, and its successive iterations, overlap: the steps
+// in a row are the longest chain of the unrolled order (472 for a 55,690-contact island of 304
+// levels and 10 iterations) instead of levels x iterations (3,040), and none waits for a barrier.
+//
+// Islands of up to kWarpIsland items run inside one warp with the tokens in shared memory
+// (k_isl_warp); larger ones over the whole grid with the tokens in global memory (k_isl_flow).
+#pragma once
+#include "pe_k_solver.cuh"
+
+namespace pe {
+
+constexpr int kMaxColors = 512;      // colours reported for an island of up to big_island_items items
+constexpr int kMaxColorsBig = 1024;  // first-fit colours of a bigger island, the last one for leftovers
+
+// an item's dynamic bodies, loaded with everything but the velocities
+template <class R, bool JOINTS> struct Item {
+    uint32_t id;
+    int ia, ib, r0, np;
+    Side<R> a, b;
+    __device__ __forceinline__ void load(uint32_t item, const Results<R>& res, const Joints<R>& J, const Bodies<R>& B, const int* row_off) {
+        id = item;
+        if (JOINTS && (item & kJointItem)) {
+            const int2 q = J.body[item & ~kJointItem];
+            ia = q.x; ib = q.y; r0 = 0; np = 0;
+        } else {
+            ia = res.a[item]; ib = res.b[item]; r0 = row_off[item]; np = res.npts[item];
+        }
+        a.load(B, ia);
+        b.load(B, ib);
+    }
+    __device__ __forceinline__ void iterate(const Joints<R>& J, const Rows<R>& rows) {
+        if (JOINTS && (id & kJointItem)) joint_iterate(J, (int)(id & ~kJointItem), a, b);
+        else si_rows(rows, r0, np, a, b);
+    }
+};
+
+// ---------------------------------------------------------------- islands inside a warp
+// Islands of up to kWarpIsland items, listed by size class: 1, 2, 3-4, 5-8, 9-16 and 17-32 items, so
+// that a warp works on islands of about one length (32, 16, 8, 4, 2 or 1 of them), one lane per item.
+constexpr int kWarpIsland = 32, kWarpClasses = 6, kWarpBlock = 128;
+__host__ __device__ inline int warp_class(int m) { return m <= 1 ? 0 : m <= 2 ? 1 : m <= 4 ? 2 : m <= 8 ? 3 : m <= 16 ? 4 : 5; }
+// first slot of class c in the island list: a class holds at most bound / (its smallest size) islands
+__host__ __device__ inline long long class_base(int c, long long bound) {
+    const int least[kWarpClasses] = {1, 2, 3, 5, 9, 17};
+    long long at = 0;
+    for (int k = 0; k < c; k++) at += bound / least[k] + 1;
+    return at;
+}
+// Sorts the islands into the size classes' lists; an island that a warp does not take (more than
+// kWarpIsland items, or above big_items, which k_isl_flow may have to colour) gets a range of flow
+// items at base[island]; those above big_items are also listed in big.
+__global__ void k_isl_classes(const int* n_isl, const int* isl_off, int bound, int big_items, int* list, int* n_list, int* base, int* n_flow,
+                              int* big, int* n_big);
+
+// One lane per item, tokens in shared memory.  A round runs every item whose tokens are there; what
+// bounds it is the chain of dependent rows of the longest island of the warp, which the rounds follow
+// item by item.  The lanes find their bodies' next items by comparing bodies across their island.
+// (One thread per island of up to 16 items, the larger ones a block each with a barrier per level:
+// 266 + 150 us of the 501-body pile's step, 1,448 + 718 us of the 4,096 piles'; together with the
+// item-sized islands in one kernel here the steps are 309 us and 1.24 ms shorter.)
+template <class R, bool JOINTS>
+__global__ void __launch_bounds__(kWarpBlock, sizeof(R) == 4 ? 4 : 2)
+k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, const uint32_t* order, Results<R> res, Joints<R> J, Bodies<R> B,
+           Rows<R> rows, const int* row_off, int iterations, int color_min, int* n_colors, int* status) {
+    constexpr int W = kWarpBlock / 32;
+    __shared__ R tok_v[W][2][6][32];     // per side and lane: the token's linear and angular velocity
+    __shared__ int tok_it[W][2][32];     // the iteration the token is for
+    __shared__ int tok_lev[W][2][32];    // its level (the first iteration's)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    int units[kWarpClasses], total = 0;
+#pragma unroll
+    for (int c = kWarpClasses - 1; c >= 0; c--) {   // the longest islands first
+        const int per = 32 >> c;
+        units[c] = (n_list[c] + per - 1) / per;
+        total += units[c];
+    }
+    const int its = iterations > 0 ? iterations : 1;   // without iterations the levels are still counted
+    int deepest = 0;
+    for (int u = blockIdx.x * W + warp; u < total; u += gridDim.x * W) {
+        int c = kWarpClasses - 1, k = u;
+        while (k >= units[c]) { k -= units[c]; c--; }
+        const int s = 1 << c;
+        const int li = k * (32 >> c) + (lane >> c), idx = lane & (s - 1), g0 = lane - idx;
+        int lo = 0, m = 0;
+        if (li < n_list[c]) {
+            const int isl = list[class_base(c, bound) + li];
+            lo = isl_off[isl];
+            m = isl_off[isl + 1] - lo;
+        }
+        const bool active = idx < m;
+        Item<R, JOINTS> t;
+        t.ia = -1; t.ib = -1;
+        if (active) t.load(order[lo + idx], res, J, B, row_off);
+        // the island's items on this item's bodies (bit per item), and on which side they hold them
+        const int da = active && !t.a.kin ? t.ia : -2, db = active && !t.b.kin ? t.ib : -2;
+        unsigned ma = 0, mab = 0, mb = 0, mbb = 0;
+        for (int j = 0; j < s; j++) {
+            const int oa = __shfl_sync(full, t.ia, g0 + j), ob = __shfl_sync(full, t.ib, g0 + j);
+            const unsigned bit = 1u << j;
+            if (oa == da) ma |= bit;
+            if (ob == da) { ma |= bit; mab |= bit; }
+            if (oa == db) mb |= bit;
+            if (ob == db) { mb |= bit; mbb |= bit; }
+        }
+        const unsigned before = (1u << idx) - 1u, after = ~(before | (1u << idx));
+        const bool wrap_a = (ma & after) == 0, wrap_b = (mb & after) == 0;
+        const int na = active && !t.a.kin ? __ffs(wrap_a ? ma : ma & after) - 1 : 0, nb = active && !t.b.kin ? __ffs(wrap_b ? mb : mb & after) - 1 : 0;
+        const int sa = (mab >> na) & 1, sb = (mbb >> nb) & 1;
+        const bool keep_a = na == idx, keep_b = nb == idx;   // the body's only item: its token stays in registers
+        tok_it[warp][0][lane] = tok_it[warp][1][lane] = -1;
+        int lev_a = 0, lev_b = 0;
+        bool have_a = !active || t.a.kin, have_b = !active || t.b.kin;
+        if (active && !t.a.kin && (ma & before) == 0) { t.a.v = B.vec(VX, t.ia); t.a.w = B.vec(WX, t.ia); have_a = true; }
+        if (active && !t.b.kin && (mb & before) == 0) { t.b.v = B.vec(VX, t.ib); t.b.w = B.vec(WX, t.ib); have_b = true; }
+        int it = active ? 0 : its;
+        __syncwarp();
+        while (__any_sync(full, it < its)) {
+            if (it < its) {
+                auto take = [&](int side, Side<R>& x, int& lev) {
+                    if (tok_it[warp][side][lane] != it) return false;
+                    const R* v = &tok_v[warp][side][0][lane];
+                    x.v = V3<R>(v[0], v[32], v[64]);
+                    x.w = V3<R>(v[96], v[128], v[160]);
+                    lev = tok_lev[warp][side][lane];
+                    return true;
+                };
+                if (!have_a) have_a = take(0, t.a, lev_a);
+                if (!have_b) have_b = take(1, t.b, lev_b);
+            }
+            const bool run = it < its && have_a && have_b;
+            if (!__any_sync(full, run)) {   // some item always holds its tokens
+                if (lane == 0) atomicOr(status, ST_FLOW_STALL);
+                break;
+            }
+            // (the vote also puts every read of this round's tokens before its writes)
+            if (run) {
+                if (iterations > 0) t.iterate(J, rows);
+                const int lev = (lev_a > lev_b ? lev_a : lev_b) + 1;
+                if (it == 0 && m > color_min) deepest = deepest > lev ? deepest : lev;
+                auto give = [&](Side<R>& x, int i, bool wrap, int nl, int side, bool keep, bool& have) {
+                    if (x.kin) return;
+                    if (wrap && it == its - 1) {
+                        B.set_vec(VX, i, x.v);
+                        B.set_vec(WX, i, x.w);
+                        return;
+                    }
+                    if (keep) return;
+                    R* v = &tok_v[warp][side][0][g0 + nl];
+                    v[0] = x.v.x; v[32] = x.v.y; v[64] = x.v.z;
+                    v[96] = x.w.x; v[128] = x.w.y; v[160] = x.w.z;
+                    tok_lev[warp][side][g0 + nl] = lev;
+                    tok_it[warp][side][g0 + nl] = it + (wrap ? 1 : 0);
+                    have = false;
+                };
+                give(t.a, t.ia, wrap_a, na, sa, keep_a, have_a);
+                give(t.b, t.ib, wrap_b, nb, sb, keep_b, have_b);
+                it++;
+            }
+            __syncwarp();
+        }
+    }
+    if (n_colors) {
+        deepest = __reduce_max_sync(full, deepest < kMaxColors ? deepest : kMaxColors);
+        if (lane == 0 && deepest > 0) atomicMax(n_colors, deepest);
+    }
+}
+
+// ---------------------------------------------------------------- islands over the grid
+// A token in global memory: 16-byte words of three payload words and a tag, each word stored and
+// loaded whole (128-bit accesses), so that a reader that finds the tag it waits for in every word
+// has the token, without a fence between payload and flag.  The tag is the iteration + 1; during the
+// first iteration the last word's tag carries the level instead, with the top bit set.
+template <class R> constexpr int token_words() { return 6 * (int)sizeof(R) / 12; }
+__device__ __forceinline__ void st_word(uint4* p, uint4 w) {
+    const unsigned long long lo = (unsigned long long)w.x | (unsigned long long)w.y << 32, hi = (unsigned long long)w.z | (unsigned long long)w.w << 32;
+    asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ uint4 ld_word(const uint4* p) {
+    unsigned long long lo, hi;
+    asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+}
+constexpr unsigned kLevelTag = 0x80000000u;
+template <class R> __device__ __forceinline__ void token_put(uint4* box, const Side<R>& x, int it, int lev) {
+    constexpr int NW = token_words<R>();
+    union { R r[6]; unsigned u[3 * NW]; } q;
+    q.r[0] = x.v.x; q.r[1] = x.v.y; q.r[2] = x.v.z; q.r[3] = x.w.x; q.r[4] = x.w.y; q.r[5] = x.w.z;
+    const unsigned tag = (unsigned)it + 1u;
+#pragma unroll
+    for (int k = 0; k < NW; k++)
+        st_word(box + k, make_uint4(q.u[3 * k], q.u[3 * k + 1], q.u[3 * k + 2], k == NW - 1 && it == 0 ? kLevelTag | (unsigned)lev : tag));
+}
+template <class R> __device__ __forceinline__ bool token_get(const uint4* box, Side<R>& x, int it, int& lev) {
+    constexpr int NW = token_words<R>();
+    union { R r[6]; unsigned u[3 * NW]; } q;
+    const unsigned tag = (unsigned)it + 1u;
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+        const uint4 w = ld_word(box + k);
+        q.u[3 * k] = w.x; q.u[3 * k + 1] = w.y; q.u[3 * k + 2] = w.z;
+        if (k == NW - 1 && it == 0) {
+            ok = ok && (w.w & kLevelTag);
+            lev = (int)(w.w & ~kLevelTag);
+        } else {
+            ok = ok && w.w == tag;
+        }
+    }
+    if (!ok) return false;
+    x.v = V3<R>(q.r[0], q.r[1], q.r[2]);
+    x.w = V3<R>(q.r[3], q.r[4], q.r[5]);
+    return true;
+}
+
+template <class R> struct FlowArgs {
+    const int* n_items;        // island items (contacts and joints) in the sorted order
+    const int* isl_scan;       // island starts before each sorted item
+    const int* isl_off;
+    const uint32_t* order;
+    const int* base;           // first flow item of each island that a warp does not take
+    const int* n_flow;         // flow items
+    const int* big;            // islands above big_items
+    const int* n_big;
+    int big_items, color_min, exact_levels, mode, iterations;
+    uint32_t* item;            // per flow item: the item,
+    int* isl;                  // its island,
+    int* color;                // and its first-fit colour, where its island runs in colour order
+    int* head;                 // per body: its entries (2 x flow item + side) as a list
+    int* next;                 // per entry: the list's next entry
+    int* succ;                 // per entry: 2 x (the entry its token goes to) + 1 when that is the next iteration's
+    uint4* box;                // per entry: its token
+    int* isl_levels;           // per island: levels,
+    int* isl_colors;           // first-fit colours in use,
+    int* isl_state;            // kFlowFirstFit, kFlowLeft
+    int* any_first_fit;
+    int* n_colors;
+    int* status;
+};
+constexpr int kFlowBlock = 128, kFlowFirstFit = 1, kFlowLeft = 2;
+constexpr int kFlowStall = 1 << 21;   // polls in a row without progress after which a warp gives up (seconds)
+
+// Islands that one warp does not take, all of them in one cooperative launch (a waiting item needs
+// the items it waits for to be resident).  Flow item j belongs to lane j mod `per` of warp j / per, with
+// as few lanes per warp as the item count allows: lanes of a warp run one after the other, and the
+// time is the latency of the longest chain, a hand-over through L2 plus one item's rows.  (A block
+// per island with a barrier per level, and one barrier over the whole grid per level for large
+// islands, took 3.4 and 11 us per level and iteration.)
+template <class R, bool JOINTS>
+__global__ void __launch_bounds__(kFlowBlock, sizeof(R) == 4 ? 4 : 2)
+k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows, const int* row_off) {
+    constexpr int NW = token_words<R>();
+    const int M = *f.n_flow;
+    if (M == 0) return;   // the same for every thread
+    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31, gw = t >> 5, GW = T >> 5;
+    const unsigned full = 0xffffffffu;
+    const int its = f.iterations > 0 ? f.iterations : 1;
+    const bool coloring = f.mode != 0 && *f.n_big > 0;
+    auto dynamic = [&](int i) { return (B.flags[i] & BF_KINEMATIC) == 0; };
+    auto island_size = [&](int s) { return f.isl_off[s + 1] - f.isl_off[s]; };
+
+    // the flow items, in island order
+    for (int k = t, n = *f.n_items; k < n; k += T) {
+        const int s = f.isl_scan[k + 1] - 1, lo = f.isl_off[s], b = f.base[s];
+        if (b < 0) continue;
+        const int j = b + k - lo;
+        const uint32_t id = f.order[k];
+        const int2 q = item_bodies(id, res, J);
+        f.item[j] = id;
+        f.isl[j] = s;
+        f.color[j] = 0;
+        f.head[q.x] = -1;
+        f.head[q.y] = -1;
+        if (k == lo) { f.isl_levels[s] = 0; f.isl_colors[s] = 0; f.isl_state[s] = 0; }
+    }
+    if (t == 0) *f.any_first_fit = 0;
+    grid.sync();
+    // every body's entries
+    for (int j = t; j < M; j += T) {
+        const int2 q = item_bodies(f.item[j], res, J);
+        if (dynamic(q.x)) f.next[2 * j] = atomicExch(&f.head[q.x], 2 * j);
+        if (dynamic(q.y)) f.next[2 * j + 1] = atomicExch(&f.head[q.y], 2 * j + 1);
+    }
+    grid.sync();
+    // Where each entry's token goes: the body's next entry by (colour, position), the first one after
+    // the last.  A body's first entry starts with its token: the velocity, or, where the island is to be
+    // coloured first, an empty colour mask.
+    auto link = [&](int e, int body, bool colors) {
+        auto key = [&](int en) { return (unsigned long long)(unsigned)f.color[en >> 1] << 32 | (unsigned)(en >> 1); };
+        const unsigned long long mine = key(e);
+        unsigned long long up = ~0ull, least = mine;
+        int eu = -1, el = e;
+        for (int en = f.head[body]; en >= 0; en = f.next[en]) {
+            const unsigned long long q = key(en);
+            if (q > mine && q < up) { up = q; eu = en; }
+            if (q < least) { least = q; el = en; }
+        }
+        f.succ[e] = eu >= 0 ? 2 * eu : 2 * el + 1;
+        uint4* box = f.box + (size_t)e * NW;
+        if (least != mine || colors)
+            for (int k = 0; k < NW; k++) box[k] = make_uint4(0, 0, 0, least == mine && k == 0 ? 1u : 0u);
+        else {
+            Side<R> x;
+            x.v = B.vec(VX, body);
+            x.w = B.vec(WX, body);
+            token_put(box, x, 0, 0);
+        }
+    };
+    for (int j = t; j < M; j += T) {
+        const int2 q = item_bodies(f.item[j], res, J);
+        const bool colors = coloring && island_size(f.isl[j]) > f.big_items;
+        if (dynamic(q.x)) link(2 * j, q.x, colors);
+        if (dynamic(q.y)) link(2 * j + 1, q.y, colors);
+    }
+    grid.sync();
+
+    const int per = min(32, max(1, (M + GW - 1) / GW)), stride = GW * per;
+    const int j0 = lane < per && gw * per + lane < M ? gw * per + lane : M;   // this lane's items: j0, j0 + stride, ..
+    int stall = 0;
+    // no progress in this round: give up after kFlowStall rounds (a lost token), else wait a little
+    // where many lanes poll
+    auto stalled = [&]() {
+        if (++stall > kFlowStall) {
+            if (lane == 0) atomicOr(f.status, ST_FLOW_STALL);
+            return true;
+        }
+        if (per > 4) __nanosleep(40);
+        return false;
+    };
+
+    if (coloring) {
+        // Levels and first-fit colours of the islands above big_items, passed on like velocities: an
+        // item's level is one above its bodies' (the round in which a colouring by rounds takes it), its
+        // colour the smallest that no earlier item of its bodies holds.  Islands within exact_levels
+        // levels keep the order of their items, the others run by colour.
+        int j = j0;
+        while (j < M && island_size(f.isl[j]) <= f.big_items) j += stride;
+        while (__any_sync(full, j < M)) {
+            bool moved = false;
+            if (j < M) {
+                const int2 q = item_bodies(f.item[j], res, J);
+                const bool da = dynamic(q.x), db = dynamic(q.y);
+                uint4 wa = make_uint4(0, 0, 0, 1), wb = wa;
+                if (da) wa = ld_word(f.box + (size_t)(2 * j) * NW);
+                if (db) wb = ld_word(f.box + (size_t)(2 * j + 1) * NW);
+                if (wa.w == 1u && wb.w == 1u) {
+                    const int s = f.isl[j], lev = (int)max(wa.x, wb.x);
+                    unsigned long long ka = (unsigned long long)wa.y | (unsigned long long)wa.z << 32;
+                    unsigned long long kb = (unsigned long long)wb.y | (unsigned long long)wb.z << 32;
+                    int c = kMaxColorsBig - 1;
+                    if (lev < kMaxColorsBig - 1) {
+                        const unsigned long long used = ka | kb;
+                        if (used != ~0ull) {
+                            c = __ffsll((long long)~used) - 1;
+                            ka |= 1ull << c;
+                            kb |= 1ull << c;
+                        }
+                        atomicMax(&f.isl_levels[s], lev + 1);
+                    } else {
+                        atomicOr(&f.isl_state[s], kFlowFirstFit);
+                    }
+                    if (c == kMaxColorsBig - 1) atomicOr(&f.isl_state[s], kFlowLeft);
+                    else atomicMax(&f.isl_colors[s], c + 1);
+                    f.color[j] = c;
+                    auto pass = [&](int e, unsigned long long k) {
+                        const int to = f.succ[e];
+                        if (!(to & 1)) st_word(f.box + (size_t)(to >> 1) * NW, make_uint4((unsigned)lev + 1u, (unsigned)k, (unsigned)(k >> 32), 1u));
+                    };
+                    if (da) pass(2 * j, ka);
+                    if (db) pass(2 * j + 1, kb);
+                    do j += stride; while (j < M && island_size(f.isl[j]) <= f.big_items);
+                    moved = true;
+                }
+            }
+            if (__any_sync(full, moved)) stall = 0;
+            else if (stalled()) break;
+        }
+        grid.sync();
+        for (int k = t; k < *f.n_big; k += T) {
+            const int s = f.big[k], lev = f.isl_levels[s];
+            const bool left = (f.isl_state[s] & kFlowLeft) != 0;
+            int used = lev;
+            if (lev > f.exact_levels || (f.isl_state[s] & kFlowFirstFit)) {
+                f.isl_state[s] |= kFlowFirstFit;
+                atomicOr(f.any_first_fit, 1);
+                used = (left ? lev : min(f.isl_colors[s], lev)) + (left ? 1 : 0);
+            }
+            atomicMax(f.n_colors, used);
+        }
+        grid.sync();
+        for (int j = t; j < M; j += T)
+            if (!(f.isl_state[f.isl[j]] & kFlowFirstFit)) f.color[j] = 0;   // item order
+        grid.sync();
+        for (int j = t; j < M; j += T) {
+            if (island_size(f.isl[j]) <= f.big_items) continue;
+            const int2 q = item_bodies(f.item[j], res, J);
+            if (dynamic(q.x)) link(2 * j, q.x, false);
+            if (dynamic(q.y)) link(2 * j + 1, q.y, false);
+        }
+        grid.sync();
+    }
+
+    const bool reorder = coloring && *(volatile int*)f.any_first_fit != 0;
+    const bool single = M <= stride;   // one item per lane: its constants stay in registers
+    Item<R, JOINTS> x;
+    int succ_a = 0, succ_b = 0, lev_a = 0, lev_b = 0, m = 0, deepest = 0;
+    bool have_a = false, have_b = false;
+    auto take_item = [&](int j) {
+        x.load(f.item[j], res, J, B, row_off);
+        have_a = x.a.kin;
+        have_b = x.b.kin;
+        if (!x.a.kin) succ_a = f.succ[2 * j];
+        if (!x.b.kin) succ_b = f.succ[2 * j + 1];
+        lev_a = 0;
+        lev_b = 0;
+        m = island_size(f.isl[j]);
+    };
+    // the lane's next item of the iteration, by position or by (colour, position); M after the last
+    auto next_item = [&](int j) {
+        if (!reorder) return j + stride < M ? j + stride : M;
+        auto key = [&](int i) { return (unsigned long long)(unsigned)f.color[i] << 32 | (unsigned)i; };
+        unsigned long long mine = j < M ? key(j) + 1 : 0ull, best = ~0ull;
+        int at = M;
+        for (int i = j0; i < M; i += stride) {
+            const unsigned long long k = key(i);
+            if (k >= mine && k < best) { best = k; at = i; }
+        }
+        return at;
+    };
+    int it = 0, j = single || !reorder ? j0 : next_item(M);
+    stall = 0;
+    if (j < M) take_item(j);
+    while (__any_sync(full, j < M)) {
+        bool moved = false;
+        if (j < M) {
+            if (!have_a) have_a = token_get(f.box + (size_t)(2 * j) * NW, x.a, it, lev_a);
+            if (!have_b) have_b = token_get(f.box + (size_t)(2 * j + 1) * NW, x.b, it, lev_b);
+            if (have_a && have_b) {
+                moved = true;
+                if (f.iterations > 0) x.iterate(J, rows);
+                const int lev = max(lev_a, lev_b) + 1;
+                auto give = [&](Side<R>& s, int i, int entry, int to, bool& have) {
+                    if (s.kin) return;
+                    if ((to & 1) && it == its - 1) {
+                        B.set_vec(VX, i, s.v);
+                        B.set_vec(WX, i, s.w);
+                    } else if (single && (to >> 1) == entry) {
+                        return;   // the body's only item: its token stays
+                    } else {
+                        token_put(f.box + (size_t)(to >> 1) * NW, s, it + (to & 1), lev);
+                    }
+                    have = false;
+                };
+                give(x.a, x.ia, 2 * j, succ_a, have_a);
+                give(x.b, x.ib, 2 * j + 1, succ_b, have_b);
+                if (it == 0) {
+                    if (m > f.big_items) { if (f.mode == 0) atomicMax(&f.isl_levels[f.isl[j]], lev); }
+                    else if (m > f.color_min) deepest = max(deepest, lev);
+                }
+                if (single) {
+                    if (++it == its) j = M;
+                } else {
+                    j = next_item(j);
+                    if (j >= M && ++it < its) j = reorder ? next_item(M) : j0;
+                    if (j < M) take_item(j);
+                }
+            }
+        }
+        if (__any_sync(full, moved)) stall = 0;
+        else if (stalled()) break;
+    }
+    if (f.mode != 0) {
+        deepest = __reduce_max_sync(full, deepest < kMaxColors ? deepest : kMaxColors);
+        if (lane == 0 && deepest > 0) atomicMax(f.n_colors, deepest);
+    }
+}
+
+} // namespace pe

@@ -1,6 +1,6 @@
-// Kernels of the rigid-body step, part 6: body-state transfer in the C ABI's layout.
+// Kernels of the rigid-body step, part 7: body-state transfer in the C ABI's layout.
 #pragma once
-#include "pe_k_solver.cuh"
+#include "pe_k_flow.cuh"
 
 namespace pe {
 

@@ -10,7 +10,6 @@ enum BodyField {
     OX = 0, OY, OZ,
     B00, B01, B02, B10, B11, B12, B20, B21, B22,
     VX, VY, VZ, WX, WY, WZ,
-    TVX, TVY, TVZ, TWX, TWY, TWZ,       // solver temporary velocities
     MNX, MNY, MNZ, MXX, MXY, MXZ,       // AABB
     I00, I01, I02, I10, I11, I12, I20, I21, I22,   // world inverse inertia
     L00, L01, L02, L10, L11, L12, L20, L21, L22,   // local inverse inertia
@@ -79,14 +78,12 @@ template <class R> struct Results {
     __host__ __device__ R& pt(int k, int slot) const { return pts[(size_t)k * cap * kSlots + slot]; }
 };
 
-// solver rows (FrictionContactConstraint::ConstraintInfo), field-major over [cap] rows
-enum RowField { RAX = 0, RAY, RAZ, RBX, RBY, RBZ, RNX, RNY, RNZ, R0X, R0Y, R0Z, R1X, R1Y, R1Z,
-                NRHS, NJMJ, T0JMJ, T1JMJ, MU, NACC, T0ACC, T1ACC, NRF };
-
+// solver rows (FrictionContactConstraint::ConstraintInfo), NRF consecutive reals per row (RowReg names
+// the fields; one is padding)
+constexpr int NRF = 24;
 template <class R> struct Rows {
     int cap;
     R* f;
-    __host__ __device__ R& at(int k, int i) const { return f[(size_t)k * cap + i]; }
 };
 
 // joint constraints (World::addConstraint, in order): Ball/Hinge/SliderJointConstraint
@@ -112,20 +109,20 @@ struct StepParams {
 
 // Scheduling settings of the step: which kernel takes which work and with how many threads.  In
 // serial-order mode no setting changes a result bit.  In coloured mode none does either while every
-// island needs at most exact_levels_colored levels (above, a big island takes first-fit colours and
-// a block-path island runs its leftover items last): the autotuner leaves that one setting alone.
+// island above big_island_items needs at most exact_levels_colored levels (one with more runs by
+// first-fit colour): the autotuner leaves that one setting alone.
 struct Tuning {
     int sat_heavy_cost = 200000;      // SAT pairs whose estimated work reaches this run on a block of warps
-    int small_island_items = 8;       // islands up to this many items run on one thread each
-    int big_island_items = 4096;      // islands above this many items are coloured and solved grid-wide
-    int color_block = 64;             // threads per island block, coloured mode
-    int level_block = 256;            // threads per island block, serial-order mode
+    int small_island_items = 8;       // islands up to this many items count no colours
+    int big_island_items = 4096;      // coloured mode: islands above this many items may run by first-fit colour
+    int color_block = 64;             // accepted; no kernel has island blocks any more
+    int level_block = 256;            // as color_block
     int exact_levels_colored = 512;   // coloured mode keeps a big island's exact levels up to this many
     int scene_sort_max = 2048;        // scenes up to this many bodies are sorted inside one block
     int side_streams = 4;             // streams the narrowphase's per-class kernels are spread over
 };
 
 // device status word bits
-enum StatusBits { ST_PAIR_OVERFLOW = 1, ST_ROW_OVERFLOW = 2, ST_COLOR_OVERFLOW = 4 };
+enum StatusBits { ST_PAIR_OVERFLOW = 1, ST_ROW_OVERFLOW = 2, ST_COLOR_OVERFLOW = 4, ST_FLOW_STALL = 8 };
 
 } // namespace pe

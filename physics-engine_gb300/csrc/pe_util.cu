@@ -247,65 +247,51 @@ __global__ void k_isl_offsets(const int* Md, const uint64_t* key, const int* sca
     }
 }
 
-// islands with more than big_items results
-__global__ void k_isl_big(const int* n_isl, const int* isl_off, int* big, int* n_big, int big_items) {
-    const int NI = *n_isl;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < NI; s += gridDim.x * blockDim.x)
-        if (isl_off[s + 1] - isl_off[s] > big_items) big[atomicAdd(n_big, 1)] = s;
+// Size classes of the islands (see k_isl_warp and k_isl_flow), one atomic per class present in a warp
+__global__ void k_isl_classes(const int* n_isl, const int* isl_off, int bound, int big_items, int* list, int* n_list, int* base, int* n_flow,
+                              int* big, int* n_big) {
+    const int NI = *n_isl, lane = threadIdx.x & 31;
+    for (int s0 = blockIdx.x * blockDim.x; s0 < NI; s0 += gridDim.x * blockDim.x) {
+        const int s = s0 + threadIdx.x;
+        int c = -1 - lane, m = 0;   // lanes without a warp-sized island match no other
+        if (s < NI) {
+            m = isl_off[s + 1] - isl_off[s];
+            if (m <= kWarpIsland && m <= big_items) c = warp_class(m);
+        }
+        const unsigned peers = __match_any_sync(0xffffffffu, c);
+        const int leader = __ffs(peers) - 1;
+        int at = 0;
+        if (c >= 0 && lane == leader) at = atomicAdd(&n_list[c], __popc(peers));
+        at = __shfl_sync(0xffffffffu, at, leader);
+        if (s >= NI) continue;
+        if (c >= 0) {
+            list[class_base(c, bound) + at + __popc(peers & ((1u << lane) - 1u))] = s;
+            base[s] = -1;
+        } else {
+            base[s] = atomicAdd(n_flow, m);
+            if (m > big_items) big[atomicAdd(n_big, 1)] = s;
+        }
+    }
 }
 
-// the step's counters gathered for one copy to the host (World::HostStat order; colours may be absent)
-__global__ void k_step_counters(const int* status, const int* rows, const int* active, const int* islands, const int* big, const int* colors,
-                                const int* cls, int* out) {
+// the step's counters gathered for one copy to the host (World::HostStat order).  Colours: those the
+// coloured mode counted; in serial order the levels of the islands above big_island_items, where they
+// are within the first-fit colours' number.
+__global__ void k_step_counters(const int* status, const int* rows, const int* active, const int* islands, const int* n_big, const int* big,
+                                const int* isl_levels, const int* colors, const int* cls, int* out) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     out[0] = *status;
     out[1] = *rows;
     out[2] = *active;
     out[3] = *islands;
-    out[4] = *big;
-    out[5] = colors ? *colors : 0;
+    out[4] = *n_big;
+    int used = colors ? *colors : 0;
+    if (!colors)
+        for (int k = 0; k < *n_big; k++)
+            if (isl_levels[big[k]] < kMaxColorsBig) used = used > isl_levels[big[k]] ? used : isl_levels[big[k]];
+    out[5] = used;
     out[6] = 0;
     for (int c = 0; c < PC_COUNT; c++) out[7 + c] = cls[c];
-}
-
-// islands of min_len + 1 .. max_len results (any order: islands share no dynamic body)
-__global__ void k_isl_pick(const int* n_isl, const int* isl_off, int min_len, int max_len, int* list, int* n_list) {
-    const int NI = *n_isl;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < NI; s += gridDim.x * blockDim.x) {
-        const int m = isl_off[s + 1] - isl_off[s];
-        if (m > min_len && m <= max_len) list[atomicAdd(n_list, 1)] = s;
-    }
-}
-
-// colour histogram of an island (cnt[c + 1] counts colour c); uncoloured results join the last colour
-__global__ void k_gc_count(int lo, int m, int* color, int* cnt) {
-    __shared__ int h[kMaxColorsBig];
-    for (int k = threadIdx.x; k < kMaxColorsBig; k += blockDim.x) h[k] = 0;
-    __syncthreads();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < m) {
-        int c = color[lo + j];
-        if (c < 0) { c = kMaxColorsBig - 1; color[lo + j] = c; }
-        atomicAdd(&h[c], 1);
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < kMaxColorsBig; k += blockDim.x)
-        if (h[k]) atomicAdd(&cnt[k + 1], h[k]);
-}
-
-// results of every colour but the last, grouped by colour (any order inside a colour)
-__global__ void k_gc_place(int lo, int m, const int* color, const uint32_t* order, int* cursor, uint32_t* corder) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const int c = j < m ? color[lo + j] : -1 - lane;
-    const bool live = c >= 0 && c < kMaxColorsBig - 1;
-    const int key = live ? c : -1 - lane;
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
-    const int leader = __ffs(peers) - 1;
-    int base = 0;
-    if (live && lane == leader) base = atomicAdd(&cursor[c], __popc(peers));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (live) corder[base + __popc(peers & ((1u << lane) - 1u))] = order[lo + j];
 }
 
 // exclusive offsets of the crowded positions' chunks (few positions: one thread)

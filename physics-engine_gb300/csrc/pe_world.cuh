@@ -250,7 +250,6 @@ private:
     template <class Tup, size_t... I> static void fill_ptrs(Tup& t, void** p, std::index_sequence<I...>) {
         ((p[I] = (void*)&std::get<I>(t)), ...);
     }
-    int coop_blocks_ = 0;   // co-resident blocks of k_gc_solve
     struct Pending { int id; cudaEvent_t e0, e1; };
     void resolve_prof() {
         if (pending_.empty()) return;
@@ -294,12 +293,16 @@ private:
     // there, and their grids come from upper bounds (the pair capacity), at most the GPU's resident
     // blocks.  The host waits twice per step: for the pair count (the capacities follow it) and for
     // the step's counters at its end.
-    enum DevCount { DC_P = 0, DC_R, DC_A, DC_M, DC_NMED, DC_MEDCUR, DC_COUNT };
+    enum DevCount { DC_P = 0, DC_R, DC_A, DC_M, DC_NLIST, DC_NFLOW = DC_NLIST + kWarpClasses, DC_NBIG, DC_COUNT };
     DBuf<int> dcnt_;
     DBuf<int2> cls_rng_;   // [first, end) of each pair class in the bucketed order
     DBuf<int> cls_work_;   // per-class work cursors of the pair-at-a-time kernels
-    DBuf<int> isl_med_;    // islands above small_island_items and up to big_island_items results
-    const uint32_t* isl_order_ = nullptr;   // island items sorted by island (points into val_)
+    // the solver's islands (pe_k_flow.cuh): the size classes' lists, and the flow items of larger islands
+    DBuf<int> isl_list_, isl_base_, isl_big_, isl_levels_, isl_colors_, isl_state_;
+    DBuf<uint32_t> flow_item_;
+    DBuf<int> flow_isl_, flow_color_, flow_head_, flow_next_, flow_succ_, flow_ff_;
+    DBuf<uint4> flow_box_;
+    template <bool JOINTS> void solve_islands(int mode, const uint32_t* order);
     // counters read back at the step's end, one copy into page-locked memory
     // (k_step_counters writes them in this order)
     enum HostStat { HS_STATUS = 0, HS_ROWS, HS_ACTIVE, HS_ISLANDS, HS_BIG, HS_COLORS, HS_P, HS_CLS, HS_COUNT = HS_CLS + PC_COUNT };
@@ -315,7 +318,7 @@ private:
     void bp_tail();                 // pair list, scene pair offsets, sweep axes
     void np_enqueue();              // narrowphase, no host waits
     void solve_enqueue(int mode);   // solver up to the velocity sync and the counters' copy, no host waits
-    void finish(int mode);          // waits for the counters; big islands; status
+    void finish();                  // waits for the counters; status
     void run_tail(int mode);        // bp_tail .. solve_enqueue, replayed from a CUDA graph when enabled
     int radix_sort_dev(int bound, int key_passes, const int* nd);
     // resident blocks of a kernel at a block size and dynamic shared memory (cached), and a grid for
@@ -440,14 +443,8 @@ private:
     int R_ = 0;
     std::vector<int> h_pair_scene_off_;
     // solver
-    DBuf<int> row_off_, active_, color_, claim_, parent_, isl_flag_, isl_off_, isl_n_, ncol_;
-    DBuf<uint32_t> isl_corder_;
-    DBuf<int> gc_big_, gc_n_, gc_cnt_, gc_cursor_, gc_cstart_, gc_ccount_;
-    DBuf<unsigned long long> gc_mask_, gc_claim_;
+    DBuf<int> row_off_, active_, color_, parent_, isl_flag_, isl_off_, isl_n_, ncol_;
     DBuf<double> xfer_;   // state transfers in the C ABI's layout
-    DBuf<int> gc_left_;   // items left after each colouring round
-    DBuf<int> gc_level_;  // coloured mode: exact levels of a big island beside its first-fit colours
-    void solve_big_islands(int nb, const uint32_t* order, bool exact);
     DBuf<R> rows_;
     int rows_cap_ = 0, n_rows_ = 0, n_active_ = 0, n_colors_ = 0, n_islands_ = 0;
     bool sat_attr_ = false;

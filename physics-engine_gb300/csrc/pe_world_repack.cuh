@@ -132,7 +132,6 @@ void World<R>::repack(const int* keep, int n_keep, const SceneData* const* adds,
     std::swap(bflags_.p, nflags.p); std::swap(bflags_.n, nflags.n);
     N_ = N;
     bcap_ = ncap;
-    claim_.ensure(N + 1);
     // scene tables (as set_scenes), then the kept axes and result offsets
     NS_ = std::max(ns, 1);
     if (ns == 0) off = {0, 0};

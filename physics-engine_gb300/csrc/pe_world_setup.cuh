@@ -406,7 +406,6 @@ void World<R>::set_bodies(int n, const int* shape, const int* flags, const doubl
     upload(bflags_, fl, st_);
     n_joints_ = 0;   // joints and ignored pairs name bodies: set them again after the bodies
     n_ign_ = 0;
-    claim_.ensure(n + 1);
     set_scenes(1, nullptr);
 }
 

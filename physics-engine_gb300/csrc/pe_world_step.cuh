@@ -171,9 +171,14 @@ template <class R> void World<R>::prepare_tail(int P) {
     const int tiles = (bound + kRadixTile - 1) / kRadixTile;
     hist_.ensure((size_t)256 * tiles + 1);
     aux_.ensure(std::max((256 * tiles + 1023) / 1024, (std::max(bound, N_) + 1 + 1023) / 1024) + 1);
-    isl_flag_.ensure(bound + 1); isl_off_.ensure(bound + 1); isl_med_.ensure(bound + 1); gc_big_.ensure(bound + 1);
-    isl_corder_.ensure(bound); color_.ensure(bound + 1);
-    isl_n_.ensure(1); ncol_.ensure(1); gc_n_.ensure(2);
+    isl_flag_.ensure(bound + 1); isl_off_.ensure(bound + 1); color_.ensure(bound + 1);
+    isl_n_.ensure(1); ncol_.ensure(1);
+    isl_list_.ensure(class_base(kWarpClasses, bound)); isl_base_.ensure(bound + 1); isl_big_.ensure(bound + 1);
+    isl_levels_.ensure(bound + 1); isl_colors_.ensure(bound + 1); isl_state_.ensure(bound + 1);
+    flow_item_.ensure(bound); flow_isl_.ensure(bound); flow_color_.ensure(bound);
+    flow_next_.ensure((size_t)2 * bound); flow_succ_.ensure((size_t)2 * bound);
+    flow_box_.ensure((size_t)2 * bound * token_words<R>());
+    flow_head_.ensure(N_ + 1); flow_ff_.ensure(1);
     parent_.ensure(N_ + 1);
     cls_count_.ensure(2 * PC_COUNT); cls_rng_.ensure(PC_COUNT); cls_work_.ensure(PC_COUNT);
     if (!sat_attr_) {   // dynamic shared memory of the staged SAT kernels (above the 48 KB default for FP64)
@@ -318,15 +323,12 @@ template <class R> void World<R>::narrowphase() {
     R_ = P_;
 }
 
-// Solver without host waits, up to the velocity sync: rows, active results, islands (union-find,
-// sort by island, offsets), the small islands one thread each, the medium ones a block each (exact
-// levels in serial-order mode, colours in coloured mode), the big islands listed for finish(); then
-// the step's counters are copied to the host in one transfer.
+// Solver without host waits: rows, active results, islands (union-find, sort by island, offsets), the
+// iterations (pe_k_flow.cuh); then the step's counters are copied to the host in one transfer.
 template <class R> void World<R>::solve_enqueue(int mode) {
     if (N_ == 0) return;
     const int cap = pair_cap_, NJ = n_joints_, bound = cap + NJ;
     const int* Rd = dcnt_.p + DC_R;
-    launch(K_SI_MISC, grid(N_), k_si_clear<R>, bodies());
     // rows: one per contact point, results' rows contiguous in result order
     launch(K_SI_MISC, pgrid(cap + 1, kBlock, k_rows_init), k_rows_init, Rd, cap, (const int*)res_np_.p, row_off_.p);
     scan_async(row_off_.p, cap + 1, rows_total_.p);
@@ -354,64 +356,57 @@ template <class R> void World<R>::solve_enqueue(int mode) {
     const int cur = radix_sort_dev(bound, label_passes, Md);
     const uint64_t* skey = key_[cur].p;
     const uint32_t* order = val_[cur].p;
-    isl_order_ = order;
     launch(K_ISLAND, pgrid(bound + 1, kBlock, k_isl_flags), k_isl_flags, (const int*)Md, bound, skey, isl_flag_.p);
     scan_async(isl_flag_.p, bound + 1, isl_n_.p);
     launch(K_ISLAND, pgrid(bound + 1, kBlock, k_isl_offsets), k_isl_offsets, (const int*)Md, skey, (const int*)isl_flag_.p, isl_off_.p,
            isl_n_.p);
-    const int small = tun_.small_island_items, big = tun_.big_island_items;
-    // islands of up to small_island_items items: one thread each
-    launch(K_SI_SERIAL, pgrid(bound, kBlock, k_isl_serial<R>), k_isl_serial<R>, (const int*)isl_n_.p, (const int*)isl_off_.p, order,
-           results(), jt, bodies(), rows(), (const int*)row_off_.p, prm_.iterations, small);
-    // islands of small_island_items + 1 .. big_island_items items: listed, then a block each
-    PE_CK(cudaMemsetAsync(dcnt_.p + DC_NMED, 0, 2 * sizeof(int), st_));
-    launch(K_ISLAND, pgrid(bound, kBlock, k_isl_pick), k_isl_pick, (const int*)isl_n_.p, (const int*)isl_off_.p, small, big, isl_med_.p,
-           dcnt_.p + DC_NMED);
-    const long long med = (long long)bound / (small + 1) + 1;   // at most this many such islands
-    if (mode == 0) {
-        // serial order: the exact level schedule
-        const int g = (int)std::min<long long>(med, resident(k_isl_levels<R>, tun_.level_block, 0));
-        launch_block(K_SI_SERIAL, g, tun_.level_block, k_isl_levels<R>, (const int*)isl_med_.p, (const int*)(dcnt_.p + DC_NMED),
-                     dcnt_.p + DC_MEDCUR, (const int*)isl_off_.p, order, results(), jt, bodies(), rows(), (const int*)row_off_.p,
-                     prm_.iterations, small, big, claim_.p, color_.p, isl_corder_.p);
-    } else {
-        PE_CK(cudaMemsetAsync(ncol_.p, 0, sizeof(int), st_));
-        const int g = (int)std::min<long long>(med, resident(k_isl_colored<R>, tun_.color_block, 0));
-        launch_block(K_SI_COLOR, g, tun_.color_block, k_isl_colored<R>, (const int*)isl_med_.p, (const int*)(dcnt_.p + DC_NMED),
-                     dcnt_.p + DC_MEDCUR, (const int*)isl_off_.p, order, results(), jt, bodies(), rows(), (const int*)row_off_.p,
-                     prm_.iterations, small, big, claim_.p, color_.p, isl_corder_.p, ncol_.p);
-    }
-    // islands above big_island_items: listed here, solved by finish() after the counters are read
-    PE_CK(cudaMemsetAsync(gc_n_.p, 0, sizeof(int), st_));
-    launch(K_SI_COLOR, pgrid(bound, kBlock, k_isl_big), k_isl_big, (const int*)isl_n_.p, (const int*)isl_off_.p, gc_big_.p, gc_n_.p, big);
-    launch(K_SI_MISC, grid(N_), k_si_sync<R>, bodies());
+    if (NJ > 0) solve_islands<true>(mode, order);
+    else solve_islands<false>(mode, order);
     launch_block(K_MISC, 1, 32, k_step_counters, (const int*)status_.p, (const int*)rows_total_.p, Ad, (const int*)isl_n_.p,
-                 (const int*)gc_n_.p, mode == 0 ? (const int*)nullptr : (const int*)ncol_.p, (const int*)cls_count_.p, dstat_.p);
+                 (const int*)(dcnt_.p + DC_NBIG), (const int*)isl_big_.p, (const int*)isl_levels_.p,
+                 mode == 0 ? (const int*)nullptr : (const int*)ncol_.p, (const int*)cls_count_.p, dstat_.p);
     PE_CK(cudaMemcpyAsync(hstat_, dstat_.p, HS_COUNT * sizeof(int), cudaMemcpyDeviceToHost, st_));
 }
 
-// The step's second host wait: its counters; then the big islands (host-driven, rare), whose
-// solve ends with a second velocity sync; then the status.
-template <class R> void World<R>::finish(int mode) {
+// The solver's iterations: the islands sorted into size classes, then those that fit a warp and those
+// that do not.
+template <class R> template <bool JOINTS> void World<R>::solve_islands(int mode, const uint32_t* order) {
+    const int bound = pair_cap_ + n_joints_, small = tun_.small_island_items, big = tun_.big_island_items;
+    int* n_list = dcnt_.p + DC_NLIST;
+    int* colors = mode == 0 ? nullptr : ncol_.p;
+    PE_CK(cudaMemsetAsync(n_list, 0, (DC_COUNT - DC_NLIST) * sizeof(int), st_));
+    if (colors) PE_CK(cudaMemsetAsync(colors, 0, sizeof(int), st_));
+    launch(K_ISLAND, pgrid(bound, kBlock, k_isl_classes), k_isl_classes, (const int*)isl_n_.p, (const int*)isl_off_.p, bound, big, isl_list_.p,
+           n_list, isl_base_.p, dcnt_.p + DC_NFLOW, isl_big_.p, dcnt_.p + DC_NBIG);
+    launch_block(K_SI_SERIAL, pgrid(bound, kWarpBlock, k_isl_warp<R, JOINTS>, kWarpBlock), kWarpBlock, k_isl_warp<R, JOINTS>,
+                 (const int*)isl_list_.p, (const int*)n_list, bound, (const int*)isl_off_.p, order, results(), joints(), bodies(), rows(),
+                 (const int*)row_off_.p, prm_.iterations, small, colors, status_.p);
+    FlowArgs<R> f;
+    f.n_items = dcnt_.p + DC_M; f.isl_scan = isl_flag_.p; f.isl_off = isl_off_.p; f.order = order;
+    f.base = isl_base_.p; f.n_flow = dcnt_.p + DC_NFLOW; f.big = isl_big_.p; f.n_big = dcnt_.p + DC_NBIG;
+    f.big_items = big; f.color_min = small; f.exact_levels = tun_.exact_levels_colored; f.mode = mode; f.iterations = prm_.iterations;
+    f.item = flow_item_.p; f.isl = flow_isl_.p; f.color = flow_color_.p; f.head = flow_head_.p; f.next = flow_next_.p; f.succ = flow_succ_.p;
+    f.box = flow_box_.p; f.isl_levels = isl_levels_.p; f.isl_colors = isl_colors_.p; f.isl_state = isl_state_.p;
+    f.any_first_fit = flow_ff_.p; f.n_colors = ncol_.p; f.status = status_.p;
+    launch_coop(K_SI_COLOR, resident(k_isl_flow<R, JOINTS>, kFlowBlock, 0), kFlowBlock, k_isl_flow<R, JOINTS>, f, results(), joints(), bodies(),
+                rows(), (const int*)row_off_.p);
+}
+
+// The step's second host wait: its counters and status.
+template <class R> void World<R>::finish() {
     PE_CK(cudaStreamSynchronize(st_));
     if (N_ == 0) return;
     n_rows_ = hstat_[HS_ROWS];
     n_active_ = hstat_[HS_ACTIVE];
     n_islands_ = hstat_[HS_ISLANDS];
-    n_colors_ = mode == 0 ? 0 : hstat_[HS_COLORS];
+    n_colors_ = hstat_[HS_COLORS];
     for (int c = 0; c < PC_COUNT; c++) h_cls_[c] = hstat_[HS_CLS + c];
-    const int status = hstat_[HS_STATUS], nb = hstat_[HS_BIG];
+    const int status = hstat_[HS_STATUS];
     if (status) {
         PE_CK(cudaMemsetAsync(status_.p, 0, sizeof(int), st_));
         PE_CK(cudaStreamSynchronize(st_));
-        throw std::runtime_error("device capacity overflow (status " + std::to_string(status) + ")");
-    }
-    if (nb > 0) {
-        solve_big_islands(nb, isl_order_, mode == 0);
-        launch(K_SI_MISC, grid(N_), k_si_sync<R>, bodies());
-        ev_end(3);   // the solve and the step end after the big islands
-        ev_end(4);
-        PE_CK(cudaGetLastError());
+        throw std::runtime_error((status & ST_FLOW_STALL ? "solver stalled (status " : "device capacity overflow (status ") +
+                                 std::to_string(status) + ")");
     }
 }
 
@@ -419,94 +414,7 @@ template <class R> void World<R>::solve(int mode) {
     prepare_tail(R_);
     solve_enqueue(mode);
     PE_CK(cudaGetLastError());
-    finish(mode);
-}
-
-// the nb islands above big_island_items results (listed in gc_big_): grid-wide colouring rounds,
-// then one launch per colour and iteration (see k_gc_*)
-template <class R> void World<R>::solve_big_islands(int nb, const uint32_t* order, bool exact) {
-    std::vector<int> big(nb);
-    PE_CK(cudaMemcpy(big.data(), gc_big_.p, nb * sizeof(int), cudaMemcpyDeviceToHost));
-    std::sort(big.begin(), big.end());
-    gc_cnt_.ensure(kMaxColorsBig + 1);
-    gc_cursor_.ensure(kMaxColorsBig);
-    const Results<R> rs = results();
-    const Joints<R> jt = joints();
-    const Bodies<R> bd = bodies();
-    const Rows<R> rw = rows();
-    std::vector<int> cnt(kMaxColorsBig + 1), start(kMaxColorsBig), cur(kMaxColorsBig);
-    for (int s : big) {
-        int lh[2];
-        PE_CK(cudaMemcpy(lh, isl_off_.p + s, 2 * sizeof(int), cudaMemcpyDeviceToHost));
-        const int lo = lh[0], m = lh[1] - lh[0], g = grid(m);
-        PE_CK(cudaMemsetAsync(color_.p + lo, 0xff, (size_t)m * sizeof(int), st_));   // -1: uncoloured
-        unsigned long long* mask = nullptr;   // exact level schedule: colour = round
-        if (!exact) {
-            gc_mask_.ensure(N_ + 1);
-            mask = gc_mask_.p;
-            launch(K_GC_COLOR, g, k_gc_mask_reset<R>, lo, m, order, rs, jt, mask);
-        }
-        // colouring rounds, the remaining count read back every 8 rounds (extra rounds find nothing to do)
-        // all rounds in one cooperative launch (up to kMaxColorsBig - 1; items left over take the last colour)
-        if (coop_blocks_ == 0) {
-            int per_sm = 0, sms = 0;
-            PE_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gc_solve<R>, kBlock, 0));
-            int per_sm2 = 0;
-            PE_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_gc_rounds<R>, kBlock, 0));
-            PE_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_));
-            coop_blocks_ = std::max(std::min(per_sm, per_sm2), 1) * sms;
-        }
-        gc_left_.ensure(kMaxColorsBig);
-        PE_CK(cudaMemsetAsync(gc_left_.p, 0, kMaxColorsBig * sizeof(int), st_));
-        gc_claim_.ensure(N_ + 1);
-        int* level = nullptr;   // coloured mode: the exact levels beside the first-fit colours
-        if (!exact) {
-            gc_level_.ensure((size_t)(lo + m));
-            level = gc_level_.p;
-            PE_CK(cudaMemsetAsync(level + lo, 0xff, (size_t)m * sizeof(int), st_));
-        }
-        launch_coop(K_GC_COLOR, coop_blocks_, kBlock, k_gc_rounds<R>, lo, m, order, rs, jt, bd, gc_claim_.p, color_.p, mask, gc_left_.p,
-                    kMaxColorsBig - 1, gc_n_.p + 1, level);
-        int ncol = 0;
-        PE_CK(cudaMemcpyAsync(&ncol, gc_n_.p + 1, sizeof(int), cudaMemcpyDeviceToHost, st_));
-        PE_CK(cudaStreamSynchronize(st_));
-        // Coloured mode keeps the exact levels (the reference's order, as in serial-order mode) when
-        // the island needs few of them; first-fit colours only bound the colour count of islands
-        // with long dependency chains (hundreds of levels), where one grid barrier per level and
-        // iteration would dominate.
-        int* col = color_.p;
-        if (!exact && ncol <= tun_.exact_levels_colored) {
-            int left_last = 0;
-            PE_CK(cudaMemcpy(&left_last, gc_left_.p + ncol - 1, sizeof(int), cudaMemcpyDeviceToHost));
-            if (left_last == 0) col = level;
-        }
-        PE_CK(cudaMemsetAsync(gc_cnt_.p, 0, (kMaxColorsBig + 1) * sizeof(int), st_));
-        launch(K_GC_COLOR, g, k_gc_count, lo, m, col, gc_cnt_.p);
-        PE_CK(cudaMemcpyAsync(cnt.data(), gc_cnt_.p, cnt.size() * sizeof(int), cudaMemcpyDeviceToHost, st_));
-        PE_CK(cudaStreamSynchronize(st_));
-        if (exact && cnt[kMaxColorsBig] > 0) {   // out of levels: the island in order on one thread
-            launch_block(K_GC_SOLVE, 1, 1, k_isl_one<R>, lo, m, order, rs, jt, bd, rw, (const int*)row_off_.p, prm_.iterations);
-            continue;
-        }
-        int run = 0, used = 0;
-        for (int c = 0; c < kMaxColorsBig; c++) {
-            start[c] = run; cur[c] = lo + run; run += cnt[c + 1];
-            if (cnt[c + 1]) used = c + 1;
-        }
-        PE_CK(cudaMemcpyAsync(gc_cursor_.p, cur.data(), cur.size() * sizeof(int), cudaMemcpyHostToDevice, st_));
-        launch(K_GC_COLOR, g, k_gc_place, lo, m, (const int*)col, order, gc_cursor_.p, isl_corder_.p);
-        const bool last = cnt[kMaxColorsBig] > 0;
-        n_colors_ = std::max(n_colors_, std::min(used, ncol) + (last ? 1 : 0));
-        // every iteration in one cooperative launch: colour lists, then the grid-wide passes
-        const int top = std::min(used, kMaxColorsBig - 1);
-        std::vector<int> cs(std::max(top, 1)), cc(std::max(top, 1));
-        for (int c = 0; c < top; c++) { cs[c] = lo + start[c]; cc[c] = cnt[c + 1]; }
-        upload(gc_cstart_, cs, st_);
-        upload(gc_ccount_, cc, st_);
-        launch_coop(K_GC_SOLVE, coop_blocks_, kBlock, k_gc_solve<R>, (const uint32_t*)isl_corder_.p, (const int*)gc_cstart_.p,
-                    (const int*)gc_ccount_.p, top, prm_.iterations, lo, m, order, (const int*)col, last ? 1 : 0, rs, jt, bd, rw,
-                    (const int*)row_off_.p);
-    }
+    finish();
 }
 
 // What a captured step graph holds fixed: buffer addresses (any reallocation changes the
@@ -627,7 +535,7 @@ template <class R> void World<R>::step(int n, int mode) {
         cur_dist_ ^= 1;
         run_tail(mode);
         R_ = P;
-        finish(mode);               // the second
+        finish();                   // the second
         ev_collect();
         last_step_launches_ = step_launches_;
     }
