@@ -75,16 +75,44 @@ template <class R> struct Cache {
 };
 
 // One pair being collided: shapes and transforms held by value (registers); the contact cache
-// (local memory, only touched by the thread that adds points) is reached through `c`.
-template <class R> struct Pair {
+// (local memory, only touched by the thread that adds points), or a recorder of the points it will be
+// given, is reached through `c`.
+template <class R, class C = Cache<R>> struct Pair {
     ShapeView<R> sa, sb;
     Xf<R> xa, xb;
     R ref_scale;
     R margin;       // the world's contact margin (ShapeTable::margin)
-    Cache<R>* c;
+    C* c;
     __device__ void add(const V3<R>& n, const V3<R>& p, R d) { c->add(n, p, d); }
     __device__ const Xf<R>& ta() const { return xa; }
     __device__ const Xf<R>& tb() const { return xb; }
+};
+
+// Points that a pair algorithm adds, kept in order to be added to a cache later (contacts never steer an
+// algorithm, so pieces of a pair can run side by side and hand their points over in the pair's order).
+// The swap flag is part of the cache's state that one algorithm may leave to the next: a point
+// recorded before the algorithm set it takes the cache's.
+constexpr int kRecReals = 8;
+template <class R> struct Recorder {
+    R* buf;          // kRecReals per point
+    int n, cap;      // n > cap: more points than fit
+    int swap;        // 0, 1, or kSwapInherit while the algorithm has not set it
+    static constexpr int kSwapInherit = 2;
+    __device__ void add(const V3<R>& wn, const V3<R>& wp, R depth) {
+        if (n < cap) {
+            R* e = buf + n * kRecReals;
+            e[0] = wn.x; e[1] = wn.y; e[2] = wn.z; e[3] = wp.x; e[4] = wp.y; e[5] = wp.z; e[6] = depth; e[7] = R(swap);
+        }
+        n++;
+    }
+    __device__ void replay(Cache<R>& c) const {
+        for (int k = 0; k < n; k++) {
+            const R* e = buf + k * kRecReals;
+            if ((int)e[7] != kSwapInherit) c.swap = (int)e[7] != 0;
+            c.add(V3<R>(e[0], e[1], e[2]), V3<R>(e[3], e[4], e[5]), e[6]);
+        }
+        if (swap != kSwapInherit) c.swap = swap != 0;
+    }
 };
 
 // ======================================================================= box-box
@@ -167,7 +195,7 @@ template <class R> __device__ void cull_points(int n, const R p[], int m, int i0
     }
 }
 
-template <class R> __device__ bool box_box(Pair<R>& c) {   // box_box_collision_algorithm.cpp:137-580
+template <class R, class C> __device__ bool box_box(Pair<R, C>& c) {   // box_box_collision_algorithm.cpp:137-580
     const R margin = c.margin, fudge = R(1.05);
     const V3<R> p1 = c.ta().o, p2 = c.tb().o;
     const M3<R>& R1 = c.ta().b;
@@ -328,7 +356,7 @@ template <class R> __device__ bool box_box(Pair<R>& c) {   // box_box_collision_
 }
 
 // ======================================================================= sphere pairs
-template <class R> __device__ bool box_sphere(Pair<R>& c) {   // box_sphere_collision_algorithm.cpp:6-141
+template <class R, class C> __device__ bool box_sphere(Pair<R, C>& c) {   // box_sphere_collision_algorithm.cpp:6-141
     const bool a_box = c.sa.type == ST_BOX;
     const ShapeView<R>& sph = a_box ? c.sb : c.sa;
     const ShapeView<R>& box = a_box ? c.sa : c.sb;
@@ -370,7 +398,7 @@ template <class R> __device__ bool box_sphere(Pair<R>& c) {   // box_sphere_coll
     return ret;
 }
 
-template <class R> __device__ bool sphere_sphere(Pair<R>& c) {   // sphere_sphere_collision_algorithm.cpp:23-37
+template <class R, class C> __device__ bool sphere_sphere(Pair<R, C>& c) {   // sphere_sphere_collision_algorithm.cpp:23-37
     const R ra = c.sa.radius, rb = c.sb.radius, margin = c.margin;
     const V3<R> rel = c.ta().o - c.tb().o;
     const R dist = norm(rel);
@@ -381,7 +409,7 @@ template <class R> __device__ bool sphere_sphere(Pair<R>& c) {   // sphere_spher
     return true;
 }
 
-template <class R> __device__ bool sphere_cylinder(Pair<R>& c) {   // sphere_cylinder_collision_algorithm.cpp:6-76
+template <class R, class C> __device__ bool sphere_cylinder(Pair<R, C>& c) {   // sphere_cylinder_collision_algorithm.cpp:6-76
     const bool a_sph = c.sa.type == ST_SPHERE;
     const ShapeView<R>& sph = a_sph ? c.sa : c.sb;
     const ShapeView<R>& cyl = a_sph ? c.sb : c.sa;
@@ -424,7 +452,7 @@ template <class R> __device__ bool sphere_cylinder(Pair<R>& c) {   // sphere_cyl
 }
 
 // ======================================================================= box-cylinder
-template <class R> __device__ void add_on_box(Pair<R>& c, const V3<R>& pc, int face, const V3<R>& he, const Xf<R>& t, R margin) {
+template <class R, class C> __device__ void add_on_box(Pair<R, C>& c, const V3<R>& pc, int face, const V3<R>& he, const Xf<R>& t, R margin) {
     if (!(face >= -3 && face <= 3 && face != 0)) return;   // box_cylinder_collision_algorithm.cpp:79-114
     for (int i = 0; i < 3; i++) if (pc[i] > he[i] || pc[i] < -he[i]) return;
     V3<R> p = pc, n(0, 0, 0);
@@ -453,7 +481,7 @@ template <class R> __device__ void cyl_contact(const V3<R>& p, const V3<R>& pos,
     wp = pw - n * margin;
     wd = -dist + 2 * margin;
 }
-template <class R> __device__ void add_on_cylinder(Pair<R>& c, const V3<R>& p, const V3<R>& pos, const V3<R>& axis, R radius, R h,
+template <class R, class C> __device__ void add_on_cylinder(Pair<R, C>& c, const V3<R>& p, const V3<R>& pos, const V3<R>& axis, R radius, R h,
                                                    const Xf<R>& t, R margin) {   // :116-139
     V3<R> n, pw;
     R d;
@@ -525,7 +553,7 @@ template <class R> __device__ bool segment_cylinder(const V3<R>& s, const V3<R>&
     return true;
 }
 
-template <class R> __device__ bool box_cylinder(Pair<R>& c) {   // box_cylinder_collision_algorithm.cpp:13-50, 306-389
+template <class R, class C> __device__ bool box_cylinder(Pair<R, C>& c) {   // box_cylinder_collision_algorithm.cpp:13-50, 306-389
     const bool a_box = c.sa.type == ST_BOX;
     const ShapeView<R>& box = a_box ? c.sa : c.sb;
     const ShapeView<R>& cyl = a_box ? c.sb : c.sa;
@@ -584,7 +612,7 @@ template <class R> __device__ bool box_cylinder(Pair<R>& c) {   // box_cylinder_
 }
 
 // ======================================================================= convex SAT + clipping
-template <class R> __device__ bool sep_test(const Pair<R>& c, const V3<R>& axis, R& depth, V3<R>& wa, V3<R>& wb) {
+template <class R, class C> __device__ bool sep_test(const Pair<R, C>& c, const V3<R>& axis, R& depth, V3<R>& wa, V3<R>& wb) {
     R min0, max0, min1, max1;   // convex_convex_collision_algorithm.cpp:216-243
     V3<R> a0, a1, b0, b1;
     shape_project(c.sa, c.ta(), axis, min0, max0, a0, a1);
@@ -601,7 +629,7 @@ template <class R> __device__ bool on_line(const V3<R>& v0, const V3<R>& v1, con
 }
 
 // findSeparatingAxis (:251-402), one thread
-template <class R> __device__ bool find_sep_axis(Pair<R>& c, V3<R>& sep) {
+template <class R, class C> __device__ bool find_sep_axis(Pair<R, C>& c, V3<R>& sep) {
     const R margin = c.margin;
     const V3<R> dc = c.ta().o - c.tb().o;
     R dmin = Lim<R>::max();
@@ -672,7 +700,7 @@ constexpr int kMaxClip = 64;   // clipped polygon capacity (incident face vertic
 
 // clipFaceAgainstHull (:63-131): the incident face fb of B clipped against the side planes of
 // the reference face fa of A; points whose depth under fa lies in [min_dist, max_dist] are kept
-template <class R> __device__ void clip_faces(Pair<R>& c, const V3<R>& sep, R min_dist, R max_dist, int fb, int fa) {
+template <class R, class C> __device__ void clip_faces(Pair<R, C>& c, const V3<R>& sep, R min_dist, R max_dist, int fb, int fa) {
     const R margin = c.margin;
     V3<R> buf[2][kMaxClip];
     int n_in = 0;
@@ -723,7 +751,7 @@ template <class R> __device__ void clip_faces(Pair<R>& c, const V3<R>& sep, R mi
 
 // clipHullAgainstHull (:133-170): incident face = first maximum of n_B.sep, reference face =
 // first minimum of n_A.sep
-template <class R> __device__ void clip_hull_hull(Pair<R>& c, const V3<R>& sep, R min_dist, R max_dist) {
+template <class R, class C> __device__ void clip_hull_hull(Pair<R, C>& c, const V3<R>& sep, R min_dist, R max_dist) {
     int fb = -1;
     {
         R dmax = Lim<R>::min();
@@ -745,7 +773,7 @@ template <class R> __device__ void clip_hull_hull(Pair<R>& c, const V3<R>& sep, 
     clip_faces(c, sep, min_dist, max_dist, fb, fa);
 }
 
-template <class R> __device__ bool convex_convex(Pair<R>& c) {   // :408-432
+template <class R, class C> __device__ bool convex_convex(Pair<R, C>& c) {   // :408-432
     V3<R> sep;
     if (!find_sep_axis(c, sep)) return false;
     clip_hull_hull(c, sep, -c.ref_scale, c.margin);   // window [-refScale, margin] (:426-429)
@@ -811,52 +839,47 @@ template <class R> __device__ bool face_hit(const ShapeView<R>& m, int f, const 
     return true;
 }
 
-// BVH::search (bvh.cpp:105-125) of a mesh's face tree for the box [aa, bb]: the right-first stack
-// walk of a tree built on index ranges meets the leaves in descending order and reports every face
-// of a leaf whose box overlaps, ascending.  Convex meshes (one face per leaf) test the face boxes.
+// BVH::search (bvh.cpp:105-125) of a convex mesh's face tree for the box [aa, bb]: the right-first stack
+// walk of a tree built on index ranges meets its single-face leaves in descending order.  (A concave
+// mesh's leaves hold several faces: k_np_mesh.)
 template <class R, class Visit>
 __device__ void mesh_query(const ShapeView<R>& m, const V3<R>& aa, const V3<R>& bb, Visit&& visit) {
-    if (m.nl == 0) {
-        for (int f = m.nf - 1; f >= 0; f--)
-            if (face_hit(m, f, aa, bb)) visit(f);
-        return;
-    }
-    for (int l = m.nl - 1; l >= 0; l--) {
-        const R* mn = m.l_min + l * 3;
-        const R* mx = m.l_max + l * 3;
-        if (mn[0] > bb.x || mn[1] > bb.y || mn[2] > bb.z) continue;
-        if (mx[0] < aa.x || mx[1] < aa.y || mx[2] < aa.z) continue;
-        for (int f = m.l_beg[l], e = m.l_beg[l] + m.l_cnt[l]; f < e; f++) visit(f);
-    }
+    for (int f = m.nf - 1; f >= 0; f--)
+        if (face_hit(m, f, aa, bb)) visit(f);
 }
-__host__ __device__ inline bool is_mesh(int t) { return t == ST_HULL || t == ST_CONCAVE; }
 
-template <class R> __device__ bool sphere_hull(Pair<R>& c) {   // sphere_convex_collision_algorithm.cpp:11-34, 165-211
-    const bool a_hull = is_mesh(c.sa.type);
+// one face of a mesh against a sphere (centre rel in the mesh's frame): its fan triangles in order
+template <class R, class C>
+__device__ bool sphere_face(Pair<R, C>& c, const ShapeView<R>& m, const Xf<R>& tm, const V3<R>& rel, R r, int f) {
+    const R margin = c.margin;
+    bool ret = false;
+    const int n = m.face_size(f);
+    for (int i = 0; i < n - 2; i++) {
+        const V3<R> vs[3] = {m.vert(m.face_vert(f, 0)), m.vert(m.face_vert(f, i + 1)), m.vert(m.face_vert(f, i + 2))};
+        V3<R> point, normal;
+        R depth = 0;
+        if (sphere_triangle(rel, r, vs, point, normal, depth)) {
+            normal = mv(tm.b, normal);
+            point = tm.apply(point);
+            c.add(normal, point - normal * margin, depth + 2 * margin);
+            ret = true;
+        }
+    }
+    return ret;
+}
+
+template <class R, class C> __device__ bool sphere_hull(Pair<R, C>& c) {   // sphere_convex_collision_algorithm.cpp:11-34, 165-211
+    const bool a_hull = c.sa.type == ST_HULL;
     const ShapeView<R>& m = a_hull ? c.sa : c.sb;
     const ShapeView<R>& sp = a_hull ? c.sb : c.sa;
     const Xf<R>& tm = a_hull ? c.ta() : c.tb();
     const Xf<R>& ts = a_hull ? c.tb() : c.ta();
-    const R margin = c.margin;
     c.c->swap = a_hull;
     const V3<R> rel = tm.inv_apply(ts.o);
     const R r = sp.radius;
     const V3<R> aa = rel - V3<R>(r, r, r), bb = rel + V3<R>(r, r, r);
     bool ret = false;
-    mesh_query(m, aa, bb, [&](int f) {
-        const int n = m.face_size(f);
-        for (int i = 0; i < n - 2; i++) {
-            const V3<R> vs[3] = {m.vert(m.face_vert(f, 0)), m.vert(m.face_vert(f, i + 1)), m.vert(m.face_vert(f, i + 2))};
-            V3<R> point, normal;
-            R depth = 0;
-            if (sphere_triangle(rel, r, vs, point, normal, depth)) {
-                normal = mv(tm.b, normal);
-                point = tm.apply(point);
-                c.add(normal, point - normal * margin, depth + 2 * margin);
-                ret = true;
-            }
-        }
-    });
+    mesh_query(m, aa, bb, [&](int f) { ret |= sphere_face(c, m, tm, rel, r, f); });
     c.c->swap = false;
     return ret;
 }
@@ -895,72 +918,86 @@ template <class R> __device__ bool segment_face(const ShapeView<R>& m, int f, co
     return true;
 }
 
-template <class R> __device__ bool cylinder_hull(Pair<R>& c) {   // cylinder_convex_collision_algorithm.cpp:11-51, 109-203
-    const bool a_hull = is_mesh(c.sa.type);
+// a cylinder in a mesh's frame (axis, centre, radius, half height) and the mesh's transform
+template <class R> struct CylinderFrame {
+    V3<R> axis, pos;
+    R cr, ch;
+    Xf<R> to;
+};
+// the cylinder's side segments against one face
+template <class R, class C>
+__device__ void cylinder_face_sides(Pair<R, C>& c, const ShapeView<R>& m, const CylinderFrame<R>& q, int f) {
+    const R margin = c.margin, cr = q.cr, ch = q.ch;
+    const V3<R>&axis = q.axis, &pos = q.pos;
+    const int dxs[4] = {1, -1, -1, 1}, dys[4] = {1, 1, -1, -1};
+    const V3<R> fn = m.face_normal(f);
+    auto seg_on_mesh = [&](const V3<R>& ps, const V3<R>& ds, R ls) {
+        R t1, t2, d1, d2;
+        if (segment_face(m, f, ps, ds, ls, margin, t1, t2, d1, d2)) {
+            const V3<R> p1 = q.to.apply(ps + ds * t1 - fn * d1);
+            const V3<R> p2 = q.to.apply(ps + ds * t2 - fn * d2);
+            const V3<R> n = mv(q.to.b, fn);
+            c.add(n, p1 - n * margin, d1 + margin * 2);
+            c.add(n, p2 - n * margin, d2 + margin * 2);
+        }
+    };
+    const R adc = dot(axis, fn);
+    V3<R> ddx, ddz;
+    const V3<R> ddy = axis;
+    bool vertical = false;
+    if (rabs(rabs(adc) - 1) < eps<R>()) {
+        ddz = normalized(cross(axis, V3<R>(1, 0, 0)));
+        ddx = normalized(cross(axis, ddz));
+        vertical = true;
+    } else {
+        ddx = normalized(cross(cross(fn, axis), axis));
+    }
+    for (int i = 0; i < 4; i++) {
+        const V3<R> ps = pos + ddx * R(dxs[i]) * cr + ddy * R(dys[i]) * ch;
+        const V3<R> ds = (dxs[i] == dys[i] ? ddy : ddx) * R(-dxs[i]);
+        const R ls = (dxs[i] == dys[i] ? ch : cr) * 2;
+        seg_on_mesh(ps, ds, ls);
+    }
+    if (vertical)
+        for (int i = 0; i < 3; i += 2) {
+            const V3<R> ps = pos + ddz * R(dxs[i]) * cr + ddy * R(dys[i]) * ch;
+            seg_on_mesh(ps, ddy * R(-dxs[i]), ch * 2);
+        }
+}
+// one face's edges against the cylinder
+template <class R, class C>
+__device__ void cylinder_face_edges(Pair<R, C>& c, const ShapeView<R>& m, const CylinderFrame<R>& q, int f) {
+    const R margin = c.margin;
+    const int n = m.face_size(f);
+    for (int i = 0; i < n; i++) {
+        const V3<R> v1 = m.vert(m.face_vert(f, i));
+        const V3<R> v2 = m.vert(m.face_vert(f, (i + 1) % n));
+        R t1, t2;
+        const V3<R> start = (v1 + v2) / R(2);
+        const R ls = norm(v2 - v1) / 2;
+        const V3<R> dir = (v2 - v1) / (ls * 2);
+        if (segment_cylinder(start, dir, ls, q.pos, q.axis, q.ch, q.cr, margin, t1, t2)) {
+            const V3<R> p1 = start + dir * t1, p2 = start + dir * t2;
+            add_on_cylinder(c, (p1 + p2) / R(2), q.pos, q.axis, q.cr, q.ch, q.to, margin);
+        }
+    }
+}
+
+template <class R, class C> __device__ bool cylinder_hull(Pair<R, C>& c) {   // cylinder_convex_collision_algorithm.cpp:11-51, 109-203
+    const bool a_hull = c.sa.type == ST_HULL;
     const ShapeView<R>& m = a_hull ? c.sa : c.sb;
     const ShapeView<R>& cy = a_hull ? c.sb : c.sa;
     const Xf<R>& to = a_hull ? c.ta() : c.tb();
     const Xf<R>& tc = a_hull ? c.tb() : c.ta();
-    const R margin = c.margin;
     c.c->swap = a_hull;
     const R cr = cy.radius, ch = cy.height / R(2.0);
     const Xf<R> rel = to.inverse() * tc;
     const V3<R> axis = rel.b.col(1), pos = rel.o;
     V3<R> aa, bb;
     shape_aabb(cy, rel, aa, bb);
-    const int dxs[4] = {1, -1, -1, 1}, dys[4] = {1, 1, -1, -1};
-    auto seg_on_mesh = [&](int f, const V3<R>& ps, const V3<R>& ds, R ls) {
-        R t1, t2, d1, d2;
-        if (segment_face(m, f, ps, ds, ls, margin, t1, t2, d1, d2)) {
-            const V3<R> fn = m.face_normal(f);
-            const V3<R> p1 = to.apply(ps + ds * t1 - fn * d1);
-            const V3<R> p2 = to.apply(ps + ds * t2 - fn * d2);
-            const V3<R> n = mv(to.b, fn);
-            c.add(n, p1 - n * margin, d1 + margin * 2);
-            c.add(n, p2 - n * margin, d2 + margin * 2);
-        }
-    };
-    mesh_query(m, aa, bb, [&](int f) {
-        const V3<R> fn = m.face_normal(f);
-        const R adc = dot(axis, fn);
-        V3<R> ddx, ddz;
-        const V3<R> ddy = axis;
-        bool vertical = false;
-        if (rabs(rabs(adc) - 1) < eps<R>()) {
-            ddz = normalized(cross(axis, V3<R>(1, 0, 0)));
-            ddx = normalized(cross(axis, ddz));
-            vertical = true;
-        } else {
-            ddx = normalized(cross(cross(fn, axis), axis));
-        }
-        for (int i = 0; i < 4; i++) {
-            const V3<R> ps = pos + ddx * R(dxs[i]) * cr + ddy * R(dys[i]) * ch;
-            const V3<R> ds = (dxs[i] == dys[i] ? ddy : ddx) * R(-dxs[i]);
-            const R ls = (dxs[i] == dys[i] ? ch : cr) * 2;
-            seg_on_mesh(f, ps, ds, ls);
-        }
-        if (vertical) {
-            for (int i = 0; i < 3; i += 2) {
-                const V3<R> ps = pos + ddz * R(dxs[i]) * cr + ddy * R(dys[i]) * ch;
-                seg_on_mesh(f, ps, ddy * R(-dxs[i]), ch * 2);
-            }
-        }
-    });
-    mesh_query(m, aa, bb, [&](int f) {
-        const int n = m.face_size(f);
-        for (int i = 0; i < n; i++) {
-            const V3<R> v1 = m.vert(m.face_vert(f, i));
-            const V3<R> v2 = m.vert(m.face_vert(f, (i + 1) % n));
-            R t1, t2;
-            const V3<R> start = (v1 + v2) / R(2);
-            const R ls = norm(v2 - v1) / 2;
-            const V3<R> dir = (v2 - v1) / (ls * 2);
-            if (segment_cylinder(start, dir, ls, pos, axis, ch, cr, margin, t1, t2)) {
-                const V3<R> p1 = start + dir * t1, p2 = start + dir * t2;
-                add_on_cylinder(c, (p1 + p2) / R(2), pos, axis, cr, ch, to, margin);
-            }
-        }
-    });
+    const CylinderFrame<R> fr{axis, pos, cr, ch, to};
+    mesh_query(m, aa, bb, [&](int f) { cylinder_face_sides(c, m, fr, f); });
+    mesh_query(m, aa, bb, [&](int f) { cylinder_face_edges(c, m, fr, f); });
     c.c->swap = false;
     return true;
 }
@@ -972,44 +1009,31 @@ template <class R> __device__ bool cylinder_hull(Pair<R>& c) {   // cylinder_con
 // face order, its normal, no unique edges: setMesh is never called on it) that the convex-convex
 // algorithm meets with the convex shape first, at the concave body's transform.
 constexpr int kFaceVerts = 32;   // longest face polygon a concave mesh may hold (checked at upload)
-template <class R> __device__ bool concave_convex(Pair<R>& c) {
-    const bool a_cc = c.sa.type == ST_CONCAVE;
-    const ShapeView<R>& cc = a_cc ? c.sa : c.sb;
-    const ShapeView<R> cv = a_cc ? c.sb : c.sa;
-    const Xf<R> tcc = a_cc ? c.xa : c.xb;
-    const Xf<R> tcv = a_cc ? c.xb : c.xa;
-    c.c->swap = a_cc;
-    V3<R> aa, bb;
-    shape_aabb(cv, tcc.inverse() * tcv, aa, bb);
+template <class R, class C>
+__device__ void concave_face(Pair<R, C>& c, const ShapeView<R>& cc, const ShapeView<R>& cv, const Xf<R>& tcc, const Xf<R>& tcv, int f) {
     R fv[kFaceVerts * 3];
     int fidx[kFaceVerts];
-    int foff[2];
     R fn[3], fmn[3], fmx[3];
-    mesh_query(cc, aa, bb, [&](int f) {
-        const int n = cc.face_size(f);
-        foff[0] = 0;
-        foff[1] = n;
-        for (int k = 0; k < 3; k++) { fmn[k] = Lim<R>::max(); fmx[k] = Lim<R>::min(); }
-        for (int i = 0; i < n; i++) {
-            const V3<R> p = cc.vert(cc.face_vert(f, i));
-            fv[i * 3] = p.x; fv[i * 3 + 1] = p.y; fv[i * 3 + 2] = p.z;
-            fidx[i] = i;
-            for (int k = 0; k < 3; k++) { fmn[k] = fmn[k] < p[k] ? fmn[k] : p[k]; fmx[k] = fmx[k] > p[k] ? fmx[k] : p[k]; }
-        }
-        const V3<R> nrm = cc.face_normal(f);
-        fn[0] = nrm.x; fn[1] = nrm.y; fn[2] = nrm.z;
-        ShapeView<R> face = cc;
-        face.type = ST_HULL;
-        face.hv = fv; face.nv = n;
-        face.f_off = foff; face.f_idx = fidx; face.f_n = fn; face.f_min = fmn; face.f_max = fmx; face.nf = 1;
-        face.e_a = nullptr; face.e_b = nullptr; face.e_d = nullptr; face.ne = 0;
-        face.nl = 0;
-        Pair<R> s = c;
-        s.sa = cv; s.sb = face; s.xa = tcv; s.xb = tcc;
-        convex_convex(s);
-    });
-    c.c->swap = false;
-    return true;
+    const int n = cc.face_size(f);
+    const int foff[2] = {0, n};
+    for (int k = 0; k < 3; k++) { fmn[k] = Lim<R>::max(); fmx[k] = Lim<R>::min(); }
+    for (int i = 0; i < n; i++) {
+        const V3<R> p = cc.vert(cc.face_vert(f, i));
+        fv[i * 3] = p.x; fv[i * 3 + 1] = p.y; fv[i * 3 + 2] = p.z;
+        fidx[i] = i;
+        for (int k = 0; k < 3; k++) { fmn[k] = fmn[k] < p[k] ? fmn[k] : p[k]; fmx[k] = fmx[k] > p[k] ? fmx[k] : p[k]; }
+    }
+    const V3<R> nrm = cc.face_normal(f);
+    fn[0] = nrm.x; fn[1] = nrm.y; fn[2] = nrm.z;
+    ShapeView<R> face = cc;
+    face.type = ST_HULL;
+    face.hv = fv; face.nv = n;
+    face.f_off = foff; face.f_idx = fidx; face.f_n = fn; face.f_min = fmn; face.f_max = fmx; face.nf = 1;
+    face.e_a = nullptr; face.e_b = nullptr; face.e_d = nullptr; face.ne = 0;
+    face.nl = 0;
+    Pair<R, C> s = c;
+    s.sa = cv; s.sb = face; s.xa = tcv; s.xb = tcc;
+    convex_convex(s);
 }
 
 // pair classes (narrow_phase_base.cpp:20-29 restricted to the four convex shape types)
@@ -1035,18 +1059,9 @@ __host__ __device__ inline int pair_class(int ta, int tb) {
     return PC_CONVEX;   // cylinder-cylinder, box-hull, hull-hull
 }
 
-// a concave mesh against any convex shape (narrow_phase_base.cpp:20-29, row and column 4);
-// concave-concave has no algorithm
-template <class R> __device__ void concave_pair(Pair<R>& c) {
-    const int o = c.sa.type == ST_CONCAVE ? c.sb.type : c.sa.type;
-    if (o == ST_SPHERE) sphere_hull(c);
-    else if (o == ST_CYLINDER) cylinder_hull(c);
-    else if (o == ST_BOX || o == ST_HULL) concave_convex(c);
-}
-
-template <class R> __device__ void collide(Pair<R>& c, int cls) {
+// the algorithm of a pair of primitives or hulls (pairs with a concave mesh run face by face, k_np_mesh)
+template <class R, class C> __device__ void collide(Pair<R, C>& c, int cls) {
     switch (cls) {
-        case PC_CONCAVE: concave_pair(c); break;
         case PC_BOX_BOX: box_box(c); break;
         case PC_BOX_SPHERE: box_sphere(c); break;
         case PC_SPHERE_SPHERE: sphere_sphere(c); break;

@@ -1,4 +1,4 @@
-// Kernels of the rigid-body step, part 6: the solver's iterations, run as a flow of body velocities
+// Kernels of the rigid-body step, part 7: the solver's iterations, run as a flow of body velocities
 // between island items.
 //
 // An island's items (contact results, then joints) act on their two bodies' temporary velocities in

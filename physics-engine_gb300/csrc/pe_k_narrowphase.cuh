@@ -166,52 +166,4 @@ __global__ void k_np_class(const int2* rng, const int* order, const int2* pairs,
     });
 }
 
-// CompoundCompoundCollisionAlgorithm::processCollision (compound_compound_collision_algorithm.cpp:8-46),
-// one thread per pair with a compound on either side.  A compound second swaps the pair (shapes,
-// transforms and the result's objects: ContactResult::setObjects(B, A), so the result names the
-// compound as object A); then every child of the compound, against every child of a second
-// compound or against the other shape, runs its shape pair's algorithm into the same contact
-// cache at the child's world transform (body transform * local transform).  Local contact
-// positions stay relative to the bodies.
-template <class R>
-__device__ __forceinline__ void compound_pair(int p, const int2* pairs, const Bodies<R>& B, const ShapeTable<R>& S, const Results<R>& res,
-                                              const int* pair_scene_off, const int* prev_off) {
-    Cache<R> cache;
-    Pair<R> pr;
-    np_setup(p, pairs, B, S, res, pair_scene_off, prev_off, cache, pr);
-    int sa = B.shape[pairs[p].x], sb = B.shape[pairs[p].y];
-    bool swapped = false;
-    if (pr.sb.type == ST_COMPOUND) {
-        const ShapeView<R> v = pr.sa; pr.sa = pr.sb; pr.sb = v;
-        const Xf<R> x = pr.xa; pr.xa = pr.xb; pr.xb = x;
-        const Xf<R> y = cache.ta; cache.ta = cache.tb; cache.tb = y;
-        const R z = cache.scale_a; cache.scale_a = cache.scale_b; cache.scale_b = z;
-        const int w = sa; sa = sb; sb = w;
-        swapped = true;
-    }
-    const Xf<R> ta = pr.xa, tb = pr.xb;
-    const bool b_comp = pr.sb.type == ST_COMPOUND;
-    for (int i = S.c_beg[sa], ie = S.c_beg[sa] + S.c_cnt[sa]; i < ie; i++) {
-        Pair<R> c = pr;
-        c.sa = S.view(S.c_shape[i]);
-        c.xa = ta * S.child_xf(i);
-        if (b_comp) {
-            for (int j = S.c_beg[sb], je = S.c_beg[sb] + S.c_cnt[sb]; j < je; j++) {
-                c.sb = S.view(S.c_shape[j]);
-                c.xb = tb * S.child_xf(j);
-                collide(c, pair_class(c.sa.type, c.sb.type));
-            }
-        } else {
-            collide(c, pair_class(c.sa.type, c.sb.type));
-        }
-    }
-    np_finish(p, pairs, B, res, cache, swapped);
-}
-
-template <class R>
-__global__ void k_np_compound(const int2* rng, const int* order, const int2* pairs, Bodies<R> B, ShapeTable<R> S, Results<R> res,
-                              const int* pair_scene_off, const int* prev_off) {
-    thread_items(*rng, [&](int t) { compound_pair(order[t], pairs, B, S, res, pair_scene_off, prev_off); });
-}
-
 } // namespace pe

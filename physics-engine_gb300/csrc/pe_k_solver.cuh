@@ -1,6 +1,6 @@
-// Kernels of the rigid-body step, part 5: sequential-impulse rows, joints and contact islands.
+// Kernels of the rigid-body step, part 6: sequential-impulse rows, joints and contact islands.
 #pragma once
-#include "pe_k_sat.cuh"
+#include "pe_k_mesh.cuh"
 
 namespace pe {
 

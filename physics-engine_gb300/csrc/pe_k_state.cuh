@@ -1,4 +1,4 @@
-// Kernels of the rigid-body step, part 7: body-state transfer in the C ABI's layout.
+// Kernels of the rigid-body step, part 8: body-state transfer in the C ABI's layout.
 #pragma once
 #include "pe_k_flow.cuh"
 

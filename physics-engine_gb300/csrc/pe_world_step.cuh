@@ -269,8 +269,10 @@ template <class R> void World<R>::np_enqueue() {
             case PC_SPHERE_SPHERE: launch(K_NP, pgrid(cap, kBlock, k_np_class<R, PC_SPHERE_SPHERE>), k_np_class<R, PC_SPHERE_SPHERE>, rg, on, pp, bd, sh, rs, pso, pro); break;
             case PC_SPHERE_CYL: launch(K_NP, pgrid(cap, kBlock, k_np_class<R, PC_SPHERE_CYL>), k_np_class<R, PC_SPHERE_CYL>, rg, on, pp, bd, sh, rs, pso, pro); break;
             case PC_BOX_CYL: launch(K_NP, pgrid(cap, kBlock, k_np_class<R, PC_BOX_CYL>), k_np_class<R, PC_BOX_CYL>, rg, on, pp, bd, sh, rs, pso, pro); break;
-            case PC_CONCAVE: launch(K_NP, pgrid(cap, kBlock, k_np_class<R, PC_CONCAVE>), k_np_class<R, PC_CONCAVE>, rg, on, pp, bd, sh, rs, pso, pro); break;
-            case PC_COMPOUND: launch(K_NP, pgrid(cap, kBlock, k_np_compound<R>), k_np_compound<R>, rg, on, pp, bd, sh, rs, pso, pro); break;
+            case PC_CONCAVE:
+            case PC_COMPOUND:
+                launch_block(K_NP, pgrid(cap, 1, k_np_mesh<R>, 32), 32, k_np_mesh<R>, rg, wk, on, pp, bd, sh, rs, pso, pro);
+                break;
             case PC_SPHERE_HULL: {
                 const int w = sphere_hull_warps<R>();
                 launch_block(K_NP, pgrid(cap, w, k_np_sphere_hull<R>, 32 * w), 32 * w, k_np_sphere_hull<R>, rg, wk, on, pp, bd, sh, rs, pso, pro);
