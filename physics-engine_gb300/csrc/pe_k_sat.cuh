@@ -35,20 +35,6 @@ template <class R> __device__ __forceinline__ V3<R> shfl3(const V3<R>& v, int sr
     return V3<R>(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src), __shfl_sync(0xffffffffu, v.z, src));
 }
 
-// ---- SAT with per-pair staging: world face normals, world unit edge directions and local hull
-// vertices of both shapes are computed once into shared memory; support intervals are computed
-// first and witness points only for an axis that becomes the current best.  Same formulas as
-// Shape::project (so the same bits); only the order of evaluation across axes differs.
-template <class R> constexpr int sat_stage_reals() { return 3 * (2 * kSatF + 2 * kSatE) + 4 * 2 * kSatV; }
-
-template <class R> struct SatStage {
-    R* nA; R* nB; R* dA; R* dB; R* vA; R* vB;   // vertices padded to 4 reals (16-byte aligned rows)
-    __device__ void bind(R* base) {
-        nA = base; nB = nA + 3 * kSatF; dA = nB + 3 * kSatF; dB = dA + 3 * kSatE; vA = dB + 3 * kSatE; vB = vA + 4 * kSatV;
-    }
-};
-template <class R> __device__ __forceinline__ V3<R> ld3(const R* p, int i) { return V3<R>(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
-template <class R> __device__ __forceinline__ void st3(R* p, int i, const V3<R>& v) { p[3 * i] = v.x; p[3 * i + 1] = v.y; p[3 * i + 2] = v.z; }
 __device__ __forceinline__ V3<float> ldv(const float* p, int i) {
     const float4 f = reinterpret_cast<const float4*>(p)[i];
     return V3<float>(f.x, f.y, f.z);
@@ -107,87 +93,6 @@ __device__ __forceinline__ void shape_interval(const ShapeView<R>& s, const Xf<R
     mxp += off;
 }
 
-// two axes at once: a hull's vertices are loaded once for both (same arithmetic per axis)
-template <class R>
-__device__ __forceinline__ void shape_interval2(const ShapeView<R>& s, const Xf<R>& t, const V3<R>* axis, const R* lv, R* mnp, R* mxp,
-                                                int* imn, int* imx) {
-    if (s.type != ST_HULL) {
-        shape_interval(s, t, axis[0], lv, mnp[0], mxp[0], imn[0], imx[0]);
-        shape_interval(s, t, axis[1], lv, mnp[1], mxp[1], imn[1], imx[1]);
-        return;
-    }
-    const V3<R> l0 = mtv(t.b, axis[0]), l1 = mtv(t.b, axis[1]);
-    R n0 = Lim<R>::max(), x0 = Lim<R>::min(), n1 = Lim<R>::max(), x1 = Lim<R>::min();
-    int in0 = -1, ix0 = -1, in1 = -1, ix1 = -1;
-    for (int i = 0; i < s.nv; i++) {
-        const V3<R> p = ldv(lv, i);
-        const R v0 = dot(p, l0), v1 = dot(p, l1);
-        if (v0 < n0) { n0 = v0; in0 = i; }
-        else if (v0 > x0) { x0 = v0; ix0 = i; }
-        if (v1 < n1) { n1 = v1; in1 = i; }
-        else if (v1 > x1) { x1 = v1; ix1 = i; }
-    }
-    const R o0 = dot(t.o, axis[0]), o1 = dot(t.o, axis[1]);
-    mnp[0] = n0 + o0; mxp[0] = x0 + o0; imn[0] = in0; imx[0] = ix0;
-    mnp[1] = n1 + o1; mxp[1] = x1 + o1; imn[1] = in1; imx[1] = ix1;
-}
-
-// Intervals of both shapes along two axes.  The larger hull's vertex loop may stop early: its
-// running minimum only falls and its (first-vertex-excluding) running maximum only rises, so the
-// overlap depths min(maxA - minB, maxB - minA) computed from a prefix of its vertices are lower
-// bounds of the final ones (IEEE rounding is monotone).  Once both depths of an axis exceed `best`
-// (an upper bound of the pair's minimum depth) the axis can neither separate nor be the minimum;
-// when that holds for both axes the loop ends and both are reported not live.  Compiled out of line:
-// the face and the edge passes share one copy, and the SAT kernels' instruction fetch stalls fell
-// with the code size (the staged SAT group 6.52 -> 5.76 ms per batched step).
-template <class R>
-__device__ __noinline__ void pair_intervals2(const Pair<R>& c, const V3<R>* ax, bool* live, R best, const R* vA, const R* vB,
-                                                R* min0, R* max0, R* min1, R* max1, int* a0, int* a1, int* b0, int* b1) {
-    const bool part_b = c.sb.type == ST_HULL && (c.sa.type != ST_HULL || c.sb.nv >= c.sa.nv);
-    const bool part_a = !part_b && c.sa.type == ST_HULL;
-    if (!part_a && !part_b) {
-        shape_interval2(c.sa, c.ta(), ax, vA, min0, max0, a0, a1);
-        shape_interval2(c.sb, c.tb(), ax, vB, min1, max1, b0, b1);
-        return;
-    }
-    // the complete side first
-    const ShapeView<R>& sp = part_b ? c.sb : c.sa;
-    const Xf<R>& tp = part_b ? c.tb() : c.ta();
-    const R* lv = part_b ? vB : vA;
-    R cmn[2], cmx[2];
-    if (part_b) { shape_interval2(c.sa, c.ta(), ax, vA, min0, max0, a0, a1); cmn[0] = min0[0]; cmn[1] = min0[1]; cmx[0] = max0[0]; cmx[1] = max0[1]; }
-    else { shape_interval2(c.sb, c.tb(), ax, vB, min1, max1, b0, b1); cmn[0] = min1[0]; cmn[1] = min1[1]; cmx[0] = max1[0]; cmx[1] = max1[1]; }
-    const V3<R> l0 = mtv(tp.b, ax[0]), l1 = mtv(tp.b, ax[1]);
-    const R o0 = dot(tp.o, ax[0]), o1 = dot(tp.o, ax[1]);
-    R n0 = Lim<R>::max(), x0 = Lim<R>::min(), n1 = Lim<R>::max(), x1 = Lim<R>::min();
-    int in0 = -1, ix0 = -1, in1 = -1, ix1 = -1;
-    bool done = false;
-    for (int i0 = 0; i0 < sp.nv; i0 += 8) {
-        const int e = i0 + 8 < sp.nv ? i0 + 8 : sp.nv;
-        for (int i = i0; i < e; i++) {
-            const V3<R> p = ldv(lv, i);
-            const R v0 = dot(p, l0), v1 = dot(p, l1);
-            if (v0 < n0) { n0 = v0; in0 = i; }
-            else if (v0 > x0) { x0 = v0; ix0 = i; }
-            if (v1 < n1) { n1 = v1; in1 = i; }
-            else if (v1 > x1) { x1 = v1; ix1 = i; }
-        }
-        if (e == sp.nv) break;
-        // partial depths: d0 = maxA - minB, d1 = maxB - minA with the partial side's running values
-        bool dec[2];
-        const R pn[2] = {n0 + o0, n1 + o1}, px[2] = {x0 + o0, x1 + o1};
-        for (int k = 0; k < 2; k++) {
-            const R d0 = part_b ? cmx[k] - pn[k] : px[k] - cmn[k];
-            const R d1 = part_b ? px[k] - cmn[k] : cmx[k] - pn[k];
-            dec[k] = !live[k] || (d0 > best && d1 > best);
-        }
-        if (dec[0] && dec[1]) { done = true; break; }
-    }
-    if (done) { live[0] = live[1] = false; return; }
-    if (part_b) { min1[0] = n0 + o0; max1[0] = x0 + o0; b0[0] = in0; b1[0] = ix0; min1[1] = n1 + o1; max1[1] = x1 + o1; b0[1] = in1; b1[1] = ix1; }
-    else { min0[0] = n0 + o0; max0[0] = x0 + o0; a0[0] = in0; a1[0] = ix0; min0[1] = n1 + o1; max0[1] = x1 + o1; a0[1] = in1; a1[1] = ix1; }
-}
-
 // witness point of Shape::project on the min (want_max = false) or max side
 template <class R>
 __device__ V3<R> shape_witness(const ShapeView<R>& s, const Xf<R>& t, const V3<R>& axis, bool want_max, int idx, const R* lv) {
@@ -203,12 +108,98 @@ __device__ V3<R> shape_witness(const ShapeView<R>& s, const Xf<R>& t, const V3<R
     return want_max ? pmax : pmin;
 }
 
+// ---- staged SAT: bounds first, exact projections for what the bounds leave.
+//
+// The pair's minimum depth decides everything, and few axes come near it.  For every candidate axis a
+// cheap lower bound of its overlap depth is taken (fused multiply-adds, unnormalised axes, a few
+// supporting points per hull), and only axes whose bound does not exceed a depth the pair is known to
+// reach are queued and projected with the reference's formulas (Shape::project, the same bits).  A
+// skipped axis is certainly above that depth, so it can neither separate the pair nor be its first
+// minimum, and candidates compare by (depth, reference axis index), the reference's first strict
+// minimum in any visiting order.
+//
+// What bounds it is instruction fetch and issue: 32 axes cost about 60 instructions for the bound (two
+// hulls' edge pairs mostly some 25, see `hulls`), and most pairs one round of exact projections for the
+// faces and one for the edges.  Per step of the 4,096 piles, before (every axis past a ball test projected
+// exactly, two per lane) and now: hull-hull 1,750 / 494 us, its heavy pairs 778 / 250, box-hull
+// 2,311 / 1,840, cylinder-cylinder 935 / 412; the whole step 8.68 / 6.30 ms, the 501-body pile's
+// 964 / 655 us (its tail was one hull pair).
+
+// One side's bound data.  rel: the support points are taken relative to the shape's own origin.
+constexpr int kSub = 8;          // supporting points per hull
+template <class R> struct SatSide {
+    V3<R> e0, e1, e2;            // box: half axes; cylinder: e0 the unit axis
+    R r, hh;                     // cylinder
+    R inner;                     // a ball about the origin inside the shape (<= 0: none)
+    R mag;                       // bound of the distances entering the projections' rounding
+};
+constexpr int kSatBase = 4 * (kSub + 2);   // reals of one hull's supporting points: kSub of them, then vertices 0 and 1
+template <class R> __device__ __forceinline__ R fma3(const V3<R>& a, const V3<R>& b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
+__device__ __forceinline__ float fast_sqrt(float x) { float r; asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ double fast_sqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ float fast_max(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double fast_max(double a, double b) { return fmax(a, b); }
+template <class R> constexpr R sat_slack() { return sizeof(R) == 4 ? R(96 * 1.1920929e-7) : R(96 * 2.220446049250313e-16); }
+
+// Lower bound of the support of a shape along y (of length ny): box and cylinder in closed form (a
+// cylinder lowered by what the reference's branches for nearly axial and nearly radial axes drop), a
+// hull by its supporting points.  For the second shape (QUIRK) a hull's bound counts only when vertex 0
+// or 1, which come before every supporting point, lies below it: the reference never lets a new
+// minimum become the maximum (convex_mesh_shape.cpp:171-175), and a point above an earlier vertex is no
+// new minimum.
+template <class R, int T, bool QUIRK>
+__device__ __forceinline__ R sat_support(int type, const SatSide<R>& s, const V3<R>& y, R ny, const R* sub, R slack) {
+    const int t = T >= 0 ? T : type;
+    if (t == ST_BOX) return rabs(fma3(y, s.e0)) + rabs(fma3(y, s.e1)) + rabs(fma3(y, s.e2));
+    if (t == ST_CYLINDER) {
+        const R c = fma3(y, s.e0);
+        const R n2 = ny * ny;   // the axis's part across the cylinder's, its square lowered by its own roundoff
+        return fma(s.hh, rabs(c), s.r * fast_sqrt(fast_max(fma(-c, c, n2) - R(0.125) * sat_slack<R>() * n2, R(0)))) - R(3e-5) * (s.r + s.hh) * ny;
+    }
+    R m = fma3(y, ldv(sub, 0));
+#pragma unroll
+    for (int k = 1; k < kSub; k++) m = fast_max(m, fma3(y, ldv(sub, k)));
+    if (QUIRK) {
+        const R u0 = fma3(y, ldv(sub, kSub)), u1 = fma3(y, ldv(sub, kSub + 1));
+        if (!(m > (u0 < u1 ? u0 : u1) + slack * ny)) m = Lim<R>::min();
+    }
+    return m;
+}
+
+// Picks the kSub vertices of a hull furthest along dir (its local frame) among those from `first` on,
+// and stores them turned into the world and multiplied by sgn.  One warp.
+template <class R>
+__device__ __forceinline__ void sat_pick(const ShapeView<R>& s, const M3<R>& b, const R* lv, const V3<R>& dir, int first, R sgn, R* sub, int lane) {
+    auto key = [&](int i) -> unsigned {   // order bits of the projection, the index in the low bits
+        if (i < first || i >= s.nv) return 0u;
+        const V3<R> p = ldv(lv, i);
+        const unsigned u = __float_as_uint((float)fma3(p, dir));
+        return (((u & 0x80000000u) ? ~u : (u | 0x80000000u)) & ~(unsigned)(kSatV - 1)) | (unsigned)i | kSatV;
+    };
+    unsigned k0 = key(lane), k1 = key(lane + 32), mine = 0, top = 0;
+#pragma unroll
+    for (int n = 0; n < kSub; n++) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, k0 > k1 ? k0 : k1);
+        if (n == 0) top = m;
+        if (k0 == m) k0 = 0;
+        if (k1 == m) k1 = 0;
+        if (lane == n) mine = m ? m : top;   // fewer vertices than points: the first again
+    }
+    if (lane < kSub + 2) {
+        const int i = lane < kSub ? (int)(mine & (unsigned)(kSatV - 1)) : lane - kSub;
+        stv(sub, lane, mv(b, ldv(lv, i)) * sgn);
+    }
+}
+
 // Group primitives of the staged SAT: a group is one warp (G = 1) or a whole block of G warps.
 // Reductions are lexicographic (value, axis index) minima/maxima, so their result does not depend
 // on the order lanes and warps are combined in.
 template <int G> __device__ __forceinline__ bool group_any(bool p) {
     if (G == 1) return __any_sync(0xffffffffu, p);
     return __syncthreads_or(p) != 0;
+}
+template <int G> __device__ __forceinline__ void group_sync() {
+    if (G == 1) __syncwarp(); else __syncthreads();
 }
 template <class R, int G> __device__ __forceinline__ void group_argmin(R& d, int& idx, int tid, R* rd, int* ri) {
     warp_argmin(d, idx);
@@ -239,54 +230,12 @@ template <class R, int G> __device__ __forceinline__ V3<R> group_bcast3(const V3
     __syncthreads();
     return r;
 }
-// reals of per-group scratch after the staging area: G reduction values, G indices, 3 broadcast,
-// the queue length
-template <class R> constexpr int sat_scratch_reals(int G) { return G == 1 ? 0 : 2 * G + 4; }
-// candidate axes per thread of one pruning pass, and the queue of surviving axis indices after the
-// scratch area (16: the batched step 0.27 ms faster than with 8, 4 slower)
-constexpr int kSatQ = 16;
-template <class R> constexpr int sat_queue_reals(int G) { return (kSatQ * 32 * G * (int)sizeof(int) + (int)sizeof(R) - 1) / (int)sizeof(R); }
-
-// Pruning bound of one shape along a world axis: lo <= the computed maximum of its projection
-// interval, hi >= the computed minimum (a hull: its inner ball about the local origin; another
-// shape: its closed-form interval), and mag bounds the magnitudes entering their rounding.
+// The inner balls' bound of an axis x of length nx, held against the depth `best`: lo <= the computed
+// maximum of a shape's projection (a hull: its inner ball about the local origin; another shape: its
+// closed-form interval), hi >= the computed minimum, mag the magnitudes entering their rounding, and 64
+// units of roundoff of those on top of `best`.
 template <class R>
-__device__ __forceinline__ void prune_side(const ShapeView<R>& s, const Xf<R>& t, const V3<R>& ax, R& lo, R& hi, R& mag) {
-    if (s.type == ST_HULL) {
-        const R o = dot(t.o, ax);
-        lo = o + s.inner;
-        hi = o - s.inner;
-        mag = rabs(o) + s.outer;
-        return;
-    }
-    int i0, i1;
-    shape_interval(s, t, ax, (const R*)nullptr, hi, lo, i0, i1);
-    mag = rabs(hi) + rabs(lo);
-}
-// True when the axis's overlap depth min(maxA - minB, maxB - minA) is certainly above `best`, a
-// depth the SAT has already computed for one of the pair's axes (so best >= 0): such an axis can
-// neither separate the pair nor be its minimum (the reference keeps the first strict minimum), and
-// skipping it leaves the result unchanged.  The bound is lowered by 64 units of roundoff of the
-// magnitudes involved, which covers the rounding of the projections the SAT would compute.  `able`
-// is false when a hull of the pair has no certified inner ball.
-template <class R>
-__device__ __forceinline__ bool sat_prunable(const Pair<R>& c, bool able, const V3<R>& ax, R best) {
-    if (!able || !(best < Lim<R>::max())) return false;
-    R loA, hiA, mA, loB, hiB, mB;
-    prune_side(c.sa, c.ta(), ax, loA, hiA, mA);
-    prune_side(c.sb, c.tb(), ax, loB, hiB, mB);
-    const R d0 = loA - hiB, d1 = loB - hiA;
-    const R lb = d0 < d1 ? d0 : d1;
-    constexpr R u = sizeof(R) == 4 ? R(1.1920929e-7) : R(2.220446049250313e-16);
-    return lb > best + R(64) * u * (mA + mB + rabs(best));
-}
-// The same test on an unnormalised axis x of length nx (computed as the reference's norm): every
-// projection scales by nx, so the bound and the slack are scaled by nx instead of dividing x by
-// it.  The normalisation the test skips changes each projection by a few units of roundoff, well
-// inside the 64-unit slack.  For boxes and hulls only (a cylinder's closed form branches on
-// near-zero components of the normalised axis).
-template <class R>
-__device__ __forceinline__ void prune_side_scaled(const ShapeView<R>& s, const Xf<R>& t, const V3<R>& x, R nx, R& lo, R& hi, R& mag) {
+__device__ __forceinline__ void ball_side(const ShapeView<R>& s, const Xf<R>& t, const V3<R>& x, R nx, R& lo, R& hi, R& mag) {
     if (s.type == ST_HULL) {
         const R o = dot(t.o, x);
         lo = o + s.inner * nx;
@@ -299,56 +248,17 @@ __device__ __forceinline__ void prune_side_scaled(const ShapeView<R>& s, const X
     mag = rabs(hi) + rabs(lo);
 }
 template <class R>
-__device__ __forceinline__ bool sat_prunable_scaled(const Pair<R>& c, bool able, const V3<R>& x, R nx, R best) {
-    if (!able || !(best < Lim<R>::max())) return false;
+__device__ __forceinline__ bool balls_above(const Pair<R>& c, const V3<R>& x, R nx, R best) {
     R loA, hiA, mA, loB, hiB, mB;
-    prune_side_scaled(c.sa, c.ta(), x, nx, loA, hiA, mA);
-    prune_side_scaled(c.sb, c.tb(), x, nx, loB, hiB, mB);
+    ball_side(c.sa, c.ta(), x, nx, loA, hiA, mA);
+    ball_side(c.sb, c.tb(), x, nx, loB, hiB, mB);
     const R d0 = loA - hiB, d1 = loB - hiA;
     const R lb = d0 < d1 ? d0 : d1;
     constexpr R u = sizeof(R) == 4 ? R(1.1920929e-7) : R(2.220446049250313e-16);
     return lb > nx * best + R(64) * u * (mA + mB + nx * rabs(best));
 }
-// Compacts the candidate axes [base, base + span) ∩ [0, n) that `keep` accepts into the group's
-// queue and returns their count (the same in every thread of the group).  With one warp the queue
-// keeps ascending order; with several, warps append in any order.
-template <int G, class F>
-__device__ __forceinline__ int sat_queue(int base, int span, int n, int tid, int* q, int* qn, F&& keep) {
-    constexpr int T = 32 * G;
-    const unsigned lt = (1u << (tid & 31)) - 1u;
-    int cnt = 0;
-    for (int j = 0; j < span; j += T) {
-        const int f = base + j + tid;
-        const bool k = f < n && keep(f);
-        const unsigned m = __ballot_sync(0xffffffffu, k);
-        if (G == 1) {
-            if (k) q[cnt + __popc(m & lt)] = f;
-            cnt += __popc(m);
-        } else {
-            int b = 0;
-            if ((tid & 31) == 0 && m) b = atomicAdd(qn, __popc(m));
-            b = __shfl_sync(0xffffffffu, b, 0);
-            if (k) q[b + __popc(m & lt)] = f;
-        }
-    }
-    if (G == 1) {
-        __syncwarp();
-        return cnt;
-    }
-    __syncthreads();
-    cnt = *qn;
-    __syncthreads();
-    if (tid == 0) *qn = 0;   // visible to the next pass's appends after sat_queue_done
-    return cnt;
-}
-// the queue is read until here; the next pass may refill it
-template <int G> __device__ __forceinline__ void sat_queue_done() {
-    if (G == 1) __syncwarp(); else __syncthreads();
-}
-
-// Staged SAT of one pair by a group of G warps (tid in [0, 32 G)).  Per pass the group tests
-// candidate axes against the pruning bound, queues the survivors and projects them two per thread;
-// it stops at the first round holding a separating axis.
+// reals of per-group scratch: G reduction values, G indices, 3 broadcast, the group's bound
+template <class R> constexpr int sat_scratch_reals(int G) { return G == 1 ? 0 : 2 * G + 4; }
 // What the staged SAT leaves for the contact step (one record of kSatOut reals per pair, written by
 // thread 0): the face-stage point, the edge-stage point, the final axis and the clipping faces,
 // in the order the reference adds them (convex_convex_collision_algorithm.cpp:300-308, :363-395,
@@ -358,86 +268,211 @@ enum SatOutField { SO_FLAGS = 0, SO_FN = 1, SO_FP = 4, SO_FD = 7, SO_EN = 8, SO_
 template <class R> __device__ __forceinline__ void so_put3(R* o, int k, const V3<R>& v) { o[k] = v.x; o[k + 1] = v.y; o[k + 2] = v.z; }
 template <class R> __device__ __forceinline__ V3<R> so_get3(const R* o, int k) { return V3<R>(o[k], o[k + 1], o[k + 2]); }
 
+// group layout in shared memory: both edge lists (the face axes before them), both shapes' vertices, the supporting points, the
+// queues (one per warp), the scratch
+constexpr int kSatFree = 64, kSatBlock = 512;   // see sat_staged's balls
+constexpr int kSatQueue = 64;    // queued axes per warp: a round's 32 and what the next 32 candidates can add
+template <class R> constexpr int sat_group_reals(int G) {
+    const int q = (kSatQueue * G * (int)sizeof(int) + (int)sizeof(R) - 1) / (int)sizeof(R);
+    return (4 * 2 * kSatE + 4 * 2 * kSatV + 2 * kSatBase + q + sat_scratch_reals<R>(G) + 3) & ~3;
+}
+
+// Staged SAT of one pair by a group of G warps (tid in [0, 32 G)).
 template <class R, int G, int TA, int TB>
 __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
     constexpr int T = 32 * G;
+    const unsigned full = 0xffffffffu;
+    const int lane = tid & 31, warp = tid >> 5;
     if (tid == 0) out[SO_FLAGS] = R(0);
     if (TA >= 0) c.sa.type = TA;   // shape types known at compile time: the other branches fold away
     if (TB >= 0) c.sb.type = TB;
     const R margin = c.margin;
-    SatStage<R> st;
-    st.bind(smem);
-    R* rd = smem + sat_stage_reals<R>();
+    R* ea = smem;
+    R* eb = ea + 4 * kSatE;
+    R* vA = eb + 4 * kSatE;
+    R* vB = vA + 4 * kSatV;
+    R* subA = vB + 4 * kSatV;
+    R* subB = subA + kSatBase;
+    int* queue = reinterpret_cast<int*>(subB + kSatBase) + warp * kSatQueue;
+    R* rd = smem + sat_group_reals<R>(G) - ((sat_scratch_reals<R>(G) + 3) & ~3);
     int* ri = reinterpret_cast<int*>(rd + G);
     R* bc = rd + 2 * G;
     const int fa = c.sa.face_count(), fb = c.sb.face_count();
     const int na = c.sa.edge_count(), nb = c.sb.edge_count();
-    for (int f = tid; f < fa; f += T) st3(st.nA, f, mv(c.ta().b, c.sa.face_normal(f)));
-    for (int f = tid; f < fb; f += T) st3(st.nB, f, mv(c.tb().b, c.sb.face_normal(f)));
-    // unit edge directions: a hull's come precomputed (k_hull_edge_dirs, the same arithmetic)
-    auto edge_unit = [](const ShapeView<R>& sh, int e) {
-        if (sh.type == ST_HULL) return sh.edge_dir(e);
-        V3<R> a0, a1;
-        sh.edge(e, a0, a1);
-        return normalized(a0 - a1);
-    };
-    for (int e = tid; e < na; e += T) st3(st.dA, e, mv(c.ta().b, edge_unit(c.sa, e)));
-    for (int e = tid; e < nb; e += T) st3(st.dB, e, mv(c.tb().b, edge_unit(c.sb, e)));
-    if (c.sa.type == ST_HULL) for (int i = tid; i < c.sa.nv; i += T) stv(st.vA, i, c.sa.vert(i));
-    if (c.sb.type == ST_HULL) for (int i = tid; i < c.sb.nv; i += T) stv(st.vB, i, c.sb.vert(i));
-    int* queue = reinterpret_cast<int*>(smem + sat_stage_reals<R>() + sat_scratch_reals<R>(G));
-    int* qn = reinterpret_cast<int*>(rd + 2 * G + 3);   // several warps: the queue length
-    if (G > 1 && tid == 0) *qn = 0;
-    if (G == 1) __syncwarp(); else __syncthreads();
+    const bool boxA = c.sa.type == ST_BOX, boxB = c.sb.type == ST_BOX;
+    if (c.sa.type == ST_HULL) for (int i = tid; i < c.sa.nv; i += T) stv(vA, i, c.sa.vert(i));
+    if (c.sb.type == ST_HULL) for (int i = tid; i < c.sb.nv; i += T) stv(vB, i, c.sb.vert(i));
+    group_sync<G>();
     const V3<R> dc = c.ta().o - c.tb().o;
-    const bool able = (c.sa.type != ST_HULL || c.sa.inner > 0) && (c.sb.type != ST_HULL || c.sb.inner > 0);
-    // ---- face axes of A, then of B (findSeparatingAxis :265-308).  Each pass compacts the axes
-    // that the running minimum does not rule out (sat_prunable) and projects those, two per thread;
-    // the first 2T axes run unpruned and give the bound.  A candidate compares by (depth, axis
-    // index), the reference's first strict minimum in any visiting order.
-    auto face_axis = [&](int f) {
-        V3<R> n = f < fa ? ld3(st.nA, f) : ld3(st.nB, f - fa);
-        if (dot(dc, n) < 0) n = n * R(-1.0);
-        return n;
+
+    // ---- bound data
+    auto side = [](const ShapeView<R>& s, const Xf<R>& t) {
+        SatSide<R> q;
+        if (s.type == ST_BOX) {
+            q.e0 = t.b.col(0) * s.half.x; q.e1 = t.b.col(1) * s.half.y; q.e2 = t.b.col(2) * s.half.z;
+            q.inner = rmin(s.half.x, rmin(s.half.y, s.half.z));
+            q.mag = s.half.x + s.half.y + s.half.z;
+        } else if (s.type == ST_CYLINDER) {
+            q.e0 = t.b.col(1); q.r = s.radius; q.hh = s.height * R(0.5);
+            q.inner = rmin(q.r, q.hh) * R(0.99);
+            q.mag = q.r + q.hh;
+        } else {
+            q.inner = s.inner;
+            q.mag = s.outer;
+        }
+        return q;
     };
+    const SatSide<R> qa = side(c.sa, c.ta()), qb = side(c.sb, c.tb());
+    // A hull's supporting points: its vertices furthest towards the other shape, from the nearest point
+    // of a box (a floor's centre says nothing about where a hull touches it), else the other's centre
+    {
+        V3<R> dir = dc;   // from B towards A
+        auto from_box = [](const ShapeView<R>& s, const Xf<R>& t, const V3<R>& o) {   // from the box's nearest point to o
+            const V3<R> p = t.inv_apply(o), h = s.half;
+            V3<R> d = p - V3<R>(rclamp(p.x, -h.x, h.x), rclamp(p.y, -h.y, h.y), rclamp(p.z, -h.z, h.z));
+            if (!(sqnorm(d) > 0)) {   // inside: out of the nearest face
+                const V3<R> g(h.x - rabs(p.x), h.y - rabs(p.y), h.z - rabs(p.z));
+                const int k = g.x <= g.y && g.x <= g.z ? 0 : g.y <= g.z ? 1 : 2;
+                d[k] = p[k] < 0 ? R(-1) : R(1);
+            }
+            return mv(t.b, d);
+        };
+        if (boxB && !boxA) dir = from_box(c.sb, c.tb(), c.ta().o);
+        else if (boxA && !boxB) dir = -from_box(c.sa, c.ta(), c.tb().o);
+        if (G == 1 || warp == 0) if (c.sa.type == ST_HULL) sat_pick(c.sa, c.ta().b, vA, mtv(c.ta().b, -dir), 0, R(-1), subA, lane);
+        if (G == 1 || warp == 0) if (c.sb.type == ST_HULL) sat_pick(c.sb, c.tb().b, vB, mtv(c.tb().b, dir), c.sb.nv > 2 ? 2 : 0, R(1), subB, lane);
+    }
+    // everything that enters a projection, in units of roundoff: the bounds' and the projections' errors
+    const R slack = sat_slack<R>() * (norm(c.ta().o) + norm(c.tb().o) + qa.mag + qb.mag);
+    const R deep = qa.inner + qb.inner - slack;   // every axis's other depth (the first shape past the second) is above this
+    const bool able = qa.inner > 0 && qb.inner > 0 && (c.sb.type != ST_HULL || c.sb.nv > 2);
+    group_sync<G>();
+    // lower bound of the depth along y, of length ny and oriented from B towards A (the reference takes the
+    // edge axes normalised and the face axes as they are: the cylinder mesh's normals are not all unit)
+    auto bound = [&](const V3<R>& y, R ny) {
+        return sat_support<R, TA, false>(c.sa.type, qa, y, ny, subA, slack) + sat_support<R, TB, true>(c.sb.type, qb, y, ny, subB, slack) - fma3(y, dc);
+    };
+    auto pruned = [&](R lb, R ny, R pb) { return able && pb < deep && lb > ny * (pb + slack); };
+    // The inner balls' bound of the same depth.  It alone also decides which axes of a hull count: the
+    // balls are certified for a projection that never takes vertex 0 as the maximum, but the reference
+    // passes over the vertices after it too while the projections keep falling, so along a few axes its
+    // depth is below the balls' bound, and those that the balls rule out stay out.  Face axes from
+    // kSatFree on are held against the least depth of the axes before them, edge axes against the least
+    // depth known when their block of kSatBlock axes begins.
+    constexpr bool has_hull = TA < 0 || TA == ST_HULL || TB == ST_HULL;
+    auto ball = [&](const V3<R>& y, R ny) {
+        auto one = [&](int type, const SatSide<R>& q) {
+            return type == ST_HULL ? q.inner * ny : rabs(fma3(y, q.e0)) + rabs(fma3(y, q.e1)) + rabs(fma3(y, q.e2));
+        };
+        return one(c.sa.type, qa) + one(c.sb.type, qb) - rabs(fma3(y, dc));
+    };
+    const bool balls = has_hull && able && (c.sa.type == ST_HULL || c.sb.type == ST_HULL);
+
+    // ---- exact projections along one axis per lane
+    R min0, max0, min1, max1;
+    int a0, a1, b0, b1;
+    auto project = [&](const V3<R>& n) {
+        shape_interval(c.sa, c.ta(), n, vA, min0, max0, a0, a1);
+        shape_interval(c.sb, c.tb(), n, vB, min1, max1, b0, b1);
+    };
+    int cnt = 0;   // queued axes, in order; a round takes the first 32
+    const unsigned lt = (1u << lane) - 1u;
+    auto push = [&](bool keep, int v) {   // at most 32 more
+        const unsigned m = __ballot_sync(full, keep);
+        if (keep) queue[cnt + __popc(m & lt)] = v;
+        cnt += __popc(m);
+    };
+    auto pop = [&](int& v) {   // this lane's axis of the round
+        __syncwarp();
+        const bool ok = lane < cnt;
+        v = ok ? queue[lane] : 0;
+        const int rest = cnt - 32, next = lane < rest ? queue[32 + lane] : 0;
+        __syncwarp();
+        if (lane < rest) queue[lane] = next;
+        cnt = rest > 0 ? rest : 0;
+        return ok;
+    };
+
+    // ---- face axes of A, then of B (findSeparatingAxis :265-308)
+    R* axes = ea;   // the face axes, until the edge lists take their place
+    for (int f = tid; f < fa + fb; f += T) {
+        V3<R> n = f < fa ? mv(c.ta().b, c.sa.face_normal(f)) : mv(c.tb().b, c.sb.face_normal(f - fa));
+        if (dot(dc, n) < 0) n = n * R(-1.0);
+        stv(axes, f, n);
+    }
+    group_sync<G>();
+    auto face_axis = [&](int f) { return ldv(axes, f); };
+    R pb = Lim<R>::max();   // a depth above which an axis is skipped
+    const int nfree = G == 1 && has_hull ? min(fa + fb, kSatFree) : fa + fb;
+    if (able) {   // the axis of the least bound, projected (upper bound of its depth): the first depth to beat
+        R least = Lim<R>::max();
+        int at = 0x7fffffff;
+        for (int f = tid; f < nfree; f += T) {
+            const V3<R> n = face_axis(f);
+            const R lb = bound(n, TA == ST_CYLINDER || TA < 0 ? fast_sqrt(fma3(n, n)) : R(1));
+            if (lb < least) { least = lb; at = f; }
+        }
+        group_argmin<R, G>(least, at, tid, rd, ri);
+        if (at < 0x7fffffff) {
+            const V3<R> y = face_axis(at);
+            auto whole = [&](const ShapeView<R>& s, const SatSide<R>& q, const Xf<R>& t, const R* lv, R sgn) {
+                if (s.type == ST_BOX) return rabs(fma3(y, q.e0)) + rabs(fma3(y, q.e1)) + rabs(fma3(y, q.e2));
+                if (s.type == ST_CYLINDER) {
+                    const R k = fma3(y, q.e0);
+                    const R n2 = fma3(y, y);
+                    return fma(q.hh, rabs(k), q.r * fast_sqrt(fast_max(fma(-k, k, n2) + R(0.125) * sat_slack<R>() * n2, R(0))));
+                }
+                const V3<R> yl = mtv(t.b, y) * sgn;
+                R m = Lim<R>::min();
+                for (int i = lane; i < s.nv; i += 32) m = fast_max(m, fma3(yl, ldv(lv, i)));
+                for (int o = 16; o > 0; o >>= 1) m = fast_max(m, __shfl_xor_sync(full, m, o));
+                return m;
+            };
+            pb = whole(c.sa, qa, c.ta(), vA, R(-1)) + whole(c.sb, qb, c.tb(), vB, R(1)) - fma3(y, dc) + slack;
+        }
+    }
     R bd = Lim<R>::max();
     int bf = 0x7fffffff, bside = 0, bia = -1, bib = -1;
-    for (int pass = 0; pass < fa + fb;) {
-        const int span = pass == 0 ? 2 * T : kSatQ * T;
-        R pb = bd;
-        warp_min(pb);
-        const int cnt = sat_queue<G>(pass, span, fa + fb, tid, queue, qn, [&](int f) { return !sat_prunable(c, able, face_axis(f), pb); });
-        for (int base = 0; base < cnt; base += 2 * T) {
-            V3<R> n[2];
-            bool ok[2];
-            int fi[2];
-            for (int k = 0; k < 2; k++) {
-                const int qi = base + T * k + tid;
-                ok[k] = qi < cnt;
-                fi[k] = ok[k] ? queue[qi] : 0x7fffffff;
-                n[k] = ok[k] ? face_axis(fi[k]) : V3<R>(0, 0, 0);
-            }
-            R min0[2], max0[2], min1[2], max1[2];
-            int a0[2], a1[2], b0[2], b1[2];
-            R best = bd;
-            warp_min(best);
-            pair_intervals2(c, n, ok, best, st.vA, st.vB, min0, max0, min1, max1, a0, a1, b0, b1);
-            bool sep = false;
-            for (int k = 0; k < 2; k++) sep |= ok[k] && (max0[k] < min1[k] || max1[k] < min0[k]);
-            if (group_any<G>(sep)) return;
-            for (int k = 0; k < 2; k++) {
-                if (!ok[k]) continue;
-                const R d0 = max0[k] - min1[k], d1 = max1[k] - min0[k];
-                const R d = d0 < d1 ? d0 : d1;
-                if (d < bd || (d == bd && fi[k] < bf)) {
-                    bd = d; bf = fi[k]; bside = d0 < d1;
-                    bia = d0 < d1 ? a1[k] : a0[k]; bib = d0 < d1 ? b0[k] : b1[k];
-                }
+    bool sepd = false;
+    R hold_f = 0;   // the least depth of the first kSatFree axes
+    // (one loop holds one copy of the bound and one of the round: the warps of an SM are at different
+    // places of this kernel, and fetching instructions was what they waited for most)
+    for (int f0 = warp * 32, end = nfree, held = 0;;) {
+        while (f0 < end && cnt <= 32) {
+            const int f = f0 + lane;
+            const V3<R> n = face_axis(f < end ? f : 0);
+            const R ny = TA == ST_CYLINDER || TA < 0 ? fast_sqrt(fma3(n, n)) : R(1);
+            bool keep = f < end && !pruned(bound(n, ny), ny, pb);
+            if (G == 1 && has_hull && held && __any_sync(full, keep)) keep = keep && !balls_above(c, n, R(1), hold_f);
+            push(keep, f);
+            f0 += T;
+        }
+        if (cnt == 0) {
+            if (end == fa + fb) break;
+            if (__any_sync(full, sepd)) return;   // G == 1
+            hold_f = bd;
+            warp_min(hold_f);
+            held = balls;
+            f0 = nfree;
+            end = fa + fb;
+            continue;
+        }
+        int f;
+        if (pop(f)) {
+            project(face_axis(f));
+            const R d0 = max0 - min1, d1 = max1 - min0;
+            const R d = d0 < d1 ? d0 : d1;
+            if (max0 < min1 || max1 < min0) sepd = true;
+            else if (d < bd || (d == bd && f < bf)) {
+                bd = d; bf = f; bside = d0 < d1;
+                bia = d0 < d1 ? a1 : a0; bib = d0 < d1 ? b0 : b1;
             }
         }
-        sat_queue_done<G>();
-        pass += span;
+        R m = bd;
+        warp_min(m);
+        pb = pb < m ? pb : m;
     }
+    if (group_any<G>(sepd)) return;
     R dmin = bd;
     int wf = bf;
     group_argmin<R, G>(dmin, wf, tid, rd, ri);
@@ -446,12 +481,11 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
     if (wf < 0x7fffffff) {
         const bool mine = bf == wf;
         if (mine) {
-            V3<R> n = wf < fa ? ld3(st.nA, wf) : ld3(st.nB, wf - fa);
-            if (dot(dc, n) < 0) n = n * R(-1.0);
+            const V3<R> n = face_axis(wf);
             sep = n;
             // testSepAxis witnesses: d0 < d1 -> (max of A, min of B), else (min of A, max of B)
-            if (!on_a) dpt = shape_witness(c.sb, c.tb(), n, !bside, bib, st.vB);
-            else dpt = shape_witness(c.sa, c.ta(), n, bside, bia, st.vA) + n * bd;
+            if (!on_a) dpt = shape_witness(c.sb, c.tb(), n, !bside, bib, vB);
+            else dpt = shape_witness(c.sa, c.ta(), n, bside, bia, vA) + n * bd;
         }
         sep = group_bcast3<R, G>(sep, mine, bc);
         dpt = group_bcast3<R, G>(dpt, mine, bc);
@@ -463,89 +497,175 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
             out[SO_FD] = -dmin + margin * 2;
         }
     }
+
     // ---- edge-pair axes (:323-361).  A box's 12 edges come in 3 classes of 4 whose direction
     // vectors are bit-identical (scaled unit-mesh differences), so they give identical axes,
     // projections and witnesses: each class is projected once, and a candidate takes the first
     // edge pair of the class (in the reference's e0-major order) whose lines hold the witnesses.
-    // Candidates compare by (depth, reference axis index), which is the reference's first strict
-    // minimum whatever order the axes are visited in.
-    R ed = dmin;
-    int ep = 0x7fffffff;
-    V3<R> ewa, ewb, en;
-    const bool boxA = c.sa.type == ST_BOX, boxB = c.sb.type == ST_BOX;
     const int ua = boxA ? 3 : na, ub = boxB ? 3 : nb;
-    const bool cyl = c.sa.type == ST_CYLINDER || c.sb.type == ST_CYLINDER;
-    const int ne = ua * ub;
-    auto edge_axis = [&](int q, V3<R>& a) {   // false for parallel edges
-        const int iu = q / ub, ju = q - iu * ub;
-        const V3<R> x = cross(ld3(st.dA, boxA ? 4 * iu : iu), ld3(st.dB, boxB ? 4 * ju : ju));
-        if (rabs(norm(x) - 0) < eps<R>()) return false;
+    // unit edge directions: a hull's come precomputed (k_hull_edge_dirs, the same arithmetic)
+    auto edge_dir = [](const ShapeView<R>& sh, const Xf<R>& t, int u) {
+        V3<R> d;
+        if (sh.type == ST_HULL) d = sh.edge_dir(u);
+        else {
+            V3<R> p0, p1;
+            sh.edge(sh.type == ST_BOX ? 4 * u : u, p0, p1);
+            d = normalized(p0 - p1);
+        }
+        return mv(t.b, d);
+    };
+    pb = pb < dmin ? pb : dmin;
+    group_sync<G>();   // the last reads of the face axes
+    // Both edge lists, without the edges whose every axis is skipped: an axis is perpendicular to its
+    // edges, so its component along the centres' line is at most that of the line's part across the
+    // edge, and the inner balls give the rest of the bound.  (The cross product of nearly parallel edges
+    // is perpendicular to them only up to a few roundoffs over its length, at least 1e-5: `lean`.)
+    const R lean = sizeof(R) == 4 ? R(0.03) : R(1e-9);
+    const R gap = able && pb < deep ? qa.inner + qb.inner - pb - slack * R(2) : R(-1);
+    auto list_edges = [&](const ShapeView<R>& s, const Xf<R>& t, int u, R* list) {   // one warp; returns the length
+        int n = 0;
+        for (int e0 = 0; e0 < u; e0 += 32) {
+            const int e = e0 + lane;
+            const V3<R> d = edge_dir(s, t, e < u ? e : 0);
+            const R k = fma3(d, dc);
+            const V3<R> w(fma(-k, d.x, dc.x), fma(-k, d.y, dc.y), fma(-k, d.z, dc.z));
+            const R g = gap - lean * rabs(k);
+            const bool keep = e < u && !(g > 0 && fma3(w, w) < g * g);
+            const unsigned m = __ballot_sync(full, keep);
+            if (keep) {
+                R* p = list + 4 * (n + __popc(m & lt));
+                p[0] = d.x; p[1] = d.y; p[2] = d.z;
+                reinterpret_cast<int*>(p + 3)[0] = e;
+            }
+            n += __popc(m);
+        }
+        return n;
+    };
+    int la = 0, lb = 0;
+    if (G == 1) {
+        la = list_edges(c.sa, c.ta(), ua, ea);
+        lb = list_edges(c.sb, c.tb(), ub, eb);
+        __syncwarp();
+    } else {
+        if (warp == 0) la = list_edges(c.sa, c.ta(), ua, ea);
+        if (warp == 1) lb = list_edges(c.sb, c.tb(), ub, eb);
+        __syncthreads();
+        if (tid == 0) ri[0] = la;
+        if (tid == 32) ri[1] = lb;
+        __syncthreads();
+        la = ri[0]; lb = ri[1];
+        if (tid == 0) bc[3] = pb;
+        __syncthreads();
+    }
+    // a queued candidate: its places in the lists; the axis index: edge of A major
+    auto list_edge = [](const R* list, int k) { return reinterpret_cast<const int*>(list + 4 * k + 3)[0]; };
+    auto edge_axis = [&](int v, V3<R>& x, R& nx, V3<R>& a) {   // false for parallel edges
+        x = cross(ldv(ea, v & 0xffff), ldv(eb, v >> 16));
+        nx = norm(x);
+        if (rabs(nx - 0) < eps<R>()) return false;
         a = normalized(x);
         if (dot(dc, a) < 0) a = a * R(-1.0);
         return true;
     };
-    for (int pass = 0; pass < ne; pass += kSatQ * T) {
-      R pb = ed;
-      warp_min(pb);
-      const int cnt = sat_queue<G>(pass, kSatQ * T, ne, tid, queue, qn, [&](int q) {
-          if (cyl) {
-              V3<R> a;
-              return edge_axis(q, a) && !sat_prunable(c, able, a, pb);
-          }
-          const int iu = q / ub, ju = q - iu * ub;
-          const V3<R> x = cross(ld3(st.dA, boxA ? 4 * iu : iu), ld3(st.dB, boxB ? 4 * ju : ju));
-          const R nx = norm(x);
-          return !(rabs(nx - 0) < eps<R>()) && !sat_prunable_scaled(c, able, x, nx, pb);   // parallel edges: no axis
-      });
-      for (int qb = 0; qb < cnt; qb += 2 * T) {
-        V3<R> cr[2];
-        bool ok[2];
-        int qa[2];
-        for (int k = 0; k < 2; k++) {
-            const int qi = qb + T * k + tid;
-            ok[k] = qi < cnt;
-            qa[k] = ok[k] ? queue[qi] : 0;
-            cr[k] = V3<R>(0, 0, 0);
-            if (ok[k]) edge_axis(qa[k], cr[k]);
-        }
-        R min0[2], max0[2], min1[2], max1[2];
-        int a0[2], a1[2], b0[2], b1[2];
-        R best = ed;
-        warp_min(best);
-        pair_intervals2(c, cr, ok, best, st.vA, st.vB, min0, max0, min1, max1, a0, a1, b0, b1);
-        bool sp = false;
-        for (int k = 0; k < 2; k++) sp |= ok[k] && (max0[k] < min1[k] || max1[k] < min0[k]);
-        if (group_any<G>(sp)) return;
-        for (int k = 0; k < 2; k++) {
-            if (!ok[k]) continue;
-            const R d0 = max0[k] - min1[k], d1 = max1[k] - min0[k];
-            const R dist = d0 < d1 ? d0 : d1;
-            if (!(dist < ed || (dist == ed && ep != 0x7fffffff))) continue;
-            const int q = qa[k];
-            const int iu = q / ub, ju = q - iu * ub;
-            const bool side = d0 < d1;
-            const V3<R> wa = shape_witness(c.sa, c.ta(), cr[k], side, side ? a1[k] : a0[k], st.vA);
-            const V3<R> wb = shape_witness(c.sb, c.tb(), cr[k], !side, side ? b0[k] : b1[k], st.vB);
-            const V3<R> la = c.ta().inv_apply(wa), lb = c.tb().inv_apply(wb);
-            int qref = 0x7fffffff;
-            for (int m0 = 0; m0 < (boxA ? 4 : 1) && qref == 0x7fffffff; m0++) {
-                const int e0 = boxA ? 4 * iu + m0 : iu;
-                V3<R> p0, p1;
-                c.sa.edge(e0, p0, p1);
-                if (!on_line(p0, p1, la)) continue;
-                for (int m1 = 0; m1 < (boxB ? 4 : 1); m1++) {
-                    const int e1 = boxB ? 4 * ju + m1 : ju;
-                    V3<R> q0, q1;
-                    c.sb.edge(e1, q0, q1);
-                    if (on_line(q0, q1, lb)) { qref = e0 * nb + e1; break; }
+    R ed = dmin;
+    int ep = 0x7fffffff;
+    V3<R> ewa, ewb, en;
+    R seen = dmin;           // this warp's least depth so far
+    R hold = dmin;           // the balls' measure of the block being resolved,
+    int block = 0;           // and which one that is
+    R measure = dmin;        // the balls' measure for the candidates: `hold` or a larger one of an earlier block
+    // candidates in the order of their index: B's list inside A's
+    const int nc = la * lb, di = lb > 0 ? T / lb : 0, dj = T - di * lb;
+    int i = lb > 0 ? tid / lb : 0, j = tid - i * lb;
+    for (int k0 = warp * 32;;) {
+        while (k0 < nc && cnt <= 32) {
+            const bool in = k0 + lane < nc;
+            const int ci = in ? i : la - 1, cj = in ? j : lb - 1;
+            const V3<R> d0 = ldv(ea, ci), d1 = ldv(eb, cj);
+            V3<R> x = cross(d0, d1);
+            const R n2 = fma3(x, x), g = fma3(x, dc);
+            bool keep = in;
+            if (able) {
+                if (G == 1 && has_hull && (list_edge(ea, __shfl_sync(full, ci, 0)) * ub + list_edge(eb, __shfl_sync(full, cj, 0))) / kSatBlock > block)
+                    measure = seen;
+                constexpr bool hulls = TA == ST_HULL && TB == ST_HULL;
+                if (hulls) {   // the balls without a square root
+                    const R t = qa.inner + qb.inner - measure - slack;
+                    keep = keep && !(t > 0 && n2 * t * t > g * g);
+                }
+                if (!hulls || __any_sync(full, keep)) {
+                    const R ny = fast_sqrt(n2);
+                    if (!hulls && has_hull && balls) keep = keep && !(ball(x, ny) > ny * (measure + slack));
+                    x = x * (g < 0 ? R(-1) : R(1));
+                    keep = keep && !pruned(bound(x, ny), ny, pb);
                 }
             }
-            if (qref == 0x7fffffff || !(dist < ed || qref < ep)) continue;
-            ed = dist; ep = qref; ewa = wa; ewb = wb; en = cr[k];
+            push(keep, ci | cj << 16);
+            k0 += T;
+            i += di;
+            j += dj;
+            if (j >= lb) { j -= lb; i++; }
         }
-      }
-      sat_queue_done<G>();
+        if (cnt == 0) break;
+        // a round: the exact projections of up to 32 queued axes
+        int v;
+        bool ok = pop(v);
+        const int iu = list_edge(ea, v & 0xffff), ju = list_edge(eb, v >> 16), q = iu * ub + ju;
+        V3<R> cr(0, 0, 0), x, wa, wb;
+        R dist = 0, nx = 0;
+        bool split = false;
+        int qref = 0x7fffffff;
+        if (ok) ok = edge_axis(v, x, nx, cr);
+        if (ok) {
+            project(cr);
+            split = max0 < min1 || max1 < min0;
+            const R d0 = max0 - min1, d1 = max1 - min0;
+            dist = d0 < d1 ? d0 : d1;
+            if (!split && (dist < ed || (dist == ed && ep != 0x7fffffff))) {
+                const bool s = d0 < d1;
+                wa = shape_witness(c.sa, c.ta(), cr, s, s ? a1 : a0, vA);
+                wb = shape_witness(c.sb, c.tb(), cr, !s, s ? b0 : b1, vB);
+                const V3<R> la = c.ta().inv_apply(wa), lb = c.tb().inv_apply(wb);
+#pragma unroll 1
+                for (int m0 = 0; m0 < (boxA ? 4 : 1) && qref == 0x7fffffff; m0++) {
+                    const int e0 = boxA ? 4 * iu + m0 : iu;
+                    V3<R> p0, p1;
+                    c.sa.edge(e0, p0, p1);
+                    if (!on_line(p0, p1, la)) continue;
+#pragma unroll 1
+                    for (int m1 = 0; m1 < (boxB ? 4 : 1); m1++) {
+                        const int e1 = boxB ? 4 * ju + m1 : ju;
+                        V3<R> q0, q1;
+                        c.sb.edge(e1, q0, q1);
+                        if (on_line(q0, q1, lb)) { qref = e0 * nb + e1; break; }
+                    }
+                }
+            }
+        }
+        // block by block (queued axes are in order), each against the depth known when it began
+        const int mine = q / kSatBlock;
+        for (unsigned todo = __ballot_sync(full, ok); todo;) {
+            const int b = __shfl_sync(full, mine, __ffs(todo) - 1);
+            if (G == 1 && has_hull && b != block) { block = b; hold = seen; }
+            const unsigned now = todo & __ballot_sync(full, mine == b);
+            todo &= ~now;
+            if (ok && mine == b && !(has_hull && balls && balls_above(c, x, nx, hold))) {
+                if (split) sepd = true;
+                else if (qref != 0x7fffffff && (dist < ed || qref < ep)) { ed = dist; ep = qref; ewa = wa; ewb = wb; en = cr; }
+            }
+            seen = ed;
+            warp_min(seen);
+        }
+        pb = pb < seen ? pb : seen;
+        if (G > 1) {   // the warps' bounds together
+            volatile R* shared = bc + 3;
+            const R o = *shared;
+            if (o < pb) pb = o;
+            else if (lane == 0 && pb < o) *shared = pb;   // any warp's bound will do
+        }
+        if (G == 1 && __any_sync(full, sepd)) return;
     }
+    if (group_any<G>(sepd)) return;
     R emin = ed;
     int wq = ep;
     group_argmin<R, G>(emin, wq, tid, rd, ri);
@@ -555,7 +675,7 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
         sep = group_bcast3<R, G>(en, mine, bc);
         if (tid == 0) {   // segmentsClosestPoints with unbounded half-lengths (:172-214, :363-395)
             const int e0 = wq / nb, e1 = wq - e0 * nb;
-            const V3<R> wea = ld3(st.dA, e0), web = ld3(st.dB, e1);
+            const V3<R> wea = edge_dir(c.sa, c.ta(), boxA ? e0 / 4 : e0), web = edge_dir(c.sb, c.tb(), boxB ? e1 / 4 : e1);
             const V3<R> tr = wpb - wpa;
             const R ab = dot(wea, web), at = dot(wea, tr), bt = dot(web, tr);
             const R d = R(1.0) - ab * ab;
@@ -585,14 +705,14 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
     R dmax = Lim<R>::min();
     int fbest = 0x7fffffff;
     for (int f = tid; f < fb; f += T) {
-        const R d = dot(ld3(st.nB, f), sep);
+        const R d = dot(mv(c.tb().b, c.sb.face_normal(f)), sep);
         if (d > dmax) { dmax = d; fbest = f; }
     }
     group_argmax<R, G>(dmax, fbest, tid, rd, ri);
     R dmn = Lim<R>::max();
     int fabest = 0x7fffffff;
     for (int f = tid; f < fa; f += T) {
-        const R d = dot(ld3(st.nA, f), sep);
+        const R d = dot(mv(c.ta().b, c.sa.face_normal(f)), sep);
         if (d < dmn) { dmn = d; fabest = f; }
     }
     group_argmin<R, G>(dmn, fabest, tid, rd, ri);
@@ -714,11 +834,8 @@ __device__ bool sat_warp(Pair<R>& c, int lane) {
 // SAT pairs: G = 1 runs kSatWarps pairs per block, one warp each, instantiated per shape pairing
 // (TA, TB; one launch per pairing); G = kSatGroup runs one heavy pair per block, any pairing (-1).
 // Only thread 0 holds the pair's contact cache.
-// per-group stride, a multiple of 4 reals so that every group's vertex rows stay 16-byte aligned
-template <class R> constexpr int sat_group_reals(int G) {
-    return (sat_stage_reals<R>() + sat_scratch_reals<R>(G) + sat_queue_reals<R>(G) + 3) & ~3;
-}
-static_assert(sat_group_reals<float>(1) % 4 == 0 && (3 * (2 * kSatF + 2 * kSatE)) % 4 == 0, "SAT staging alignment");
+static_assert(2 * kSatF <= 2 * kSatE, "the face axes fit the edge lists' room");
+static_assert(sat_group_reals<float>(1) % 4 == 0 && kSatBase % 4 == 0, "SAT staging alignment");
 template <class R, int G, int TA, int TB>
 __global__ void __launch_bounds__(G == 1 ? 32 * kSatWarps : 32 * G, G == 1 ? kSatBlocksPerSm : 2)
 k_np_sat(const int2* rng, int* cursor, const int* order, const int2* pairs, Bodies<R> B, ShapeTable<R> S, R* sat_out) {
