@@ -115,6 +115,47 @@ __global__ void k_bp_gather(Bodies<R> B, const uint32_t* order, R* smn, R* smx, 
 // Pass 0 counts the pairs of each position and keeps its first kStage partners; pass 1 writes the
 // pairs at the scanned offsets, copying staged partners and re-sweeping only crowded positions.
 constexpr int kStage = 4;
+// U chunks of 32 candidates from j0 on, tested in order after all their loads are under way; false
+// once a chunk is not full.  (c is the position's pairs so far.)
+template <class R, bool WRITE, int U>
+__device__ __forceinline__ bool sweep_chunks(int i, int j0, int n, int lane, int sc, const R* amin, R maxi_ax, const V3<R>& mn, const V3<R>& mx,
+                                             int fi, const R* smn, const R* smx, const int* sflag, const int* sscene, int* stage, int2* out,
+                                             int a, const uint32_t* order, const IgnoreLists& ign, int& c) {
+    R am[U];
+    V3<R> lo[U], hi[U];
+    int fl[U], scn[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int j = min(j0 + 32 * u + lane, n - 1);   // past the end: the last one, not `in` below
+        am[u] = amin[j];
+        scn[u] = sscene[j];
+        fl[u] = sflag[j];
+        lo[u] = V3<R>(smn[j], smn[n + j], smn[2 * (size_t)n + j]);
+        hi[u] = V3<R>(smx[j], smx[n + j], smx[2 * (size_t)n + j]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int j = j0 + 32 * u + lane;
+        const bool in = j < n && !(am[u] > maxi_ax) && scn[u] == sc;
+        const unsigned live = __ballot_sync(0xffffffffu, in);
+        bool hit = in && !(fl[u] & BF_IGNORE) && !((fi & BF_KINEMATIC) && (fl[u] & BF_KINEMATIC)) &&
+                   !(mn.x > hi[u].x || lo[u].x > mx.x) && !(mn.y > hi[u].y || lo[u].y > mx.y) && !(mn.z > hi[u].z || lo[u].z > mx.z);
+        if (hit && ign.off && ((fi | fl[u]) & BF_IGN_LIST)) hit = !ign.ignored(i, j);
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) {
+            const int k = c + __popc(m & ((1u << lane) - 1u));
+            if (WRITE) out[k] = make_int2(a, (int)order[j]);
+            else if (k < kStage) stage[(size_t)i * kStage + k] = j;
+        }
+        c += __popc(m);
+        if (live != 0xffffffffu) return false;
+    }
+    return true;
+}
+// The sweep of one position by a warp.  A window is a chain of chunks, each some 3 us of dependent
+// loads and votes when taken alone: the floor of a 1,600-body scene, 50 chunks, held the count for
+// 81 us and the write for 169 us.  Most windows end in the first two chunks; longer ones go four
+// chunks at a time, loads first.
 template <class R, bool WRITE>
 __device__ __forceinline__ int sweep_warp(int i, int n, int lane, const int* scene_axis, const R* smn, const R* smx,
                                           const int* sflag, const int* sscene, int* stage, int2* out, const uint32_t* order,
@@ -123,93 +164,37 @@ __device__ __forceinline__ int sweep_warp(int i, int n, int lane, const int* sce
     const int ax = scene_axis[sc];
     const R* amin = smn + (size_t)ax * n;
     const R maxi_ax = smx[(size_t)ax * n + i];
-    const R mnx = smn[i], mny = smn[n + i], mnz = smn[2 * (size_t)n + i];
-    const R mxx = smx[i], mxy = smx[n + i], mxz = smx[2 * (size_t)n + i];
+    const V3<R> mn(smn[i], smn[n + i], smn[2 * (size_t)n + i]), mx(smx[i], smx[n + i], smx[2 * (size_t)n + i]);
     const int fi = sflag[i];
     if (fi & BF_IGNORE) return 0;
     const int a = WRITE ? (int)order[i] : 0;
-    const unsigned lt = (1u << lane) - 1u;
-    int c = 0;
-    for (int j0 = i + 1; j0 < n; j0 += 32) {
-        const int j = j0 + lane;
-        const bool in = j < n && !(amin[j] > maxi_ax) && sscene[j] == sc;
-        const unsigned live = __ballot_sync(0xffffffffu, in);
-        bool hit = false;
-        if (in) {
-            const int fj = sflag[j];
-            hit = !(fj & BF_IGNORE) && !((fi & BF_KINEMATIC) && (fj & BF_KINEMATIC)) &&
-                  !(mnx > smx[j] || smn[j] > mxx) && !(mny > smx[n + j] || smn[n + j] > mxy) &&
-                  !(mnz > smx[2 * (size_t)n + j] || smn[2 * (size_t)n + j] > mxz);
-            if (hit && ign.off && ((fi | fj) & BF_IGN_LIST)) hit = !ign.ignored(i, j);
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (hit) {
-            const int k = c + __popc(m & lt);
-            if (WRITE) out[k] = make_int2(a, (int)order[j]);
-            else if (k < kStage) stage[(size_t)i * kStage + k] = j;
-        }
-        c += __popc(m);
-        if (live != 0xffffffffu) break;
-    }
+    int c = 0, j0 = i + 1;
+    for (int k = 0; k < 2; k++, j0 += 32)
+        if (j0 >= n || !sweep_chunks<R, WRITE, 1>(i, j0, n, lane, sc, amin, maxi_ax, mn, mx, fi, smn, smx, sflag, sscene, stage, out, a, order, ign, c))
+            return c;
+    for (; j0 < n; j0 += 128)
+        if (!sweep_chunks<R, WRITE, 4>(i, j0, n, lane, sc, amin, maxi_ax, mn, mx, fi, smn, smx, sflag, sscene, stage, out, a, order, ign, c)) break;
     return c;
 }
 
 // A position whose window along the axis holds more than kBigWindow candidates (a floor or a wall
-// spanning the scene) is swept by a whole block instead of a warp: 256 candidates per iteration,
-// warp ballots plus a block prefix of the warp counts keep the pairs in ascending j.
-constexpr int kBigWindow = 32768;
+// spanning the scene) is swept by blocks instead of a warp: 256 candidates per iteration, warp
+// ballots plus a block prefix of the warp counts keep the pairs in ascending j.
+constexpr int kBigWindow = 4096;        // about 32 steps of four chunks for a warp
+constexpr int kNoBigWindow = 1 << 30;   // limit of a caller without the chunk kernels
 template <class R>
-__device__ __forceinline__ bool big_window(int i, int n, const int* scene_axis, const R* smn, const R* smx, const int* sscene) {
-    const int j = i + kBigWindow;
-    if (j >= n) return false;
+__device__ __forceinline__ bool big_window(int i, int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sscene) {
+    if (limit >= n - i) return false;
+    const int j = i + limit;
     const int sc = sscene[i], ax = scene_axis[sc];
     return sscene[j] == sc && !(smn[(size_t)ax * n + j] > smx[(size_t)ax * n + i]);
 }
-template <class R, bool WRITE>
-__device__ int sweep_block(int i, int n, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
-                           int2* out, const uint32_t* order, int* wcnt, const IgnoreLists& ign) {
-    const int sc = sscene[i];
-    const int ax = scene_axis[sc];
-    const R* amin = smn + (size_t)ax * n;
-    const R maxi_ax = smx[(size_t)ax * n + i];
-    const R mnx = smn[i], mny = smn[n + i], mnz = smn[2 * (size_t)n + i];
-    const R mxx = smx[i], mxy = smx[n + i], mxz = smx[2 * (size_t)n + i];
-    const int fi = sflag[i];
-    if (fi & BF_IGNORE) return 0;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-    const int a = WRITE ? (int)order[i] : 0;
-    const unsigned lt = (1u << lane) - 1u;
-    int c = 0;
-    for (int j0 = i + 1; j0 < n; j0 += blockDim.x) {
-        const int j = j0 + tid;
-        const bool in = j < n && !(amin[j] > maxi_ax) && sscene[j] == sc;
-        bool hit = false;
-        if (in) {
-            const int fj = sflag[j];
-            hit = !(fj & BF_IGNORE) && !((fi & BF_KINEMATIC) && (fj & BF_KINEMATIC)) &&
-                  !(mnx > smx[j] || smn[j] > mxx) && !(mny > smx[n + j] || smn[n + j] > mxy) &&
-                  !(mnz > smx[2 * (size_t)n + j] || smn[2 * (size_t)n + j] > mxz);
-            if (hit && ign.off && ((fi | fj) & BF_IGN_LIST)) hit = !ign.ignored(i, j);
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) wcnt[w] = __popc(m);
-        const int all_in = __syncthreads_and(in);
-        int before = 0, total = 0;
-        for (int k = 0; k < nw; k++) { if (k < w) before += wcnt[k]; total += wcnt[k]; }
-        if (WRITE && hit) out[c + before + __popc(m & lt)] = make_int2(a, (int)order[j]);
-        c += total;
-        __syncthreads();   // wcnt is rewritten next iteration
-        if (!all_in) break;
-    }
-    return c;
-}
-
 // A crowded position's window (the candidates j > i of its scene whose minimum along the axis does
 // not exceed i's maximum: a prefix of the scene's sorted positions, found by binary search) swept in
 // up to kMaxChunks chunks of at least kChunk candidates, one block per chunk: chunk counts are summed
 // per position, and each chunk writes its pairs after those of the chunks before it, so the pairs
 // keep ascending j.
-constexpr int kChunk = 4096;
+constexpr int kChunk = 1024;
 constexpr int kMaxChunks = 32;
 template <class R, bool WRITE>
 __device__ int sweep_range_block(int i, int jb, int je, int n, const R* smn, const R* smx, const int* sflag, int2* out,
@@ -306,57 +291,27 @@ __global__ void k_bp_write_chunks(int n, const R* smn, const R* smx, const int* 
 }
 
 template <class R>
-__global__ void k_bp_count(int n, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene, int* count,
+__global__ void k_bp_count(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene, int* count,
                            int* stage, int* big, int* n_big, IgnoreLists ign) {
     const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= n) return;
-    if (big_window(i, n, scene_axis, smn, smx, sscene)) {   // left to k_bp_count_big
+    if (big_window(i, n, limit, scene_axis, smn, smx, sscene)) {   // left to k_bp_count_chunks
         if (lane == 0) big[atomicAdd(n_big, 1)] = i;
         return;
     }
     const int c = sweep_warp<R, false>(i, n, lane, scene_axis, smn, smx, sflag, sscene, stage, nullptr, nullptr, ign);
     if (lane == 0) count[i] = c;
 }
-// one block per listed position (blocks loop over the list)
 template <class R>
-__global__ void k_bp_count_big(int n, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
-                               int* count, const int* big, const int* n_big, IgnoreLists ign) {
-    __shared__ int wcnt[32];
-    for (int b = blockIdx.x; b < *n_big; b += gridDim.x) {
-        const int i = big[b];
-        const int c = sweep_block<R, false>(i, n, scene_axis, smn, smx, sflag, sscene, nullptr, nullptr, wcnt, ign);
-        if (threadIdx.x == 0) count[i] = c;
-        __syncthreads();
-    }
-}
-template <class R>
-__global__ void k_bp_write_big(int n, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
-                               const uint32_t* order, const int* offset, int2* pairs, int pair_cap, int* status, const int* big,
-                               const int* n_big, IgnoreLists ign) {
-    __shared__ int wcnt[32];
-    for (int b = blockIdx.x; b < *n_big; b += gridDim.x) {
-        const int i = big[b];
-        const int base = offset[i], c = offset[i + 1] - base;
-        if (c == 0) continue;   // uniform in the block
-        if (base + c > pair_cap) {
-            if (threadIdx.x == 0) atomicOr(status, ST_PAIR_OVERFLOW);
-            continue;
-        }
-        sweep_block<R, true>(i, n, scene_axis, smn, smx, sflag, sscene, pairs + base, order, wcnt, ign);
-        __syncthreads();
-    }
-}
-
-template <class R>
-__global__ void k_bp_write(int n, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
+__global__ void k_bp_write(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
                            const uint32_t* order, const int* offset, const int* stage, int2* pairs, int pair_cap, int* status,
                            IgnoreLists ign) {
     const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= n) return;
     const int base = offset[i], c = offset[i + 1] - base;
-    if (c == 0 || big_window(i, n, scene_axis, smn, smx, sscene)) return;   // big windows: k_bp_write_big
+    if (c == 0 || big_window(i, n, limit, scene_axis, smn, smx, sscene)) return;   // big windows: k_bp_write_chunks
     if (base + c > pair_cap) {
         if (lane == 0) atomicOr(status, ST_PAIR_OVERFLOW);
         return;

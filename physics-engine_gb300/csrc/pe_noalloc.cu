@@ -22,7 +22,6 @@ namespace {
 constexpr int kSapMaxBodies = 16384;
 // no window of a scene this small can exceed the world's crowded-window threshold, so the warp
 // sweep alone gives the world's pairs (the block sweeps of crowded windows never have work here)
-static_assert(kSapMaxBodies <= kBigWindow, "crowded-window sweeps would be needed");
 constexpr size_t kAlign = 256;
 constexpr size_t al(size_t b) { return (b + kAlign - 1) / kAlign * kAlign; }
 constexpr int kSapTiles = (kSapMaxBodies + kRadixTile - 1) / kRadixTile;
@@ -219,12 +218,12 @@ extern "C" int pe_gpu_sap_pairs_noalloc(int device, int n, const float* aabb_min
     k_sap_gather<<<g, kBlock, 0, st>>>(n, aabb_min, aabb_max, flags, order, smn, smx, sflag, sscene, count, status, n_big);
     const int gw = (int)(((size_t)n * 32 + kBlock - 1) / kBlock);
     const IgnoreLists no_lists;   // this entry point takes no ignored-pair lists
-    k_bp_count<float><<<gw, kBlock, 0, st>>>(n, scene_axis, smn, smx, sflag, sscene, count, stage, big, n_big, no_lists);
+    k_bp_count<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, count, stage, big, n_big, no_lists);
     const int ct = (n + 1 + 1023) / 1024;
     k_scan_tiles<<<ct, kBlock, 0, st>>>(count, n + 1, aux);
     k_scan_aux<<<1, kBlock, 0, st>>>(aux, ct, total);
     k_scan_add<<<ct, kBlock, 0, st>>>(count, n + 1, aux);
-    k_bp_write<float><<<gw, kBlock, 0, st>>>(n, scene_axis, smn, smx, sflag, sscene, order, count, stage, reinterpret_cast<int2*>(pairs),
+    k_bp_write<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, order, count, stage, reinterpret_cast<int2*>(pairs),
                                              pair_cap, status, no_lists);
     k_sap_total<<<1, 1, 0, st>>>(total, n_pairs);
     const cudaError_t e = cudaGetLastError();

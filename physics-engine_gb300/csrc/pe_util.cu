@@ -294,12 +294,16 @@ __global__ void k_step_counters(const int* status, const int* rows, const int* a
     for (int c = 0; c < PC_COUNT; c++) out[7 + c] = cls[c];
 }
 
-// exclusive offsets of the crowded positions' chunks (few positions: one thread)
+// exclusive offsets of the crowded positions' chunks (one warp)
 __global__ void k_bp_chunk_offsets(const int* n_big, const int* nchunk, int* choff, int* total) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    const int lane = threadIdx.x & 31, nb = *n_big;
     int run = 0;
-    for (int b = 0; b < *n_big; b++) { choff[b] = run; run += nchunk[b]; }
-    *total = run;
+    for (int b0 = 0; b0 < nb; b0 += 32) {
+        const int b = b0 + lane, v = b < nb ? nchunk[b] : 0, incl = warp_incl_scan(v);
+        if (b < nb) choff[b] = run + incl - v;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) *total = run;
 }
 __global__ void k_bp_chunk_sums(const int* big, const int* n_big, const int* choff, const int* nchunk, const int* ccount, int* cpref,
                                 int* count) {

@@ -215,6 +215,8 @@ private:
     cudaStream_t side_[kSideStreams] = {};
     cudaEvent_t fork_ev_ = nullptr, join_ev_[kSideStreams] = {};
     cudaStream_t cur_ = nullptr;
+    cudaStream_t axis_st_ = nullptr;   // the sweep axes' stream
+    cudaEvent_t axis_ev_[2] = {};
     void fork_streams() {
         PE_CK(cudaEventRecord(fork_ev_, st_));
         for (int k = 0; k < kSideStreams; k++) PE_CK(cudaStreamWaitEvent(side_[k], fork_ev_, 0));
@@ -315,7 +317,10 @@ private:
     void bp_count_enqueue();        // its launches, ending with the count's copy to the host
     void run_head();                // integrate and bp_count_enqueue, replayed from a CUDA graph when enabled
     void prepare_tail(int P);       // every capacity the rest of the step needs, before any launch of it
-    void bp_tail();                 // pair list, scene pair offsets, sweep axes
+    void bp_tail();                 // pair list, scene pair offsets
+    void bp_axis();                 // the scenes' next sweep axes,
+    void bp_axis_begin();           // started on their own stream (after bp_tail)
+    void bp_axis_end();             // and waited for by the world's
     void np_enqueue();              // narrowphase, no host waits
     void solve_enqueue(int mode);   // solver up to the velocity sync and the counters' copy, no host waits
     void finish();                  // waits for the counters; status

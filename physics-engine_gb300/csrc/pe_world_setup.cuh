@@ -14,6 +14,8 @@ template <class R> World<R>::World(int device) : dev_(device) {
         PE_CK(cudaEventCreateWithFlags(&join_ev_[k], cudaEventDisableTiming));
     }
     PE_CK(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
+    PE_CK(cudaStreamCreateWithFlags(&axis_st_, cudaStreamNonBlocking));
+    for (auto& e : axis_ev_) PE_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& e : ev_) { PE_CK(cudaEventCreate(&e[0])); PE_CK(cudaEventCreate(&e[1])); }
     UnitMeshes u;
     std::memset(&u, 0, sizeof(u));
@@ -49,6 +51,8 @@ template <class R> World<R>::~World() {
         if (join_ev_[k]) cudaEventDestroy(join_ev_[k]);
     }
     if (fork_ev_) cudaEventDestroy(fork_ev_);
+    if (axis_st_) { cudaStreamSynchronize(axis_st_); cudaStreamDestroy(axis_st_); }
+    for (auto e : axis_ev_) if (e) cudaEventDestroy(e);
     if (st_) cudaStreamDestroy(st_);
 }
 

@@ -1,0 +1,67 @@
+"""Pair lists of the sweep against the oracle where its windows change hands: ends at
+every edge of a warp's first chunks of 32 and of its groups of four, windows past the length that
+blocks sweep in chunks, several scenes in one world (a window ends with its scene), and the sweep axis
+that the next step takes, computed beside the rest of the step."""
+import numpy as np
+import pytest
+
+import orc
+import pe_gb300 as pg
+from pe_gb300 import scene as sc
+
+pytestmark = pytest.mark.gpu
+
+
+def _line(n, lengths, bits, seed, dense=False):
+    """Unit boxes one apart along x, and for each length a kinematic slab that starts just left of a
+    box and spans that many of them."""
+    r = np.random.default_rng(seed)
+    sb = sc.SceneBuilder(dt=1.0 / 60.0, iterations=2, gravity=(0.0, 0.0, 0.0))
+    box = sb.shape(sc.BOX, (0.9, 0.9, 0.9))
+    for i in range(n):
+        z = 0.0 if dense else float(r.uniform(-3, 3))   # not every box of a window overlaps its slab
+        sb.body(box, (float(i), float(r.uniform(-0.4, 0.4)), z), mass=1.0)
+    for k, m in enumerate(lengths):
+        start = int(r.integers(0, max(1, n - m)))
+        sb.body(sb.shape(sc.BOX, (float(m), 1.0, 2.0)), (start - 0.5 + m / 2 - 0.01, 0.0, 0.0), mass=0.0, kinematic=True)
+    return sb.build(bits)
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("lengths", [(1, 31, 32, 33, 63), (64, 65, 95, 96, 97, 127, 128), (191, 192, 193, 320, 321, 449)])
+def test_windows_of_a_warp(lengths, bits):
+    s = _line(460, lengths, bits, seed=len(lengths) + bits)
+    g, o = pg.GpuWorld(s, bits), orc.OracleWorld(s, bits, stable_ties=True)
+    for _ in range(3):
+        g.step(1, pg.SERIAL_ORDER)
+        o.step(1)
+        assert np.array_equal(g.pairs(), o.pairs())
+        assert g.axis == o.axis
+    g.close()
+
+
+def test_windows_of_blocks():
+    # 4,095 to 5,121 candidates: the last that one warp sweeps, the first in chunks, and a second chunk round
+    s = _line(5400, (4095, 4096, 4097, 5119, 5121), 32, seed=3)
+    g, o = pg.GpuWorld(s, 32), orc.OracleWorld(s, 32, stable_ties=True)
+    for _ in range(2):
+        g.step(1, pg.SERIAL_ORDER)
+        o.step(1)
+        assert np.array_equal(g.pairs(), o.pairs())
+        assert g.axis == o.axis
+    g.close()
+
+
+def test_windows_end_with_their_scene():
+    sizes = (40, 2, 130, 33, 1, 260)
+    parts = [_line(n, (max(1, n - 3),), 32, seed=n, dense=True) for n in sizes]
+    whole, offs = sc.concat(parts)
+    g = pg.GpuWorld(whole, 32, scenes=offs)
+    g.step(2, pg.SERIAL_ORDER)
+    want = []
+    for k, p in enumerate(parts):
+        alone = orc.OracleWorld(p, 32, stable_ties=True)
+        alone.step(2)
+        want.append(alone.pairs().reshape(-1, 2) + int(offs[k]))
+    assert np.array_equal(g.pairs().reshape(-1, 2), np.concatenate(want))
+    g.close()
