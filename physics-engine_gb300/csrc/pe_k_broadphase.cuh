@@ -1,39 +1,15 @@
-// Kernels of the rigid-body step, part 2: scan, the LSD radix sort and the sweep-and-prune broadphase.
+// Kernels of the rigid-body step, part 3: the sweep-and-prune broadphase.
 #pragma once
-#include "pe_k_integrate.cuh"
+#include "pe_k_sort.cuh"
 
 namespace pe {
 
-// ===================================================================== scan
-// exclusive scan of n ints, in place, three phases; totals of each tile in aux
-__global__ void k_scan_tiles(int* data, int n, int* aux);
-__global__ void k_scan_aux(int* aux, int m, int* total);
-__global__ void k_scan_add(int* data, int n, const int* aux);
-constexpr int kSmallScanTiles = 16;   // scans of up to 16 tiles of 1024 run in one block (k_scan_aux in place)
-
-// ===================================================================== radix sort
-// Sort (key, value) pairs by a 64-bit key and then, more significantly, by a 32-bit
-// secondary key (scene id); stable, least-significant digit first, 8-bit digits.
-constexpr int kRadixItems = 16;                      // items per thread per tile
-constexpr int kRadixTile = kBlock * kRadixItems;     // 4096 items per tile
-// The item count is n, or *nd when nd is set (a count the device computed: the grid then covers an
-// upper bound, tiles past the count do nothing, and with `small` >= 0 the passes do nothing at all
-// when the count is at most `small`, the inputs that k_sort_pairs_block sorts instead).
-__global__ void k_radix_hist(const uint64_t* key, const uint32_t* key2, int n, const int* nd, int small, int shift, int use2, int* hist,
-                             int n_tiles);
-// a sort of n <= kSceneSortMax (key, value) pairs inside one block (bitonic over (key, position)): the
-// order of the stable LSD radix sort, in one launch instead of five per pass, for small inputs.  With
-// nd set the count is *nd and the kernel does nothing when it is above kSceneSortMax; the output
-// may be the input (all reads precede all writes).
-__global__ void k_sort_pairs_block(const uint64_t* key, const uint32_t* val, int n, const int* nd, uint64_t* key_out, uint32_t* val_out);
-__global__ void k_radix_scatter(const uint64_t* key_in, const uint32_t* key2_in, const uint32_t* val_in, uint64_t* key_out,
-                                uint32_t* key2_out, uint32_t* val_out, int n, const int* nd, int small, int shift, int use2,
-                                const int* hist, int n_tiles);
-
-__device__ inline uint64_t order_bits(float x) {
+template <class R> struct KeyOf { using type = uint32_t; };
+template <> struct KeyOf<double> { using type = uint64_t; };
+__device__ inline uint32_t order_bits(float x) {
     if (x == 0.0f) x = 0.0f;   // -0 and +0 compare equal: give them one key
     const uint32_t u = __float_as_uint(x);
-    return (uint64_t)((u & 0x80000000u) ? ~u : (u | 0x80000000u));
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ inline uint64_t order_bits(double x) {
     if (x == 0.0) x = 0.0;
@@ -43,12 +19,11 @@ __device__ inline uint64_t order_bits(double x) {
 
 // sort key of each body: its AABB minimum along its scene's sweep axis
 template <class R>
-__global__ void k_bp_keys(Bodies<R> B, const int* scene_axis, uint64_t* key, uint32_t* key2, uint32_t* val) {
+__global__ void k_bp_keys(Bodies<R> B, const int* scene_axis, typename KeyOf<R>::type* key, uint32_t* val) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B.n) return;
     const int ax = scene_axis[B.scene[i]];
     key[i] = order_bits(B.at(MNX + ax, i));
-    key2[i] = (uint32_t)B.scene[i];
     val[i] = (uint32_t)i;
 }
 

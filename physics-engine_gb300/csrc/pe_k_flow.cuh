@@ -25,13 +25,13 @@ template <class R, bool JOINTS> struct Item {
     uint32_t id;
     int ia, ib, r0, np;
     Side<R> a, b;
-    __device__ __forceinline__ void load(uint32_t item, const Results<R>& res, const Joints<R>& J, const Bodies<R>& B, const int* row_off) {
+    __device__ __forceinline__ void load(uint32_t item, const Results<R>& res, const Joints<R>& J, const Bodies<R>& B) {
         id = item;
         if (JOINTS && (item & kJointItem)) {
             const int2 q = J.body[item & ~kJointItem];
             ia = q.x; ib = q.y; r0 = 0; np = 0;
         } else {
-            ia = res.a[item]; ib = res.b[item]; r0 = row_off[item]; np = res.npts[item];
+            ia = res.a[item]; ib = res.b[item]; r0 = (int)item * kSlots; np = res.npts[item];
         }
         a.load(B, ia);
         b.load(B, ib);
@@ -54,11 +54,9 @@ __host__ __device__ inline long long class_base(int c, long long bound) {
     for (int k = 0; k < c; k++) at += bound / least[k] + 1;
     return at;
 }
-// Sorts the islands into the size classes' lists; an island that a warp does not take (more than
-// kWarpIsland items, or above big_items, which k_isl_flow may have to colour) gets a range of flow
-// items at base[island]; those above big_items are also listed in big.
-__global__ void k_isl_classes(const int* n_isl, const int* isl_off, int bound, int big_items, int* list, int* n_list, int* base, int* n_flow,
-                              int* big, int* n_big);
+// An island that a warp does not take (more than kWarpIsland items, or above big_items, which
+// k_isl_flow may have to colour) gets a range of flow items at base[island]; those above big_items
+// are also listed in big (k_isl_classes).
 
 // One lane per item, tokens in shared memory.  A round runs every item whose tokens are there; what
 // bounds it is the chain of dependent rows of the longest island of the warp, which the rounds follow
@@ -69,7 +67,7 @@ __global__ void k_isl_classes(const int* n_isl, const int* isl_off, int bound, i
 template <class R, bool JOINTS>
 __global__ void __launch_bounds__(kWarpBlock, sizeof(R) == 4 ? 4 : 2)
 k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, const uint32_t* order, Results<R> res, Joints<R> J, Bodies<R> B,
-           Rows<R> rows, const int* row_off, int iterations, int color_min, int* n_colors, int* status) {
+           Rows<R> rows, int iterations, int color_min, int* n_colors, int* status) {
     constexpr int W = kWarpBlock / 32;
     __shared__ R tok_v[W][2][6][32];     // per side and lane: the token's linear and angular velocity
     __shared__ int tok_it[W][2][32];     // the iteration the token is for
@@ -99,7 +97,7 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
         const bool active = idx < m;
         Item<R, JOINTS> t;
         t.ia = -1; t.ib = -1;
-        if (active) t.load(order[lo + idx], res, J, B, row_off);
+        if (active) t.load(order[lo + idx], res, J, B);
         // the island's items on this item's bodies (bit per item), and on which side they hold them
         const int da = active && !t.a.kin ? t.ia : -2, db = active && !t.b.kin ? t.ib : -2;
         unsigned ma = 0, mab = 0, mb = 0, mbb = 0;
@@ -256,7 +254,7 @@ constexpr int kFlowStall = 1 << 21;   // polls in a row without progress after w
 // islands, took 3.4 and 11 us per level and iteration.)
 template <class R, bool JOINTS>
 __global__ void __launch_bounds__(kFlowBlock, sizeof(R) == 4 ? 4 : 2)
-k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows, const int* row_off) {
+k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows) {
     constexpr int NW = token_words<R>();
     const int M = *f.n_flow;
     if (M == 0) return;   // the same for every thread
@@ -416,7 +414,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
     int succ_a = 0, succ_b = 0, lev_a = 0, lev_b = 0, m = 0, deepest = 0;
     bool have_a = false, have_b = false;
     auto take_item = [&](int j) {
-        x.load(f.item[j], res, J, B, row_off);
+        x.load(f.item[j], res, J, B);
         have_a = x.a.kin;
         have_b = x.b.kin;
         if (!x.a.kin) succ_a = f.succ[2 * j];

@@ -62,8 +62,8 @@ __device__ __forceinline__ void row_store(const Rows<double>& rows, int r, const
 
 // FrictionContactConstraint::initSequentialImpulse (friction_contact_constraint.cpp:9-73), one thread per result
 template <class R>
-__device__ __forceinline__ void si_setup_result(int p, const Results<R>& res, const Bodies<R>& B, const Rows<R>& rows, const int* row_off,
-                                                const StepParams& prm, int* status) {
+__device__ __forceinline__ void si_setup_result(int p, const Results<R>& res, const Bodies<R>& B, const Rows<R>& rows,
+                                                const StepParams& prm) {
     const int np = res.npts[p];
     if (np == 0) return;
     const int ia = res.a[p], ib = res.b[p];
@@ -75,8 +75,7 @@ __device__ __forceinline__ void si_setup_result(int p, const Results<R>& res, co
     const V3<R> va0 = B.vec(VX, ia), wa0 = B.vec(WX, ia), vb0 = B.vec(VX, ib), wb0 = B.vec(WX, ib);
     const R dt = R(prm.dt), kerp = R(0.2), pen_th = R(0.3), rest_th = R(0.1);
     const R mu = res.fr[p], e = res.re[p];
-    const int r0 = row_off[p];
-    if (r0 + np > rows.cap) { atomicOr(status, ST_ROW_OVERFLOW); return; }
+    const int r0 = p * kSlots;
     for (int k = 0; k < np; k++) {
         const int o = p * kSlots + k;
         const V3<R> la(res.pt(LAX, o), res.pt(LAY, o), res.pt(LAZ, o));
@@ -104,9 +103,9 @@ __device__ __forceinline__ void si_setup_result(int p, const Results<R>& res, co
     }
 }
 template <class R>
-__global__ void k_si_setup(const int* Rd, Results<R> res, Bodies<R> B, Rows<R> rows, const int* row_off, StepParams prm, int* status) {
+__global__ void k_si_setup(const int* Rd, Results<R> res, Bodies<R> B, Rows<R> rows, StepParams prm) {
     const int P = *Rd;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) si_setup_result(p, res, B, rows, row_off, prm, status);
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) si_setup_result(p, res, B, rows, prm);
 }
 
 // One body of an item while the solver works on it: temporary velocities and the constants its
@@ -346,65 +345,10 @@ __device__ __forceinline__ void uf_union(int* parent, int a, int b) {
     }
 }
 
-__global__ void k_isl_init(int n, int* parent);
-template <class R>
-__global__ void k_isl_union(const int* Ad, const int* active, Results<R> res, Bodies<R> B, int* parent) {
-    const int A = *Ad;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < A; t += gridDim.x * blockDim.x) {
-        const int p = active[t];
-        const int ia = res.a[p], ib = res.b[p];
-        if ((B.flags[ia] & BF_KINEMATIC) || (B.flags[ib] & BF_KINEMATIC)) continue;
-        uf_union(parent, ia, ib);
-    }
-}
-// joints link their bodies like contact results do
-template <class R>
-__global__ void k_isl_union_joints(Joints<R> J, Bodies<R> B, int* parent) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= J.n) return;
-    const int ia = J.body[j].x, ib = J.body[j].y;
-    if ((B.flags[ia] & BF_KINEMATIC) || (B.flags[ib] & BF_KINEMATIC)) return;
-    uf_union(parent, ia, ib);
-}
-// sort keys of the joints, after the A active results: the island label of a dynamic body; a joint
-// between two kinematic bodies (which moves nothing) gets the label n_bodies, an island of its own
-template <class R>
-__global__ void k_isl_keys_joints(Joints<R> J, Bodies<R> B, const int* parent, const int* Ad, uint64_t* key, uint32_t* key2, uint32_t* val) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= J.n) return;
-    const int A = *Ad;
-    const int ia = J.body[j].x, ib = J.body[j].y;
-    const bool ka = (B.flags[ia] & BF_KINEMATIC) != 0, kb = (B.flags[ib] & BF_KINEMATIC) != 0;
-    key[A + j] = ka && kb ? (uint64_t)B.n : (uint64_t)uf_find(parent, ka ? ib : ia);
-    key2[A + j] = 0;
-    val[A + j] = kJointItem | (uint32_t)j;
-}
-// sort keys: island label (smallest body index of the island) of each active result
-template <class R>
-__global__ void k_isl_keys(const int* Ad, const int* active, Results<R> res, Bodies<R> B, const int* parent, uint64_t* key, uint32_t* key2,
-                           uint32_t* val) {
-    const int A = *Ad;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < A; t += gridDim.x * blockDim.x) {
-        const int p = active[t];
-        const int ia = res.a[p], ib = res.b[p];
-        const int dyn = (B.flags[ia] & BF_KINEMATIC) ? ib : ia;
-        key[t] = (uint64_t)uf_find(parent, dyn);
-        key2[t] = 0;
-        val[t] = (uint32_t)p;
-    }
-}
-// M = *Md sorted items (active results, then joints): island starts, and the islands' first slots
-__global__ void k_isl_flags(const int* Md, int bound, const uint64_t* key, int* flag);
-__global__ void k_isl_offsets(const int* Md, const uint64_t* key, const int* scan, int* isl_off, int* n_isl_out);
-__global__ void k_count_add(const int* a, int add, int* out);
 __global__ void k_step_counters(const int* status, const int* rows, const int* active, const int* islands, const int* n_big, const int* big,
                                 const int* isl_levels, const int* colors, const int* cls, int* out);
 
 // first sorted position of each scene -> offset of its first pair
 __global__ void k_scene_pair_off(int n_scenes, const int* scene_off, const int* pair_scan, int n, int* pair_scene_off);
-// results with at least one point, compacted
-__global__ void k_rows_init(const int* Rd, int bound, const int* npts, int* row_off);
-__global__ void k_active_flags(const int* Rd, int bound, const int* npts, int* flag);
-__global__ void k_active_compact(const int* Rd, const int* npts, const int* scan, int* active);
 
 } // namespace pe

@@ -6,4 +6,5 @@
 // The kernels live in eight parts, each including the one before it:
 // pe_k_integrate, pe_k_broadphase, pe_k_narrowphase, pe_k_sat, pe_k_mesh, pe_k_solver, pe_k_flow, pe_k_state.
 #pragma once
+#include "pe_k_islands.cuh"
 #include "pe_k_state.cuh"

@@ -24,19 +24,19 @@ constexpr int kSapMaxBodies = 16384;
 // sweep alone gives the world's pairs (the block sweeps of crowded windows never have work here)
 constexpr size_t kAlign = 256;
 constexpr size_t al(size_t b) { return (b + kAlign - 1) / kAlign * kAlign; }
-constexpr int kSapTiles = (kSapMaxBodies + kRadixTile - 1) / kRadixTile;
-constexpr int kSapAux = (256 * kSapTiles + 1023) / 1024 + (kSapMaxBodies + 1 + 1023) / 1024 + 2;
+constexpr int kSapTiles = kSapMaxBodies / (kBlock * kRadixItems);
+static_assert(kSapTiles <= kRadixFused, "a radix pass would need its offsets kernel");
+constexpr int kSapAux = kSapMaxBodies / kScanTile + 1;
 
 // byte layout of the scratch array
 struct SapLayout {
-    size_t key[2], key2[2], val[2], hist, aux, total, axis, status, nbig, smn, smx, sflag, sscene, count, stage, big, end;
+    size_t key[2], val[2], hist, aux, total, axis, status, nbig, smn, smx, sflag, sscene, count, stage, big, end;
 };
 constexpr SapLayout sap_layout() {
     SapLayout L{};
     size_t o = 0;
     const size_t n = kSapMaxBodies;
-    for (int k = 0; k < 2; k++) { L.key[k] = o; o += al(n * 8); }
-    for (int k = 0; k < 2; k++) { L.key2[k] = o; o += al(n * 4); }
+    for (int k = 0; k < 2; k++) { L.key[k] = o; o += al(n * 4); }
     for (int k = 0; k < 2; k++) { L.val[k] = o; o += al(n * 4); }
     L.hist = o; o += al((256 * kSapTiles + 1) * 4);
     L.aux = o; o += al(kSapAux * 4);
@@ -62,12 +62,11 @@ __device__ __align__(256) unsigned char g_sap_scratch[kSapScratchBytes];
 
 // sort keys of the bodies (AABB minimum along the axis, as in k_bp_keys); also the per-call
 // values that must start known: the scene axis, one scene id for every key
-__global__ void k_sap_keys(int n, const float* mn, int axis, uint64_t* key, uint32_t* key2, uint32_t* val, int* scene_axis) {
+__global__ void k_sap_keys(int n, const float* mn, int axis, uint32_t* key, uint32_t* val, int* scene_axis) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) scene_axis[0] = axis;
     if (i >= n) return;
     key[i] = order_bits(mn[3 * i + axis]);
-    key2[i] = 0u;
     val[i] = (uint32_t)i;
 }
 
@@ -182,8 +181,7 @@ extern "C" int pe_gpu_sap_pairs_noalloc(int device, int n, const float* aabb_min
         if (e != cudaSuccess) return done(PE_GPU_ERR_CUDA, "cudaMemsetAsync", e);
         return done(PE_GPU_OK, nullptr, cudaSuccess);
     }
-    uint64_t* key[2] = {reinterpret_cast<uint64_t*>(base + kL.key[0]), reinterpret_cast<uint64_t*>(base + kL.key[1])};
-    uint32_t* key2[2] = {reinterpret_cast<uint32_t*>(base + kL.key2[0]), reinterpret_cast<uint32_t*>(base + kL.key2[1])};
+    uint32_t* key[2] = {reinterpret_cast<uint32_t*>(base + kL.key[0]), reinterpret_cast<uint32_t*>(base + kL.key[1])};
     uint32_t* val[2] = {reinterpret_cast<uint32_t*>(base + kL.val[0]), reinterpret_cast<uint32_t*>(base + kL.val[1])};
     int* hist = reinterpret_cast<int*>(base + kL.hist);
     int* aux = reinterpret_cast<int*>(base + kL.aux);
@@ -200,29 +198,25 @@ extern "C" int pe_gpu_sap_pairs_noalloc(int device, int n, const float* aabb_min
     int* n_big = reinterpret_cast<int*>(base + kL.nbig);
 
     const int g = (n + kBlock - 1) / kBlock;
-    k_sap_keys<<<g, kBlock, 0, st>>>(n, aabb_min, axis, key[0], key2[0], val[0], scene_axis);
-    // stable LSD radix sort of the 32-bit keys (as World::radix_sort_keys)
-    const int tiles = (n + kRadixTile - 1) / kRadixTile;
+    k_sap_keys<<<g, kBlock, 0, st>>>(n, aabb_min, axis, key[0], val[0], scene_axis);
     int cur = 0;
-    for (int shift = 0; shift < 32; shift += 8) {
-        k_radix_hist<<<tiles, kBlock, 0, st>>>(key[cur], key2[cur], n, nullptr, -1, shift, 0, hist, tiles);
-        const int m = 256 * tiles, ht = (m + 1023) / 1024;
-        k_scan_tiles<<<ht, kBlock, 0, st>>>(hist, m, aux);
-        k_scan_aux<<<1, kBlock, 0, st>>>(aux, ht, total);
-        k_scan_add<<<ht, kBlock, 0, st>>>(hist, m, aux);
-        k_radix_scatter<<<tiles, kBlock, 0, st>>>(key[cur], key2[cur], val[cur], key[cur ^ 1], key2[cur ^ 1], val[cur ^ 1], n, nullptr, -1, shift, 0,
-                                                 hist, tiles);
-        cur ^= 1;
+    for (int shift = 0; shift < 32; shift += 8, cur ^= 1) {   // as World::radix_pass
+        const RadixArgs<uint32_t> a{key[cur], val[cur], key[cur ^ 1], val[cur ^ 1], nullptr, n, nullptr, -1, shift, hist, radix_tiles(n)};
+        k_radix_hist<uint32_t, kRadixItems><<<a.tiles, kBlock, 0, st>>>(a);
+        k_radix_scatter<uint32_t, kRadixItems><<<a.tiles, kBlock, 0, st>>>(a);
     }
     const uint32_t* order = val[cur];
     k_sap_gather<<<g, kBlock, 0, st>>>(n, aabb_min, aabb_max, flags, order, smn, smx, sflag, sscene, count, status, n_big);
     const int gw = (int)(((size_t)n * 32 + kBlock - 1) / kBlock);
     const IgnoreLists no_lists;   // this entry point takes no ignored-pair lists
     k_bp_count<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, count, stage, big, n_big, no_lists);
-    const int ct = (n + 1 + 1023) / 1024;
-    k_scan_tiles<<<ct, kBlock, 0, st>>>(count, n + 1, aux);
-    k_scan_aux<<<1, kBlock, 0, st>>>(aux, ct, total);
-    k_scan_add<<<ct, kBlock, 0, st>>>(count, n + 1, aux);
+    if (n + 1 <= kScanOne) {
+        k_scan_one<<<1, kScanOneBlock, 0, st>>>(count, n + 1, total);
+    } else {
+        const int ct = scan_tiles(n + 1);
+        k_scan_sums<<<ct, kBlock, 0, st>>>(count, n + 1, aux);
+        k_scan_apply<<<ct, kBlock, 0, st>>>(count, n + 1, aux, total);
+    }
     k_bp_write<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, order, count, stage, reinterpret_cast<int2*>(pairs),
                                              pair_cap, status, no_lists);
     k_sap_total<<<1, 1, 0, st>>>(total, n_pairs);

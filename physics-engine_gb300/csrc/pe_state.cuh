@@ -79,10 +79,9 @@ template <class R> struct Results {
 };
 
 // solver rows (FrictionContactConstraint::ConstraintInfo), NRF consecutive reals per row (RowReg names
-// the fields; one is padding)
+// the fields; one is padding); row k of result p is row p * kSlots + k
 constexpr int NRF = 24;
 template <class R> struct Rows {
-    int cap;
     R* f;
 };
 

@@ -1,163 +1,63 @@
-// Precision-independent device utilities: exclusive scan, stable LSD radix sort passes,
-// pair bucketing, and the constant-memory unit meshes.
+// Precision-independent device utilities: exclusive scan, stable LSD radix sort passes, pair bucketing,
+// contact islands, and the constant-memory unit meshes.
 #include "pe_kernels.cuh"
 
 namespace pe {
 
 // ---------------------------------------------------------------- scan
-// tile = kBlock * 4 elements
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kBlock * kScanItems;
-
-__device__ __forceinline__ int warp_incl_scan(int v) {
-    const int lane = threadIdx.x & 31;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += u;
-    }
-    return v;
-}
-
-// block-wide exclusive scan of one value per thread; returns the block total in *total
-__device__ int block_excl_scan(int v, int* total) {
-    __shared__ int warp_sums[kBlock / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int incl = warp_incl_scan(v);
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < kBlock / 32 ? warp_sums[lane] : 0;
-        w = warp_incl_scan(w);
-        if (lane < kBlock / 32) warp_sums[lane] = w;
-    }
-    __syncthreads();
-    const int before = warp == 0 ? 0 : warp_sums[warp - 1];
-    *total = warp_sums[kBlock / 32 - 1];
-    __syncthreads();
-    return before + incl - v;
-}
-
-__global__ void k_scan_tiles(int* data, int n, int* aux) {
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    int v[kScanItems], s = 0;
-    for (int k = 0; k < kScanItems; k++) { v[k] = base + k < n ? data[base + k] : 0; s += v[k]; }
-    int total;
-    int run = block_excl_scan(s, &total);
-    for (int k = 0; k < kScanItems; k++) { if (base + k < n) data[base + k] = run; run += v[k]; }
-    if (threadIdx.x == 0) aux[blockIdx.x] = total;
-}
-
-// single block: exclusive scan of the m tile totals, grand total into *total
-__global__ void k_scan_aux(int* aux, int m, int* total) {
+__global__ void __launch_bounds__(kScanOneBlock) k_scan_one(int* data, int n, int* total) {
     int carry = 0;
-    for (int base = 0; base < m; base += kBlock) {
-        const int i = base + threadIdx.x;
-        const int v = i < m ? aux[i] : 0;
-        int t;
-        const int ex = block_excl_scan(v, &t);
-        if (i < m) aux[i] = carry + ex;
+    for (int r = 0; r < n; r += kScanOneBlock * kScanOneItems) {
+        const int base = r + threadIdx.x * kScanOneItems;
+        int v[kScanOneItems], s = 0, t;
+#pragma unroll
+        for (int k = 0; k < kScanOneItems; k++) { v[k] = base + k < n ? data[base + k] : 0; s += v[k]; }
+        int run = carry + block_excl_scan<kScanOneBlock>(s, &t);
+#pragma unroll
+        for (int k = 0; k < kScanOneItems; k++) { if (base + k < n) data[base + k] = run; run += v[k]; }
         carry += t;
     }
     if (threadIdx.x == 0) *total = carry;
 }
 
-__global__ void k_scan_add(int* data, int n, const int* aux) {
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    const int add = aux[blockIdx.x];
-    for (int k = 0; k < kScanItems; k++) if (base + k < n) data[base + k] += add;
+__global__ void k_scan_sums(const int* data, int n, int* aux) {
+    int s = 0, t;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        const int i = blockIdx.x * kScanTile + k * kBlock + threadIdx.x;
+        s += i < n ? data[i] : 0;
+    }
+    block_excl_scan<kBlock>(s, &t);
+    if (threadIdx.x == 0) aux[blockIdx.x] = t;
 }
 
-// ---------------------------------------------------------------- small sorts
-__global__ void __launch_bounds__(kSceneSortBlock) k_sort_pairs_block(const uint64_t* key, const uint32_t* val, int n0, const int* nd,
-                                                                     uint64_t* key_out, uint32_t* val_out) {
-    __shared__ uint64_t k[kSceneSortMax];
-    __shared__ uint32_t pos[kSceneSortMax];
-    const int n = nd ? *nd : n0;
-    if (n > kSceneSortMax) return;   // the radix passes sort this count
-    int P = 1;
-    while (P < n) P <<= 1;
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        if (i < n) { k[i] = key[i]; pos[i] = (uint32_t)i; }
-        else { k[i] = ~0ull; pos[i] = 0xffffffffu; }   // padding sorts last
-    }
-    __syncthreads();
-    for (int size = 2; size <= P; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
-                const int i = 2 * t - (t & (stride - 1)), j = i + stride;
-                const bool up = (i & size) == 0;
-                const uint64_t ki = k[i], kj = k[j];
-                const uint32_t pi = pos[i], pj = pos[j];
-                const bool gt = ki > kj || (ki == kj && pi > pj);
-                if (gt == up) { k[i] = kj; k[j] = ki; pos[i] = pj; pos[j] = pi; }
-            }
-            __syncthreads();
-        }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) pos[i] = val[pos[i]];   // every read of the input before any write
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) { key_out[i] = k[i]; val_out[i] = pos[i]; }
+__global__ void k_scan_apply(int* data, int n, const int* aux, int* total) {
+    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    int v[kScanItems], s = 0, t;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) { v[k] = base + k < n ? data[base + k] : 0; s += v[k]; }
+    const int before = tiles_before<kBlock>(aux, blockIdx.x);
+    int run = before + block_excl_scan<kBlock>(s, &t);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) { if (base + k < n) data[base + k] = run; run += v[k]; }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + t;
 }
 
 // ---------------------------------------------------------------- radix sort
-__device__ __forceinline__ int digit_of(const uint64_t* key, const uint32_t* key2, int i, int shift, int use2) {
-    return use2 ? (int)((key2[i] >> shift) & 0xffu) : (int)((key[i] >> shift) & 0xffull);
-}
-
-// per-tile digit histogram, stored digit-major: hist[d * n_tiles + tile]
-__global__ void k_radix_hist(const uint64_t* key, const uint32_t* key2, int n0, const int* nd, int small, int shift, int use2, int* hist,
-                             int n_tiles) {
-    __shared__ int cnt[256];
-    const int n = nd ? *nd : n0;
+// one block per digit: its counts in the tiles become the counts of the tiles before, its total goes to the last row
+__global__ void __launch_bounds__(kBlock) k_radix_offsets(int* hist, int tiles, int tile_items, int n0, const int* nd, int small) {
+    const int n = nd ? *nd : n0, d = blockIdx.x;
     if (n <= small) return;
-    cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const int base = blockIdx.x * kRadixTile;
-    for (int r = 0; r < kRadixItems; r++) {
-        const int i = base + r * kBlock + threadIdx.x;
-        if (i < n) atomicAdd(&cnt[digit_of(key, key2, i, shift, use2)], 1);
+    const int live = (n + tile_items - 1) / tile_items;
+    int carry = 0;
+    for (int t0 = 0; t0 < live; t0 += kBlock) {
+        const int t = t0 + threadIdx.x, v = t < live ? hist[t * 256 + d] : 0;
+        int all;
+        const int ex = block_excl_scan<kBlock>(v, &all);
+        if (t < live) hist[t * 256 + d] = carry + ex;
+        carry += all;
     }
-    __syncthreads();
-    hist[threadIdx.x * n_tiles + blockIdx.x] = cnt[threadIdx.x];
-}
-
-// stable scatter: items of a tile keep their order within each digit
-__global__ void k_radix_scatter(const uint64_t* key_in, const uint32_t* key2_in, const uint32_t* val_in, uint64_t* key_out,
-                                uint32_t* key2_out, uint32_t* val_out, int n0, const int* nd, int small, int shift, int use2,
-                                const int* hist, int n_tiles) {
-    __shared__ int base_d[256];          // running output position of each digit for this tile
-    const int n = nd ? *nd : n0;
-    if (n <= small) return;
-    __shared__ int warp_cnt[kBlock / 32][256];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    base_d[threadIdx.x] = hist[threadIdx.x * n_tiles + blockIdx.x];
-    const int tile = blockIdx.x * kRadixTile;
-    for (int r = 0; r < kRadixItems; r++) {
-        for (int w = 0; w < kBlock / 32; w++) warp_cnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        const int i = tile + r * kBlock + threadIdx.x;
-        const bool live = i < n;
-        const int d = live ? digit_of(key_in, key2_in, i, shift, use2) : 256 + lane;   // dead lanes never match live ones
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (live && rank == 0) warp_cnt[warp][d] = __popc(peers);
-        __syncthreads();
-        // exclusive prefix over warps for each digit (thread = digit)
-        {
-            int run = 0;
-            for (int w = 0; w < kBlock / 32; w++) { const int c = warp_cnt[w][threadIdx.x]; warp_cnt[w][threadIdx.x] = run; run += c; }
-            // stash the round total in the digit base after use below
-            __syncthreads();
-            if (live) {
-                const int pos = base_d[d] + warp_cnt[warp][d] + rank;
-                key_out[pos] = key_in[i];
-                key2_out[pos] = key2_in[i];
-                val_out[pos] = val_in[i];
-            }
-            __syncthreads();
-            base_d[threadIdx.x] += run;
-        }
-        __syncthreads();
-    }
+    if (threadIdx.x == 0) hist[tiles * 256 + d] = carry;
 }
 
 // ---------------------------------------------------------------- narrowphase bucketing
@@ -203,73 +103,259 @@ __global__ void k_scene_pair_off(int n_scenes, const int* scene_off, const int* 
     pair_scene_off[s] = pair_scan[scene_off[s]];
 }
 
-// rows of each result before the scan: its point count; zero from the result count up to `bound`
-__global__ void k_rows_init(const int* Rd, int bound, const int* npts, int* row_off) {
-    const int P = *Rd;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= bound; p += gridDim.x * blockDim.x) row_off[p] = p < P ? npts[p] : 0;
+// ---------------------------------------------------------------- islands
+// a result's or joint's part in the union-find: its bodies are of one island when both are dynamic
+__device__ __forceinline__ void isl_union(const IslandArgs& a, int* parent, int ia, int ib) {
+    if ((a.flags[ia] & BF_KINEMATIC) || (a.flags[ib] & BF_KINEMATIC)) return;
+    uf_union(parent, ia, ib);
+}
+// an item's island label: the smallest body of its island (N for a joint that moves nothing)
+__device__ __forceinline__ uint32_t isl_label(const IslandArgs& a, const int* parent, uint32_t item) {
+    if (item & kJointItem) {
+        const int2 q = a.jbody[item & ~kJointItem];
+        const bool ka = (a.flags[q.x] & BF_KINEMATIC) != 0, kb = (a.flags[q.y] & BF_KINEMATIC) != 0;
+        return ka && kb ? (uint32_t)a.N : (uint32_t)uf_find(parent, ka ? q.y : q.x);
+    }
+    const int ia = a.res_a[item];
+    return (uint32_t)uf_find(parent, (a.flags[ia] & BF_KINEMATIC) ? a.res_b[item] : ia);
+}
+// an active result counts one item (high half) and its points (low half)
+__device__ __forceinline__ unsigned long long act_value(int np) { return np > 0 ? 1ull << 32 | (unsigned)np : 0ull; }
+
+__global__ void __launch_bounds__(kIslandBlock) k_islands_one(IslandArgs a, int label_passes) {
+    constexpr int W = kIslandBlock / 32;
+    extern __shared__ int s_dyn[];
+    uint32_t* key = (uint32_t*)s_dyn;                 // [kIslandOne]
+    uint32_t* val = key + kIslandOne;                 // [kIslandOne]
+    int* off = (int*)(val + kIslandOne);              // [kIslandOne + 1]
+    unsigned short* cnt = (unsigned short*)(off + kIslandOne + 2);   // [W][256]
+    int* parent = (int*)(cnt + W * 256);              // [N]
+    __shared__ int digit_base[256], n_cls[kWarpClasses + 2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int P = *a.P;
+    for (int k = tid; k < a.N; k += kIslandBlock) parent[k] = k;
+    if (tid < kWarpClasses + 2) n_cls[tid] = 0;
+    // active results in order, then the joints; their unions
+    unsigned long long v[2], all;
+#pragma unroll
+    for (int k = 0; k < 2; k++) v[k] = 2 * tid + k < P ? act_value(a.npts[2 * tid + k]) : 0ull;
+    unsigned long long run = block_excl_scan<kIslandBlock>(v[0] + v[1], &all);
+    const int A = (int)(all >> 32), M = A + a.NJ;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        if (v[k]) {
+            const int p = 2 * tid + k;
+            val[run >> 32] = (uint32_t)p;
+            isl_union(a, parent, a.res_a[p], a.res_b[p]);
+        }
+        run += v[k];
+    }
+    for (int j = tid; j < a.NJ; j += kIslandBlock) {
+        val[A + j] = kJointItem | (uint32_t)j;
+        const int2 q = a.jbody[j];
+        isl_union(a, parent, q.x, q.y);
+    }
+    __syncthreads();
+    // items warp * 64 + r * 32 + lane, sorted by label
+    uint32_t kr[2], vr[2];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const int i = warp * 64 + r * 32 + lane;
+        vr[r] = i < M ? val[i] : 0u;
+        kr[r] = i < M ? isl_label(a, parent, vr[r]) : 0u;
+    }
+    for (int pass = 0; pass < label_passes; pass++) {
+        for (int k = tid; k < W * 128; k += kIslandBlock) ((unsigned*)cnt)[k] = 0u;
+        __syncthreads();
+        int digit[2], rank[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const bool live = warp * 64 + r * 32 + lane < M;
+            digit[r] = live ? (int)(kr[r] >> (8 * pass)) & 0xff : 256 + lane;
+            const unsigned peers = __match_any_sync(0xffffffffu, digit[r]);
+            rank[r] = live ? cnt[warp * 256 + digit[r]] + __popc(peers & ((1u << lane) - 1u)) : 0;
+            __syncwarp();
+            if (live && lane == __ffs(peers) - 1) cnt[warp * 256 + digit[r]] += (unsigned short)__popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        int total = 0, sum;
+        if (tid < 256)
+            for (int w = 0; w < W; w++) { const int c = cnt[w * 256 + tid]; cnt[w * 256 + tid] = (unsigned short)total; total += c; }
+        const int before = block_excl_scan<kIslandBlock>(total, &sum);
+        if (tid < 256) digit_base[tid] = before;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+            if (warp * 64 + r * 32 + lane < M) {
+                const int pos = digit_base[digit[r]] + cnt[warp * 256 + digit[r]] + rank[r];
+                key[pos] = kr[r];
+                val[pos] = vr[r];
+            }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int i = warp * 64 + r * 32 + lane;
+            if (i < M) { kr[r] = key[i]; vr[r] = val[i]; }
+        }
+    }
+    // islands of the sorted items
+    int head[2], n_isl;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 2 * tid + k;
+        head[k] = i < M && (i == 0 || key[i] != key[i - 1]) ? 1 : 0;
+    }
+    int at = block_excl_scan<kIslandBlock>(head[0] + head[1], &n_isl);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 2 * tid + k;
+        if (i < M) {
+            a.val[0][i] = val[i];
+            a.isl_scan[i] = at;
+            if (head[k]) off[at] = a.isl_off[at] = i;
+        }
+        at += head[k];
+    }
+    if (tid == 0) {
+        off[n_isl] = a.isl_off[n_isl] = M;
+        a.isl_scan[M] = n_isl;
+        *a.n_active = A;
+        *a.n_items = M;
+        *a.n_rows = (int)(all & 0xffffffffull);
+        *a.n_isl = n_isl;
+        if (a.n_colors) *a.n_colors = 0;
+    }
+    __syncthreads();
+    for (int s = tid; s < n_isl; s += kIslandBlock) {
+        const int m = off[s + 1] - off[s];
+        if (m <= kWarpIsland && m <= a.big_items) {
+            const int c = warp_class(m);
+            a.list[class_base(c, a.bound) + atomicAdd(&n_cls[c], 1)] = s;
+            a.base[s] = -1;
+        } else {
+            a.base[s] = atomicAdd(&n_cls[kWarpClasses], m);
+            if (m > a.big_items) a.big[atomicAdd(&n_cls[kWarpClasses + 1], 1)] = s;
+        }
+    }
+    __syncthreads();
+    if (tid < kWarpClasses + 2) a.n_list[tid] = n_cls[tid];
 }
 
-// 1 for the results with points, 0 from the result count up to `bound`
-__global__ void k_active_flags(const int* Rd, int bound, const int* npts, int* flag) {
-    const int P = *Rd;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= bound; p += gridDim.x * blockDim.x) flag[p] = p < P && npts[p] > 0 ? 1 : 0;
-}
-
-__global__ void k_active_compact(const int* Rd, const int* npts, const int* scan, int* active) {
-    const int P = *Rd;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x)
-        if (npts[p] > 0) active[scan[p]] = p;
-}
-
-// *out = *a + add (one thread)
-__global__ void k_count_add(const int* a, int add, int* out) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *out = *a + add;
-}
-
-__global__ void k_isl_init(int n, int* parent) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) parent[i] = i;
-}
-
-// island starts among the M = *Md sorted items; 0 from M up to `bound`
-__global__ void k_isl_flags(const int* Md, int bound, const uint64_t* key, int* flag) {
-    const int M = *Md;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= bound; k += gridDim.x * blockDim.x)
-        flag[k] = k < M && (k == 0 || key[k] != key[k - 1]) ? 1 : 0;
-}
-
-// after an exclusive scan of the flags: island id = scan value at each island's first slot
-__global__ void k_isl_offsets(const int* Md, const uint64_t* key, const int* scan, int* isl_off, int* n_isl_out) {
-    const int M = *Md;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k <= M; k += gridDim.x * blockDim.x) {
-        if (k < M && (k == 0 || key[k] != key[k - 1])) isl_off[scan[k]] = k;
-        if (k == M) { isl_off[scan[M]] = M; *n_isl_out = scan[M]; }
+__global__ void __launch_bounds__(kBlock) k_act_sums(IslandArgs a) {
+    const int P = *a.P;
+    const int t = blockIdx.x * kBlock + threadIdx.x;
+    for (int k = t; k < a.N; k += gridDim.x * kBlock) a.parent[k] = k;
+    if (t < kWarpClasses + 2) a.n_list[t] = 0;
+    if (t == 0 && a.n_colors) *a.n_colors = 0;
+    for (int tile = blockIdx.x; tile * kScanTile < P; tile += gridDim.x) {   // a block's tiles one after the other
+        unsigned long long s = 0, all;
+#pragma unroll
+        for (int k = 0; k < kScanItems; k++) {
+            const int p = tile * kScanTile + k * kBlock + threadIdx.x;
+            s += p < P ? act_value(a.npts[p]) : 0ull;
+        }
+        block_excl_scan<kBlock>(s, &all);
+        if (threadIdx.x == 0) a.aux[tile] = all;
     }
 }
 
-// Size classes of the islands (see k_isl_warp and k_isl_flow), one atomic per class present in a warp
-__global__ void k_isl_classes(const int* n_isl, const int* isl_off, int bound, int big_items, int* list, int* n_list, int* base, int* n_flow,
-                              int* big, int* n_big) {
-    const int NI = *n_isl, lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(kBlock) k_act_apply(IslandArgs a) {
+    const int P = *a.P, tiles = max((P + kScanTile - 1) / kScanTile, 1), tile = blockIdx.x;
+    for (int j = blockIdx.x * kBlock + threadIdx.x; j < a.NJ; j += gridDim.x * kBlock) {
+        const int2 q = a.jbody[j];
+        isl_union(a, a.parent, q.x, q.y);
+    }
+    if (tile >= tiles) return;
+    const int base = tile * kScanTile + threadIdx.x * kScanItems;
+    unsigned long long v[kScanItems], s = 0, all;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) { v[k] = base + k < P ? act_value(a.npts[base + k]) : 0ull; s += v[k]; }
+    const unsigned long long before = tiles_before<kBlock>(a.aux, tile);
+    unsigned long long run = before + block_excl_scan<kBlock>(s, &all);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (v[k]) {
+            const int p = base + k;
+            a.active[run >> 32] = p;
+            isl_union(a, a.parent, a.res_a[p], a.res_b[p]);
+        }
+        run += v[k];
+    }
+    if (tile == tiles - 1 && threadIdx.x == 0) {
+        const int A = (int)((before + all) >> 32);
+        *a.n_active = A;
+        *a.n_items = A + a.NJ;
+        *a.n_rows = (int)((before + all) & 0xffffffffull);
+    }
+}
+
+__global__ void k_isl_keys(IslandArgs a) {
+    const int A = *a.n_active, M = A + a.NJ;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < M; t += gridDim.x * blockDim.x) {
+        const uint32_t item = t < A ? (uint32_t)a.active[t] : kJointItem | (uint32_t)(t - A);
+        a.key[0][t] = isl_label(a, a.parent, item);
+        a.val[0][t] = item;
+    }
+}
+
+__device__ __forceinline__ int isl_head(const uint32_t* key, int k, int M) { return k < M && (k == 0 || key[k] != key[k - 1]) ? 1 : 0; }
+__global__ void __launch_bounds__(kBlock) k_head_sums(IslandArgs a, const uint32_t* key) {
+    const int M = *a.n_items;
+    if ((int)blockIdx.x * kScanTile >= M) return;
+    unsigned long long s = 0, all;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) s += (unsigned)isl_head(key, blockIdx.x * kScanTile + k * kBlock + threadIdx.x, M);
+    block_excl_scan<kBlock>(s, &all);
+    if (threadIdx.x == 0) a.aux[blockIdx.x] = all;
+}
+__global__ void __launch_bounds__(kBlock) k_head_apply(IslandArgs a, const uint32_t* key) {
+    const int M = *a.n_items, tiles = max((M + kScanTile - 1) / kScanTile, 1), tile = blockIdx.x;
+    if (tile >= tiles) return;
+    const int base = tile * kScanTile + threadIdx.x * kScanItems;
+    int v[kScanItems];
+    unsigned long long s = 0, all;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) { v[k] = isl_head(key, base + k, M); s += (unsigned)v[k]; }
+    const unsigned long long before = tiles_before<kBlock>(a.aux, tile);
+    int run = (int)(before + block_excl_scan<kBlock>(s, &all));
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (base + k < M) a.isl_scan[base + k] = run;
+        if (v[k]) a.isl_off[run] = base + k;
+        run += v[k];
+    }
+    if (tile == tiles - 1 && threadIdx.x == 0) {
+        const int n = (int)(before + all);
+        a.isl_scan[M] = n;
+        a.isl_off[n] = M;
+        *a.n_isl = n;
+    }
+}
+
+// size classes of the islands (see k_isl_warp and k_isl_flow), one atomic per class present in a warp
+__global__ void k_isl_classes(IslandArgs a) {
+    const int NI = *a.n_isl, lane = threadIdx.x & 31;
+    int *n_flow = a.n_list + kWarpClasses, *n_big = n_flow + 1;
     for (int s0 = blockIdx.x * blockDim.x; s0 < NI; s0 += gridDim.x * blockDim.x) {
         const int s = s0 + threadIdx.x;
         int c = -1 - lane, m = 0;   // lanes without a warp-sized island match no other
         if (s < NI) {
-            m = isl_off[s + 1] - isl_off[s];
-            if (m <= kWarpIsland && m <= big_items) c = warp_class(m);
+            m = a.isl_off[s + 1] - a.isl_off[s];
+            if (m <= kWarpIsland && m <= a.big_items) c = warp_class(m);
         }
         const unsigned peers = __match_any_sync(0xffffffffu, c);
         const int leader = __ffs(peers) - 1;
         int at = 0;
-        if (c >= 0 && lane == leader) at = atomicAdd(&n_list[c], __popc(peers));
+        if (c >= 0 && lane == leader) at = atomicAdd(&a.n_list[c], __popc(peers));
         at = __shfl_sync(0xffffffffu, at, leader);
         if (s >= NI) continue;
         if (c >= 0) {
-            list[class_base(c, bound) + at + __popc(peers & ((1u << lane) - 1u))] = s;
-            base[s] = -1;
+            a.list[class_base(c, a.bound) + at + __popc(peers & ((1u << lane) - 1u))] = s;
+            a.base[s] = -1;
         } else {
-            base[s] = atomicAdd(n_flow, m);
-            if (m > big_items) big[atomicAdd(n_big, 1)] = s;
+            a.base[s] = atomicAdd(n_flow, m);
+            if (m > a.big_items) a.big[atomicAdd(n_big, 1)] = s;
         }
     }
 }

@@ -300,6 +300,7 @@ private:
     DBuf<int2> cls_rng_;   // [first, end) of each pair class in the bucketed order
     DBuf<int> cls_work_;   // per-class work cursors of the pair-at-a-time kernels
     // the solver's islands (pe_k_flow.cuh): the size classes' lists, and the flow items of larger islands
+    DBuf<unsigned long long> isl_aux_;
     DBuf<int> isl_list_, isl_base_, isl_big_, isl_levels_, isl_colors_, isl_state_;
     DBuf<uint32_t> flow_item_;
     DBuf<int> flow_isl_, flow_color_, flow_head_, flow_next_, flow_succ_, flow_ff_;
@@ -325,7 +326,6 @@ private:
     void solve_enqueue(int mode);   // solver up to the velocity sync and the counters' copy, no host waits
     void finish();                  // waits for the counters; status
     void run_tail(int mode);        // bp_tail .. solve_enqueue, replayed from a CUDA graph when enabled
-    int radix_sort_dev(int bound, int key_passes, const int* nd);
     // resident blocks of a kernel at a block size and dynamic shared memory (cached), and a grid for
     // `items` items of `per_block` items per block, at most four times those (the work loops stride
     // or take items from a cursor; blocks beyond the resident ones let the block scheduler mix the
@@ -351,7 +351,7 @@ private:
     struct GraphSig {
         unsigned long long gen;
         const void* order;
-        int n, ns, pair_cap, rows_cap, nj, n_ign, s, side;
+        int n, ns, pair_cap, nj, n_ign, s, side;
         int plan[PC_COUNT];
         StepParams prm;
         R margin;
@@ -372,8 +372,7 @@ private:
     R* staging(size_t n);         // pinned host buffer of at least n reals
     R* stage_ = nullptr;
     size_t stage_n_ = 0;
-    void radix_sort(int n, int n_scene_passes);
-    int radix_sort_keys(int n, int key_passes, int scene_passes);   // returns the buffer holding the result
+    template <class K> void radix_pass(RadixArgs<K>& a);
     void ensure_pair_capacity(int P);
     void ev_begin(int phase);
     void ev_end(int phase);
@@ -430,8 +429,8 @@ private:
     DBuf<int> scene_off_, scene_axis_, pair_scene_off_, res_scene_off_, prev_res_off_;
     // broadphase
     DBuf<uint64_t> key_[2];
-    DBuf<uint32_t> key2_[2], val_[2];
-    DBuf<int> hist_, aux_, total_, count_, status_;
+    DBuf<uint32_t> val_[2];
+    DBuf<int> hist_, aux_, count_, status_;
     DBuf<R> smn_, smx_;
     DBuf<int> sflag_, ssc_, bp_stage_, bp_big_, bp_nbig_;
     DBuf<int> bp_wend_, bp_csize_, bp_nch_, bp_choff_, bp_ctot_, bp_ccount_, bp_cpref_;   // crowded windows in chunks
@@ -448,10 +447,10 @@ private:
     int R_ = 0;
     std::vector<int> h_pair_scene_off_;
     // solver
-    DBuf<int> row_off_, active_, color_, parent_, isl_flag_, isl_off_, isl_n_, ncol_;
+    DBuf<int> active_, parent_, isl_flag_, isl_off_, isl_n_, ncol_;
     DBuf<double> xfer_;   // state transfers in the C ABI's layout
     DBuf<R> rows_;
-    int rows_cap_ = 0, n_rows_ = 0, n_active_ = 0, n_colors_ = 0, n_islands_ = 0;
+    int n_rows_ = 0, n_active_ = 0, n_colors_ = 0, n_islands_ = 0;
     bool sat_attr_ = false;
 };
 

@@ -23,7 +23,6 @@ template <class R> World<R>::World(int device) : dev_(device) {
     PE_CK(cudaMemcpyToSymbol(g_unit, &u, sizeof(u)));
     status_.ensure(1);
     PE_CK(cudaMemset(status_.p, 0, sizeof(int)));
-    total_.ensure(1);
     rows_total_.ensure(1);
     dcnt_.ensure(DC_COUNT);
     PE_CK(cudaMemset(dcnt_.p, 0, DC_COUNT * sizeof(int)));
@@ -106,7 +105,6 @@ template <class R> Results<R> World<R>::results() {
 
 template <class R> Rows<R> World<R>::rows() {
     Rows<R> r;
-    r.cap = rows_cap_;
     r.f = rows_.p;
     return r;
 }

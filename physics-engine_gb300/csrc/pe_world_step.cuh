@@ -7,67 +7,30 @@ namespace pe {
 
 // ------------------------------------------------------------------ utilities
 template <class R> void World<R>::scan_async(int* data, int n, int* total) {
-    const int tiles = (n + 1023) / 1024;
-    if (tiles <= kSmallScanTiles) {
-        launch(K_SCAN, 1, k_scan_aux, data, n, total);
+    if (n <= kScanOne) {
+        launch_block(K_SCAN, 1, kScanOneBlock, k_scan_one, data, n, total);
     } else {
-        aux_.ensure(tiles + 1);
-        launch(K_SCAN, tiles, k_scan_tiles, data, n, aux_.p);
-        launch(K_SCAN, 1, k_scan_aux, aux_.p, tiles, total);
-        launch(K_SCAN, tiles, k_scan_add, data, n, aux_.p);
+        const int tiles = scan_tiles(n);
+        aux_.ensure(tiles);
+        launch(K_SCAN, tiles, k_scan_sums, (const int*)data, n, aux_.p);
+        launch(K_SCAN, tiles, k_scan_apply, data, n, (const int*)aux_.p, total);
     }
 }
 
-template <class R> void World<R>::radix_sort(int n, int scene_passes) {
-    order_ = val_[radix_sort_keys(n, (int)sizeof(R), scene_passes)].p;
-}
-
-template <class R> int World<R>::radix_sort_keys(int n, int key_passes, int scene_passes) {
-    if (scene_passes == 0 && n <= kSceneSortMax) {   // small: one block, one launch
-        launch_block(K_RADIX, 1, kSceneSortBlock, k_sort_pairs_block, (const uint64_t*)key_[0].p, (const uint32_t*)val_[0].p, n,
-                     (const int*)nullptr, key_[1].p, val_[1].p);
-        return 1;
-    }
-    const int tiles = (n + kRadixTile - 1) / kRadixTile;
-    hist_.ensure((size_t)256 * tiles + 1);
-    aux_.ensure((256 * tiles + 1023) / 1024 + 1);
-    int cur = 0;
-    auto pass = [&](int shift, int use2) {
-        launch(K_RADIX, tiles, k_radix_hist, (const uint64_t*)key_[cur].p, (const uint32_t*)key2_[cur].p, n, (const int*)nullptr, -1, shift,
-               use2, hist_.p, tiles);
-        scan_async(hist_.p, 256 * tiles, total_.p);
-        launch(K_RADIX, tiles, k_radix_scatter, (const uint64_t*)key_[cur].p, (const uint32_t*)key2_[cur].p, (const uint32_t*)val_[cur].p,
-               key_[cur ^ 1].p, key2_[cur ^ 1].p, val_[cur ^ 1].p, n, (const int*)nullptr, -1, shift, use2, (const int*)hist_.p, tiles);
-        cur ^= 1;
-    };
-    for (int s = 0; s < key_passes * 8; s += 8) pass(s, 0);
-    for (int s = 0; s < scene_passes * 8; s += 8) pass(s, 1);
-    return cur;
-}
-
-// Sort of up to `bound` keys whose count is on the device (*nd): one block when it is at most
-// kSceneSortMax, the radix passes above (each launch does nothing for the other case).  Both end
-// in the buffer returned.
-template <class R> int World<R>::radix_sort_dev(int bound, int key_passes, const int* nd) {
-    if (bound <= kSceneSortMax) {
-        launch_block(K_RADIX, 1, kSceneSortBlock, k_sort_pairs_block, (const uint64_t*)key_[0].p, (const uint32_t*)val_[0].p, bound, nd,
-                     key_[1].p, val_[1].p);
-        return 1;
-    }
-    const int fin = key_passes & 1;   // the buffer the passes end in (the block sort may write its input)
-    launch_block(K_RADIX, 1, kSceneSortBlock, k_sort_pairs_block, (const uint64_t*)key_[0].p, (const uint32_t*)val_[0].p, bound, nd,
-                 key_[fin].p, val_[fin].p);
-    const int tiles = (bound + kRadixTile - 1) / kRadixTile;
-    int cur = 0;
-    for (int s = 0; s < key_passes * 8; s += 8) {
-        launch(K_RADIX, tiles, k_radix_hist, (const uint64_t*)key_[cur].p, (const uint32_t*)key2_[cur].p, bound, nd, kSceneSortMax, s, 0,
-               hist_.p, tiles);
-        scan_async(hist_.p, 256 * tiles, total_.p);
-        launch(K_RADIX, tiles, k_radix_scatter, (const uint64_t*)key_[cur].p, (const uint32_t*)key2_[cur].p, (const uint32_t*)val_[cur].p,
-               key_[cur ^ 1].p, key2_[cur ^ 1].p, val_[cur ^ 1].p, bound, nd, kSceneSortMax, s, 0, (const int*)hist_.p, tiles);
-        cur ^= 1;
-    }
-    return fin;
+// one pass of the radix sort over up to n items; the buffers a holds are swapped
+template <class R> template <class K> void World<R>::radix_pass(RadixArgs<K>& a) {
+    a.tiles = radix_tiles(a.n);
+    a.hist = hist_.p;
+    const bool big = radix_big(a.n);
+    launch(K_RADIX, a.tiles, big ? k_radix_hist<K, kRadixItemsBig> : k_radix_hist<K, kRadixItems>, a);
+    if (a.tiles > kRadixFused) launch(K_RADIX, 256, k_radix_offsets, a.hist, a.tiles, radix_tile(a.n), a.n, a.nd, a.small);
+    launch(K_RADIX, a.tiles, big ? k_radix_scatter<K, kRadixItemsBig> : k_radix_scatter<K, kRadixItems>, a);
+    K* key = a.key_out;
+    uint32_t* val = a.val_out;
+    a.key_out = const_cast<K*>(a.key);
+    a.val_out = const_cast<uint32_t*>(a.val);
+    a.key = key;
+    a.val = val;
 }
 
 template <class R> void World<R>::ensure_pair_capacity(int P) {
@@ -81,7 +44,7 @@ template <class R> void World<R>::ensure_pair_capacity(int P) {
     // result slot distances survive between steps: grow both generations keeping contents
     res_dist_[0].ensure((size_t)cap * kSlots, true);
     res_dist_[1].ensure((size_t)cap * kSlots, true);
-    row_off_.ensure(cap + 1); active_.ensure(cap + 1); color_.ensure(cap + 1);
+    active_.ensure(cap + 1);
     sat_out_.ensure((size_t)cap * kSatOut);
     // point buffer: field-major over the capacity; its contents live for one step only
     pair_cap_ = cap;
@@ -107,7 +70,7 @@ template <class R> int World<R>::bp_count() {
 template <class R> void World<R>::bp_count_enqueue() {
     const int n = N_;
     if (n < 2) return;
-    for (int k = 0; k < 2; k++) { key_[k].ensure(n); key2_[k].ensure(n); val_[k].ensure(n); }
+    for (int k = 0; k < 2; k++) { key_[k].ensure(n); val_[k].ensure(n); }
     smn_.ensure((size_t)3 * n); smx_.ensure((size_t)3 * n); sflag_.ensure(n); ssc_.ensure(n);
     count_.ensure(n + 1);
     max_scene_ = 0;
@@ -117,10 +80,16 @@ template <class R> void World<R>::bp_count_enqueue() {
                      val_[0].p);
         order_ = val_[0].p;
     } else {
-        launch(K_BP_KEYS, grid(n), k_bp_keys<R>, bodies(), scene_axis_.p, key_[0].p, key2_[0].p, val_[0].p);
-        int scene_passes = 0;
-        for (int m = NS_ - 1; m > 0; m >>= 8) scene_passes++;
-        radix_sort(n, scene_passes);
+        using K = typename KeyOf<R>::type;
+        K* key[2] = {reinterpret_cast<K*>(key_[0].p), reinterpret_cast<K*>(key_[1].p)};
+        launch(K_BP_KEYS, grid(n), k_bp_keys<R>, bodies(), scene_axis_.p, key[0], val_[0].p);
+        RadixArgs<K> a{key[0], val_[0].p, key[1], val_[1].p, nullptr, n, nullptr, -1, 0, nullptr, 0};
+        hist_.ensure(radix_hist_ints(n));
+        for (a.shift = 0; a.shift < (int)sizeof(K) * 8; a.shift += 8) radix_pass(a);
+        a.scene = bscene_.p;
+        a.shift = 0;
+        for (int m = NS_ - 1; m > 0; m >>= 8, a.shift += 8) radix_pass(a);
+        order_ = const_cast<uint32_t*>(a.val);
     }
     launch(K_BP_GATHER, grid(n), k_bp_gather<R>, bodies(), order_, smn_.p, smx_.p, sflag_.p, ssc_.p);
     bp_stage_.ensure((size_t)n * kStage);
@@ -145,7 +114,6 @@ template <class R> void World<R>::bp_count_enqueue() {
     if (crowded) launch(K_BP_SWEEP, kBigSweepBlocks, k_bp_chunk_sums, (const int*)bp_big_.p, (const int*)bp_nbig_.p, (const int*)bp_choff_.p,
            (const int*)bp_nch_.p, (const int*)bp_ccount_.p, bp_cpref_.p, count_.p);
     PE_CK(cudaMemsetAsync(count_.p + n, 0, sizeof(int), st_));
-    aux_.ensure((n + 1 + 1023) / 1024 + 1);
     scan_async(count_.p, n + 1, dcnt_.p + DC_P);
     PE_CK(cudaMemcpyAsync(hstat_ + HS_P, dcnt_.p + DC_P, sizeof(int), cudaMemcpyDeviceToHost, st_));
 }
@@ -155,23 +123,19 @@ template <class R> void World<R>::bp_count_enqueue() {
 // are bounded by the pair capacity plus the joints.
 template <class R> void World<R>::prepare_tail(int P) {
     ensure_pair_capacity(std::max(P, 1));
-    // a result has at most kSlots points, so kSlots rows per pair slot always fit
-    if ((long long)kSlots * pair_cap_ > rows_cap_) {
-        rows_cap_ = kSlots * pair_cap_ + kSlots * pair_cap_ / 4;
-        rows_.ensure((size_t)NRF * rows_cap_);
-    }
+    // a result has at most kSlots points: its rows start at kSlots times its index
+    rows_.ensure((size_t)NRF * kSlots * pair_cap_);
     const int bound = pair_cap_ + n_joints_;
     const int keys = std::max(N_, bound);
     // the sort buffers also hold the broadphase's body order until the pair list is written: a
     // growth keeps their contents and order_ follows its buffer
     const int oi = order_ == val_[1].p ? 1 : 0;
     const bool ordered = order_ != nullptr;
-    for (int k = 0; k < 2; k++) { key_[k].ensure(keys); key2_[k].ensure(keys); val_[k].ensure(keys, true); }
+    for (int k = 0; k < 2; k++) { key_[k].ensure(keys); val_[k].ensure(keys, true); }
     if (ordered) order_ = val_[oi].p;
-    const int tiles = (bound + kRadixTile - 1) / kRadixTile;
-    hist_.ensure((size_t)256 * tiles + 1);
-    aux_.ensure(std::max((256 * tiles + 1023) / 1024, (std::max(bound, N_) + 1 + 1023) / 1024) + 1);
-    isl_flag_.ensure(bound + 1); isl_off_.ensure(bound + 1); color_.ensure(bound + 1);
+    hist_.ensure(radix_hist_ints(bound));
+    isl_aux_.ensure(scan_tiles(bound) + 1);
+    isl_flag_.ensure(bound + 1); isl_off_.ensure(bound + 1);
     isl_n_.ensure(1); ncol_.ensure(1);
     isl_list_.ensure(class_base(kWarpClasses, bound)); isl_base_.ensure(bound + 1); isl_big_.ensure(bound + 1);
     isl_levels_.ensure(bound + 1); isl_colors_.ensure(bound + 1); isl_state_.ensure(bound + 1);
@@ -189,6 +153,7 @@ template <class R> void World<R>::prepare_tail(int P) {
         PE_CK(cudaFuncSetAttribute(k_np_sat<R, 1, ST_CYLINDER, ST_CYLINDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, light));
         PE_CK(cudaFuncSetAttribute(k_np_sat<R, kSatGroup, -1, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(sat_group_reals<R>(kSatGroup) * sizeof(R))));
+        PE_CK(cudaFuncSetAttribute(k_islands_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)island_one_smem(kIslandOneBodies)));
         sat_attr_ = true;
     }
 }
@@ -344,43 +309,48 @@ template <class R> void World<R>::narrowphase() {
     R_ = P_;
 }
 
-// Solver without host waits: rows, active results, islands (union-find, sort by island, offsets), the
-// iterations (pe_k_flow.cuh); then the step's counters are copied to the host in one transfer.
+// Solver without host waits: rows (on a side stream), islands (pe_k_islands.cuh), the iterations
+// (pe_k_flow.cuh); then the step's counters are copied to the host in one transfer.
 template <class R> void World<R>::solve_enqueue(int mode) {
     if (N_ == 0) return;
     const int cap = pair_cap_, NJ = n_joints_, bound = cap + NJ;
     const int* Rd = dcnt_.p + DC_R;
-    // rows: one per contact point, results' rows contiguous in result order
-    launch(K_SI_MISC, pgrid(cap + 1, kBlock, k_rows_init), k_rows_init, Rd, cap, (const int*)res_np_.p, row_off_.p);
-    scan_async(row_off_.p, cap + 1, rows_total_.p);
-    launch(K_SI_SETUP, pgrid(cap, kBlock, k_si_setup<R>), k_si_setup<R>, Rd, results(), bodies(), rows(), (const int*)row_off_.p, prm_,
-           status_.p);
-    // results with points, in result order
-    launch(K_SI_MISC, pgrid(cap + 1, kBlock, k_active_flags), k_active_flags, Rd, cap, (const int*)res_np_.p, color_.p);
-    scan_async(color_.p, cap + 1, dcnt_.p + DC_A);
-    launch(K_SI_MISC, pgrid(cap, kBlock, k_active_compact), k_active_compact, Rd, (const int*)res_np_.p, (const int*)color_.p, active_.p);
+    int *Ad = dcnt_.p + DC_A, *Md = dcnt_.p + DC_M;
     const Joints<R> jt = joints();
+    PE_CK(cudaEventRecord(fork_ev_, st_));
+    PE_CK(cudaStreamWaitEvent(side_[0], fork_ev_, 0));
+    use_stream(0);
+    launch(K_SI_SETUP, pgrid(cap, kBlock, k_si_setup<R>), k_si_setup<R>, Rd, results(), bodies(), rows(), prm_);
     if (NJ > 0) launch(K_SI_SETUP, grid(NJ), k_joint_init<R>, jt, bodies(), prm_);
-    // islands: union-find over dynamic bodies linked by contacts and joints; items (active results
-    // in result order, then joints in order) sorted by island label, stably
-    const int* Ad = dcnt_.p + DC_A;
-    int* Md = dcnt_.p + DC_M;
-    launch_block(K_ISLAND, 1, 32, k_count_add, Ad, NJ, Md);
-    launch(K_ISLAND, grid(N_), k_isl_init, N_, parent_.p);
-    launch(K_ISLAND, pgrid(cap, kBlock, k_isl_union<R>), k_isl_union<R>, Ad, (const int*)active_.p, results(), bodies(), parent_.p);
-    if (NJ > 0) launch(K_ISLAND, grid(NJ), k_isl_union_joints<R>, jt, bodies(), parent_.p);
-    launch(K_ISLAND, pgrid(cap, kBlock, k_isl_keys<R>), k_isl_keys<R>, Ad, (const int*)active_.p, results(), bodies(), (const int*)parent_.p,
-           key_[0].p, key2_[0].p, val_[0].p);
-    if (NJ > 0) launch(K_ISLAND, grid(NJ), k_isl_keys_joints<R>, jt, bodies(), (const int*)parent_.p, Ad, key_[0].p, key2_[0].p, val_[0].p);
+    cur_ = nullptr;
+    IslandArgs a;
+    a.P = Rd; a.NJ = NJ; a.N = N_; a.bound = bound;
+    a.res_a = res_a_.p; a.res_b = res_b_.p; a.npts = res_np_.p; a.flags = bflags_.p; a.jbody = jbody_.p;
+    a.parent = parent_.p; a.active = active_.p; a.n_active = Ad; a.n_items = Md; a.n_rows = rows_total_.p;
+    for (int k = 0; k < 2; k++) { a.key[k] = reinterpret_cast<uint32_t*>(key_[k].p); a.val[k] = val_[k].p; }
+    a.aux = isl_aux_.p; a.isl_scan = isl_flag_.p; a.isl_off = isl_off_.p; a.n_isl = isl_n_.p;
+    a.big_items = tun_.big_island_items;
+    a.list = isl_list_.p; a.n_list = dcnt_.p + DC_NLIST; a.base = isl_base_.p; a.big = isl_big_.p;
+    a.n_colors = mode == 0 ? nullptr : ncol_.p;
+    const uint32_t* order = val_[0].p;
     int label_passes = 0;
     for (int m = NJ > 0 ? N_ : N_ - 1; m > 0; m >>= 8) label_passes++;   // joint labels reach n_bodies
-    const int cur = radix_sort_dev(bound, label_passes, Md);
-    const uint64_t* skey = key_[cur].p;
-    const uint32_t* order = val_[cur].p;
-    launch(K_ISLAND, pgrid(bound + 1, kBlock, k_isl_flags), k_isl_flags, (const int*)Md, bound, skey, isl_flag_.p);
-    scan_async(isl_flag_.p, bound + 1, isl_n_.p);
-    launch(K_ISLAND, pgrid(bound + 1, kBlock, k_isl_offsets), k_isl_offsets, (const int*)Md, skey, (const int*)isl_flag_.p, isl_off_.p,
-           isl_n_.p);
+    if (bound <= kIslandOne && N_ <= kIslandOneBodies) {
+        const size_t smem = island_one_smem(N_);
+        launch_smem(K_ISLAND, 1, kIslandBlock, smem, k_islands_one, a, label_passes);
+    } else {
+        launch(K_ISLAND, pgrid(std::max(cap, N_), kScanTile, k_act_sums), k_act_sums, a);
+        launch(K_ISLAND, scan_tiles(cap), k_act_apply, a);
+        launch(K_ISLAND, pgrid(bound, kBlock, k_isl_keys), k_isl_keys, a);
+        RadixArgs<uint32_t> r{a.key[0], a.val[0], a.key[1], a.val[1], nullptr, bound, Md, -1, 0, nullptr, 0};
+        for (int k = 0; k < label_passes; k++, r.shift += 8) radix_pass(r);
+        order = r.val;
+        launch(K_ISLAND, scan_tiles(bound), k_head_sums, a, r.key);
+        launch(K_ISLAND, scan_tiles(bound), k_head_apply, a, r.key);
+        launch(K_ISLAND, pgrid(bound, kBlock, k_isl_classes), k_isl_classes, a);
+    }
+    PE_CK(cudaEventRecord(join_ev_[0], side_[0]));
+    PE_CK(cudaStreamWaitEvent(st_, join_ev_[0], 0));
     if (NJ > 0) solve_islands<true>(mode, order);
     else solve_islands<false>(mode, order);
     launch_block(K_MISC, 1, 32, k_step_counters, (const int*)status_.p, (const int*)rows_total_.p, Ad, (const int*)isl_n_.p,
@@ -389,19 +359,14 @@ template <class R> void World<R>::solve_enqueue(int mode) {
     PE_CK(cudaMemcpyAsync(hstat_, dstat_.p, HS_COUNT * sizeof(int), cudaMemcpyDeviceToHost, st_));
 }
 
-// The solver's iterations: the islands sorted into size classes, then those that fit a warp and those
-// that do not.
+// The solver's iterations: the islands that fit a warp, then those that do not.
 template <class R> template <bool JOINTS> void World<R>::solve_islands(int mode, const uint32_t* order) {
     const int bound = pair_cap_ + n_joints_, small = tun_.small_island_items, big = tun_.big_island_items;
     int* n_list = dcnt_.p + DC_NLIST;
     int* colors = mode == 0 ? nullptr : ncol_.p;
-    PE_CK(cudaMemsetAsync(n_list, 0, (DC_COUNT - DC_NLIST) * sizeof(int), st_));
-    if (colors) PE_CK(cudaMemsetAsync(colors, 0, sizeof(int), st_));
-    launch(K_ISLAND, pgrid(bound, kBlock, k_isl_classes), k_isl_classes, (const int*)isl_n_.p, (const int*)isl_off_.p, bound, big, isl_list_.p,
-           n_list, isl_base_.p, dcnt_.p + DC_NFLOW, isl_big_.p, dcnt_.p + DC_NBIG);
     launch_block(K_SI_SERIAL, pgrid(bound, kWarpBlock, k_isl_warp<R, JOINTS>, kWarpBlock), kWarpBlock, k_isl_warp<R, JOINTS>,
                  (const int*)isl_list_.p, (const int*)n_list, bound, (const int*)isl_off_.p, order, results(), joints(), bodies(), rows(),
-                 (const int*)row_off_.p, prm_.iterations, small, colors, status_.p);
+                 prm_.iterations, small, colors, status_.p);
     FlowArgs<R> f;
     f.n_items = dcnt_.p + DC_M; f.isl_scan = isl_flag_.p; f.isl_off = isl_off_.p; f.order = order;
     f.base = isl_base_.p; f.n_flow = dcnt_.p + DC_NFLOW; f.big = isl_big_.p; f.n_big = dcnt_.p + DC_NBIG;
@@ -410,7 +375,7 @@ template <class R> template <bool JOINTS> void World<R>::solve_islands(int mode,
     f.box = flow_box_.p; f.isl_levels = isl_levels_.p; f.isl_colors = isl_colors_.p; f.isl_state = isl_state_.p;
     f.any_first_fit = flow_ff_.p; f.n_colors = ncol_.p; f.status = status_.p;
     launch_coop(K_SI_COLOR, resident(k_isl_flow<R, JOINTS>, kFlowBlock, 0), kFlowBlock, k_isl_flow<R, JOINTS>, f, results(), joints(), bodies(),
-                rows(), (const int*)row_off_.p);
+                rows());
 }
 
 // The step's second host wait: its counters and status.
@@ -445,7 +410,7 @@ template <class R> void World<R>::graph_sig(GraphSig& g) const {
     std::memset(&g, 0, sizeof g);
     g.gen = dbuf_generation().load();
     g.order = order_;
-    g.n = N_; g.ns = NS_; g.pair_cap = pair_cap_; g.rows_cap = rows_cap_; g.nj = n_joints_; g.n_ign = n_ign_; g.s = S_;
+    g.n = N_; g.ns = NS_; g.pair_cap = pair_cap_; g.nj = n_joints_; g.n_ign = n_ign_; g.s = S_;
     g.side = bcap_ * 4 + (max_scene_ > kBigWindow ? 1 : 0);
     std::memcpy(g.plan, stream_of_, sizeof g.plan);
     std::memcpy(&g.prm, &prm_, sizeof prm_);
