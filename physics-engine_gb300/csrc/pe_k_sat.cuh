@@ -344,7 +344,7 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
     }
     // everything that enters a projection, in units of roundoff: the bounds' and the projections' errors
     const R slack = sat_slack<R>() * (norm(c.ta().o) + norm(c.tb().o) + qa.mag + qb.mag);
-    const R deep = qa.inner + qb.inner - slack;   // every axis's other depth (the first shape past the second) is above this
+    const R deep = qa.inner + qb.inner - slack;   // the inner balls keep every axis's other depth (the first shape past the second) above this
     const bool able = qa.inner > 0 && qb.inner > 0 && (c.sb.type != ST_HULL || c.sb.nv > 2);
     group_sync<G>();
     // lower bound of the depth along y, of length ny and oriented from B towards A (the reference takes the
@@ -352,7 +352,27 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
     auto bound = [&](const V3<R>& y, R ny) {
         return sat_support<R, TA, false>(c.sa.type, qa, y, ny, subA, slack) + sat_support<R, TB, true>(c.sb.type, qb, y, ny, subB, slack) - fma3(y, dc);
     };
-    auto pruned = [&](R lb, R ny, R pb) { return able && pb < deep && lb > ny * (pb + slack); };
+    // The other depth, the first shape past the second, has its own quirk: the reference's projection of
+    // the first shape passes over the vertices of its first falling run, so its maximum may lie below
+    // the inner ball's.  Among the first kCertain vertices, one that certainly lies above an earlier
+    // one is never passed over; an axis is skipped only if such a vertex keeps the other depth above pb,
+    // or if the run ends with vertex 0, which the inner ball leaves out.
+    constexpr int kCertain = 8;
+    auto certain = [&](const V3<R>& y, R ny, R pb) {
+        if (c.sa.type != ST_HULL) return true;
+        const V3<R> yl = mtv(c.ta().b, y);
+        const R tol = R(2) * slack * ny, need = ny * (pb - qb.inner) - fma3(y, dc) + tol;
+        const int n = min(c.sa.nv, kCertain);
+        R low = fma3(yl, ldv(vA, 0));
+#pragma unroll 1
+        for (int i = 1; i < n; i++) {   // (most axes end at the first or second)
+            const R u = fma3(yl, ldv(vA, i));
+            if (u > low + tol && (i == 1 || u > need)) return true;   // the inner ball leaves out vertex 0 only
+            low = low < u ? low : u;
+        }
+        return false;
+    };
+    auto pruned = [&](const V3<R>& y, R ny, R pb) { return able && pb < deep && bound(y, ny) > ny * (pb + slack) && certain(y, ny, pb); };
     // The inner balls' bound of the same depth.  It alone also decides which axes of a hull count: the
     // balls are certified for a projection that never takes vertex 0 as the maximum, but the reference
     // passes over the vertices after it too while the projections keep falling, so along a few axes its
@@ -442,7 +462,7 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
             const int f = f0 + lane;
             const V3<R> n = face_axis(f < end ? f : 0);
             const R ny = TA == ST_CYLINDER || TA < 0 ? fast_sqrt(fma3(n, n)) : R(1);
-            bool keep = f < end && !pruned(bound(n, ny), ny, pb);
+            bool keep = f < end && !pruned(n, ny, pb);
             if (G == 1 && has_hull && held && __any_sync(full, keep)) keep = keep && !balls_above(c, n, R(1), hold_f);
             push(keep, f);
             f0 += T;
@@ -597,7 +617,7 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
                     const R ny = fast_sqrt(n2);
                     if (!hulls && has_hull && balls) keep = keep && !(ball(x, ny) > ny * (measure + slack));
                     x = x * (g < 0 ? R(-1) : R(1));
-                    keep = keep && !pruned(bound(x, ny), ny, pb);
+                    keep = keep && !pruned(x, ny, pb);
                 }
             }
             push(keep, ci | cj << 16);
