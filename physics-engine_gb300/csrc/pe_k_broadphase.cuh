@@ -27,18 +27,34 @@ __global__ void k_bp_keys(Bodies<R> B, const int* scene_axis, typename KeyOf<R>:
     val[i] = (uint32_t)i;
 }
 
+// sorted copy of the sweep inputs (coalesced reads in the sweep)
+template <class R> struct SweepBoxes {
+    R *mn, *mx;
+    int *flag, *scene;
+    __device__ __forceinline__ void copy(const Bodies<R>& B, int k, int i) const {
+        for (int d = 0; d < 3; d++) {
+            mn[(size_t)d * B.n + k] = B.at(MNX + d, i);
+            mx[(size_t)d * B.n + k] = B.at(MXX + d, i);
+        }
+        flag[k] = B.flags[i];
+        scene[k] = B.scene[i];
+    }
+};
+
 // Sort of every scene's bodies by the AABB minimum along the scene's axis, one block per scene of
 // at most kSceneSortMax bodies: a bitonic sort in shared memory of (key, body index) pairs, whose
 // order, ties by body index, is the stable LSD radix sort's.  Replaces the radix passes (four
 // per key byte plus one per scene-id byte, five launches each) when every scene fits a block.
 constexpr int kSceneSortMax = 2048;
 constexpr int kSceneSortBlock = 512;
+// The block then copies the sweep's inputs in that order (k_bp_gather's work).
 template <class R>
 __global__ void __launch_bounds__(kSceneSortBlock) k_bp_sort_scenes(Bodies<R> B, const int* scene_axis, const int* scene_off,
-                                                                   uint32_t* order) {
+                                                                   uint32_t* order, SweepBoxes<R> out, int* n_big) {
     __shared__ uint64_t key[kSceneSortMax];
     __shared__ uint32_t idx[kSceneSortMax];
     const int s = blockIdx.x;
+    if (s == 0 && threadIdx.x == 0) *n_big = 0;
     const int lo = scene_off[s], cnt = scene_off[s + 1] - lo;
     if (cnt <= 0) return;   // whole block
     int P = 1;
@@ -62,21 +78,17 @@ __global__ void __launch_bounds__(kSceneSortBlock) k_bp_sort_scenes(Bodies<R> B,
             __syncthreads();
         }
     }
-    for (int k = threadIdx.x; k < cnt; k += blockDim.x) order[lo + k] = (uint32_t)lo + idx[k];
-}
-
-// sorted copy of the sweep inputs (coalesced reads in the sweep)
-template <class R>
-__global__ void k_bp_gather(Bodies<R> B, const uint32_t* order, R* smn, R* smx, int* sflag, int* sscene) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= B.n) return;
-    const int i = (int)order[k];
-    for (int d = 0; d < 3; d++) {
-        smn[(size_t)d * B.n + k] = B.at(MNX + d, i);
-        smx[(size_t)d * B.n + k] = B.at(MXX + d, i);
+    for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
+        const int i = lo + (int)idx[k];
+        order[lo + k] = (uint32_t)i;
+        out.copy(B, lo + k, i);
     }
-    sflag[k] = B.flags[i];
-    sscene[k] = B.scene[i];
+}
+template <class R>
+__global__ void k_bp_gather(Bodies<R> B, const uint32_t* order, SweepBoxes<R> out, int* n_big) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) *n_big = 0;
+    if (k < B.n) out.copy(B, k, (int)order[k]);
 }
 
 // BroadPhaseSweepAndPrune::calcCollisionPairs sweep (broad_phase_sweep_and_prune.cpp:24-35)
@@ -271,6 +283,7 @@ __global__ void k_bp_count(int n, int limit, const int* scene_axis, const R* smn
     const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= n) return;
+    if (i == 0 && lane == 0) count[n] = 0;   // the scan's last place
     if (big_window(i, n, limit, scene_axis, smn, smx, sscene)) {   // left to k_bp_count_chunks
         if (lane == 0) big[atomicAdd(n_big, 1)] = i;
         return;
@@ -281,9 +294,11 @@ __global__ void k_bp_count(int n, int limit, const int* scene_axis, const R* smn
 template <class R>
 __global__ void k_bp_write(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
                            const uint32_t* order, const int* offset, const int* stage, int2* pairs, int pair_cap, int* status,
-                           IgnoreLists ign) {
+                           IgnoreLists ign, int n_scenes, const int* scene_off, int* pair_scene_off) {
     const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
+    // each scene's first pair: that of its first sorted position
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s <= n_scenes; s += gridDim.x * blockDim.x) pair_scene_off[s] = offset[scene_off[s]];
     if (i >= n) return;
     const int base = offset[i], c = offset[i + 1] - base;
     if (c == 0 || big_window(i, n, limit, scene_axis, smn, smx, sscene)) return;   // big windows: k_bp_write_chunks

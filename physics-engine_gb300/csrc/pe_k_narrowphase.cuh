@@ -31,28 +31,83 @@ template <class R> __device__ __forceinline__ int sat_class(const ShapeView<R>& 
     return a.type == ST_BOX ? PC_CONVEX : PC_CONVEX_HULL_BOX;
 }
 
-// The pair count is on the device (*Pd); whole warps stride over it, so that every lane takes part
-// in the warp votes.
+// The narrowphase's plan of a step: the pairs grouped by class, and the last results' offsets kept as
+// the pool that the new ones draw stale slots from.
+struct NpPlan {
+    const int* P;
+    int n_scenes;
+    const int* pair_off;       // each scene's first pair, which is its first result from now on
+    int *res_off, *prev_off;
+    int* n_res;
+    int *count, *cursor, *last, *work;   // per class: counts (zero between steps), cursors, the counts kept
+    int2* range;
+    int* order;                // pairs by class
+};
+__device__ __forceinline__ void np_plan_scenes(const NpPlan& a, int t, int T) {
+    for (int s = t; s <= a.n_scenes; s += T) {
+        a.prev_off[s] = a.res_off[s];
+        a.res_off[s] = a.pair_off[s];
+    }
+    if (t == 0) *a.n_res = *a.P;
+}
+template <class R> __device__ __forceinline__ int np_pair_class(int2 q, const Bodies<R>& B, const ShapeTable<R>& S, long long heavy) {
+    const ShapeView<R> sa = S.view(B.shape[q.x]), sb = S.view(B.shape[q.y]);
+    const int c = pair_class(sa.type, sb.type);
+    return c == PC_CONVEX ? sat_class(sa, sb, heavy) : c;
+}
+// Up to kPlanOne pairs: the plan in one block (three launches and five copies before, some 20 us of a
+// 12-body scene's step).
+constexpr int kPlanOne = 2048, kPlanBlock = 1024;
+template <class R> __global__ void __launch_bounds__(kPlanBlock) k_np_plan_one(NpPlan a, const int2* pairs, Bodies<R> B, ShapeTable<R> S, long long heavy) {
+    constexpr int PER = kPlanOne / kPlanBlock;
+    __shared__ int count[32], first[32];
+    if (threadIdx.x < 32) count[threadIdx.x] = 0;
+    np_plan_scenes(a, threadIdx.x, kPlanBlock);
+    __syncthreads();
+    const int P = *a.P;
+    int c[PER], at[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int p = k * kPlanBlock + threadIdx.x;
+        c[k] = p < P ? np_pair_class(pairs[p], B, S, heavy) : -1;
+        at[k] = c[k] >= 0 ? atomicAdd(&count[c[k]], 1) : 0;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int v = count[threadIdx.x], end = warp_incl_scan(v);
+        first[threadIdx.x] = end - v;
+        if (threadIdx.x < PC_COUNT) {
+            a.range[threadIdx.x] = make_int2(end - v, end);
+            a.work[threadIdx.x] = end - v;
+            a.last[threadIdx.x] = v;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < PER; k++)
+        if (c[k] >= 0) a.order[first[c[k]] + at[k]] = k * kPlanBlock + threadIdx.x;
+}
+
+// More pairs: classify, ranges, bucket.  The pair count is on the device; whole warps stride over it,
+// so that every lane takes part in the warp votes.
 template <class R>
-__global__ void k_np_classify(const int* Pd, const int2* pairs, Bodies<R> B, ShapeTable<R> S, int* cls, int* cls_count, long long heavy) {
-    const int P = *Pd;
+__global__ void k_np_classify(NpPlan a, const int2* pairs, Bodies<R> B, ShapeTable<R> S, int* cls, long long heavy) {
+    const int P = *a.P;
+    np_plan_scenes(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     for (int base = blockIdx.x * blockDim.x; base < P; base += gridDim.x * blockDim.x) {
         const int p = base + threadIdx.x;
         int c = -1 - (int)(threadIdx.x & 31);   // lanes past the end never match a class
         if (p < P) {
-            const int2 q = pairs[p];
-            const ShapeView<R> sa = S.view(B.shape[q.x]), sb = S.view(B.shape[q.y]);
-            c = pair_class(sa.type, sb.type);
-            if (c == PC_CONVEX) c = sat_class(sa, sb, heavy);
+            c = np_pair_class(pairs[p], B, S, heavy);
             cls[p] = c;
         }
         // one atomic per class present in the warp
         const unsigned peers = __match_any_sync(0xffffffffu, c);
-        if (c >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&cls_count[c], __popc(peers));
+        if (c >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&a.count[c], __popc(peers));
     }
 }
-__global__ void k_np_bucket(const int* Pd, const int* cls, int* cursor, int* order);
-__global__ void k_np_ranges(const int* count, int* cursor, int2* range, int* work);
+__global__ void k_np_bucket(NpPlan a, const int* cls);
+__global__ void k_np_ranges(NpPlan a);
 
 // Work loops over a class's range [rng.x, rng.y) of the bucketed order, whose size only the device
 // knows: the grids are sized by an upper bound, at most the GPU's resident blocks.

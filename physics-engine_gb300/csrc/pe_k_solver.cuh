@@ -348,7 +348,4 @@ __device__ __forceinline__ void uf_union(int* parent, int a, int b) {
 __global__ void k_step_counters(const int* status, const int* rows, const int* active, const int* islands, const int* n_big, const int* big,
                                 const int* isl_levels, const int* colors, const int* cls, int* out);
 
-// first sorted position of each scene -> offset of its first pair
-__global__ void k_scene_pair_off(int n_scenes, const int* scene_off, const int* pair_scan, int n, int* pair_scene_off);
-
 } // namespace pe

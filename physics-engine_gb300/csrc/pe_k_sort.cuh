@@ -5,15 +5,15 @@
 namespace pe {
 
 // ===================================================================== scan
-// Exclusive scan of n ints in place, the total to *total: up to kScanOne in one block, else tile sums
+// Exclusive scan of n ints in place, the total to *total (and to page-locked *host_total, if set): up to kScanOne in one block, else tile sums
 // and a second launch whose blocks add up the tile sums before their own (no third launch for the
 // sums' scan: a block's share is some hundred loads).  16 tiles of 1,024 took 29 us as rounds of one
 // 256-thread block; 16,384 now take four rounds of 1,024 threads.
 constexpr int kScanItems = 8, kScanTile = kBlock * kScanItems;
 constexpr int kScanOne = 16384, kScanOneBlock = 1024, kScanOneItems = 4;
-__global__ void k_scan_one(int* data, int n, int* total);
+__global__ void k_scan_one(int* data, int n, int* total, int* host_total);
 __global__ void k_scan_sums(const int* data, int n, int* aux);
-__global__ void k_scan_apply(int* data, int n, const int* aux, int* total);
+__global__ void k_scan_apply(int* data, int n, const int* aux, int* total, int* host_total);
 inline int scan_tiles(long long n) { return (int)((n + kScanTile - 1) / kScanTile); }
 
 #ifdef __CUDACC__

@@ -211,14 +211,14 @@ extern "C" int pe_gpu_sap_pairs_noalloc(int device, int n, const float* aabb_min
     const IgnoreLists no_lists;   // this entry point takes no ignored-pair lists
     k_bp_count<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, count, stage, big, n_big, no_lists);
     if (n + 1 <= kScanOne) {
-        k_scan_one<<<1, kScanOneBlock, 0, st>>>(count, n + 1, total);
+        k_scan_one<<<1, kScanOneBlock, 0, st>>>(count, n + 1, total, nullptr);
     } else {
         const int ct = scan_tiles(n + 1);
         k_scan_sums<<<ct, kBlock, 0, st>>>(count, n + 1, aux);
-        k_scan_apply<<<ct, kBlock, 0, st>>>(count, n + 1, aux, total);
+        k_scan_apply<<<ct, kBlock, 0, st>>>(count, n + 1, aux, total, nullptr);
     }
     k_bp_write<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, order, count, stage, reinterpret_cast<int2*>(pairs),
-                                             pair_cap, status, no_lists);
+                                             pair_cap, status, no_lists, -1, nullptr, nullptr);
     k_sap_total<<<1, 1, 0, st>>>(total, n_pairs);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return done(PE_GPU_ERR_CUDA, "kernel launch", e);

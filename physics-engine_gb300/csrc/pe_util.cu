@@ -5,7 +5,7 @@
 namespace pe {
 
 // ---------------------------------------------------------------- scan
-__global__ void __launch_bounds__(kScanOneBlock) k_scan_one(int* data, int n, int* total) {
+__global__ void __launch_bounds__(kScanOneBlock) k_scan_one(int* data, int n, int* total, int* host_total) {
     int carry = 0;
     for (int r = 0; r < n; r += kScanOneBlock * kScanOneItems) {
         const int base = r + threadIdx.x * kScanOneItems;
@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(kScanOneBlock) k_scan_one(int* data, int n, in
         for (int k = 0; k < kScanOneItems; k++) { if (base + k < n) data[base + k] = run; run += v[k]; }
         carry += t;
     }
-    if (threadIdx.x == 0) *total = carry;
+    if (threadIdx.x == 0) { *total = carry; if (host_total) *host_total = carry; }
 }
 
 __global__ void k_scan_sums(const int* data, int n, int* aux) {
@@ -31,7 +31,7 @@ __global__ void k_scan_sums(const int* data, int n, int* aux) {
     if (threadIdx.x == 0) aux[blockIdx.x] = t;
 }
 
-__global__ void k_scan_apply(int* data, int n, const int* aux, int* total) {
+__global__ void k_scan_apply(int* data, int n, const int* aux, int* total, int* host_total) {
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems], s = 0, t;
 #pragma unroll
@@ -40,7 +40,7 @@ __global__ void k_scan_apply(int* data, int n, const int* aux, int* total) {
     int run = before + block_excl_scan<kBlock>(s, &t);
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) { if (base + k < n) data[base + k] = run; run += v[k]; }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + t;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) { *total = before + t; if (host_total) *host_total = before + t; }
 }
 
 // ---------------------------------------------------------------- radix sort
@@ -64,8 +64,9 @@ __global__ void __launch_bounds__(kBlock) k_radix_offsets(int* hist, int tiles, 
 // pairs grouped by class (order inside a class is free: every pair's result has its own slot);
 // one atomic per class present in a warp.  The pair count is on the device; whole warps stride
 // over it (the loop bound is block-uniform, so every lane takes part in the warp votes).
-__global__ void k_np_bucket(const int* Pd, const int* cls, int* cursor, int* order) {
-    const int P = *Pd;
+__global__ void k_np_bucket(NpPlan a, const int* cls) {
+    const int P = *a.P;
+    int *cursor = a.cursor, *order = a.order;
     const int lane = threadIdx.x & 31;
     for (int base = blockIdx.x * blockDim.x; base < P; base += gridDim.x * blockDim.x) {
         const int p = base + threadIdx.x;
@@ -79,29 +80,24 @@ __global__ void k_np_bucket(const int* Pd, const int* cls, int* cursor, int* ord
     }
 }
 
-// class ranges from the class counts (one thread): range[c] = [first, end) of class c in the
-// bucketed order, the bucketing cursors at each class's first slot, and the work cursors of the
-// kernels that hand pairs out one at a time (they start at the class's first slot)
-__global__ void k_np_ranges(const int* count, int* cursor, int2* range, int* work) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    int run = 0;
-    for (int c = 0; c < PC_COUNT; c++) {
-        range[c] = make_int2(run, run + count[c]);
-        cursor[c] = run;
-        work[c] = run;
-        run += count[c];
-    }
+// class ranges from the class counts, by one warp: range[c] = [first, end) of class c in the bucketed
+// order, the bucketing cursors at each class's first slot, and the work cursors of the kernels that
+// hand pairs out one at a time (they start at the class's first slot).  The counts are kept for the
+// step's counters and cleared for the next step.
+__device__ void np_ranges(const NpPlan& a, int count) {   // lane c: class c's count
+    const int c = threadIdx.x & 31, v = c < PC_COUNT ? count : 0, end = warp_incl_scan(v);
+    if (c >= PC_COUNT) return;
+    a.range[c] = make_int2(end - v, end);
+    a.cursor[c] = end - v;
+    a.work[c] = end - v;
+    a.last[c] = v;
+    a.count[c] = 0;
 }
+__global__ void k_np_ranges(NpPlan a) { np_ranges(a, threadIdx.x < PC_COUNT ? a.count[threadIdx.x] : 0); }
 
 } // namespace pe
 
 namespace pe {
-
-__global__ void k_scene_pair_off(int n_scenes, const int* scene_off, const int* pair_scan, int n, int* pair_scene_off) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s > n_scenes) return;
-    pair_scene_off[s] = pair_scan[scene_off[s]];
-}
 
 // ---------------------------------------------------------------- islands
 // a result's or joint's part in the union-find: its bodies are of one island when both are dynamic
@@ -360,24 +356,22 @@ __global__ void k_isl_classes(IslandArgs a) {
     }
 }
 
-// the step's counters gathered for one copy to the host (World::HostStat order).  Colours: those the
+// the step's counters, by one warp into page-locked host memory (World::HostStat order).  Colours: those the
 // coloured mode counted; in serial order the levels of the islands above big_island_items, where they
 // are within the first-fit colours' number.
 __global__ void k_step_counters(const int* status, const int* rows, const int* active, const int* islands, const int* n_big, const int* big,
                                 const int* isl_levels, const int* colors, const int* cls, int* out) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    out[0] = *status;
-    out[1] = *rows;
-    out[2] = *active;
-    out[3] = *islands;
-    out[4] = *n_big;
-    int used = colors ? *colors : 0;
-    if (!colors)
-        for (int k = 0; k < *n_big; k++)
-            if (isl_levels[big[k]] < kMaxColorsBig) used = used > isl_levels[big[k]] ? used : isl_levels[big[k]];
-    out[5] = used;
-    out[6] = 0;
-    for (int c = 0; c < PC_COUNT; c++) out[7 + c] = cls[c];
+    const int lane = threadIdx.x & 31;
+    int used = 0;
+    if (colors) used = *colors;
+    else
+        for (int k = lane; k < *n_big; k += 32)
+            if (isl_levels[big[k]] < kMaxColorsBig) used = max(used, isl_levels[big[k]]);
+    used = __reduce_max_sync(0xffffffffu, used);
+    const int* head[5] = {status, rows, active, islands, n_big};
+    if (lane < 5) out[lane] = *head[lane];
+    if (lane == 5) out[5] = used;
+    if (lane < PC_COUNT) out[7 + lane] = cls[lane];
 }
 
 // exclusive offsets of the crowded positions' chunks (one warp)

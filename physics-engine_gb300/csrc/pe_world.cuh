@@ -287,7 +287,7 @@ private:
                    const double* o, const double* b, const double* v, const double* w) const;
     Results<R> results();
     Rows<R> rows();
-    void scan_async(int* data, int n, int* total);   // exclusive scan in place, total to device memory
+    void scan_async(int* data, int n, int* total, int* host_total = nullptr);   // exclusive scan in place
     DBuf<int> rows_total_;
 
     // ---- the step without host waits between its phases.  The device holds the sizes the phases
@@ -306,10 +306,9 @@ private:
     DBuf<int> flow_isl_, flow_color_, flow_head_, flow_next_, flow_succ_, flow_ff_;
     DBuf<uint4> flow_box_;
     template <bool JOINTS> void solve_islands(int mode, const uint32_t* order);
-    // counters read back at the step's end, one copy into page-locked memory
+    // the pair count and the step's counters, written by kernels to page-locked memory
     // (k_step_counters writes them in this order)
     enum HostStat { HS_STATUS = 0, HS_ROWS, HS_ACTIVE, HS_ISLANDS, HS_BIG, HS_COLORS, HS_P, HS_CLS, HS_COUNT = HS_CLS + PC_COUNT };
-    DBuf<int> dstat_;
     int* hstat_ = nullptr;
     int h_cls_[PC_COUNT] = {};   // the last step's pair-class counts (the side-stream plan)
     int stream_of_[PC_COUNT] = {};

@@ -30,7 +30,8 @@ template <class R> World<R>::World(int device) : dev_(device) {
     std::memset(&last_sig_, 0xff, sizeof last_sig_);
     std::memset(&gsig_head_, 0, sizeof gsig_head_);
     std::memset(&last_sig_head_, 0xff, sizeof last_sig_head_);
-    dstat_.ensure(HS_COUNT);
+    cls_count_.ensure(3 * PC_COUNT);
+    PE_CK(cudaMemset(cls_count_.p, 0, 3 * PC_COUNT * sizeof(int)));
     PE_CK(cudaMallocHost(&hstat_, HS_COUNT * sizeof(int)));
     std::memset(hstat_, 0, HS_COUNT * sizeof(int));
     set_scenes(1, nullptr);

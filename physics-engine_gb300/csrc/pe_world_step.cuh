@@ -6,14 +6,14 @@
 namespace pe {
 
 // ------------------------------------------------------------------ utilities
-template <class R> void World<R>::scan_async(int* data, int n, int* total) {
+template <class R> void World<R>::scan_async(int* data, int n, int* total, int* host_total) {
     if (n <= kScanOne) {
-        launch_block(K_SCAN, 1, kScanOneBlock, k_scan_one, data, n, total);
+        launch_block(K_SCAN, 1, kScanOneBlock, k_scan_one, data, n, total, host_total);
     } else {
         const int tiles = scan_tiles(n);
         aux_.ensure(tiles);
         launch(K_SCAN, tiles, k_scan_sums, (const int*)data, n, aux_.p);
-        launch(K_SCAN, tiles, k_scan_apply, data, n, (const int*)aux_.p, total);
+        launch(K_SCAN, tiles, k_scan_apply, data, n, (const int*)aux_.p, total, host_total);
     }
 }
 
@@ -66,18 +66,23 @@ template <class R> int World<R>::bp_count() {
     return hstat_[HS_P];
 }
 
-// the launches of bp_count, ending with the count's copy into page-locked memory (no wait)
+// the launches of bp_count, the last of which writes the count to page-locked memory (no wait)
 template <class R> void World<R>::bp_count_enqueue() {
     const int n = N_;
     if (n < 2) return;
     for (int k = 0; k < 2; k++) { key_[k].ensure(n); val_[k].ensure(n); }
     smn_.ensure((size_t)3 * n); smx_.ensure((size_t)3 * n); sflag_.ensure(n); ssc_.ensure(n);
     count_.ensure(n + 1);
+    bp_stage_.ensure((size_t)n * kStage);
+    bp_big_.ensure(n + 1);
+    bp_nbig_.ensure(1);
+    SweepBoxes<R> boxes;
+    boxes.mn = smn_.p; boxes.mx = smx_.p; boxes.flag = sflag_.p; boxes.scene = ssc_.p;
     max_scene_ = 0;
     for (int s = 0; s < NS_; s++) max_scene_ = std::max(max_scene_, h_scene_off_[s + 1] - h_scene_off_[s]);
     if (max_scene_ <= std::min(tun_.scene_sort_max, kSceneSortMax)) {   // every scene sorted inside one block
         launch_block(K_RADIX, NS_, kSceneSortBlock, k_bp_sort_scenes<R>, bodies(), (const int*)scene_axis_.p, (const int*)scene_off_.p,
-                     val_[0].p);
+                     val_[0].p, boxes, bp_nbig_.p);
         order_ = val_[0].p;
     } else {
         using K = typename KeyOf<R>::type;
@@ -90,12 +95,8 @@ template <class R> void World<R>::bp_count_enqueue() {
         a.shift = 0;
         for (int m = NS_ - 1; m > 0; m >>= 8, a.shift += 8) radix_pass(a);
         order_ = const_cast<uint32_t*>(a.val);
+        launch(K_BP_GATHER, grid(n), k_bp_gather<R>, bodies(), (const uint32_t*)order_, boxes, bp_nbig_.p);
     }
-    launch(K_BP_GATHER, grid(n), k_bp_gather<R>, bodies(), order_, smn_.p, smx_.p, sflag_.p, ssc_.p);
-    bp_stage_.ensure((size_t)n * kStage);
-    bp_big_.ensure(n + 1);
-    bp_nbig_.ensure(1);
-    PE_CK(cudaMemsetAsync(bp_nbig_.p, 0, sizeof(int), st_));
     IgnoreLists ign;
     if (n_ign_ > 0) { ign.off = ign_off_.p; ign.ids = ign_ids_.p; ign.order = order_; }
     launch(K_BP_SWEEP, grid_warps(n), k_bp_count<R>, n, kBigWindow, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, count_.p, bp_stage_.p,
@@ -113,9 +114,7 @@ template <class R> void World<R>::bp_count_enqueue() {
            (const int*)bp_ctot_.p, bp_ccount_.p, ign);
     if (crowded) launch(K_BP_SWEEP, kBigSweepBlocks, k_bp_chunk_sums, (const int*)bp_big_.p, (const int*)bp_nbig_.p, (const int*)bp_choff_.p,
            (const int*)bp_nch_.p, (const int*)bp_ccount_.p, bp_cpref_.p, count_.p);
-    PE_CK(cudaMemsetAsync(count_.p + n, 0, sizeof(int), st_));
-    scan_async(count_.p, n + 1, dcnt_.p + DC_P);
-    PE_CK(cudaMemcpyAsync(hstat_ + HS_P, dcnt_.p + DC_P, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    scan_async(count_.p, n + 1, dcnt_.p + DC_P, hstat_ + HS_P);
 }
 
 // Every buffer the rest of the step writes, sized for P pairs before any of its launches, so that
@@ -144,7 +143,7 @@ template <class R> void World<R>::prepare_tail(int P) {
     flow_box_.ensure((size_t)2 * bound * token_words<R>());
     flow_head_.ensure(N_ + 1); flow_ff_.ensure(1);
     parent_.ensure(N_ + 1);
-    cls_count_.ensure(2 * PC_COUNT); cls_rng_.ensure(PC_COUNT); cls_work_.ensure(PC_COUNT);
+    cls_rng_.ensure(PC_COUNT); cls_work_.ensure(PC_COUNT);
     if (!sat_attr_) {   // dynamic shared memory of the staged SAT kernels (above the 48 KB default for FP64)
         const int light = (int)(kSatWarps * sat_group_reals<R>(1) * sizeof(R));
         PE_CK(cudaFuncSetAttribute(k_np_sat<R, 1, ST_BOX, ST_HULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, light));
@@ -165,13 +164,12 @@ template <class R> void World<R>::bp_tail() {
     IgnoreLists ign;
     if (n_ign_ > 0) { ign.off = ign_off_.p; ign.ids = ign_ids_.p; ign.order = order_; }
     launch(K_BP_SWEEP, grid_warps(n), k_bp_write<R>, n, kBigWindow, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, order_, count_.p, bp_stage_.p,
-           pairs_.p, pair_cap_, status_.p, ign);
+           pairs_.p, pair_cap_, status_.p, ign, NS_, (const int*)scene_off_.p, pair_scene_off_.p);
     if (max_scene_ > kBigWindow)
         launch(K_BP_SWEEP, 2 * kBigSweepBlocks, k_bp_write_chunks<R>, n, (const R*)smn_.p, (const R*)smx_.p, (const int*)sflag_.p,
                (const uint32_t*)order_, (const int*)count_.p, (const int*)bp_big_.p, (const int*)bp_nbig_.p, (const int*)bp_wend_.p,
                (const int*)bp_csize_.p, (const int*)bp_choff_.p, (const int*)bp_ctot_.p, (const int*)bp_cpref_.p, pairs_.p, pair_cap_,
                status_.p, ign);
-    launch(K_MISC, grid(NS_ + 1), k_scene_pair_off, NS_, scene_off_.p, count_.p, n, pair_scene_off_.p);
 }
 
 // The scenes' next sweep axes, from the sorted boxes.  A sum of all bodies in order is a chain (378 us
@@ -224,18 +222,24 @@ template <class R> void World<R>::plan_streams(int* plan) const {
 // ranges computed there, and every class's kernel launched over its range (grids from the pair
 // capacity, persistent up to the resident blocks), side by side on the side streams.
 template <class R> void World<R>::np_enqueue() {
-    // the results of the previous step become the pool the new step draws stale slots from
-    PE_CK(cudaMemcpyAsync(prev_res_off_.p, res_scene_off_.p, (NS_ + 1) * sizeof(int), cudaMemcpyDeviceToDevice, st_));
     const int cap = pair_cap_;
     const int* Pd = dcnt_.p + DC_P;
     const Results<R> rs = results();
     const Bodies<R> bd = bodies();
     const ShapeTable<R> sh = shapes();
-    PE_CK(cudaMemsetAsync(cls_count_.p, 0, PC_COUNT * sizeof(int), st_));
-    launch(K_NP_BUCKET, pgrid(cap, kBlock, k_np_classify<R>), k_np_classify<R>, Pd, (const int2*)pairs_.p, bd, sh, cls_.p, cls_count_.p,
-           (long long)tun_.sat_heavy_cost);
-    launch_block(K_NP_BUCKET, 1, 32, k_np_ranges, (const int*)cls_count_.p, cls_count_.p + PC_COUNT, cls_rng_.p, cls_work_.p);
-    launch(K_NP_BUCKET, pgrid(cap, kBlock, k_np_bucket), k_np_bucket, Pd, (const int*)cls_.p, cls_count_.p + PC_COUNT, order_np_.p);
+    NpPlan plan;
+    plan.P = Pd; plan.n_scenes = NS_;
+    plan.pair_off = pair_scene_off_.p; plan.res_off = res_scene_off_.p; plan.prev_off = prev_res_off_.p; plan.n_res = dcnt_.p + DC_R;
+    plan.count = cls_count_.p; plan.cursor = cls_count_.p + PC_COUNT; plan.last = cls_count_.p + 2 * PC_COUNT; plan.work = cls_work_.p;
+    plan.range = cls_rng_.p; plan.order = order_np_.p;
+    const long long heavy = tun_.sat_heavy_cost;
+    if (cap <= kPlanOne) {
+        launch_block(K_NP_BUCKET, 1, kPlanBlock, k_np_plan_one<R>, plan, (const int2*)pairs_.p, bd, sh, heavy);
+    } else {
+        launch(K_NP_BUCKET, pgrid(cap, kBlock, k_np_classify<R>), k_np_classify<R>, plan, (const int2*)pairs_.p, bd, sh, cls_.p, heavy);
+        launch_block(K_NP_BUCKET, 1, 32, k_np_ranges, plan);
+        launch(K_NP_BUCKET, pgrid(cap, kBlock, k_np_bucket), k_np_bucket, plan, (const int*)cls_.p);
+    }
     // The classes' kernels touch disjoint pairs and results: they run side by side on the side
     // streams, so the long tails of the per-pair kernels overlap the other classes.
     fork_streams();
@@ -296,8 +300,6 @@ template <class R> void World<R>::np_enqueue() {
         }
     }
     join_streams();
-    PE_CK(cudaMemcpyAsync(res_scene_off_.p, pair_scene_off_.p, (NS_ + 1) * sizeof(int), cudaMemcpyDeviceToDevice, st_));
-    PE_CK(cudaMemcpyAsync(dcnt_.p + DC_R, dcnt_.p + DC_P, sizeof(int), cudaMemcpyDeviceToDevice, st_));
 }
 
 template <class R> void World<R>::narrowphase() {
@@ -310,7 +312,7 @@ template <class R> void World<R>::narrowphase() {
 }
 
 // Solver without host waits: rows (on a side stream), islands (pe_k_islands.cuh), the iterations
-// (pe_k_flow.cuh); then the step's counters are copied to the host in one transfer.
+// (pe_k_flow.cuh); then the step's counters, written to host memory by the last kernel.
 template <class R> void World<R>::solve_enqueue(int mode) {
     if (N_ == 0) return;
     const int cap = pair_cap_, NJ = n_joints_, bound = cap + NJ;
@@ -355,8 +357,7 @@ template <class R> void World<R>::solve_enqueue(int mode) {
     else solve_islands<false>(mode, order);
     launch_block(K_MISC, 1, 32, k_step_counters, (const int*)status_.p, (const int*)rows_total_.p, Ad, (const int*)isl_n_.p,
                  (const int*)(dcnt_.p + DC_NBIG), (const int*)isl_big_.p, (const int*)isl_levels_.p,
-                 mode == 0 ? (const int*)nullptr : (const int*)ncol_.p, (const int*)cls_count_.p, dstat_.p);
-    PE_CK(cudaMemcpyAsync(hstat_, dstat_.p, HS_COUNT * sizeof(int), cudaMemcpyDeviceToHost, st_));
+                 mode == 0 ? (const int*)nullptr : (const int*)ncol_.p, (const int*)cls_count_.p + 2 * PC_COUNT, hstat_);
 }
 
 // The solver's iterations: the islands that fit a warp, then those that do not.
