@@ -25,20 +25,22 @@ template <class R, bool JOINTS> struct Item {
     uint32_t id;
     int ia, ib, r0, np;
     Side<R> a, b;
-    __device__ __forceinline__ void load(uint32_t item, const Results<R>& res, const Joints<R>& J, const Bodies<R>& B) {
+    RowReg<R> q;   // a result's first row
+    __device__ __forceinline__ void load(uint32_t item, const Results<R>& res, const Joints<R>& J, const Bodies<R>& B, const Rows<R>& rows) {
         id = item;
         if (JOINTS && (item & kJointItem)) {
             const int2 q = J.body[item & ~kJointItem];
             ia = q.x; ib = q.y; r0 = 0; np = 0;
         } else {
             ia = res.a[item]; ib = res.b[item]; r0 = (int)item * kSlots; np = res.npts[item];
+            row_load(rows, r0, q);
         }
         a.load(B, ia);
         b.load(B, ib);
     }
     __device__ __forceinline__ void iterate(const Joints<R>& J, const Rows<R>& rows) {
         if (JOINTS && (id & kJointItem)) joint_iterate(J, (int)(id & ~kJointItem), a, b);
-        else si_rows(rows, r0, np, a, b);
+        else si_rows(rows, r0, np, q, a, b);
     }
 };
 
@@ -97,7 +99,7 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
         const bool active = idx < m;
         Item<R, JOINTS> t;
         t.ia = -1; t.ib = -1;
-        if (active) t.load(order[lo + idx], res, J, B);
+        if (active) t.load(order[lo + idx], res, J, B, rows);
         // the island's items on this item's bodies (bit per item), and on which side they hold them
         const int da = active && !t.a.kin ? t.ia : -2, db = active && !t.b.kin ? t.ib : -2;
         unsigned ma = 0, mab = 0, mb = 0, mbb = 0;
@@ -414,7 +416,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
     int succ_a = 0, succ_b = 0, lev_a = 0, lev_b = 0, m = 0, deepest = 0;
     bool have_a = false, have_b = false;
     auto take_item = [&](int j) {
-        x.load(f.item[j], res, J, B);
+        x.load(f.item[j], res, J, B, rows);
         have_a = x.a.kin;
         have_b = x.b.kin;
         if (!x.a.kin) succ_a = f.succ[2 * j];

@@ -132,7 +132,7 @@ template <class R> __device__ __forceinline__ void si_row(RowReg<R>& q, Side<R>&
     q.nacc += ni;
     R tt0 = q.t0acc - dot(q.t0, vr) * q.t0jmj;
     R tt1 = q.t1acc - dot(q.t1, vr) * q.t1jmj;
-    const R scale = q.mu * q.nacc / real_sqrt(tt0 * tt0 + tt1 * tt1);
+    const R scale = friction_scale(q.mu * q.nacc, tt0 * tt0 + tt1 * tt1);
     if (scale < 1) { tt0 *= scale; tt1 *= scale; }
     const V3<R> imp = ni * q.n + (tt0 - q.t0acc) * q.t0 + (tt1 - q.t1acc) * q.t1;
     q.t0acc = tt0;
@@ -141,13 +141,16 @@ template <class R> __device__ __forceinline__ void si_row(RowReg<R>& q, Side<R>&
     const V3<R> nimp = -imp;
     if (!b.kin) { b.v = b.v + nimp * b.im; b.w = b.w + mv(b.I, cross(q.rb, nimp)); }
 }
-// all points of one result, in order
-template <class R> __device__ __forceinline__ void si_rows(const Rows<R>& rows, int r0, int np, Side<R>& a, Side<R>& b) {
-    for (int r = r0; r < r0 + np; r++) {
-        RowReg<R> q;
-        row_load(rows, r, q);
+// All points of one result, in order; q holds the first row, before and after.  The next row is loaded
+// while one is worked on: its loads would otherwise wait behind the stores of the accumulators, and
+// the first row's until the bodies' velocities arrive.
+template <class R> __device__ __forceinline__ void si_rows(const Rows<R>& rows, int r0, int np, RowReg<R>& q, Side<R>& a, Side<R>& b) {
+    for (int k = 0; k < np; k++) {
+        RowReg<R> next;
+        if (np > 1) row_load(rows, r0 + (k + 1 < np ? k + 1 : 0), next);
         si_row(q, a, b);
-        row_store_acc(rows, r, q);
+        row_store_acc(rows, r0 + k, q);
+        if (np > 1) q = next;
     }
 }
 

@@ -41,6 +41,19 @@ PE_HD float real_sqrt(float x) { return sqrtf(x); }
 PE_HD double real_sqrt(double x) { return sqrt(x); }
 PE_HD float rabs(float x) { return fabsf(x); }
 PE_HD double rabs(double x) { return fabs(x); }
+// The friction scale of a row, bound / sqrt(q2), where it is below 1 (else any value that is not).  The
+// reference takes the root and the quotient for every row, the longest two links of a row's chain; most
+// contacts hold: bound^2 certainly above q2 means bound >= the rounded root, hence a quotient of at
+// least 1, and a bound of zero over a positive root is zero.  The factor covers the squares' and the
+// root's roundoff, and the limits keep the squares clear of overflow and of denormals.
+template <class R> PE_HD R friction_scale(R bound, R q2) {
+    constexpr R near = sizeof(R) == 4 ? R(1 + 1e-6) : R(1 + 4e-15), lo = sizeof(R) == 4 ? R(1e-30) : R(1e-280), hi = sizeof(R) == 4 ? R(1e30) : R(1e280);
+    if (q2 >= lo && q2 <= hi) {
+        if (bound > R(0) && bound * bound >= q2 * near) return R(1);
+        if (bound == R(0)) return bound;
+    }
+    return bound / real_sqrt(q2);
+}
 template <class R> PE_HD R rmin(R a, R b) { return a < b ? a : b; }
 template <class R> PE_HD R rmax(R a, R b) { return a > b ? a : b; }
 template <class R> PE_HD R rclamp(R x, R lo, R hi) { return rmax(rmin(x, hi), lo); }
