@@ -902,20 +902,89 @@ __global__ void k_np_sat_finish(const int2* rng, const int* order, const int2* p
     });
 }
 
-// CylinderConvexCollisionAlgorithm (cylinder_convex_collision_algorithm.cpp:109-203), one warp
-// per pair: in rounds of 32 faces (in the reference's descending face order, lane i taking the
-// i-th face of the round), each lane computes the contact points its face contributes, and lane 0
-// then adds them to the pair's cache in face order and, inside a face, in the reference's segment
-// order: the cache's merging depends on that order, the candidate points do not.
-constexpr int kCylHullCand = 12;   // points a face can give: 6 cylinder segments x 2 ends
+// ---------------------------------------------------------------- cylinder or sphere against a hull
+// One warp per pair.  The reference walks the faces that the other shape's box reaches in descending
+// index (the face tree's order for a hull) and adds the points a face gives one after the other: the
+// cache's merging depends on that order, the candidate points do not.  The hit faces are queued in
+// order, up to 32 at a time, and their pieces of work (a face and a cylinder segment, a hull edge, or a
+// fan triangle) go to the lanes one each; lane 0 then adds the points the pieces gave, in order.  (With a
+// whole face per lane, its four to six segments or its edges one after the other, a lone pair took 97 us,
+// and the room for all points of 32 faces kept two blocks on an SM.)
+template <class R> struct HullFaces {
+    int nf, lane;
+    int* queue;   // [64]
+    // hit(f): is face f reached; work(n): the first n <= 32 queued faces
+    template <class H, class F> __device__ __forceinline__ void each(H&& hit, F&& work) const {
+        const unsigned full = 0xffffffffu;
+        int cnt = 0;
+        for (int base = 0; base < nf || cnt > 0;) {
+            while (base < nf && cnt < 32) {
+                const int f = nf - 1 - base - lane;
+                const bool h = f >= 0 && hit(f);
+                const unsigned m = __ballot_sync(full, h);
+                if (h) queue[cnt + __popc(m & ((1u << lane) - 1u))] = f;
+                cnt += __popc(m);
+                base += 32;
+            }
+            __syncwarp();
+            const int n = cnt < 32 ? cnt : 32;
+            if (n) work(n);
+            __syncwarp();
+            const int rest = cnt - n, v = lane < rest ? queue[32 + lane] : 0;
+            __syncwarp();
+            if (lane < rest) queue[lane] = v;
+            cnt = rest;
+        }
+    }
+    // the pieces of n queued faces, size(f) of face f: piece(f, k) for each, 32 at a time, then done()
+    template <class S, class F, class D> __device__ __forceinline__ void pieces(int n, S&& size, F&& piece, D&& done) const {
+        const int mine = lane < n ? size(queue[lane]) : 0, end = warp_incl_scan(mine);
+        const int total = __shfl_sync(0xffffffffu, end, 31);
+        for (int t0 = 0; t0 < total; t0 += 32) {
+            const int t = t0 + lane;
+            int lo = 0;   // the first face whose pieces end after t
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (__shfl_sync(0xffffffffu, end, lo + o - 1) <= t) lo += o;
+            const int first = __shfl_sync(0xffffffffu, end - mine, lo < 32 ? lo : 31);
+            if (t < total) piece(queue[lo], t - first);
+            done();
+        }
+    }
+};
+// a piece's points, for lane 0 to add (P points of 7 reals per lane)
+template <class R, int P> struct PieceOut {
+    R* buf;   // this lane's
+    int n;
+    __device__ __forceinline__ void push(const V3<R>& nrm, const V3<R>& pt, R d) {
+        R* e = buf + 7 * n++;
+        e[0] = nrm.x; e[1] = nrm.y; e[2] = nrm.z; e[3] = pt.x; e[4] = pt.y; e[5] = pt.z; e[6] = d;
+    }
+    __device__ __forceinline__ void drain(Pair<R>& c, int lane) {   // the warp's points in order, into lane 0's cache
+        __syncwarp();
+        const unsigned one = __ballot_sync(0xffffffffu, n > 0), two = __ballot_sync(0xffffffffu, n > 1);
+        if (lane == 0)
+            for (unsigned m = one; m; m &= m - 1) {
+                const int l = __ffs(m) - 1;
+                for (int k = 0; k < 1 + (int)((two >> l) & 1u); k++) {
+                    const R* e = buf + l * (7 * P) + 7 * k;
+                    c.add(V3<R>(e[0], e[1], e[2]), V3<R>(e[3], e[4], e[5]), e[6]);
+                }
+            }
+        __syncwarp();
+        n = 0;
+    }
+};
+
+// CylinderConvexCollisionAlgorithm (cylinder_convex_collision_algorithm.cpp:109-203)
 template <class R> constexpr int cyl_hull_warps() { return sizeof(R) == 4 ? 4 : 2; }
 template <class R>
 __global__ void __launch_bounds__(32 * cyl_hull_warps<R>())
 k_np_cyl_hull(const int2* rng, int* cursor, const int* order, const int2* pairs, Bodies<R> B, ShapeTable<R> S, Results<R> res,
               const int* pair_scene_off, const int* prev_off) {
-    constexpr int W = cyl_hull_warps<R>(), K = kCylHullCand;
-    __shared__ R cand[W][32 * K][7];
-    __shared__ int ccnt[W][32];
+    constexpr int W = cyl_hull_warps<R>();
+    __shared__ R cand[W][32 * 14];
+    __shared__ int queue[W][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     warp_items(*rng, cursor, [&](int t) {
     const int p = order[t];
@@ -934,116 +1003,61 @@ k_np_cyl_hull(const int2* rng, int* cursor, const int* order, const int2* pairs,
     const V3<R> axis = rel.b.col(1), pos = rel.o;
     V3<R> aa, bb;
     shape_aabb(cy, rel, aa, bb);
-    const int dxs[4] = {1, -1, -1, 1}, dys[4] = {1, 1, -1, -1};
-    auto push = [&](int& k, const V3<R>& n, const V3<R>& pt, R d) {
-        R* e = cand[warp][lane * K + k];
-        e[0] = n.x; e[1] = n.y; e[2] = n.z; e[3] = pt.x; e[4] = pt.y; e[5] = pt.z; e[6] = d;
-        k++;
-    };
-    auto drain = [&]() {   // lane 0 adds the round's points in face order
-        __syncwarp();
-        if (lane == 0)
-            for (int l = 0; l < 32; l++)
-                for (int k = 0; k < ccnt[warp][l]; k++) {
-                    const R* e = cand[warp][l * K + k];
-                    c.add(V3<R>(e[0], e[1], e[2]), V3<R>(e[3], e[4], e[5]), e[6]);
-                }
-        __syncwarp();
-    };
-    // cylinder side segments against the faces the cylinder's box reaches
-    for (int base = 0; base < m.nf; base += 32) {
-        const int f = m.nf - 1 - base - lane;
-        int k = 0;
-        if (f >= 0 && face_hit(m, f, aa, bb)) {
+    HullFaces<R> faces;
+    faces.nf = m.nf; faces.lane = lane; faces.queue = queue[warp];
+    PieceOut<R, 2> out;
+    out.buf = cand[warp] + lane * 14; out.n = 0;
+    auto hit = [&](int f) { return face_hit(m, f, aa, bb); };
+    auto done = [&]() { out.drain(c, lane); };
+    // cylinder side segments against the faces the cylinder's box reaches: four of a face, and two more
+    // when its normal is the axis
+    faces.each(hit, [&](int n) {
+        faces.pieces(n, [](int) { return 6; }, [&](int f, int k) {
             const V3<R> fn = m.face_normal(f);
             const R adc = dot(axis, fn);
-            V3<R> ddx, ddz;
             const V3<R> ddy = axis;
-            bool vertical = false;
-            if (rabs(rabs(adc) - 1) < eps<R>()) {
+            const bool vertical = rabs(rabs(adc) - 1) < eps<R>();
+            if (k >= 4 && !vertical) return;
+            V3<R> ddx, ddz;
+            if (vertical) {
                 ddz = normalized(cross(axis, V3<R>(1, 0, 0)));
                 ddx = normalized(cross(axis, ddz));
-                vertical = true;
             } else {
                 ddx = normalized(cross(cross(fn, axis), axis));
             }
-            auto seg = [&](const V3<R>& ps, const V3<R>& ds, R ls) {
-                R t1, t2, d1, d2;
-                if (segment_face(m, f, ps, ds, ls, margin, t1, t2, d1, d2)) {
-                    const V3<R> p1 = to.apply(ps + ds * t1 - fn * d1);
-                    const V3<R> p2 = to.apply(ps + ds * t2 - fn * d2);
-                    const V3<R> n = mv(to.b, fn);
-                    push(k, n, p1 - n * margin, d1 + margin * 2);
-                    push(k, n, p2 - n * margin, d2 + margin * 2);
-                }
-            };
-            for (int i = 0; i < 4; i++) {
-                const V3<R> ps = pos + ddx * R(dxs[i]) * cr + ddy * R(dys[i]) * ch;
-                const V3<R> ds = (dxs[i] == dys[i] ? ddy : ddx) * R(-dxs[i]);
-                const R ls = (dxs[i] == dys[i] ? ch : cr) * 2;
-                seg(ps, ds, ls);
+            const int i = k < 4 ? k : 2 * (k - 4);
+            const int dx = i == 0 || i == 3 ? 1 : -1, dy = i < 2 ? 1 : -1;   // (1,1) (-1,1) (-1,-1) (1,-1)
+            const V3<R> ps = pos + (k < 4 ? ddx : ddz) * R(dx) * cr + ddy * R(dy) * ch;
+            const V3<R> ds = (k >= 4 || dx == dy ? ddy : ddx) * R(-dx);
+            const R ls = (k >= 4 || dx == dy ? ch : cr) * 2;
+            R t1, t2, d1, d2;
+            if (segment_face(m, f, ps, ds, ls, margin, t1, t2, d1, d2)) {
+                const V3<R> p1 = to.apply(ps + ds * t1 - fn * d1);
+                const V3<R> p2 = to.apply(ps + ds * t2 - fn * d2);
+                const V3<R> nw = mv(to.b, fn);
+                out.push(nw, p1 - nw * margin, d1 + margin * 2);
+                out.push(nw, p2 - nw * margin, d2 + margin * 2);
             }
-            if (vertical)
-                for (int i = 0; i < 3; i += 2) {
-                    const V3<R> ps = pos + ddz * R(dxs[i]) * cr + ddy * R(dys[i]) * ch;
-                    seg(ps, ddy * R(-dxs[i]), ch * 2);
-                }
-        }
-        ccnt[warp][lane] = k;
-        drain();
-    }
-    // hull edges of those faces against the cylinder (a face with more than K edges is left to
-    // lane 0, in its turn)
-    for (int base = 0; base < m.nf; base += 32) {
-        const int f = m.nf - 1 - base - lane;
-        int k = 0;
-        if (f >= 0 && face_hit(m, f, aa, bb)) {
-            const int n = m.face_size(f);
-            if (n > K) k = -1;
-            else
-                for (int i = 0; i < n; i++) {
-                    const V3<R> v1 = m.vert(m.face_vert(f, i));
-                    const V3<R> v2 = m.vert(m.face_vert(f, (i + 1) % n));
-                    R t1, t2;
-                    const V3<R> start = (v1 + v2) / R(2);
-                    const R ls = norm(v2 - v1) / 2;
-                    const V3<R> dir = (v2 - v1) / (ls * 2);
-                    if (segment_cylinder(start, dir, ls, pos, axis, ch, cr, margin, t1, t2)) {
-                        const V3<R> p1 = start + dir * t1, p2 = start + dir * t2;
-                        V3<R> wn, wp;
-                        R wd;
-                        cyl_contact((p1 + p2) / R(2), pos, axis, cr, ch, to, margin, wn, wp, wd);
-                        push(k, wn, wp, wd);
-                    }
-                }
-        }
-        ccnt[warp][lane] = k;
-        __syncwarp();
-        if (lane == 0)
-            for (int l = 0; l < 32; l++) {
-                if (ccnt[warp][l] >= 0) {
-                    for (int q = 0; q < ccnt[warp][l]; q++) {
-                        const R* e = cand[warp][l * K + q];
-                        c.add(V3<R>(e[0], e[1], e[2]), V3<R>(e[3], e[4], e[5]), e[6]);
-                    }
-                    continue;
-                }
-                const int g = m.nf - 1 - base - l, n = m.face_size(g);
-                for (int i = 0; i < n; i++) {
-                    const V3<R> v1 = m.vert(m.face_vert(g, i));
-                    const V3<R> v2 = m.vert(m.face_vert(g, (i + 1) % n));
-                    R t1, t2;
-                    const V3<R> start = (v1 + v2) / R(2);
-                    const R ls = norm(v2 - v1) / 2;
-                    const V3<R> dir = (v2 - v1) / (ls * 2);
-                    if (segment_cylinder(start, dir, ls, pos, axis, ch, cr, margin, t1, t2)) {
-                        const V3<R> p1 = start + dir * t1, p2 = start + dir * t2;
-                        add_on_cylinder(c, (p1 + p2) / R(2), pos, axis, cr, ch, to, margin);
-                    }
-                }
+        }, done);
+    });
+    // hull edges of those faces against the cylinder
+    faces.each(hit, [&](int n) {
+        faces.pieces(n, [&](int f) { return m.face_size(f); }, [&](int f, int i) {
+            const V3<R> v1 = m.vert(m.face_vert(f, i));
+            const V3<R> v2 = m.vert(m.face_vert(f, (i + 1) % m.face_size(f)));
+            R t1, t2;
+            const V3<R> start = (v1 + v2) / R(2);
+            const R ls = norm(v2 - v1) / 2;
+            const V3<R> dir = (v2 - v1) / (ls * 2);
+            if (segment_cylinder(start, dir, ls, pos, axis, ch, cr, margin, t1, t2)) {
+                const V3<R> p1 = start + dir * t1, p2 = start + dir * t2;
+                V3<R> wn, wp;
+                R wd;
+                cyl_contact((p1 + p2) / R(2), pos, axis, cr, ch, to, margin, wn, wp, wd);
+                out.push(wn, wp, wd);
             }
-        __syncwarp();
-    }
+        }, done);
+    });
     if (lane == 0) {
         cache.swap = false;
         np_finish(p, pairs, B, res, cache);
@@ -1051,21 +1065,16 @@ k_np_cyl_hull(const int2* rng, int* cursor, const int* order, const int2* pairs,
     });
 }
 
-// SphereConvexCollisionAlgorithm (sphere_convex_collision_algorithm.cpp:185-210) for a convex hull,
-// one warp per pair: in rounds of 32 faces (the face tree's order for a hull, descending face
-// index; lane i takes the i-th face of the round) each lane tests its face's box and runs the
-// sphere-triangle test on its face's fan triangles; lane 0 then adds the points to the pair's cache
-// in face order and, inside a face, in triangle order, as the reference's query callback does.  A
-// face with more than kSphereHullCand triangles is left to lane 0 in its turn.
-constexpr int kSphereHullCand = 8;
+// SphereConvexCollisionAlgorithm (sphere_convex_collision_algorithm.cpp:185-210) for a convex hull: the
+// sphere against the fan triangles of the faces its box reaches
 template <class R> constexpr int sphere_hull_warps() { return sizeof(R) == 4 ? 4 : 2; }
 template <class R>
 __global__ void __launch_bounds__(32 * sphere_hull_warps<R>())
 k_np_sphere_hull(const int2* rng, int* cursor, const int* order, const int2* pairs, Bodies<R> B, ShapeTable<R> S, Results<R> res,
                  const int* pair_scene_off, const int* prev_off) {
-    constexpr int W = sphere_hull_warps<R>(), K = kSphereHullCand;
-    __shared__ R cand[W][32 * K][7];
-    __shared__ int ccnt[W][32];
+    constexpr int W = sphere_hull_warps<R>();
+    __shared__ R cand[W][32 * 7];
+    __shared__ int queue[W][64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     warp_items(*rng, cursor, [&](int t) {
     const int p = order[t];
@@ -1082,47 +1091,22 @@ k_np_sphere_hull(const int2* rng, int* cursor, const int* order, const int2* pai
     const V3<R> rel = tm.inv_apply(ts.o);
     const R r = sp.radius;
     const V3<R> aa = rel - V3<R>(r, r, r), bb = rel + V3<R>(r, r, r);
-    // the points of face f's fan triangles, in order, through emit
-    auto face_points = [&](int f, auto&& emit) {
-        const int n = m.face_size(f);
-        for (int i = 0; i < n - 2; i++) {
+    HullFaces<R> faces;
+    faces.nf = m.nf; faces.lane = lane; faces.queue = queue[warp];
+    PieceOut<R, 1> out;
+    out.buf = cand[warp] + lane * 7; out.n = 0;
+    faces.each([&](int f) { return face_hit(m, f, aa, bb); }, [&](int n) {
+        faces.pieces(n, [&](int f) { const int k = m.face_size(f) - 2; return k > 0 ? k : 0; }, [&](int f, int i) {
             const V3<R> vs[3] = {m.vert(m.face_vert(f, 0)), m.vert(m.face_vert(f, i + 1)), m.vert(m.face_vert(f, i + 2))};
             V3<R> point, normal;
             R depth = 0;
             if (sphere_triangle(rel, r, vs, point, normal, depth)) {
                 normal = mv(tm.b, normal);
                 point = tm.apply(point);
-                emit(normal, point - normal * margin, depth + 2 * margin);
+                out.push(normal, point - normal * margin, depth + 2 * margin);
             }
-        }
-    };
-    for (int base = 0; base < m.nf; base += 32) {
-        const int f = m.nf - 1 - base - lane;
-        int k = 0;
-        if (f >= 0 && face_hit(m, f, aa, bb)) {
-            if (m.face_size(f) - 2 > K) k = -1;
-            else
-                face_points(f, [&](const V3<R>& n, const V3<R>& pt, R d) {
-                    R* e = cand[warp][lane * K + k];
-                    e[0] = n.x; e[1] = n.y; e[2] = n.z; e[3] = pt.x; e[4] = pt.y; e[5] = pt.z; e[6] = d;
-                    k++;
-                });
-        }
-        ccnt[warp][lane] = k;
-        __syncwarp();
-        if (lane == 0)
-            for (int l = 0; l < 32; l++) {
-                if (ccnt[warp][l] >= 0) {
-                    for (int q = 0; q < ccnt[warp][l]; q++) {
-                        const R* e = cand[warp][l * K + q];
-                        c.add(V3<R>(e[0], e[1], e[2]), V3<R>(e[3], e[4], e[5]), e[6]);
-                    }
-                } else {
-                    face_points(m.nf - 1 - base - l, [&](const V3<R>& n, const V3<R>& pt, R d) { c.add(n, pt, d); });
-                }
-            }
-        __syncwarp();
-    }
+        }, [&]() { out.drain(c, lane); });
+    });
     if (lane == 0) {
         cache.swap = false;
         np_finish(p, pairs, B, res, cache);
