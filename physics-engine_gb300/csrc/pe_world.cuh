@@ -185,12 +185,12 @@ public:
 private:
     // every kernel of the step goes through here: counts launches, and in profiling mode
     // brackets the launch with events on the world's stream
-    template <class Kern, class... A> void launch(int id, int g, Kern kern, A... args) { launch_smem(id, g, kBlock, 0, kern, args...); }
+    template <class Kern, class... A> void launch(int id, dim3 g, Kern kern, A... args) { launch_smem(id, g, kBlock, 0, kern, args...); }
     template <class Kern, class... A> void launch_block(int id, int g, int block, Kern kern, A... args) {
         launch_smem(id, g, block, 0, kern, args...);
     }
-    template <class Kern, class... A> void launch_smem(int id, int g, int block, size_t smem, Kern kern, A... args) {
-        if (g <= 0) return;
+    template <class Kern, class... A> void launch_smem(int id, dim3 g, int block, size_t smem, Kern kern, A... args) {
+        if (g.x == 0) return;
         klaunch_[id]++;
         step_launches_++;
         cudaStream_t s = cur_ ? cur_ : st_;   // a side stream while a fork is open (fork_streams)
@@ -278,11 +278,11 @@ private:
         return b;
     }
     ShapeTable<R> shapes() const;
-    // appends shapes; returns the first new index.  With `remap`, convex meshes identical to one
-    // appended this way before are not appended again: remap[s] is shape s's index in the tables.
+    // appends shapes; returns the first new index.  With `remap`, shapes identical to one appended this
+    // way before are not appended again: remap[s] is shape s's index in the tables.
     int append_shapes(int S, const int* type, const double* param, const int* vbeg, const int* vcnt, const int* fbeg,
                       const int* fcnt, const double* hv, const int* foff, const int* fidx, std::vector<int>* remap = nullptr);
-    std::unordered_map<std::string, int> hull_by_content_;
+    std::unordered_map<std::string, int> shape_by_content_;
     void fill_body(R* f, size_t stride, int j, int shape, double mass, double fr, double re, double ld, double ad,
                    const double* o, const double* b, const double* v, const double* w) const;
     Results<R> results();
@@ -447,6 +447,9 @@ private:
     std::vector<int> h_pair_scene_off_;
     // solver
     DBuf<int> active_, parent_, isl_flag_, isl_off_, isl_n_, ncol_;
+    // repacking: the spare body arrays (swapped with bf_, bshape_, bflags_), the added bodies, the tables
+    DBuf<R> rp_f_, rp_blk_;
+    DBuf<int> rp_shape_, rp_flags_, rp_tab_[4];
     DBuf<double> xfer_;   // state transfers in the C ABI's layout
     DBuf<R> rows_;
     int n_rows_ = 0, n_active_ = 0, n_colors_ = 0, n_islands_ = 0;

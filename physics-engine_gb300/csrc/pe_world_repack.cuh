@@ -6,7 +6,6 @@ namespace pe {
 
 // ------------------------------------------------------------------ serving: scene repacking
 namespace {
-// kept bodies: field-major gather from the old layout (stride ocap) into the new one (stride ncap)
 // scene whose [off[s], off[s + 1]) holds r (the last such s when empty scenes share an offset)
 __device__ __forceinline__ int segment_of(const int* off, int ns, int r) {
     int lo = 0, hi = ns;
@@ -17,6 +16,9 @@ __device__ __forceinline__ int segment_of(const int* off, int ns, int r) {
     }
     return lo;
 }
+constexpr int kRepackFields = 8;   // fields per block of k_repack_bodies
+// kept bodies: field-major gather from the old layout (stride ocap) into the new one (stride ncap), some
+// fields per block: all of a body's fields in one thread took 26 us for any number of bodies
 template <class R>
 __global__ void k_repack_bodies(const R* of, int ocap, const int* oshape, const int* oflags, R* nf, int ncap, int* nshape,
                                 int* nflags, const int* koff, const int* first, int nk, int n) {
@@ -24,9 +26,13 @@ __global__ void k_repack_bodies(const R* of, int ocap, const int* oshape, const 
     if (j >= n) return;
     const int s = segment_of(koff, nk, j);
     const int i = first[s] + j - koff[s];
-    for (int k = 0; k < NBF; k++) nf[(size_t)k * ncap + j] = of[(size_t)k * ocap + i];
-    nshape[j] = oshape[i];
-    nflags[j] = oflags[i];
+    if (blockIdx.y == 0) {
+        nshape[j] = oshape[i];
+        nflags[j] = oflags[i];
+    }
+#pragma unroll
+    for (int k = blockIdx.y * kRepackFields; k < (int)(blockIdx.y + 1) * kRepackFields; k++)
+        if (k < NBF) nf[(size_t)k * ncap + j] = of[(size_t)k * ocap + i];
 }
 // added bodies: a compact field-major block [NBF x n] placed at new index `at`
 template <class R>
@@ -87,21 +93,23 @@ void World<R>::repack(const int* keep, int n_keep, const SceneData* const* adds,
                       &d.origin[(size_t)i * 3], &d.basis[(size_t)i * 9], &d.lin_vel[(size_t)i * 3], &d.ang_vel[(size_t)i * 3]);
         }
     }
-    DBuf<R> nf;
-    DBuf<int> nshape, nflags, dkoff, dfirst;
+    // the spare set of body arrays and the tables below stay allocated: eight allocations and frees
+    // per repack otherwise
+    DBuf<R>& nf = rp_f_;
+    DBuf<int>&nshape = rp_shape_, &nflags = rp_flags_;
     nf.ensure((size_t)NBF * ncap);
     nshape.ensure(ncap + 1);
     nflags.ensure(ncap + 1);
     if (n_kept) {
-        upload(dkoff, std::vector<int>(off.begin(), off.begin() + n_keep + 1), st_);
-        upload(dfirst, first, st_);
-        launch(K_MISC, grid(n_kept), k_repack_bodies<R>, (const R*)bf_.p, bcap_, (const int*)bshape_.p, (const int*)bflags_.p, nf.p,
-               ncap, nshape.p, nflags.p, (const int*)dkoff.p, (const int*)dfirst.p, n_keep, n_kept);
+        upload(rp_tab_[0], std::vector<int>(off.begin(), off.begin() + n_keep + 1), st_);
+        upload(rp_tab_[1], first, st_);
+        launch(K_MISC, dim3(grid(n_kept), (NBF + kRepackFields - 1) / kRepackFields), k_repack_bodies<R>, (const R*)bf_.p, bcap_,
+               (const int*)bshape_.p, (const int*)bflags_.p, nf.p, ncap, nshape.p, nflags.p, (const int*)rp_tab_[0].p,
+               (const int*)rp_tab_[1].p, n_keep, n_kept);
     }
-    DBuf<R> dblk;
     if (n_new) {
-        upload(dblk, blk, st_);
-        launch(K_MISC, grid(n_new), k_place_bodies<R>, (const R*)dblk.p, n_new, nf.p, ncap, n_kept);
+        upload(rp_blk_, blk, st_);
+        launch(K_MISC, grid(n_new), k_place_bodies<R>, (const R*)rp_blk_.p, n_new, nf.p, ncap, n_kept);
         PE_CK(cudaMemcpyAsync(nshape.p + n_kept, ashape.data(), n_new * sizeof(int), cudaMemcpyHostToDevice, st_));
         PE_CK(cudaMemcpyAsync(nflags.p + n_kept, aflags.data(), n_new * sizeof(int), cudaMemcpyHostToDevice, st_));
     }
@@ -118,18 +126,17 @@ void World<R>::repack(const int* keep, int n_keep, const SceneData* const* adds,
     const int T = new_res[ns];
     ensure_pair_capacity(std::max(T, 1));   // grows both pool generations keeping their contents
     if (T) {
-        DBuf<int> dnew, dold;
-        upload(dnew, new_res, st_);
-        upload(dold, old_start, st_);
+        upload(rp_tab_[2], new_res, st_);
+        upload(rp_tab_[3], old_start, st_);
         launch(K_MISC, grid(T * kSlots), k_repack_pool<R>, (const R*)res_dist_[cur_dist_].p, res_dist_[cur_dist_ ^ 1].p,
-               (const int*)dnew.p, (const int*)dold.p, ns, T * kSlots);
-        PE_CK(cudaStreamSynchronize(st_));
+               (const int*)rp_tab_[2].p, (const int*)rp_tab_[3].p, ns, T * kSlots);
         cur_dist_ ^= 1;
     }
     PE_CK(cudaStreamSynchronize(st_));
     std::swap(bf_.p, nf.p); std::swap(bf_.n, nf.n);
     std::swap(bshape_.p, nshape.p); std::swap(bshape_.n, nshape.n);
     std::swap(bflags_.p, nflags.p); std::swap(bflags_.n, nflags.n);
+    dbuf_generation()++;   // a captured graph holds the other set's addresses
     N_ = N;
     bcap_ = ncap;
     // scene tables (as set_scenes), then the kept axes and result offsets

@@ -131,7 +131,7 @@ void World<R>::set_shapes(int S, const int* type, const double* param, const int
     h_stype_.clear(); h_sparam_.clear(); h_sinertia_.clear(); h_shull_.clear();
     h_hvb_.clear(); h_hvc_.clear(); h_hfb_.clear(); h_hfc_.clear(); h_heb_.clear(); h_hec_.clear(); h_foff_.clear(); h_fidx_.clear();
     h_hv_.clear(); h_fn_.clear(); h_fmn_.clear(); h_fmx_.clear(); h_ea_.clear(); h_eb_.clear(); h_hrad_.clear();
-    hull_by_content_.clear();
+    shape_by_content_.clear();
     h_cbeg_.clear(); h_ccnt_.clear(); h_cshape_.clear(); h_cready_.clear(); h_cxf_.clear();
     h_hlb_.clear(); h_hlc_.clear(); h_lfb_.clear(); h_lfc_.clear(); h_lfmn_.clear(); h_lfmx_.clear();
     append_shapes(S, type, param, vbeg, vcnt, fbeg, fcnt, hv, foff, fidx);
@@ -145,6 +145,7 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
                  o_fi = h_fidx_.size(), o_l = h_lfb_.size();
     if (remap) remap->assign(S, -1);
     int added = 0;
+    std::unordered_map<std::string, int> fresh;   // known to later requests once all of this one's are accepted
     for (int s = 0; s < S; s++) {
         const int t = type[s];
         std::string key;
@@ -158,12 +159,19 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
                 key.append(reinterpret_cast<const char*>(&n), sizeof n);
                 key.append(reinterpret_cast<const char*>(fidx + foff[fbeg[s] + f]), (size_t)n * sizeof(int));
             }
-            auto it = hull_by_content_.find(key);
-            if (it != hull_by_content_.end()) { (*remap)[s] = it->second; continue; }
+        } else if (remap) {   // kind and parameters
+            key.append(reinterpret_cast<const char*>(&t), sizeof t);
+            key.append(reinterpret_cast<const char*>(param + (size_t)s * 3), 3 * sizeof(double));
+        }
+        if (remap) {
+            auto it = shape_by_content_.find(key);
+            if (it != shape_by_content_.end()) { (*remap)[s] = it->second; continue; }
+            it = fresh.find(key);
+            if (it != fresh.end()) { (*remap)[s] = it->second; continue; }
         }
         const int gs = s0 + added++;
         if (remap) (*remap)[s] = gs;
-        if (!key.empty()) hull_by_content_.emplace(std::move(key), gs);
+        if (remap) fresh.emplace(std::move(key), gs);
         V3<R> p;
         for (int k = 0; k < 3; k++) h_sparam_.push_back(R(param[s * 3 + k]));
         p = V3<R>(h_sparam_[(size_t)gs * 3], h_sparam_[(size_t)gs * 3 + 1], h_sparam_[(size_t)gs * 3 + 2]);
@@ -221,6 +229,10 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
     // hull face offsets are global per face: face f of hull h sits at hfb[h] + f, its offsets at
     // f_off[hfb[h] + f] .. f_off[hfb[h] + f + 1]
     S_ = s0 + added;
+    shape_by_content_.merge(fresh);
+    // a request whose shapes are all known already (each one's primitives were appended again, five
+    // uploads, a launch and two waits per request)
+    if (remap && added == 0) return s0;
     PE_CK(cudaStreamSynchronize(st_));   // growth copies below run outside the stream
     upload_tail(stype_, h_stype_, s0, st_); upload_tail(sparam_, h_sparam_, (size_t)s0 * 3, st_); upload_tail(shull_, h_shull_, s0, st_);
     upload_tail(hvbeg_, h_hvb_, o_h, st_); upload_tail(hvcnt_, h_hvc_, o_h, st_); upload_tail(hfbeg_, h_hfb_, o_h, st_);
