@@ -116,6 +116,10 @@ public:
     std::string err;
 };
 
+// State arrays up to this size are read and written in place when they are page-locked: above it the copy
+// engines move them at least as fast as the kernels do.
+constexpr size_t kDirectBytes = (size_t)1 << 20;
+
 template <class R> class World : public WorldBase {
 public:
     explicit World(int device);
@@ -153,6 +157,13 @@ public:
                    const float* iw) override {
         set_state_t(o, b, v, w, mn, mx, iw);
     }
+    template <class T> struct Xfer {   // a state transfer's groups (xfer_groups)
+        XferGroups<T> G{};
+        T* staged[8] = {};
+        size_t size[8] = {};
+        int at[7] = {-1, -1, -1, -1, -1, -1, -1}, widest = 1;
+    };
+    template <class T> Xfer<T> xfer_groups(T* const* arrays);
     template <class T> void get_state_t(T* o, T* b, T* v, T* w, T* mn, T* mx, T* iw);
     template <class T> void set_state_t(const T* o, const T* b, const T* v, const T* w, const T* mn, const T* mx, const T* iw);
     void get_axes(int* a) override;
@@ -376,7 +387,7 @@ private:
     void ev_begin(int phase);
     void ev_end(int phase);
     void ev_collect();
-    int grid(int n) const { return (n + kBlock - 1) / kBlock; }
+    int grid(long long n) const { return (int)((n + kBlock - 1) / kBlock); }
     int grid_warps(int n) const { return (int)(((size_t)n * 32 + kBlock - 1) / kBlock); }   // one warp per item
 
     int dev_;

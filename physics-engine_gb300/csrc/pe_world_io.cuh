@@ -6,8 +6,9 @@
 namespace pe {
 
 // ------------------------------------------------------------------ transfers
-// The body state moves through a device staging buffer in the caller's layout (k_state_pack /
-// k_state_unpack convert precision and layout on the device); pairs copy straight into the caller's
+// The body state is converted on the device (k_state_pack / k_state_unpack), in place in page-locked arrays
+// of up to kDirectBytes and through a device staging buffer otherwise: in place one launch does what
+// took a copy per array too; pairs copy straight into the caller's
 // array, contact results through host vectors (their layout changes on the host), and the serving
 // reads of finished scenes through pinned host memory (staging).  These are the host<->device copies
 // a drop-in caller pays.
@@ -21,52 +22,70 @@ template <class R> R* World<R>::staging(size_t n) {
     return stage_;
 }
 
+// The device's address of a caller's array of `bytes` bytes that kernels may use in place: page-locked
+// memory from end to end, aligned for its values.  nullptr: it goes through the staging buffer.
+static void* direct_address(const void* p, size_t bytes, size_t align) {
+    if (bytes == 0 || bytes > kDirectBytes || reinterpret_cast<uintptr_t>(p) % align != 0) return nullptr;
+    cudaPointerAttributes at, end;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess || cudaPointerGetAttributes(&end, static_cast<const char*>(p) + bytes - 1) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    if (at.type != cudaMemoryTypeHost || end.type != cudaMemoryTypeHost || !at.devicePointer || !end.devicePointer ||
+        static_cast<char*>(end.devicePointer) - static_cast<char*>(at.devicePointer) != (ptrdiff_t)(bytes - 1))
+        return nullptr;
+    return at.devicePointer;
+}
+
+// The groups of the arrays given (null: left out), each in place or in the staging buffer: src[g] is the
+// caller's array of a staged group, its bytes size[g].
+template <class R> template <class T>
+typename World<R>::template Xfer<T> World<R>::xfer_groups(T* const* arrays) {
+    static const int k0[7] = {OX, B00, VX, WX, MNX, MXX, I00}, nk[7] = {3, 9, 3, 3, 3, 3, 9};
+    Xfer<T> x;
+    size_t tot = 0, off[7];
+    for (int g = 0; g < 7; g++) {
+        if (!arrays[g]) continue;
+        const int n = x.G.n++;
+        x.at[g] = n;
+        x.G.k0[n] = k0[g]; x.G.nk[n] = nk[g];
+        x.size[n] = (size_t)nk[g] * N_ * sizeof(T);
+        x.G.ptr[n] = static_cast<T*>(direct_address(arrays[g], x.size[n], sizeof(T)));
+        x.staged[n] = x.G.ptr[n] ? nullptr : arrays[g];
+        off[n] = tot;
+        if (x.staged[n]) tot += (size_t)nk[g] * N_;
+        x.widest = std::max(x.widest, nk[g]);
+    }
+    if (tot) xfer_.ensure((tot * sizeof(T) + sizeof(double) - 1) / sizeof(double));
+    for (int n = 0; n < x.G.n; n++)
+        if (x.staged[n]) x.G.ptr[n] = reinterpret_cast<T*>(xfer_.p) + off[n];
+    return x;
+}
+
 template <class R> template <class T>
 void World<R>::get_state_t(T* o, T* b, T* v, T* w, T* mn, T* mx, T* iw) {
-    T* dst[7] = {o, b, v, w, mn, mx, iw};
-    const int k0[7] = {OX, B00, VX, WX, MNX, MXX, I00}, nk[7] = {3, 9, 3, 3, 3, 3, 9};
-    XferGroups G{};
-    size_t tot = 0;
-    int map[7];
-    for (int g = 0; g < 7; g++) {
-        if (!dst[g]) continue;
-        map[G.n] = g;
-        G.k0[G.n] = k0[g]; G.nk[G.n] = nk[g]; G.off[G.n] = tot;
-        tot += (size_t)nk[g] * N_;
-        G.n++;
-    }
-    if (!N_ || !G.n) return;
-    xfer_.ensure((tot * sizeof(T) + sizeof(double) - 1) / sizeof(double));
-    T* x = reinterpret_cast<T*>(xfer_.p);
-    launch(K_MISC, grid(N_), k_state_pack<R, T>, bodies(), G, x);
-    for (int q = 0; q < G.n; q++)
-        PE_CK(cudaMemcpyAsync(dst[map[q]], x + G.off[q], (size_t)G.nk[q] * N_ * sizeof(T), cudaMemcpyDeviceToHost, st_));
+    T* const dst[7] = {o, b, v, w, mn, mx, iw};
+    if (!N_) return;
+    const Xfer<T> x = xfer_groups(dst);
+    if (!x.G.n) return;
+    launch(K_MISC, dim3(grid(N_ * (long long)x.widest), x.G.n), k_state_pack<R, T>, bodies(), x.G);
+    for (int n = 0; n < x.G.n; n++)
+        if (x.staged[n]) PE_CK(cudaMemcpyAsync(x.staged[n], x.G.ptr[n], x.size[n], cudaMemcpyDeviceToHost, st_));
     PE_CK(cudaStreamSynchronize(st_));
 }
 
 template <class R> template <class T>
 void World<R>::set_state_t(const T* o, const T* b, const T* v, const T* w, const T* mn, const T* mx, const T* iw) {
-    const T* src[7] = {o, b, v, w, mn, mx, iw};
-    const int k0[7] = {OX, B00, VX, WX, MNX, MXX, I00}, nk[7] = {3, 9, 3, 3, 3, 3, 9};
-    XferGroups G{};
-    size_t tot = 0;
-    int at[7] = {-1, -1, -1, -1, -1, -1, -1};
-    for (int g = 0; g < 7; g++) {
-        if (!src[g]) continue;
-        at[g] = G.n;
-        G.k0[G.n] = k0[g]; G.nk[G.n] = nk[g]; G.off[G.n] = tot;
-        tot += (size_t)nk[g] * N_;
-        G.n++;
-    }
-    if (!N_ || !G.n) return;
-    xfer_.ensure((tot * sizeof(T) + sizeof(double) - 1) / sizeof(double));
-    T* x = reinterpret_cast<T*>(xfer_.p);
-    for (int g = 0; g < 7; g++)
-        if (src[g])
-            PE_CK(cudaMemcpyAsync(x + G.off[at[g]], src[g], (size_t)nk[g] * N_ * sizeof(T), cudaMemcpyHostToDevice, st_));
+    T* const src[7] = {const_cast<T*>(o), const_cast<T*>(b), const_cast<T*>(v), const_cast<T*>(w), const_cast<T*>(mn),
+                       const_cast<T*>(mx), const_cast<T*>(iw)};   // only read
+    if (!N_) return;
+    const Xfer<T> x = xfer_groups(src);
+    if (!x.G.n) return;
+    for (int n = 0; n < x.G.n; n++)
+        if (x.staged[n]) PE_CK(cudaMemcpyAsync(x.G.ptr[n], x.staged[n], x.size[n], cudaMemcpyHostToDevice, st_));
     const bool scale = mn && mx && o;   // the injected box's AABB scale
-    launch(K_MISC, grid(N_), k_state_unpack<R, T>, bodies(), G, (const T*)x, scale ? at[0] : -1, scale ? at[4] : -1,
-           scale ? at[5] : -1);
+    launch(K_MISC, dim3(grid(N_ * (long long)x.widest), x.G.n), k_state_unpack<R, T>, bodies(), x.G, scale ? x.at[0] : -1,
+           scale ? x.at[4] : -1, scale ? x.at[5] : -1);
     PE_CK(cudaStreamSynchronize(st_));
 }
 
