@@ -323,6 +323,10 @@ private:
     int* hstat_ = nullptr;
     int h_cls_[PC_COUNT] = {};   // the last step's pair-class counts (the side-stream plan)
     int stream_of_[PC_COUNT] = {};
+    // what the shape tables hold: kinds (bit per ShapeType), and the most faces, edges and vertices of a hull
+    unsigned kinds_ = 0;
+    int most_faces_ = 0, most_edges_ = 0, most_verts_ = 0;
+    unsigned possible_classes() const;
     void plan_streams(int* plan) const;
     int bp_count();                 // integrate's successor up to the pair count (waits for it)
     void bp_count_enqueue();        // its launches, ending with the count's copy to the host
@@ -362,6 +366,7 @@ private:
         unsigned long long gen;
         const void* order;
         int n, ns, pair_cap, nj, n_ign, s, side;
+        unsigned classes;
         int plan[PC_COUNT];
         StepParams prm;
         R margin;

@@ -128,6 +128,8 @@ void World<R>::set_shapes(int S, const int* type, const double* param, const int
                           const int* fcnt, int HV, const double* hv, int HF, const int* foff, const int* fidx) {
     (void)HV; (void)HF;
     S_ = 0;
+    kinds_ = 0;
+    most_faces_ = most_edges_ = most_verts_ = 0;
     h_stype_.clear(); h_sparam_.clear(); h_sinertia_.clear(); h_shull_.clear();
     h_hvb_.clear(); h_hvc_.clear(); h_hfb_.clear(); h_hfc_.clear(); h_heb_.clear(); h_hec_.clear(); h_foff_.clear(); h_fidx_.clear();
     h_hv_.clear(); h_fn_.clear(); h_fmn_.clear(); h_fmx_.clear(); h_ea_.clear(); h_eb_.clear(); h_hrad_.clear();
@@ -229,6 +231,12 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
     // hull face offsets are global per face: face f of hull h sits at hfb[h] + f, its offsets at
     // f_off[hfb[h] + f] .. f_off[hfb[h] + f + 1]
     S_ = s0 + added;
+    for (size_t s = s0; s < h_stype_.size(); s++) kinds_ |= 1u << h_stype_[s];
+    for (size_t h = o_h; h < h_hvc_.size(); h++) {
+        most_faces_ = std::max(most_faces_, h_hfc_[h]);
+        most_edges_ = std::max(most_edges_, h_hec_[h]);
+        most_verts_ = std::max(most_verts_, h_hvc_[h]);
+    }
     shape_by_content_.merge(fresh);
     // a request whose shapes are all known already (each one's primitives were appended again, five
     // uploads, a launch and two waits per request)

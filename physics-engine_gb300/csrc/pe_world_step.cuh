@@ -218,6 +218,27 @@ template <class R> void World<R>::plan_streams(int* plan) const {
     }
 }
 
+// The pair classes (bit per class) that pairs of the tables' shapes can have (k_np_classify).  The others'
+// kernels, up to 17 of 20, are not launched: each is a node of some 2 us in one of four chains.
+template <class R> unsigned World<R>::possible_classes() const {
+    static_assert(kCylF <= kSatF && kCylE <= kSatE && kBoxE <= kSatE, "boxes and cylinders fit the staged SAT");
+    auto has = [&](int t) { return (kinds_ >> t & 1u) != 0; };
+    unsigned m = 0;
+    for (int a = 0; a < 32; a++)
+        for (int b = 0; b <= a; b++)
+            if (has(a) && has(b)) m |= 1u << pair_class(a, b);
+    if (!(m >> PC_CONVEX & 1u)) return m;
+    const bool hull = has(ST_HULL);
+    if (!(hull && has(ST_BOX))) m &= ~(1u << PC_CONVEX);
+    else m |= 1u << PC_CONVEX_HULL_BOX;
+    if (hull) m |= 1u << PC_CONVEX_HULL_HULL;
+    if (has(ST_CYLINDER)) m |= 1u << PC_CONVEX_CYL_CYL;
+    if (most_faces_ > kSatF || most_edges_ > kSatE || most_verts_ > kSatV) m |= 1u << PC_CONVEX_BIG;
+    const long long f = std::max(most_faces_, kCylF), e = std::max(most_edges_, kCylE), v = std::max(most_verts_, 12);
+    if ((2 * f + e * e) * (2 * v) >= tun_.sat_heavy_cost) m |= 1u << PC_CONVEX_HEAVY;
+    return m;
+}
+
 // Narrowphase without host waits: pairs classified and bucketed by class on the device, the class
 // ranges computed there, and every class's kernel launched over its range (grids from the pair
 // capacity, persistent up to the resident blocks), side by side on the side streams.
@@ -243,7 +264,9 @@ template <class R> void World<R>::np_enqueue() {
     // The classes' kernels touch disjoint pairs and results: they run side by side on the side
     // streams, so the long tails of the per-pair kernels overlap the other classes.
     fork_streams();
+    const unsigned possible = possible_classes();
     for (int c = 0; c < PC_COUNT; c++) {
+        if (!(possible >> c & 1u)) continue;
         use_stream(stream_of_[c] % tun_.side_streams);
         const int2* rg = cls_rng_.p + c;
         int* wk = cls_work_.p + c;
@@ -412,6 +435,7 @@ template <class R> void World<R>::graph_sig(GraphSig& g) const {
     g.gen = dbuf_generation().load();
     g.order = order_;
     g.n = N_; g.ns = NS_; g.pair_cap = pair_cap_; g.nj = n_joints_; g.n_ign = n_ign_; g.s = S_;
+    g.classes = possible_classes();
     g.side = bcap_ * 4 + (max_scene_ > kBigWindow ? 1 : 0);
     std::memcpy(g.plan, stream_of_, sizeof g.plan);
     std::memcpy(&g.prm, &prm_, sizeof prm_);
