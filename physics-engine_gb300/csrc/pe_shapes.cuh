@@ -13,23 +13,42 @@ namespace pe {
 
 enum ShapeType { ST_BOX = 0, ST_SPHERE = 1, ST_CYLINDER = 2, ST_HULL = 3, ST_CONCAVE = 4, ST_COMPOUND = 5 };
 
-// unit meshes (host builds them; device reads them from constant memory)
+// unit meshes (host builds them in double precision; the device reads them in the world's real type)
 constexpr int kBoxV = 24, kBoxF = 6, kBoxE = 12;
 constexpr int kCylV = 80, kCylF = 42, kCylE = 80, kCylFIdx = 20 + 20 + 40 * 3;
-struct UnitMeshes {
-    double box_v[kBoxV][3];
-    double box_n[kBoxF][3];
-    double box_e[kBoxE][6];
-    double cyl_v[kCylV][3];
-    double cyl_n[kCylF][3];
+template <class R> struct UnitMeshesOf {
+    R box_v[kBoxV][3];
+    R box_n[kBoxF][3];
+    R box_e[kBoxE][6];
+    R cyl_v[kCylV][3];
+    R cyl_n[kCylF][3];
     int cyl_foff[kCylF + 1];
     int cyl_fidx[kCylFIdx];
     int cyl_e[kCylE][2];   // unique edges as vertex index pairs
 };
+struct UnitMeshes : UnitMeshesOf<double> {};
 
 #ifdef __CUDACC__
-// one copy per translation unit; each world implementation uploads its own at creation
-static __constant__ UnitMeshes g_unit;
+// One copy per translation unit and real type; each world uploads its own at creation.  In global
+// memory: the lanes of a warp read different edges and faces, which constant memory serves one after
+// the other, and a float world converted every value from double, on a pipe that takes two lanes a clock.
+static __device__ UnitMeshesOf<float> g_unit_f32;
+static __device__ UnitMeshesOf<double> g_unit_f64;
+template <class R> __device__ __forceinline__ const UnitMeshesOf<R>& unit_meshes() {
+    if constexpr (sizeof(R) == 4) return g_unit_f32;
+    else return g_unit_f64;
+}
+inline void round_unit_meshes(const UnitMeshes& u, UnitMeshesOf<float>& o) {
+    auto all = [](const auto& from, auto& to) {
+        for (size_t i = 0; i < sizeof(from) / sizeof(from[0]); i++)
+            for (size_t k = 0; k < sizeof(from[0]) / sizeof(from[0][0]); k++)
+                to[i][k] = static_cast<std::remove_reference_t<decltype(to[0][0])>>(from[i][k]);
+    };
+    all(u.box_v, o.box_v); all(u.box_n, o.box_n); all(u.box_e, o.box_e);
+    all(u.cyl_v, o.cyl_v); all(u.cyl_n, o.cyl_n); all(u.cyl_e, o.cyl_e);
+    for (int k = 0; k <= kCylF; k++) o.cyl_foff[k] = u.cyl_foff[k];
+    for (int k = 0; k < kCylFIdx; k++) o.cyl_fidx[k] = u.cyl_fidx[k];
+}
 #endif
 
 // device view of one shape
@@ -64,35 +83,35 @@ template <class R> struct ShapeView {
     __device__ int edge_count() const { return type == ST_BOX ? kBoxE : (type == ST_CYLINDER ? kCylE : ne); }
     __device__ int vert_count() const { return type == ST_BOX ? kBoxV : (type == ST_CYLINDER ? kCylV : nv); }
     __device__ V3<R> vert(int i) const {
-        if (type == ST_BOX) return cmul(V3<R>(R(g_unit.box_v[i][0]), R(g_unit.box_v[i][1]), R(g_unit.box_v[i][2])), size);
+        if (type == ST_BOX) return cmul(V3<R>(unit_meshes<R>().box_v[i][0], unit_meshes<R>().box_v[i][1], unit_meshes<R>().box_v[i][2]), size);
         if (type == ST_CYLINDER)
-            return V3<R>(R(g_unit.cyl_v[i][0]) * r2, R(g_unit.cyl_v[i][1]) * height, R(g_unit.cyl_v[i][2]) * r2);
+            return V3<R>(unit_meshes<R>().cyl_v[i][0] * r2, unit_meshes<R>().cyl_v[i][1] * height, unit_meshes<R>().cyl_v[i][2] * r2);
         return V3<R>(hv[i * 3], hv[i * 3 + 1], hv[i * 3 + 2]);
     }
     __device__ int face_size(int f) const {
         if (type == ST_BOX) return 4;
-        if (type == ST_CYLINDER) return g_unit.cyl_foff[f + 1] - g_unit.cyl_foff[f];
+        if (type == ST_CYLINDER) return unit_meshes<R>().cyl_foff[f + 1] - unit_meshes<R>().cyl_foff[f];
         return f_off[f + 1] - f_off[f];
     }
     __device__ int face_vert(int f, int k) const {
         if (type == ST_BOX) return f * 4 + k;
-        if (type == ST_CYLINDER) return g_unit.cyl_fidx[g_unit.cyl_foff[f] + k];
+        if (type == ST_CYLINDER) return unit_meshes<R>().cyl_fidx[unit_meshes<R>().cyl_foff[f] + k];
         return f_idx[f_off[f] + k];
     }
     __device__ V3<R> face_normal(int f) const {
-        if (type == ST_BOX) return V3<R>(R(g_unit.box_n[f][0]), R(g_unit.box_n[f][1]), R(g_unit.box_n[f][2]));
-        if (type == ST_CYLINDER) return V3<R>(R(g_unit.cyl_n[f][0]), R(g_unit.cyl_n[f][1]), R(g_unit.cyl_n[f][2]));
+        if (type == ST_BOX) return V3<R>(unit_meshes<R>().box_n[f][0], unit_meshes<R>().box_n[f][1], unit_meshes<R>().box_n[f][2]);
+        if (type == ST_CYLINDER) return V3<R>(unit_meshes<R>().cyl_n[f][0], unit_meshes<R>().cyl_n[f][1], unit_meshes<R>().cyl_n[f][2]);
         return V3<R>(f_n[f * 3], f_n[f * 3 + 1], f_n[f * 3 + 2]);
     }
     // unit direction of hull edge e: normalized(a - b) of edge(e, a, b), as stored by k_hull_edge_dirs
     __device__ V3<R> edge_dir(int e) const { return V3<R>(e_d[e * 3], e_d[e * 3 + 1], e_d[e * 3 + 2]); }
     __device__ void edge(int e, V3<R>& a, V3<R>& b) const {
         if (type == ST_BOX) {
-            a = cmul(V3<R>(R(g_unit.box_e[e][0]), R(g_unit.box_e[e][1]), R(g_unit.box_e[e][2])), size);
-            b = cmul(V3<R>(R(g_unit.box_e[e][3]), R(g_unit.box_e[e][4]), R(g_unit.box_e[e][5])), size);
+            a = cmul(V3<R>(unit_meshes<R>().box_e[e][0], unit_meshes<R>().box_e[e][1], unit_meshes<R>().box_e[e][2]), size);
+            b = cmul(V3<R>(unit_meshes<R>().box_e[e][3], unit_meshes<R>().box_e[e][4], unit_meshes<R>().box_e[e][5]), size);
         } else if (type == ST_CYLINDER) {
-            a = vert(g_unit.cyl_e[e][0]);
-            b = vert(g_unit.cyl_e[e][1]);
+            a = vert(unit_meshes<R>().cyl_e[e][0]);
+            b = vert(unit_meshes<R>().cyl_e[e][1]);
         } else {
             a = V3<R>(e_a[e * 3], e_a[e * 3 + 1], e_a[e * 3 + 2]);
             b = V3<R>(e_b[e * 3], e_b[e * 3 + 1], e_b[e * 3 + 2]);

@@ -20,7 +20,13 @@ template <class R> World<R>::World(int device) : dev_(device) {
     UnitMeshes u;
     std::memset(&u, 0, sizeof(u));
     build_unit_meshes(u);
-    PE_CK(cudaMemcpyToSymbol(g_unit, &u, sizeof(u)));
+    if constexpr (sizeof(R) == 4) {
+        UnitMeshesOf<float> f;
+        round_unit_meshes(u, f);
+        PE_CK(cudaMemcpyToSymbol(g_unit_f32, &f, sizeof f));
+    } else {
+        PE_CK(cudaMemcpyToSymbol(g_unit_f64, &u, sizeof(UnitMeshesOf<double>)));
+    }
     status_.ensure(1);
     PE_CK(cudaMemset(status_.p, 0, sizeof(int)));
     rows_total_.ensure(1);
