@@ -1009,30 +1009,36 @@ template <class R, class C> __device__ bool cylinder_hull(Pair<R, C>& c) {   // 
 // face order, its normal, no unique edges: setMesh is never called on it) that the convex-convex
 // algorithm meets with the convex shape first, at the concave body's transform.
 constexpr int kFaceVerts = 32;   // longest face polygon a concave mesh may hold (checked at upload)
+template <class R> struct FaceBuf { R v[kFaceVerts * 3], n[3], mn[3], mx[3]; int idx[kFaceVerts], off[2]; };
+// the pair that face f of the mesh cc makes with the convex shape cv
 template <class R, class C>
-__device__ void concave_face(Pair<R, C>& c, const ShapeView<R>& cc, const ShapeView<R>& cv, const Xf<R>& tcc, const Xf<R>& tcv, int f) {
-    R fv[kFaceVerts * 3];
-    int fidx[kFaceVerts];
-    R fn[3], fmn[3], fmx[3];
+__device__ Pair<R, C> face_pair(const Pair<R, C>& c, const ShapeView<R>& cc, const ShapeView<R>& cv, const Xf<R>& tcc, const Xf<R>& tcv, int f,
+                                FaceBuf<R>& b) {
     const int n = cc.face_size(f);
-    const int foff[2] = {0, n};
-    for (int k = 0; k < 3; k++) { fmn[k] = Lim<R>::max(); fmx[k] = Lim<R>::min(); }
+    b.off[0] = 0; b.off[1] = n;
+    for (int k = 0; k < 3; k++) { b.mn[k] = Lim<R>::max(); b.mx[k] = Lim<R>::min(); }
     for (int i = 0; i < n; i++) {
         const V3<R> p = cc.vert(cc.face_vert(f, i));
-        fv[i * 3] = p.x; fv[i * 3 + 1] = p.y; fv[i * 3 + 2] = p.z;
-        fidx[i] = i;
-        for (int k = 0; k < 3; k++) { fmn[k] = fmn[k] < p[k] ? fmn[k] : p[k]; fmx[k] = fmx[k] > p[k] ? fmx[k] : p[k]; }
+        b.v[i * 3] = p.x; b.v[i * 3 + 1] = p.y; b.v[i * 3 + 2] = p.z;
+        b.idx[i] = i;
+        for (int k = 0; k < 3; k++) { b.mn[k] = b.mn[k] < p[k] ? b.mn[k] : p[k]; b.mx[k] = b.mx[k] > p[k] ? b.mx[k] : p[k]; }
     }
     const V3<R> nrm = cc.face_normal(f);
-    fn[0] = nrm.x; fn[1] = nrm.y; fn[2] = nrm.z;
+    b.n[0] = nrm.x; b.n[1] = nrm.y; b.n[2] = nrm.z;
     ShapeView<R> face = cc;
     face.type = ST_HULL;
-    face.hv = fv; face.nv = n;
-    face.f_off = foff; face.f_idx = fidx; face.f_n = fn; face.f_min = fmn; face.f_max = fmx; face.nf = 1;
+    face.hv = b.v; face.nv = n;
+    face.f_off = b.off; face.f_idx = b.idx; face.f_n = b.n; face.f_min = b.mn; face.f_max = b.mx; face.nf = 1;
     face.e_a = nullptr; face.e_b = nullptr; face.e_d = nullptr; face.ne = 0;
     face.nl = 0;
     Pair<R, C> s = c;
     s.sa = cv; s.sb = face; s.xa = tcv; s.xb = tcc;
+    return s;
+}
+template <class R, class C>
+__device__ void concave_face(Pair<R, C>& c, const ShapeView<R>& cc, const ShapeView<R>& cv, const Xf<R>& tcc, const Xf<R>& tcv, int f) {
+    FaceBuf<R> b;
+    Pair<R, C> s = face_pair(c, cc, cv, tcc, tcv, f, b);
     convex_convex(s);
 }
 

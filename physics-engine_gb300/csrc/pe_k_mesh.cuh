@@ -24,8 +24,9 @@ constexpr int kMeshPoints = 12, kMeshQueue = 64;
 struct MeshPiece {
     int i, j;      // child of A, of B; -1: the shape itself
     int face;      // kPieceWhole: the whole pair of shapes; kPieceEnd: a mesh's faces are done
-    int pass;      // cylinder against a face: 0 sides, 1 edges
+    int pass;      // cylinder against a face: 0 sides, 1 edges; kPassHull: a hull against a face
 };
+constexpr int kPassHull = 2;
 constexpr int kPieceWhole = -1, kPieceEnd = -2;
 
 // the mesh's face f against the convex shape on the other side; `c` names the pair's shapes in order
@@ -67,6 +68,35 @@ template <class R, class C> __device__ __noinline__ void mesh_piece(const MeshPi
     if (q.face == kPieceWhole) collide(c, pair_class(c.sa.type, c.sb.type));
     else mesh_face(c, q.face, q.pass);
 }
+// A mesh's face against a hull is the work of up to 128 axes, each projecting every vertex: by one lane,
+// hundreds of microseconds.  The lanes first hold a face each against its own normal, which most faces
+// near a hull are apart along (an axis that separates ends the reference's test, and nothing has been
+// added before the edge axes, which a face has none of); the faces left meet the hull by the whole warp,
+// one after the other in their turn.
+template <class R, class F> __device__ __forceinline__ void mesh_hull_pair(const MeshPiece& q, const Pair<R>& pr, const ShapeTable<R>& S, Cache<R>* cache, F&& f) {
+    Pair<R> c;
+    mesh_place(pr, S, q.i, q.j, cache, c);
+    const bool a_mesh = c.sa.type == ST_CONCAVE;
+    FaceBuf<R> b;
+    Pair<R> s = face_pair(c, a_mesh ? c.sa : c.sb, a_mesh ? c.sb : c.sa, a_mesh ? c.xa : c.xb, a_mesh ? c.xb : c.xa, q.face, b);
+    f(s, a_mesh);
+}
+template <class R> __device__ __noinline__ bool mesh_hull_near(const MeshPiece& q, const Pair<R>& pr, const ShapeTable<R>& S, Cache<R>* cache) {
+    bool near = true;
+    mesh_hull_pair(q, pr, S, cache, [&](Pair<R>& s, bool) {
+        V3<R> n = mv(s.tb().b, s.sb.face_normal(0)), wa, wb;
+        if (dot(s.ta().o - s.tb().o, n) < 0) n = n * R(-1.0);
+        R d;
+        near = sep_test(s, n, d, wa, wb);
+    });
+    return near;
+}
+template <class R> __device__ __noinline__ void mesh_hull_face(const MeshPiece& q, const Pair<R>& pr, const ShapeTable<R>& S, Cache<R>* cache, int lane) {
+    mesh_hull_pair(q, pr, S, cache, [&](Pair<R>& s, bool a_mesh) {
+        if (lane == 0) cache->swap = a_mesh;
+        sat_warp(s, lane);
+    });
+}
 template <class R> __device__ __noinline__ void mesh_sat(const Pair<R>& pr, const ShapeTable<R>& S, int i, int j, Cache<R>* cache, int lane) {
     Pair<R> c;
     mesh_place(pr, S, i, j, cache, c);
@@ -102,18 +132,32 @@ k_np_mesh(const int2* rng, int* cursor, const int* order, const int2* pairs, Bod
         int qn = 0;   // queued pieces
         auto flush = [&](int n) {   // runs the first n (at most 32) queued pieces
             __syncwarp();
+            bool by_warp = false;
             if (lane < n) {
-                Recorder<R> r{rec[lane], 0, kMeshPoints, Recorder<R>::kSwapInherit};
-                mesh_piece(queue[lane], pr, S, &r);
-                rec_n[lane] = r.n;
-                rec_swap[lane] = r.swap;
-            }
-            __syncwarp();
-            if (lane == 0)
-                for (int l = 0; l < n; l++) {
-                    if (rec_n[l] > kMeshPoints) mesh_piece(queue[l], pr, S, &cache);
-                    else Recorder<R>{rec[l], rec_n[l], kMeshPoints, rec_swap[l]}.replay(cache);
+                if (queue[lane].pass == kPassHull) {
+                    by_warp = mesh_hull_near(queue[lane], pr, S, &cache);
+                    rec_n[lane] = 0;
+                    rec_swap[lane] = Recorder<R>::kSwapInherit;
+                } else {
+                    Recorder<R> r{rec[lane], 0, kMeshPoints, Recorder<R>::kSwapInherit};
+                    mesh_piece(queue[lane], pr, S, &r);
+                    rec_n[lane] = r.n;
+                    rec_swap[lane] = r.swap;
                 }
+            }
+            unsigned whole = __ballot_sync(full, by_warp);
+            for (int l = 0; l < n;) {
+                const int stop = whole ? __ffs(whole) - 1 : n;
+                if (lane == 0)
+                    for (; l < stop; l++) {
+                        if (rec_n[l] > kMeshPoints) mesh_piece(queue[l], pr, S, &cache);
+                        else Recorder<R>{rec[l], rec_n[l], kMeshPoints, rec_swap[l]}.replay(cache);
+                    }
+                __syncwarp();
+                if (stop < n) mesh_hull_face(queue[stop], pr, S, &cache, lane);
+                whole &= whole - 1;
+                l = stop + 1;
+            }
             __syncwarp();
             if (lane < qn - n) queue[lane] = queue[n + lane];   // at most 31 stay
             qn -= n;
@@ -153,22 +197,30 @@ k_np_mesh(const int2* rng, int* cursor, const int* order, const int2* pairs, Bod
             } else {
                 shape_aabb(o, tm.inverse() * to, aa, bb);
             }
-            const int passes = o.type == ST_CYLINDER ? 2 : 1;
+            const int passes = o.type == ST_CYLINDER ? 2 : 1, hull = o.type == ST_HULL ? kPassHull : 0;
             // mesh_query: leaves in descending order, the faces of an overlapping leaf ascending
+            // (four rounds of 32 leaves at a time, their boxes loaded first: 16 rounds of the 512 leaves of a
+            // 4,608-triangle terrain, once per child and pass, each waited for memory otherwise)
+            constexpr int U = 4;
             for (int pass = 0; pass < passes; pass++)
-                for (int l0 = m.nl - 1; l0 >= 0; l0 -= 32) {
-                    const int l = l0 - lane;
-                    bool hit = false;
-                    if (l >= 0) {
-                        const R* mn = m.l_min + l * 3;
-                        const R* mx = m.l_max + l * 3;
-                        hit = !(mn[0] > bb.x || mn[1] > bb.y || mn[2] > bb.z) && !(mx[0] < aa.x || mx[1] < aa.y || mx[2] < aa.z);
+                for (int l0 = m.nl - 1; l0 >= 0; l0 -= 32 * U) {
+                    unsigned hit = 0;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int l = l0 - 32 * u - lane, k = l >= 0 ? l : 0;
+                        const R* mn = m.l_min + k * 3;
+                        const R* mx = m.l_max + k * 3;
+                        const V3<R> lo(mn[0], mn[1], mn[2]), hi(mx[0], mx[1], mx[2]);
+                        if (l >= 0 && !(lo.x > bb.x || lo.y > bb.y || lo.z > bb.z) && !(hi.x < aa.x || hi.y < aa.y || hi.z < aa.z)) hit |= 1u << u;
                     }
-                    for (unsigned hits = __ballot_sync(full, hit); hits; hits &= hits - 1) {
-                        const int leaf = l0 - (__ffs(hits) - 1), first = m.l_beg[leaf], cnt = m.l_cnt[leaf];
-                        for (int f0 = 0; f0 < cnt; f0 += 32)
-                            push(f0 + lane < cnt, lane, min(32, cnt - f0), MeshPiece{i, j, first + f0 + lane, pass});
-                    }
+                    if (!__any_sync(full, hit)) continue;
+#pragma unroll 1
+                    for (int u = 0; u < U; u++)
+                        for (unsigned hits = __ballot_sync(full, hit >> u & 1u); hits; hits &= hits - 1) {
+                            const int leaf = l0 - 32 * u - (__ffs(hits) - 1), first = m.l_beg[leaf], cnt = m.l_cnt[leaf];
+                            for (int f0 = 0; f0 < cnt; f0 += 32)
+                                push(f0 + lane < cnt, lane, min(32, cnt - f0), MeshPiece{i, j, first + f0 + lane, pass + hull});
+                        }
                 }
             push(lane == 0, 0, 1, MeshPiece{i, j, kPieceEnd, 0});
         };
