@@ -37,6 +37,8 @@ struct IslandArgs {
 //   k_isl_keys                 labels; then the radix sort
 //   k_head_sums, k_head_apply  islands of the sorted items
 //   k_isl_classes              their size classes
+constexpr int kActItems = 2, kActTile = kBlock * kActItems;   // small tiles: a thread's unions are a chain (8 of them took 34 us for 6,500 results)
+inline int act_tiles(long long n) { return (int)((n + kActTile - 1) / kActTile); }
 constexpr int kIslandOne = 2048, kIslandBlock = 1024, kIslandOneBodies = 8192;
 inline size_t island_one_smem(int n_bodies) {   // sorted keys and values, island offsets, digit counters, union-find
     return (size_t)(3 * kIslandOne + 2) * 4 + (size_t)(kIslandBlock / 32) * 256 * 2 + (size_t)n_bodies * 4;

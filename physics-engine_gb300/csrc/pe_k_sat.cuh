@@ -271,10 +271,11 @@ template <class R> __device__ __forceinline__ V3<R> so_get3(const R* o, int k) {
 // group layout in shared memory: both edge lists (the face axes before them), both shapes' vertices, the supporting points, the
 // queues (one per warp), the scratch
 constexpr int kSatFree = 64, kSatBlock = 512;   // see sat_staged's balls
+constexpr int kCertain = 5;      // the first shape's first vertices, turned into the world (see sat_staged's certain)
 constexpr int kSatQueue = 64;    // queued axes per warp: a round's 32 and what the next 32 candidates can add
 template <class R> constexpr int sat_group_reals(int G) {
     const int q = (kSatQueue * G * (int)sizeof(int) + (int)sizeof(R) - 1) / (int)sizeof(R);
-    return (4 * 2 * kSatE + 4 * 2 * kSatV + 2 * kSatBase + q + sat_scratch_reals<R>(G) + 3) & ~3;
+    return (4 * 2 * kSatE + 4 * 2 * kSatV + 2 * kSatBase + 4 * kCertain + q + sat_scratch_reals<R>(G) + 3) & ~3;
 }
 
 // Staged SAT of one pair by a group of G warps (tid in [0, 32 G)).
@@ -293,7 +294,8 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
     R* vB = vA + 4 * kSatV;
     R* subA = vB + 4 * kSatV;
     R* subB = subA + kSatBase;
-    int* queue = reinterpret_cast<int*>(subB + kSatBase) + warp * kSatQueue;
+    R* cerA = subB + kSatBase;
+    int* queue = reinterpret_cast<int*>(cerA + 4 * kCertain) + warp * kSatQueue;
     R* rd = smem + sat_group_reals<R>(G) - ((sat_scratch_reals<R>(G) + 3) & ~3);
     int* ri = reinterpret_cast<int*>(rd + G);
     R* bc = rd + 2 * G;
@@ -341,6 +343,7 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
         else if (boxA && !boxB) dir = -from_box(c.sa, c.ta(), c.tb().o);
         if (G == 1 || warp == 0) if (c.sa.type == ST_HULL) sat_pick(c.sa, c.ta().b, vA, mtv(c.ta().b, -dir), 0, R(-1), subA, lane);
         if (G == 1 || warp == 0) if (c.sb.type == ST_HULL) sat_pick(c.sb, c.tb().b, vB, mtv(c.tb().b, dir), c.sb.nv > 2 ? 2 : 0, R(1), subB, lane);
+        if (c.sa.type == ST_HULL && tid < kCertain) stv(cerA, tid, mv(c.ta().b, ldv(vA, min(tid, c.sa.nv - 1))));
     }
     // everything that enters a projection, in units of roundoff: the bounds' and the projections' errors
     const R slack = sat_slack<R>() * (norm(c.ta().o) + norm(c.tb().o) + qa.mag + qb.mag);
@@ -356,21 +359,22 @@ __device__ void sat_staged(Pair<R>& c, int tid, R* smem, R* out) {
     // the first shape passes over the vertices of its first falling run, so its maximum may lie below
     // the inner ball's.  Among the first kCertain vertices, one that certainly lies above an earlier
     // one is never passed over; an axis is skipped only if such a vertex keeps the other depth above pb,
-    // or if the run ends with vertex 0, which the inner ball leaves out.
-    constexpr int kCertain = 8;
+    // or if the run ends with vertex 0, which the inner ball leaves out.  (One axis in a hundred has a
+    // longer run and is projected; a loop over eight vertices cost the longest pair of a 501-body pile 50 us.)
     auto certain = [&](const V3<R>& y, R ny, R pb) {
         if (c.sa.type != ST_HULL) return true;
-        const V3<R> yl = mtv(c.ta().b, y);
         const R tol = R(2) * slack * ny, need = ny * (pb - qb.inner) - fma3(y, dc) + tol;
-        const int n = min(c.sa.nv, kCertain);
-        R low = fma3(yl, ldv(vA, 0));
-#pragma unroll 1
-        for (int i = 1; i < n; i++) {   // (most axes end at the first or second)
-            const R u = fma3(yl, ldv(vA, i));
-            if (u > low + tol && (i == 1 || u > need)) return true;   // the inner ball leaves out vertex 0 only
-            low = low < u ? low : u;
+        R u[kCertain];
+#pragma unroll
+        for (int i = 0; i < kCertain; i++) u[i] = fma3(y, ldv(cerA, i));
+        bool ok = u[1] > u[0] + tol;
+        R low = u[0] < u[1] ? u[0] : u[1];
+#pragma unroll
+        for (int i = 2; i < kCertain; i++) {
+            ok = ok || (u[i] > low + tol && u[i] > need);
+            low = low < u[i] ? low : u[i];
         }
-        return false;
+        return ok;
     };
     auto pruned = [&](const V3<R>& y, R ny, R pb) { return able && pb < deep && bound(y, ny) > ny * (pb + slack) && certain(y, ny, pb); };
     // The inner balls' bound of the same depth.  It alone also decides which axes of a hull count: the

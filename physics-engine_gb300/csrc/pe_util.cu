@@ -244,11 +244,11 @@ __global__ void __launch_bounds__(kBlock) k_act_sums(IslandArgs a) {
     for (int k = t; k < a.N; k += gridDim.x * kBlock) a.parent[k] = k;
     if (t < kWarpClasses + 2) a.n_list[t] = 0;
     if (t == 0 && a.n_colors) *a.n_colors = 0;
-    for (int tile = blockIdx.x; tile * kScanTile < P; tile += gridDim.x) {   // a block's tiles one after the other
+    for (int tile = blockIdx.x; tile * kActTile < P; tile += gridDim.x) {   // a block's tiles one after the other
         unsigned long long s = 0, all;
 #pragma unroll
-        for (int k = 0; k < kScanItems; k++) {
-            const int p = tile * kScanTile + k * kBlock + threadIdx.x;
+        for (int k = 0; k < kActItems; k++) {
+            const int p = tile * kActTile + k * kBlock + threadIdx.x;
             s += p < P ? act_value(a.npts[p]) : 0ull;
         }
         block_excl_scan<kBlock>(s, &all);
@@ -257,20 +257,20 @@ __global__ void __launch_bounds__(kBlock) k_act_sums(IslandArgs a) {
 }
 
 __global__ void __launch_bounds__(kBlock) k_act_apply(IslandArgs a) {
-    const int P = *a.P, tiles = max((P + kScanTile - 1) / kScanTile, 1), tile = blockIdx.x;
+    const int P = *a.P, tiles = max((P + kActTile - 1) / kActTile, 1), tile = blockIdx.x;
     for (int j = blockIdx.x * kBlock + threadIdx.x; j < a.NJ; j += gridDim.x * kBlock) {
         const int2 q = a.jbody[j];
         isl_union(a, a.parent, q.x, q.y);
     }
     if (tile >= tiles) return;
-    const int base = tile * kScanTile + threadIdx.x * kScanItems;
-    unsigned long long v[kScanItems], s = 0, all;
+    const int base = tile * kActTile + threadIdx.x * kActItems;
+    unsigned long long v[kActItems], s = 0, all;
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) { v[k] = base + k < P ? act_value(a.npts[base + k]) : 0ull; s += v[k]; }
+    for (int k = 0; k < kActItems; k++) { v[k] = base + k < P ? act_value(a.npts[base + k]) : 0ull; s += v[k]; }
     const unsigned long long before = tiles_before<kBlock>(a.aux, tile);
     unsigned long long run = before + block_excl_scan<kBlock>(s, &all);
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
+    for (int k = 0; k < kActItems; k++) {
         if (v[k]) {
             const int p = base + k;
             a.active[run >> 32] = p;

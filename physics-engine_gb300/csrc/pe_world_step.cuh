@@ -133,7 +133,7 @@ template <class R> void World<R>::prepare_tail(int P) {
     for (int k = 0; k < 2; k++) { key_[k].ensure(keys); val_[k].ensure(keys, true); }
     if (ordered) order_ = val_[oi].p;
     hist_.ensure(radix_hist_ints(bound));
-    isl_aux_.ensure(scan_tiles(bound) + 1);
+    isl_aux_.ensure(std::max(scan_tiles(bound), act_tiles(pair_cap_)) + 1);
     isl_flag_.ensure(bound + 1); isl_off_.ensure(bound + 1);
     isl_n_.ensure(1); ncol_.ensure(1);
     isl_list_.ensure(class_base(kWarpClasses, bound)); isl_base_.ensure(bound + 1); isl_big_.ensure(bound + 1);
@@ -364,8 +364,8 @@ template <class R> void World<R>::solve_enqueue(int mode) {
         const size_t smem = island_one_smem(N_);
         launch_smem(K_ISLAND, 1, kIslandBlock, smem, k_islands_one, a, label_passes);
     } else {
-        launch(K_ISLAND, pgrid(std::max(cap, N_), kScanTile, k_act_sums), k_act_sums, a);
-        launch(K_ISLAND, scan_tiles(cap), k_act_apply, a);
+        launch(K_ISLAND, pgrid(std::max(cap, N_), kActTile, k_act_sums), k_act_sums, a);
+        launch(K_ISLAND, act_tiles(cap), k_act_apply, a);
         launch(K_ISLAND, pgrid(bound, kBlock, k_isl_keys), k_isl_keys, a);
         RadixArgs<uint32_t> r{a.key[0], a.val[0], a.key[1], a.val[1], nullptr, bound, Md, -1, 0, nullptr, 0};
         for (int k = 0; k < label_passes; k++, r.shift += 8) radix_pass(r);
