@@ -101,7 +101,7 @@ __global__ void k_bp_gather(Bodies<R> B, const uint32_t* order, SweepBoxes<R> ou
 // ascending j with a ballot and a prefix popcount, which is the reference's pair order.
 // Pass 0 counts the pairs of each position and keeps its first kStage partners; pass 1 writes the
 // pairs at the scanned offsets, copying staged partners and re-sweeping only crowded positions.
-constexpr int kStage = 4;
+constexpr int kStage = 8;   // a position with more pairs is swept again to write them
 // U chunks of 32 candidates from j0 on, tested in order after all their loads are under way; false
 // once a chunk is not full.  (c is the position's pairs so far.)
 template <class R, bool WRITE, int U>
@@ -291,6 +291,69 @@ __global__ void k_bp_count(int n, int limit, const int* scene_axis, const R* smn
     const int c = sweep_warp<R, false>(i, n, lane, scene_axis, smn, smx, sflag, sscene, stage, nullptr, nullptr, ign);
     if (lane == 0) count[i] = c;
 }
+// The count of kSweepShare consecutive positions by one warp: their windows nearly coincide, so each
+// chunk of candidates is loaded once for all of them.  With a warp per position, 65,536 scattered
+// bodies read 23 chunks each, some 1.5 GB out of the L2 cache.  From kSweepSharedFrom bodies on: below
+// that a warp per position fills the GPU, and the longest window decides.
+constexpr int kSweepShare = 4, kSweepSharedFrom = 16384;
+template <class R>
+__global__ void k_bp_count_shared(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
+                                  int* count, int* stage, int* big, int* n_big, IgnoreLists ign) {
+    constexpr int U = kSweepShare;
+    const int i0 = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5) * U;
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    if (i0 >= n) return;
+    if (i0 == 0 && lane == 0) count[n] = 0;   // the scan's last place
+    V3<R> mn[U], mx[U];
+    R top[U];
+    int sc[U], ax[U], fi[U], c[U];
+    unsigned alive = 0;   // bit u: position i0 + u's window goes on
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int i = min(i0 + u, n - 1);
+        mn[u] = V3<R>(smn[i], smn[n + i], smn[2 * (size_t)n + i]);
+        mx[u] = V3<R>(smx[i], smx[n + i], smx[2 * (size_t)n + i]);
+        sc[u] = sscene[i];
+        ax[u] = scene_axis[sc[u]];
+        fi[u] = sflag[i];
+        top[u] = ax[u] == 0 ? mx[u].x : ax[u] == 1 ? mx[u].y : mx[u].z;
+        c[u] = 0;
+        if (i0 + u >= n) continue;
+        if (big_window(i, n, limit, scene_axis, smn, smx, sscene)) {   // left to k_bp_count_chunks
+            if (lane == 0) big[atomicAdd(n_big, 1)] = i;
+            c[u] = -1;
+        } else if (!(fi[u] & BF_IGNORE)) {
+            alive |= 1u << u;
+        }
+    }
+    for (int j0 = i0 + 1; alive && j0 < n; j0 += 32) {
+        const int j = j0 + lane, k = min(j, n - 1);
+        const V3<R> lo(smn[k], smn[n + k], smn[2 * (size_t)n + k]), hi(smx[k], smx[n + k], smx[2 * (size_t)n + k]);
+        const int fj = sflag[k], sj = sscene[k];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (!(alive >> u & 1u)) continue;   // the same for the whole warp
+            const R low = ax[u] == 0 ? lo.x : ax[u] == 1 ? lo.y : lo.z;
+            const bool past = j <= i0 + u, in = j < n && !(low > top[u]) && sj == sc[u];
+            const unsigned live = __ballot_sync(full, past || in);
+            bool hit = in && !past && !(fj & BF_IGNORE) && !((fi[u] & BF_KINEMATIC) && (fj & BF_KINEMATIC)) &&
+                       !(mn[u].x > hi.x || lo.x > mx[u].x) && !(mn[u].y > hi.y || lo.y > mx[u].y) && !(mn[u].z > hi.z || lo.z > mx[u].z);
+            if (hit && ign.off && ((fi[u] | fj) & BF_IGN_LIST)) hit = !ign.ignored(i0 + u, j);
+            const unsigned m = __ballot_sync(full, hit);
+            if (hit) {
+                const int at = c[u] + __popc(m & ((1u << lane) - 1u));
+                if (at < kStage) stage[(size_t)(i0 + u) * kStage + at] = j;
+            }
+            c[u] += __popc(m);
+            if (live != full) alive &= ~(1u << u);
+        }
+    }
+    if (lane == 0)
+        for (int u = 0; u < U; u++)
+            if (i0 + u < n && c[u] >= 0) count[i0 + u] = c[u];
+}
+
 template <class R>
 __global__ void k_bp_write(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
                            const uint32_t* order, const int* offset, const int* stage, int2* pairs, int pair_cap, int* status,

@@ -99,7 +99,8 @@ template <class R> void World<R>::bp_count_enqueue() {
     }
     IgnoreLists ign;
     if (n_ign_ > 0) { ign.off = ign_off_.p; ign.ids = ign_ids_.p; ign.order = order_; }
-    launch(K_BP_SWEEP, grid_warps(n), k_bp_count<R>, n, kBigWindow, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, count_.p, bp_stage_.p,
+    const bool share = n >= kSweepSharedFrom;
+    launch(K_BP_SWEEP, grid_warps(share ? (n + kSweepShare - 1) / kSweepShare : n), share ? k_bp_count_shared<R> : k_bp_count<R>, n, kBigWindow, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, count_.p, bp_stage_.p,
            bp_big_.p, bp_nbig_.p, ign);
     // crowded positions: windows in chunks of one block each (at most kMaxChunks per position); a
     // window holds at most the scene's other bodies, so scenes of at most kBigWindow bodies have none

@@ -65,3 +65,32 @@ def test_windows_end_with_their_scene():
         want.append(alone.pairs().reshape(-1, 2) + int(offs[k]))
     assert np.array_equal(g.pairs().reshape(-1, 2), np.concatenate(want))
     g.close()
+
+
+@pytest.mark.parametrize("n", [16383, 16384, 16387])
+def test_windows_of_four_positions(n):
+    """From 16,384 bodies on a warp counts four positions: windows that end inside and at the edges of its
+    chunks, the last positions of the world, and scenes that end between a warp's positions."""
+    s = _line(n - 40, [m for m in range(1, 80, 2)], 32, seed=n)
+    g, o = pg.GpuWorld(s, 32), orc.OracleWorld(s, 32, stable_ties=True)
+    for _ in range(2):
+        g.step(1, pg.SERIAL_ORDER)
+        o.step(1)
+        assert np.array_equal(g.pairs(), o.pairs())
+    g.close()
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+def test_windows_of_four_positions_end_with_their_scene(bits):
+    parts = [_line(int(m), (3, 5, 17, 33), bits, seed=k, dense=k % 2 == 0) for k, m in enumerate(np.resize([61, 36, 50, 127, 43], 260))]
+    whole, offs = sc.concat(parts)
+    assert whole.n_bodies >= 16384
+    g = pg.GpuWorld(whole, bits, scenes=offs)
+    g.step(1, pg.SERIAL_ORDER)
+    want = []
+    for k, p in enumerate(parts):
+        alone = orc.OracleWorld(p, bits, stable_ties=True)
+        alone.step(1)
+        want.append(alone.pairs().reshape(-1, 2) + int(offs[k]))
+    assert np.array_equal(g.pairs().reshape(-1, 2), np.concatenate(want))
+    g.close()
