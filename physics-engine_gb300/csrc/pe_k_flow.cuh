@@ -44,6 +44,69 @@ template <class R, bool JOINTS> struct Item {
     }
 };
 
+// ---------------------------------------------------------------- one result by a whole warp (FP64)
+// A double-precision instruction holds a warp for 64 cycles on this chip, with one lane in it or 32,
+// and the next one waits even if it does not depend on it (measured: dependent and independent chains
+// alike), so a row costs its instruction count: some 170, 5 us, when one lane runs it.  Here lanes 0 to 8
+// share a row: lane 3 s + k holds component k of body s's velocities, lane 3 q + k component k of
+// direction q (normal, tangents), some 40 instructions with shuffles between them.  Operations and
+// their order are si_row's.
+struct WarpRow {   // what a lane holds of one row
+    double r1, r2, d, jmj, base, mu, nacc;
+    __device__ __forceinline__ void load(const Rows<double>& rows, int row, int s, int q, int k) {
+        const double* p = rows.f + (size_t)row * NRF;
+        const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+        r1 = p[4 * s + k1]; r2 = p[4 * s + k2];
+        d = p[8 + 4 * q + k];
+        jmj = p[q == 0 ? 3 : q == 1 ? 11 : 15];
+        base = p[q == 0 ? 7 : 21 + q];
+        mu = p[20]; nacc = p[21];
+    }
+};
+constexpr int kWarpItem = 32;   // doubles of an item in shared memory: velocities of a and b (6 each), inverse inertias (9 each), inverse masses
+__device__ __forceinline__ double shfl_d(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
+// item's rows r0 .. r0 + np - 1 (every lane's arguments the same); its velocities are updated in `item`
+__device__ __forceinline__ void si_rows_warp(const Rows<double>& rows, int r0, int np, bool kin_a, bool kin_b, double* item, int lane) {
+    const int l = lane < 9 ? lane : 8, q = l / 3, k = l - 3 * q, s = q < 2 ? q : 1;   // lanes past the last role repeat one
+    const int k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1, at = 3 * s;
+    double v = item[6 * s + k], w = item[6 * s + 3 + k];
+    const double i0 = item[12 + 9 * s + 3 * k], i1 = item[13 + 9 * s + 3 * k], i2 = item[14 + 9 * s + 3 * k], im = item[30 + s];
+    const bool kin = s == 0 ? kin_a : kin_b;
+    WarpRow row;
+    row.load(rows, r0, s, q, k);
+    for (int n = 0; n < np; n++) {
+        WarpRow next;
+        if (n + 1 < np) next.load(rows, r0 + n + 1, s, q, k);
+        const double w1 = shfl_d(w, at + k1), w2 = shfl_d(w, at + k2);
+        const double turn = w1 * row.r2 - w2 * row.r1;
+        const double vr = ((shfl_d(v, k) + shfl_d(turn, k)) - shfl_d(v, 3 + k)) - shfl_d(turn, 3 + k);
+        const double part = row.d * vr;
+        const double dotq = (shfl_d(part, 3 * q) + shfl_d(part, 3 * q + 1)) + shfl_d(part, 3 * q + 2);
+        double val = row.base - dotq * row.jmj;
+        double ni = shfl_d(val, 0);
+        ni = ni > -row.nacc ? ni : -row.nacc;
+        const double nacc = row.nacc + ni;
+        const double sq = val * val;
+        const double scale = friction_scale(row.mu * nacc, shfl_d(sq, 3) + shfl_d(sq, 6));
+        if (scale < 1) val = val * scale;
+        const double push = (q == 0 ? ni : val - row.base) * row.d;
+        double imp = (shfl_d(push, k) + shfl_d(push, 3 + k)) + shfl_d(push, 6 + k);
+        if (s == 1) imp = -imp;
+        const double p1 = shfl_d(imp, at + k1), p2 = shfl_d(imp, at + k2);
+        const double x = row.r1 * p2 - row.r2 * p1;
+        const double m0 = i0 * shfl_d(x, at), m1 = i1 * shfl_d(x, at + 1), m2 = i2 * shfl_d(x, at + 2);
+        const double turned = ((k < 2 ? m0 : m1) + (k < 2 ? m1 : m2)) + (k < 2 ? m2 : m0);   // mv: the last row right to left
+        if (!kin) { v = v + imp * im; w = w + turned; }
+        double* p = rows.f + (size_t)(r0 + n) * NRF;
+        if (lane == 0) p[21] = nacc;
+        else if (lane == 3 || lane == 6) p[21 + q] = val;
+        row = next;
+    }
+    __syncwarp();
+    if (lane < 6) { item[6 * s + k] = v; item[6 * s + 3 + k] = w; }
+    __syncwarp();
+}
+
 // ---------------------------------------------------------------- islands inside a warp
 // Islands of up to kWarpIsland items, listed by size class: 1, 2, 3-4, 5-8, 9-16 and 17-32 items, so
 // that a warp works on islands of about one length (32, 16, 8, 4, 2 or 1 of them), one lane per item.
@@ -246,6 +309,7 @@ template <class R> struct FlowArgs {
     int* status;
 };
 constexpr int kFlowBlock = 128, kFlowFirstFit = 1, kFlowLeft = 2;
+constexpr int kByWarpMost = 4;   // ready results of a warp up to which each takes the whole warp: 4 x 40 instructions, against 170 for all at once
 constexpr int kFlowStall = 1 << 21;   // polls in a row without progress after which a warp gives up (seconds)
 
 // Islands that one warp does not take, all of them in one cooperative launch (a waiting item needs
@@ -410,6 +474,9 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
         grid.sync();
     }
 
+    // FP64: a warp with few ready results runs them one by one, all lanes on each (si_rows_warp)
+    constexpr bool kByWarp = sizeof(R) == 8;
+    __shared__ R shared_item[kByWarp ? kFlowBlock : 1][kByWarp ? kWarpItem : 1];
     const bool reorder = coloring && *(volatile int*)f.any_first_fit != 0;
     const bool single = M <= stride;   // one item per lane: its constants stay in registers
     Item<R, JOINTS> x;
@@ -424,6 +491,12 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
         lev_a = 0;
         lev_b = 0;
         m = island_size(f.isl[j]);
+        if constexpr (kByWarp) {
+            R* it = shared_item[threadIdx.x];
+            for (int a = 0; a < 3; a++)
+                for (int b = 0; b < 3; b++) { it[12 + 3 * a + b] = x.a.I.m[a][b]; it[21 + 3 * a + b] = x.b.I.m[a][b]; }
+            it[30] = x.a.im; it[31] = x.b.im;
+        }
     };
     // the lane's next item of the iteration, by position or by (colour, position); M after the last
     auto next_item = [&](int j) {
@@ -441,13 +514,42 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
     stall = 0;
     if (j < M) take_item(j);
     while (__any_sync(full, j < M)) {
-        bool moved = false;
+        bool moved = false, done = false;
         if (j < M) {
             if (!have_a) have_a = token_get(f.box + (size_t)(2 * j) * NW, x.a, it, lev_a);
             if (!have_b) have_b = token_get(f.box + (size_t)(2 * j + 1) * NW, x.b, it, lev_b);
+        }
+        if constexpr (kByWarp) {
+            const bool ready = j < M && have_a && have_b && f.iterations > 0 && !(JOINTS && (x.id & kJointItem));
+            unsigned todo = __ballot_sync(full, ready);
+            if (__popc(todo) <= kByWarpMost) {
+                done = ready;
+                if (ready) {
+                    R* p = shared_item[threadIdx.x];
+                    p[0] = x.a.v.x; p[1] = x.a.v.y; p[2] = x.a.v.z; p[3] = x.a.w.x; p[4] = x.a.w.y; p[5] = x.a.w.z;
+                    p[6] = x.b.v.x; p[7] = x.b.v.y; p[8] = x.b.v.z; p[9] = x.b.w.x; p[10] = x.b.w.y; p[11] = x.b.w.z;
+                }
+                __syncwarp();
+                for (; todo; todo &= todo - 1) {
+                    const int o = __ffs(todo) - 1;
+                    const int r0 = __shfl_sync(full, x.r0, o), np = __shfl_sync(full, x.np, o);
+                    const int kins = __shfl_sync(full, (x.a.kin ? 1 : 0) | (x.b.kin ? 2 : 0), o);
+                    si_rows_warp(rows, r0, np, kins & 1, kins & 2, shared_item[(threadIdx.x & ~31) + o], lane);
+                }
+                if (ready) {
+                    const R* p = shared_item[threadIdx.x];
+                    x.a.v = V3<R>(p[0], p[1], p[2]); x.a.w = V3<R>(p[3], p[4], p[5]);
+                    x.b.v = V3<R>(p[6], p[7], p[8]); x.b.w = V3<R>(p[9], p[10], p[11]);
+                }
+            }
+        }
+        if (j < M) {
             if (have_a && have_b) {
                 moved = true;
-                if (f.iterations > 0) x.iterate(J, rows);
+                if (f.iterations > 0 && !done) {
+                    if (kByWarp && !(JOINTS && (x.id & kJointItem))) row_load(rows, x.r0, x.q);   // the warp keeps no row in registers
+                    x.iterate(J, rows);
+                }
                 const int lev = max(lev_a, lev_b) + 1;
                 auto give = [&](Side<R>& s, int i, int entry, int to, bool& have) {
                     if (s.kin) return;
