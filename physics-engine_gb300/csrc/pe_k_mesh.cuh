@@ -19,7 +19,7 @@ namespace pe {
 // recorder holds runs again on lane 0.  The leaves of a concave mesh's face tree are tested 32 at a
 // time.  (What bounds a pair is the serial code of one piece; with one thread per pair, walking some
 // 2,000 leaves and then face after face, a step of 300 bodies on a terrain of 4,608 triangles spent 13.9 ms
-// on its compound pairs and 4.5 ms on the others beside them, and took 18.9 ms; it takes 1.2 ms so.)
+// on its compound pairs and 4.5 ms on the others beside them, and took 18.9 ms; it takes 0.7 ms so.)
 constexpr int kMeshPoints = 12, kMeshQueue = 64;
 struct MeshPiece {
     int i, j;      // child of A, of B; -1: the shape itself
