@@ -141,8 +141,8 @@ __device__ __forceinline__ bool sweep_chunks(int i, int j0, int n, int lane, int
 }
 // The sweep of one position by a warp.  A window is a chain of chunks, each some 3 us of dependent
 // loads and votes when taken alone: the floor of a 1,600-body scene, 50 chunks, held the count for
-// 81 us and the write for 169 us.  Most windows end in the first two chunks; longer ones go four
-// chunks at a time, loads first.
+// 81 us and the write for 169 us (now 31 and 46).  Most windows end in the first two chunks; longer
+// ones go four chunks at a time, loads first.
 template <class R, bool WRITE>
 __device__ __forceinline__ int sweep_warp(int i, int n, int lane, const int* scene_axis, const R* smn, const R* smx,
                                           const int* sflag, const int* sscene, int* stage, int2* out, const uint32_t* order,
@@ -293,7 +293,8 @@ __global__ void k_bp_count(int n, int limit, const int* scene_axis, const R* smn
 }
 // The count of kSweepShare consecutive positions by one warp: their windows nearly coincide, so each
 // chunk of candidates is loaded once for all of them.  With a warp per position, 65,536 scattered
-// bodies read 23 chunks each, some 1.5 GB out of the L2 cache.  From kSweepSharedFrom bodies on: below
+// bodies read 23 chunks each, some 1.5 GB out of the L2 cache (their step 1,469 / 1,454 us, that of
+// 40,000 poured ones and 4,096 piles each some 2 % shorter).  From kSweepSharedFrom bodies on: below
 // that a warp per position fills the GPU, and the longest window decides.
 constexpr int kSweepShare = 4, kSweepSharedFrom = 16384;
 template <class R>

@@ -121,9 +121,8 @@ __device__ V3<R> shape_witness(const ShapeView<R>& s, const Xf<R>& t, const V3<R
 // What bounds it is instruction fetch and issue: 32 axes cost about 60 instructions for the bound (two
 // hulls' edge pairs mostly some 25, see `hulls`), and most pairs one round of exact projections for the
 // faces and one for the edges.  Per step of the 4,096 piles, before (every axis past a ball test projected
-// exactly, two per lane) and now: hull-hull 1,750 / 494 us, its heavy pairs 778 / 250, box-hull
-// 2,311 / 1,840, cylinder-cylinder 935 / 412; the whole step 8.68 / 6.30 ms, the 501-body pile's
-// 964 / 655 us (its tail was one hull pair).
+// exactly, two per lane) and now: hull-hull 1,750 / 521 us, its heavy pairs 778 / 297, box-hull
+// 2,311 / 1,286, hull-box 699 / 411, cylinder-cylinder 935 / 245.
 
 // One side's bound data.  rel: the support points are taken relative to the shape's own origin.
 constexpr int kSub = 8;          // supporting points per hull
