@@ -140,22 +140,36 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
     __shared__ int tok_lev[W][2][32];    // its level (the first iteration's)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
-    int units[kWarpClasses], total = 0;
+    // Islands per warp: as many as its lanes hold, and fewer while there are warps to spare.  A warp takes
+    // as long as its slowest lanes in every round, and its lanes' joints and rows of different length run
+    // one after the other (200 FP64 chains, four islands a warp before and one now: 921 / 857 us).
+    int units[kWarpClasses], total = 0, spread = 0;
+    for (int sp = 0; sp <= 5; sp++) {
+        int sum = 0;
+#pragma unroll
+        for (int c = 0; c < kWarpClasses; c++) {
+            const int per = max(1, 32 >> (c + sp));
+            sum += (n_list[c] + per - 1) / per;
+        }
+        if (sp > 0 && sum > (int)gridDim.x) break;   // the grid is up to four times the resident blocks, four warps each
+        spread = sp;
+    }
 #pragma unroll
     for (int c = kWarpClasses - 1; c >= 0; c--) {   // the longest islands first
-        const int per = 32 >> c;
+        const int per = max(1, 32 >> (c + spread));
         units[c] = (n_list[c] + per - 1) / per;
         total += units[c];
     }
     const int its = iterations > 0 ? iterations : 1;   // without iterations the levels are still counted
     int deepest = 0;
-    for (int u = blockIdx.x * W + warp; u < total; u += gridDim.x * W) {
+    // neighbours in a block, or over the SMs first while there are warps to spare
+    for (int u = spread ? warp * gridDim.x + blockIdx.x : blockIdx.x * W + warp; u < total; u += gridDim.x * W) {
         int c = kWarpClasses - 1, k = u;
         while (k >= units[c]) { k -= units[c]; c--; }
-        const int s = 1 << c;
-        const int li = k * (32 >> c) + (lane >> c), idx = lane & (s - 1), g0 = lane - idx;
+        const int s = 1 << c, per = max(1, 32 >> (c + spread));
+        const int li = k * per + (lane >> c), idx = lane & (s - 1), g0 = lane - idx;
         int lo = 0, m = 0;
-        if (li < n_list[c]) {
+        if ((lane >> c) < per && li < n_list[c]) {
             const int isl = list[class_base(c, bound) + li];
             lo = isl_off[isl];
             m = isl_off[isl + 1] - lo;

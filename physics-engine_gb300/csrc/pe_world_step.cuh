@@ -389,7 +389,8 @@ template <class R> template <bool JOINTS> void World<R>::solve_islands(int mode,
     const int bound = pair_cap_ + n_joints_, small = tun_.small_island_items, big = tun_.big_island_items;
     int* n_list = dcnt_.p + DC_NLIST;
     int* colors = mode == 0 ? nullptr : ncol_.p;
-    launch_block(K_SI_SERIAL, pgrid(bound, kWarpBlock, k_isl_warp<R, JOINTS>, kWarpBlock), kWarpBlock, k_isl_warp<R, JOINTS>,
+    // (a warp for every island, up to the resident ones: see the islands per warp)
+    launch_block(K_SI_SERIAL, pgrid(bound, kWarpBlock / 32, k_isl_warp<R, JOINTS>, kWarpBlock), kWarpBlock, k_isl_warp<R, JOINTS>,
                  (const int*)isl_list_.p, (const int*)n_list, bound, (const int*)isl_off_.p, order, results(), joints(), bodies(), rows(),
                  prm_.iterations, small, colors, status_.p);
     FlowArgs<R> f;
