@@ -141,8 +141,9 @@ __device__ __forceinline__ double fast_max(double a, double b) { return fmax(a, 
 template <class R> constexpr R sat_slack() { return sizeof(R) == 4 ? R(96 * 1.1920929e-7) : R(96 * 2.220446049250313e-16); }
 
 // Lower bound of the support of a shape along y (of length ny): box and cylinder in closed form (a
-// cylinder lowered by what the reference's branches for nearly axial and nearly radial axes drop), a
-// hull by its supporting points.  For the second shape (QUIRK) a hull's bound counts only when vertex 0
+// cylinder lowered by what the reference's branches for nearly axial and nearly radial axes drop: they
+// take the half height or the radius whatever the axis's length, and one normal of the cylinder mesh is
+// 1.0188 long), a hull by its supporting points.  For the second shape (QUIRK) a hull's bound counts only when vertex 0
 // or 1, which come before every supporting point, lies below it: the reference never lets a new
 // minimum become the maximum (convex_mesh_shape.cpp:171-175), and a point above an earlier vertex is no
 // new minimum.
@@ -153,7 +154,8 @@ __device__ __forceinline__ R sat_support(int type, const SatSide<R>& s, const V3
     if (t == ST_CYLINDER) {
         const R c = fma3(y, s.e0);
         const R n2 = ny * ny;   // the axis's part across the cylinder's, its square lowered by its own roundoff
-        return fma(s.hh, rabs(c), s.r * fast_sqrt(fast_max(fma(-c, c, n2) - R(0.125) * sat_slack<R>() * n2, R(0)))) - R(3e-5) * (s.r + s.hh) * ny;
+        return fma(s.hh, rabs(c), s.r * fast_sqrt(fast_max(fma(-c, c, n2) - R(0.125) * sat_slack<R>() * n2, R(0)))) -
+               (s.r + s.hh) * fma(R(3e-5), ny, fast_max(ny - R(1), R(0)));
     }
     R m = fma3(y, ldv(sub, 0));
 #pragma unroll
