@@ -365,7 +365,7 @@ private:
     struct GraphSig {
         unsigned long long gen;
         const void* order;
-        int n, ns, pair_cap, nj, n_ign, s, side;
+        int n, ns, pair_cap, nj, n_ign, s, bcap, max_scene;
         unsigned classes;
         int plan[PC_COUNT];
         StepParams prm;
@@ -441,6 +441,7 @@ private:
     // scenes
     int NS_ = 1;
     std::vector<int> h_scene_off_;
+    void scene_offsets_changed();   // what follows from h_scene_off_
     DBuf<int> scene_off_, scene_axis_, pair_scene_off_, res_scene_off_, prev_res_off_;
     // broadphase
     DBuf<uint64_t> key_[2];
@@ -451,7 +452,7 @@ private:
     DBuf<int> bp_wend_, bp_csize_, bp_nch_, bp_choff_, bp_ctot_, bp_ccount_, bp_cpref_;   // crowded windows in chunks
     static constexpr int kBigSweepBlocks = 152;   // blocks that share the crowded positions
     uint32_t* order_ = nullptr;   // sorted body order (points into val_)
-    int max_scene_ = 0;           // bodies of the largest scene (the crowded-window kernels run above kBigWindow)
+    int max_scene_ = 0;           // bodies of the largest scene (set with h_scene_off_; the crowded-window kernels run above kBigWindow)
     DBuf<int2> pairs_;
     int P_ = 0, pair_cap_ = 0;
     // narrowphase

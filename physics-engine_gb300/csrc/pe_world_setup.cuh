@@ -438,6 +438,11 @@ void World<R>::set_bodies(int n, const int* shape, const int* flags, const doubl
     set_scenes(1, nullptr);
 }
 
+template <class R> void World<R>::scene_offsets_changed() {
+    max_scene_ = 0;
+    for (int s = 0; s < NS_; s++) max_scene_ = std::max(max_scene_, h_scene_off_[s + 1] - h_scene_off_[s]);
+}
+
 template <class R> void World<R>::set_scenes(int ns, const int* off) {
     std::vector<int> so(ns + 1);
     if (off) for (int s = 0; s <= ns; s++) so[s] = off[s];
@@ -446,6 +451,7 @@ template <class R> void World<R>::set_scenes(int ns, const int* off) {
     for (int s = 0; s < ns; s++) if (so[s + 1] < so[s]) throw std::runtime_error("scene offsets must not decrease");
     NS_ = ns;
     h_scene_off_ = so;
+    scene_offsets_changed();
     std::vector<int> sc(std::max(N_, 1), 0);
     for (int s = 0; s < ns; s++) for (int i = so[s]; i < so[s + 1]; i++) sc[i] = s;
     upload(bscene_, sc, st_);

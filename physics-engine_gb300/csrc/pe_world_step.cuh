@@ -78,8 +78,6 @@ template <class R> void World<R>::bp_count_enqueue() {
     bp_nbig_.ensure(1);
     SweepBoxes<R> boxes;
     boxes.mn = smn_.p; boxes.mx = smx_.p; boxes.flag = sflag_.p; boxes.scene = ssc_.p;
-    max_scene_ = 0;
-    for (int s = 0; s < NS_; s++) max_scene_ = std::max(max_scene_, h_scene_off_[s + 1] - h_scene_off_[s]);
     if (max_scene_ <= std::min(tun_.scene_sort_max, kSceneSortMax)) {   // every scene sorted inside one block
         launch_block(K_RADIX, NS_, kSceneSortBlock, k_bp_sort_scenes<R>, bodies(), (const int*)scene_axis_.p, (const int*)scene_off_.p,
                      val_[0].p, boxes, bp_nbig_.p);
@@ -438,7 +436,8 @@ template <class R> void World<R>::graph_sig(GraphSig& g) const {
     g.order = order_;
     g.n = N_; g.ns = NS_; g.pair_cap = pair_cap_; g.nj = n_joints_; g.n_ign = n_ign_; g.s = S_;
     g.classes = possible_classes();
-    g.side = bcap_ * 4 + (max_scene_ > kBigWindow ? 1 : 0);
+    g.bcap = bcap_;
+    g.max_scene = max_scene_;   // which sort the scenes take, and whether windows are swept in chunks
     std::memcpy(g.plan, stream_of_, sizeof g.plan);
     std::memcpy(&g.prm, &prm_, sizeof prm_);
     std::memcpy(&g.margin, &margin_, sizeof margin_);
