@@ -250,7 +250,8 @@ int pe_gpu_server_create(const pe_gpu_config* cfg, double dt, double gx, double 
                          double hbm_budget_bytes, pe_gpu_server** out);
 int pe_gpu_server_destroy(pe_gpu_server* s);
 const char* pe_gpu_server_last_error(const pe_gpu_server* s);
-/* copies the scene; *id identifies the request.  n_steps must be at least 1 (PE_GPU_ERR_ARG otherwise). */
+/* copies the scene; *id identifies the request.  n_steps must be at least 1, and the scene's shapes ones that a
+ * request may have: no compounds, and what pe_gpu_set_shapes takes (PE_GPU_ERR_ARG otherwise). */
 int pe_gpu_server_submit(pe_gpu_server* s, const pe_gpu_scene* scene, int n_steps, long long* id);
 /* retire, admit, one batched step of all live scenes */
 int pe_gpu_server_step(pe_gpu_server* s, int* n_live, int* n_queued);

@@ -1008,7 +1008,6 @@ template <class R, class C> __device__ bool cylinder_hull(Pair<R, C>& c) {   // 
 // selects faces through the face tree; each face becomes a one-face convex shape (its vertices in
 // face order, its normal, no unique edges: setMesh is never called on it) that the convex-convex
 // algorithm meets with the convex shape first, at the concave body's transform.
-constexpr int kFaceVerts = 32;   // longest face polygon a concave mesh may hold (checked at upload)
 template <class R> struct FaceBuf { R v[kFaceVerts * 3], n[3], mn[3], mx[3]; int idx[kFaceVerts], off[2]; };
 // the pair that face f of the mesh cc makes with the convex shape cv
 template <class R, class C>

@@ -1,6 +1,7 @@
 // Host-side preprocessing shared by the world implementations: unit meshes, convex-mesh
 // preparation and per-body mass properties.  Runs once per scene upload, never per step.
 #pragma once
+#include <string>
 #include <vector>
 #include "pe_math.cuh"
 
@@ -28,6 +29,10 @@ template <class R> struct HullPrep {
 // ConvexMeshShape::setMesh, or ConcaveMeshShape::setMesh with `concave`
 template <class R> HullPrep<R> prepare_hull(const double* verts, int nv, const int* face_off, const int* face_idx, int nf,
                                             bool concave = false);
+
+// Why a shape is refused ("" when it is not): its type, its face count and its faces' offsets, `batched`
+// for a request of the serving loop.
+std::string shape_fault(int type, int n_faces, const int* face_off, bool batched);
 
 // A scene as a caller describes it (the arrays of pe_gpu_set_shapes and pe_gpu_set_bodies), owned
 // on the host; shape indices of the bodies and hull indices are local to the scene.

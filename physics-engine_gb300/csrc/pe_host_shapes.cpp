@@ -87,6 +87,16 @@ void build_unit_meshes(UnitMeshes& u) {
     }
 }
 
+std::string shape_fault(int type, int n_faces, const int* face_off, bool batched) {
+    if (type == ST_COMPOUND) return batched ? "compound shapes are not supported in batched requests" : "";
+    if (type < ST_BOX || type > ST_COMPOUND) return "unsupported shape type " + std::to_string(type);
+    if (type == ST_HULL && n_faces > kHullFaces) return "convex mesh with more than " + std::to_string(kHullFaces) + " faces is not supported";
+    if (type == ST_CONCAVE)
+        for (int f = 0; f < n_faces; f++)
+            if (face_off[f + 1] - face_off[f] > kFaceVerts) return "concave mesh face with more than " + std::to_string(kFaceVerts) + " vertices";
+    return "";
+}
+
 template <class R> M3<R> box_inertia(const V3<R>& s) {
     const R x2 = s.x * s.x, y2 = s.y * s.y, z2 = s.z * s.z;
     M3<R> m;

@@ -50,21 +50,21 @@ public:
         return id;
     }
 
+    // (requests change their state once the world has been repacked: a repack that fails leaves them as
+    // they were)
     void step(int* n_live, int* n_queued) {
         const std::vector<int> off = w_->scene_body_offsets();
         std::vector<int> keep;
-        std::vector<long long> still;
-        bool changed = false;
+        std::vector<long long> still, retired;
+        double used = used_;
         for (size_t k = 0; k < live_.size(); k++) {
             Req& q = reqs_[live_[k]];
             if (q.done >= q.k) {   // retire: read the final state back
                 const int n = off[k + 1] - off[k];
                 q.o.resize((size_t)n * 3); q.b.resize((size_t)n * 9); q.v.resize((size_t)n * 3); q.w.resize((size_t)n * 3);
                 w_->get_state_range(off[k], n, q.o.data(), q.b.data(), q.v.data(), q.w.data());
-                q.state = 2;
-                used_ -= q.bytes;
-                finished_++;
-                changed = true;
+                used -= q.bytes;
+                retired.push_back(live_[k]);
             } else {
                 keep.push_back((int)k);
                 still.push_back(live_[k]);
@@ -72,21 +72,26 @@ public:
         }
         std::vector<const SceneData*> adds;
         std::vector<long long> added;
-        while (!queue_.empty()) {   // admission in arrival order, by footprint
-            Req& q = reqs_[queue_.front()];
-            if (used_ + q.bytes > budget_) break;
-            used_ += q.bytes;
-            q.state = 1;
+        for (long long id : queue_) {   // admission in arrival order, by footprint
+            Req& q = reqs_[id];
+            if (used + q.bytes > budget_) break;
+            used += q.bytes;
             adds.push_back(&q.d);
-            added.push_back(queue_.front());
-            queue_.pop_front();
-            admitted_++;
+            added.push_back(id);
         }
-        if (changed || !adds.empty()) {
+        if (!retired.empty() || !adds.empty()) {
             w_->repack(keep.data(), (int)keep.size(), adds.data(), (int)adds.size());
+            for (long long id : retired) reqs_[id].state = 2;
+            for (long long id : added) {
+                reqs_[id].state = 1;
+                reqs_[id].d = SceneData();   // uploaded: free the host copy
+                queue_.pop_front();
+            }
             live_ = still;
             live_.insert(live_.end(), added.begin(), added.end());
-            for (long long id : added) reqs_[id].d = SceneData();   // uploaded: free the host copy
+            used_ = used;
+            finished_ += (long long)retired.size();
+            admitted_ += (long long)added.size();
         }
         peak_used_ = std::max(peak_used_, used_);
         if (!live_.empty()) {
@@ -172,6 +177,9 @@ template <class F> int sguard(pe_gpu_server* h, F&& f) {
     } catch (const std::bad_alloc&) {
         h->err = "host allocation failed";
         return PE_GPU_ERR_CAPACITY;
+    } catch (const std::invalid_argument& e) {
+        h->err = e.what();
+        return PE_GPU_ERR_ARG;
     } catch (const std::exception& e) {
         h->err = e.what();
         return PE_GPU_ERR_STATE;
@@ -227,10 +235,15 @@ int pe_gpu_server_submit(pe_gpu_server* h, const pe_gpu_scene* sc, int n_steps, 
             d.hull_face_idx.assign(sc->hull_face_idx, sc->hull_face_idx + sc->hull_face_off[sc->n_hull_faces]);
         }
         for (int k = 0; k < S; k++)
-            if (d.shape_type[k] == PE_GPU_SHAPE_CONVEX_MESH &&
+            if ((d.shape_type[k] == PE_GPU_SHAPE_CONVEX_MESH || d.shape_type[k] == PE_GPU_SHAPE_CONCAVE_MESH) &&
                 (d.hull_vbeg[k] < 0 || d.hull_vbeg[k] + d.hull_vcnt[k] > sc->n_hull_verts || d.hull_fbeg[k] < 0 ||
                  d.hull_fbeg[k] + d.hull_fcnt[k] > sc->n_hull_faces))
                 return PE_GPU_ERR_ARG;
+        for (int k = 0; k < S; k++) {   // what the world would refuse, before the request is in the queue
+            const bool mesh = d.shape_type[k] == PE_GPU_SHAPE_CONVEX_MESH || d.shape_type[k] == PE_GPU_SHAPE_CONCAVE_MESH;
+            const std::string why = pe::shape_fault(d.shape_type[k], mesh ? d.hull_fcnt[k] : 0, mesh ? d.hull_face_off.data() + d.hull_fbeg[k] : nullptr, true);
+            if (!why.empty()) throw std::invalid_argument(why);
+        }
         d.body_shape.assign(sc->body_shape, sc->body_shape + N);
         d.body_flags.assign(sc->body_flags, sc->body_flags + N);
         d.mass.assign(sc->mass, sc->mass + N);

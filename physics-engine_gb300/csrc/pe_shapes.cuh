@@ -12,6 +12,8 @@
 namespace pe {
 
 enum ShapeType { ST_BOX = 0, ST_SPHERE = 1, ST_CYLINDER = 2, ST_HULL = 3, ST_CONCAVE = 4, ST_COMPOUND = 5 };
+constexpr int kHullFaces = 16381;   // most faces of a convex mesh
+constexpr int kFaceVerts = 32;      // longest face polygon of a concave mesh
 
 // unit meshes (host builds them in double precision; the device reads them in the world's real type)
 constexpr int kBoxV = 24, kBoxF = 6, kBoxE = 12;

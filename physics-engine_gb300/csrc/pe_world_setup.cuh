@@ -2,6 +2,7 @@
 // compounds, joints, ignored pairs, bodies, scenes, parameters).
 #pragma once
 #include <algorithm>
+#include <functional>
 #include "pe_world.cuh"
 
 namespace pe {
@@ -129,6 +130,13 @@ template <class T> static void upload_tail(DBuf<T>& d, const std::vector<T>& h, 
     if (h.size() > from) PE_CK(cudaMemcpyAsync(d.p + from, h.data() + from, (h.size() - from) * sizeof(T), cudaMemcpyHostToDevice, st));
 }
 
+// truncates tables that only grew since `keep` to the sizes they had then, unless `back` is cleared before
+struct TableUndo {
+    std::vector<std::function<void()>> back;
+    template <class... V> void keep(V&... v) { (back.push_back([&v, n = v.size()] { v.resize(n); }), ...); }
+    ~TableUndo() { for (auto& f : back) f(); }
+};
+
 template <class R>
 void World<R>::set_shapes(int S, const int* type, const double* param, const int* vbeg, const int* vcnt, const int* fbeg,
                           const int* fcnt, int HV, const double* hv, int HF, const int* foff, const int* fidx) {
@@ -149,8 +157,16 @@ template <class R>
 int World<R>::append_shapes(int S, const int* type, const double* param, const int* vbeg, const int* vcnt, const int* fbeg,
                             const int* fcnt, const double* hv, const int* foff, const int* fidx, std::vector<int>* remap) {
     const int s0 = S_;
+    for (int s = 0; s < S; s++) {   // all of them before the tables change
+        const bool mesh = type[s] == ST_HULL || type[s] == ST_CONCAVE;
+        const std::string why = shape_fault(type[s], mesh ? fcnt[s] : 0, mesh ? foff + fbeg[s] : nullptr, remap != nullptr);
+        if (!why.empty()) throw std::runtime_error(why);
+    }
     const size_t o_h = h_hvb_.size(), o_v = h_hv_.size(), o_f = h_fn_.size(), o_e = h_ea_.size(), o_fo = h_foff_.size(),
                  o_fi = h_fidx_.size(), o_l = h_lfb_.size();
+    TableUndo undo;   // an allocation that fails below leaves the tables as they were
+    undo.keep(h_stype_, h_sparam_, h_sinertia_, h_shull_, h_hvb_, h_hvc_, h_hfb_, h_hfc_, h_heb_, h_hec_, h_foff_, h_fidx_, h_hv_, h_fn_,
+              h_fmn_, h_fmx_, h_ea_, h_eb_, h_hrad_, h_hlb_, h_hlc_, h_lfb_, h_lfc_, h_lfmn_, h_lfmx_, h_cbeg_, h_ccnt_, h_cready_);
     if (remap) remap->assign(S, -1);
     int added = 0;
     std::unordered_map<std::string, int> fresh;   // known to later requests once all of this one's are accepted
@@ -193,11 +209,6 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
             // local face offsets of this shape
             std::vector<int> lo(fcnt[s] + 1);
             for (int f = 0; f <= fcnt[s]; f++) lo[f] = foff[fbeg[s] + f] - foff[fbeg[s]];
-            if (t == ST_HULL && fcnt[s] >= 16382) throw std::runtime_error("convex mesh with more than 16381 faces is not supported");
-            if (t == ST_CONCAVE)
-                for (int f = 0; f < fcnt[s]; f++)
-                    if (lo[f + 1] - lo[f] > kFaceVerts)
-                        throw std::runtime_error("concave mesh face with more than " + std::to_string(kFaceVerts) + " vertices");
             HullPrep<R> h = prepare_hull<R>(hv + (size_t)vbeg[s] * 3, vcnt[s], lo.data(), fidx + foff[fbeg[s]], fcnt[s],
                                             t == ST_CONCAVE);
             inertia = h.inertia;
@@ -222,11 +233,8 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
             h_fmx_.insert(h_fmx_.end(), h.f_max.begin(), h.f_max.end());
             h_ea_.insert(h_ea_.end(), h.e_a.begin(), h.e_a.end());
             h_eb_.insert(h_eb_.end(), h.e_b.begin(), h.e_b.end());
-        } else if (t == ST_COMPOUND && !remap) {
-            inertia = M3<R>();   // set by set_compounds (CompoundShape::init)
-        } else {
-            throw std::runtime_error(t == ST_COMPOUND ? "compound shapes are not supported in batched requests"
-                                                      : "unsupported shape type " + std::to_string(t));
+        } else {   // a compound: set by set_compounds (CompoundShape::init)
+            inertia = M3<R>();
         }
         h_cbeg_.push_back(0);
         h_ccnt_.push_back(0);
@@ -236,14 +244,6 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
     }
     // hull face offsets are global per face: face f of hull h sits at hfb[h] + f, its offsets at
     // f_off[hfb[h] + f] .. f_off[hfb[h] + f + 1]
-    S_ = s0 + added;
-    for (size_t s = s0; s < h_stype_.size(); s++) kinds_ |= 1u << h_stype_[s];
-    for (size_t h = o_h; h < h_hvc_.size(); h++) {
-        most_faces_ = std::max(most_faces_, h_hfc_[h]);
-        most_edges_ = std::max(most_edges_, h_hec_[h]);
-        most_verts_ = std::max(most_verts_, h_hvc_[h]);
-    }
-    shape_by_content_.merge(fresh);
     // a request whose shapes are all known already (each one's primitives were appended again, five
     // uploads, a launch and two waits per request)
     if (remap && added == 0) return s0;
@@ -262,6 +262,15 @@ int World<R>::append_shapes(int S, const int* type, const double* param, const i
     hed_.ensure((size_t)std::max(n_edges, 1) * 3);
     if (n_edges > 0) launch(K_MISC, grid(n_edges), k_hull_edge_dirs<R>, n_edges, (const R*)hea_.p, (const R*)heb_.p, hed_.p);
     PE_CK(cudaStreamSynchronize(st_));
+    undo.back.clear();
+    S_ = s0 + added;
+    for (size_t s = s0; s < h_stype_.size(); s++) kinds_ |= 1u << h_stype_[s];
+    for (size_t h = o_h; h < h_hvc_.size(); h++) {
+        most_faces_ = std::max(most_faces_, h_hfc_[h]);
+        most_edges_ = std::max(most_edges_, h_hec_[h]);
+        most_verts_ = std::max(most_verts_, h_hvc_[h]);
+    }
+    shape_by_content_.merge(fresh);
     return s0;
 }
 
