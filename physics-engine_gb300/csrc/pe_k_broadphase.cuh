@@ -164,10 +164,15 @@ __device__ __forceinline__ int sweep_warp(int i, int n, int lane, const int* sce
     return c;
 }
 
-// A position whose window along the axis holds more than kBigWindow candidates (a floor or a wall
+// A position whose window along the axis holds more than big_window_limit candidates (a floor or a wall
 // spanning the scene) is swept by blocks instead of a warp: 256 candidates per iteration, warp
 // ballots plus a block prefix of the warp counts keep the pairs in ascending j.
-constexpr int kBigWindow = 4096;        // about 32 steps of four chunks for a warp
+// The limit: what a warp sweeps in some 32 steps of four chunks, and at least an eighth of the largest
+// scene, so that only bodies that span the scene exceed it.  Where bodies lie so close that ordinary
+// windows hold thousands, nearly every position would go to the blocks, two searches and a chunk each
+// (POUR_FIGURES).
+constexpr int kBigWindow = 4096;
+inline int big_window_limit(int largest_scene) { return kBigWindow > largest_scene / 8 ? kBigWindow : largest_scene / 8; }
 constexpr int kNoBigWindow = 1 << 30;   // limit of a caller without the chunk kernels
 template <class R>
 __device__ __forceinline__ bool big_window(int i, int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sscene) {

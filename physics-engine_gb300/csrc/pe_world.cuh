@@ -452,7 +452,7 @@ private:
     DBuf<int> bp_wend_, bp_csize_, bp_nch_, bp_choff_, bp_ctot_, bp_ccount_, bp_cpref_;   // crowded windows in chunks
     static constexpr int kBigSweepBlocks = 152;   // blocks that share the crowded positions
     uint32_t* order_ = nullptr;   // sorted body order (points into val_)
-    int max_scene_ = 0;           // bodies of the largest scene (set with h_scene_off_; the crowded-window kernels run above kBigWindow)
+    int max_scene_ = 0;           // bodies of the largest scene (set with h_scene_off_; the crowded-window kernels run above big_window_limit)
     DBuf<int2> pairs_;
     int P_ = 0, pair_cap_ = 0;
     // narrowphase

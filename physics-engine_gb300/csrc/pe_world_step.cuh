@@ -98,11 +98,12 @@ template <class R> void World<R>::bp_count_enqueue() {
     IgnoreLists ign;
     if (n_ign_ > 0) { ign.off = ign_off_.p; ign.ids = ign_ids_.p; ign.order = order_; }
     const bool share = n >= kSweepSharedFrom;
-    launch(K_BP_SWEEP, grid_warps(share ? (n + kSweepShare - 1) / kSweepShare : n), share ? k_bp_count_shared<R> : k_bp_count<R>, n, kBigWindow, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, count_.p, bp_stage_.p,
+    const int limit = big_window_limit(max_scene_);
+    launch(K_BP_SWEEP, grid_warps(share ? (n + kSweepShare - 1) / kSweepShare : n), share ? k_bp_count_shared<R> : k_bp_count<R>, n, limit, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, count_.p, bp_stage_.p,
            bp_big_.p, bp_nbig_.p, ign);
     // crowded positions: windows in chunks of one block each (at most kMaxChunks per position); a
-    // window holds at most the scene's other bodies, so scenes of at most kBigWindow bodies have none
-    const bool crowded = max_scene_ > kBigWindow;
+    // window holds at most the scene's other bodies, so scenes of at most `limit` bodies have none
+    const bool crowded = max_scene_ > limit;
     bp_wend_.ensure(n + 1); bp_csize_.ensure(n + 1); bp_nch_.ensure(n + 1); bp_choff_.ensure(n + 1); bp_ctot_.ensure(1);
     bp_ccount_.ensure((size_t)kMaxChunks * n + 1); bp_cpref_.ensure((size_t)kMaxChunks * n + 1);
     if (crowded) launch(K_BP_SWEEP, kBigSweepBlocks, k_bp_big_windows<R>, n, (const int*)scene_axis_.p, (const int*)scene_off_.p, (const R*)smn_.p,
@@ -158,13 +159,13 @@ template <class R> void World<R>::prepare_tail(int P) {
 
 // the pair list from the counted sweep, and each scene's first pair
 template <class R> void World<R>::bp_tail() {
-    const int n = N_;
+    const int n = N_, limit = big_window_limit(max_scene_);
     if (n < 2) return;
     IgnoreLists ign;
     if (n_ign_ > 0) { ign.off = ign_off_.p; ign.ids = ign_ids_.p; ign.order = order_; }
-    launch(K_BP_SWEEP, grid_warps(n), k_bp_write<R>, n, kBigWindow, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, order_, count_.p, bp_stage_.p,
+    launch(K_BP_SWEEP, grid_warps(n), k_bp_write<R>, n, limit, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, order_, count_.p, bp_stage_.p,
            pairs_.p, pair_cap_, status_.p, ign, NS_, (const int*)scene_off_.p, pair_scene_off_.p);
-    if (max_scene_ > kBigWindow)
+    if (max_scene_ > limit)
         launch(K_BP_SWEEP, 2 * kBigSweepBlocks, k_bp_write_chunks<R>, n, (const R*)smn_.p, (const R*)smx_.p, (const int*)sflag_.p,
                (const uint32_t*)order_, (const int*)count_.p, (const int*)bp_big_.p, (const int*)bp_nbig_.p, (const int*)bp_wend_.p,
                (const int*)bp_csize_.p, (const int*)bp_choff_.p, (const int*)bp_ctot_.p, (const int*)bp_cpref_.p, pairs_.p, pair_cap_,

@@ -94,3 +94,17 @@ def test_windows_of_four_positions_end_with_their_scene(bits):
         want.append(alone.pairs().reshape(-1, 2) + int(offs[k]))
     assert np.array_equal(g.pairs().reshape(-1, 2), np.concatenate(want))
     g.close()
+
+
+def test_windows_of_blocks_in_a_large_scene():
+    """A scene of 40,000 bodies: blocks take windows of more than an eighth of it, warps shared by four
+    positions those of 4,097 to 5,000."""
+    s = _line(39993, (4096, 4097, 4999, 5000, 5001, 6200, 39000), 32, seed=9)
+    assert s.n_bodies == 40000
+    g, o = pg.GpuWorld(s, 32), orc.OracleWorld(s, 32, stable_ties=True)
+    for _ in range(2):
+        g.step(1, pg.SERIAL_ORDER)
+        o.step(1)
+        assert np.array_equal(g.pairs(), o.pairs())
+        assert g.axis == o.axis
+    g.close()
