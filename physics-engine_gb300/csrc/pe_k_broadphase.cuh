@@ -31,10 +31,13 @@ __global__ void k_bp_keys(Bodies<R> B, const int* scene_axis, typename KeyOf<R>:
 template <class R> struct SweepBoxes {
     R *mn, *mx;
     int *flag, *scene;
+    int* lost;   // set where a box's minimum is not a number (cleared by k_bp_axis)
     __device__ __forceinline__ void copy(const Bodies<R>& B, int k, int i) const {
         for (int d = 0; d < 3; d++) {
-            mn[(size_t)d * B.n + k] = B.at(MNX + d, i);
+            const R m = B.at(MNX + d, i);
+            mn[(size_t)d * B.n + k] = m;
             mx[(size_t)d * B.n + k] = B.at(MXX + d, i);
+            if (m != m) *lost = 1;
         }
         flag[k] = B.flags[i];
         scene[k] = B.scene[i];
@@ -174,6 +177,12 @@ __device__ __forceinline__ int sweep_warp(int i, int n, int lane, const int* sce
 constexpr int kBigWindow = 4096;
 inline int big_window_limit(int largest_scene) { return kBigWindow > largest_scene / 8 ? kBigWindow : largest_scene / 8; }
 constexpr int kNoBigWindow = 1 << 30;   // limit of a caller without the chunk kernels
+// A box that is not a number compares as overlapping everything and lies anywhere in the order.  What a
+// position meets of it past its window's end depends on where the window's chunks of 32 begin and on
+// which kernel sweeps it; so in a world with one every window up to kLostWindow is swept by a warp of
+// its own, in chunks from the position on, by the count and the write alike.
+constexpr int kLostWindow = 32768;
+__device__ __forceinline__ int window_limit(int limit, const int* lost) { return lost && *lost ? max(limit, kLostWindow) : limit; }
 template <class R>
 __device__ __forceinline__ bool big_window(int i, int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sscene) {
     if (limit >= n - i) return false;
@@ -283,8 +292,9 @@ __global__ void k_bp_write_chunks(int n, const R* smn, const R* smx, const int* 
 }
 
 template <class R>
-__global__ void k_bp_count(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene, int* count,
-                           int* stage, int* big, int* n_big, IgnoreLists ign) {
+__global__ void k_bp_count(int n, int limit0, const int* lost, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
+                           int* count, int* stage, int* big, int* n_big, IgnoreLists ign) {
+    const int limit = window_limit(limit0, lost);
     const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (i >= n) return;
@@ -303,8 +313,9 @@ __global__ void k_bp_count(int n, int limit, const int* scene_axis, const R* smn
 // that a warp per position fills the GPU, and the longest window decides.
 constexpr int kSweepShare = 4, kSweepSharedFrom = 16384;
 template <class R>
-__global__ void k_bp_count_shared(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
-                                  int* count, int* stage, int* big, int* n_big, IgnoreLists ign) {
+__global__ void k_bp_count_shared(int n, int limit0, const int* lost, const int* scene_axis, const R* smn, const R* smx, const int* sflag,
+                                  const int* sscene, int* count, int* stage, int* big, int* n_big, IgnoreLists ign) {
+    const int limit = window_limit(limit0, lost);
     constexpr int U = kSweepShare;
     const int i0 = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5) * U;
     const int lane = threadIdx.x & 31;
@@ -333,26 +344,31 @@ __global__ void k_bp_count_shared(int n, int limit, const int* scene_axis, const
             alive |= 1u << u;
         }
     }
-    for (int j0 = i0 + 1; alive && j0 < n; j0 += 32) {
-        const int j = j0 + lane, k = min(j, n - 1);
-        const V3<R> lo(smn[k], smn[n + k], smn[2 * (size_t)n + k]), hi(smx[k], smx[n + k], smx[2 * (size_t)n + k]);
-        const int fj = sflag[k], sj = sscene[k];
+    const bool alone = *lost != 0;   // one position after the other then (see window_limit)
+    for (unsigned left = alive; left;) {
+        alive = alone ? left & (0u - left) : left;
+        left &= ~alive;
+        for (int j0 = i0 + __ffs(alive); alive && j0 < n; j0 += 32) {
+            const int j = j0 + lane, k = min(j, n - 1);
+            const V3<R> lo(smn[k], smn[n + k], smn[2 * (size_t)n + k]), hi(smx[k], smx[n + k], smx[2 * (size_t)n + k]);
+            const int fj = sflag[k], sj = sscene[k];
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (!(alive >> u & 1u)) continue;   // the same for the whole warp
-            const R low = ax[u] == 0 ? lo.x : ax[u] == 1 ? lo.y : lo.z;
-            const bool past = j <= i0 + u, in = j < n && !(low > top[u]) && sj == sc[u];
-            const unsigned live = __ballot_sync(full, past || in);
-            bool hit = in && !past && !(fj & BF_IGNORE) && !((fi[u] & BF_KINEMATIC) && (fj & BF_KINEMATIC)) &&
-                       !(mn[u].x > hi.x || lo.x > mx[u].x) && !(mn[u].y > hi.y || lo.y > mx[u].y) && !(mn[u].z > hi.z || lo.z > mx[u].z);
-            if (hit && ign.off && ((fi[u] | fj) & BF_IGN_LIST)) hit = !ign.ignored(i0 + u, j);
-            const unsigned m = __ballot_sync(full, hit);
-            if (hit) {
-                const int at = c[u] + __popc(m & ((1u << lane) - 1u));
-                if (at < kStage) stage[(size_t)(i0 + u) * kStage + at] = j;
+            for (int u = 0; u < U; u++) {
+                if (!(alive >> u & 1u)) continue;   // the same for the whole warp
+                const R low = ax[u] == 0 ? lo.x : ax[u] == 1 ? lo.y : lo.z;
+                const bool past = j <= i0 + u, in = j < n && !(low > top[u]) && sj == sc[u];
+                const unsigned live = __ballot_sync(full, past || in);
+                bool hit = in && !past && !(fj & BF_IGNORE) && !((fi[u] & BF_KINEMATIC) && (fj & BF_KINEMATIC)) &&
+                           !(mn[u].x > hi.x || lo.x > mx[u].x) && !(mn[u].y > hi.y || lo.y > mx[u].y) && !(mn[u].z > hi.z || lo.z > mx[u].z);
+                if (hit && ign.off && ((fi[u] | fj) & BF_IGN_LIST)) hit = !ign.ignored(i0 + u, j);
+                const unsigned m = __ballot_sync(full, hit);
+                if (hit) {
+                    const int at = c[u] + __popc(m & ((1u << lane) - 1u));
+                    if (at < kStage) stage[(size_t)(i0 + u) * kStage + at] = j;
+                }
+                c[u] += __popc(m);
+                if (live != full) alive &= ~(1u << u);
             }
-            c[u] += __popc(m);
-            if (live != full) alive &= ~(1u << u);
         }
     }
     if (lane == 0)
@@ -361,7 +377,7 @@ __global__ void k_bp_count_shared(int n, int limit, const int* scene_axis, const
 }
 
 template <class R>
-__global__ void k_bp_write(int n, int limit, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
+__global__ void k_bp_write(int n, int limit0, const int* lost, const int* scene_axis, const R* smn, const R* smx, const int* sflag, const int* sscene,
                            const uint32_t* order, const int* offset, const int* stage, int2* pairs, int pair_cap, int* status,
                            IgnoreLists ign, int n_scenes, const int* scene_off, int* pair_scene_off) {
     const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
@@ -369,6 +385,7 @@ __global__ void k_bp_write(int n, int limit, const int* scene_axis, const R* smn
     // each scene's first pair: that of its first sorted position
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s <= n_scenes; s += gridDim.x * blockDim.x) pair_scene_off[s] = offset[scene_off[s]];
     if (i >= n) return;
+    const int limit = window_limit(limit0, lost);
     const int base = offset[i], c = offset[i + 1] - base;
     if (c == 0 || big_window(i, n, limit, scene_axis, smn, smx, sscene)) return;   // big windows: k_bp_write_chunks
     if (base + c > pair_cap) {
@@ -392,12 +409,13 @@ __global__ void k_bp_write(int n, int limit, const int* scene_axis, const R* smn
 // bodies keeps its axis (the reference returns before updating it).
 template <class R> constexpr int axis_chunk() { return sizeof(R) == 4 ? 1024 : 512; }   // centres per staged chunk
 template <class R>
-__global__ void __launch_bounds__(64) k_bp_axis(const R* smn, const R* smx, int n, const int* scene_off, int* scene_axis) {
+__global__ void __launch_bounds__(64) k_bp_axis(const R* smn, const R* smx, int n, const int* scene_off, int* scene_axis, int* lost) {
     constexpr int CH = axis_chunk<R>(), PAD = CH + 1;   // the padding puts the three rows in different banks
     __shared__ R cbuf[2][3 * PAD];
     __shared__ R sums[6];
     const int s = blockIdx.x, tid = threadIdx.x;
     const int lo = scene_off[s], hi = scene_off[s + 1], cnt = hi - lo;
+    if (s == 0 && tid == 0) *lost = 0;   // (the last kernel of a broadphase)
     if (cnt < 2) return;   // whole block
     auto stage = [&](int buf, int base, int t) {   // t in [0, 32): the staging warp's lane
         const int e = min(CH, hi - base);

@@ -209,7 +209,7 @@ extern "C" int pe_gpu_sap_pairs_noalloc(int device, int n, const float* aabb_min
     k_sap_gather<<<g, kBlock, 0, st>>>(n, aabb_min, aabb_max, flags, order, smn, smx, sflag, sscene, count, status, n_big);
     const int gw = (int)(((size_t)n * 32 + kBlock - 1) / kBlock);
     const IgnoreLists no_lists;   // this entry point takes no ignored-pair lists
-    k_bp_count<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, count, stage, big, n_big, no_lists);
+    k_bp_count<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, nullptr, scene_axis, smn, smx, sflag, sscene, count, stage, big, n_big, no_lists);
     if (n + 1 <= kScanOne) {
         k_scan_one<<<1, kScanOneBlock, 0, st>>>(count, n + 1, total, nullptr);
     } else {
@@ -217,7 +217,7 @@ extern "C" int pe_gpu_sap_pairs_noalloc(int device, int n, const float* aabb_min
         k_scan_sums<<<ct, kBlock, 0, st>>>(count, n + 1, aux);
         k_scan_apply<<<ct, kBlock, 0, st>>>(count, n + 1, aux, total, nullptr);
     }
-    k_bp_write<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, scene_axis, smn, smx, sflag, sscene, order, count, stage, reinterpret_cast<int2*>(pairs),
+    k_bp_write<float><<<gw, kBlock, 0, st>>>(n, kNoBigWindow, nullptr, scene_axis, smn, smx, sflag, sscene, order, count, stage, reinterpret_cast<int2*>(pairs),
                                              pair_cap, status, no_lists, -1, nullptr, nullptr);
     k_sap_total<<<1, 1, 0, st>>>(total, n_pairs);
     const cudaError_t e = cudaGetLastError();

@@ -448,7 +448,7 @@ private:
     DBuf<uint32_t> val_[2];
     DBuf<int> hist_, aux_, count_, status_;
     DBuf<R> smn_, smx_;
-    DBuf<int> sflag_, ssc_, bp_stage_, bp_big_, bp_nbig_;
+    DBuf<int> sflag_, ssc_, bp_stage_, bp_big_, bp_nbig_;   // bp_nbig_: crowded positions; SweepBoxes::lost
     DBuf<int> bp_wend_, bp_csize_, bp_nch_, bp_choff_, bp_ctot_, bp_ccount_, bp_cpref_;   // crowded windows in chunks
     static constexpr int kBigSweepBlocks = 152;   // blocks that share the crowded positions
     uint32_t* order_ = nullptr;   // sorted body order (points into val_)

@@ -28,6 +28,8 @@ template <class R> World<R>::World(int device) : dev_(device) {
     } else {
         PE_CK(cudaMemcpyToSymbol(g_unit_f64, &u, sizeof(UnitMeshesOf<double>)));
     }
+    bp_nbig_.ensure(2);
+    PE_CK(cudaMemset(bp_nbig_.p, 0, 2 * sizeof(int)));
     status_.ensure(1);
     PE_CK(cudaMemset(status_.p, 0, sizeof(int)));
     rows_total_.ensure(1);

@@ -75,9 +75,8 @@ template <class R> void World<R>::bp_count_enqueue() {
     count_.ensure(n + 1);
     bp_stage_.ensure((size_t)n * kStage);
     bp_big_.ensure(n + 1);
-    bp_nbig_.ensure(1);
     SweepBoxes<R> boxes;
-    boxes.mn = smn_.p; boxes.mx = smx_.p; boxes.flag = sflag_.p; boxes.scene = ssc_.p;
+    boxes.mn = smn_.p; boxes.mx = smx_.p; boxes.flag = sflag_.p; boxes.scene = ssc_.p; boxes.lost = bp_nbig_.p + 1;
     if (max_scene_ <= std::min(tun_.scene_sort_max, kSceneSortMax)) {   // every scene sorted inside one block
         launch_block(K_RADIX, NS_, kSceneSortBlock, k_bp_sort_scenes<R>, bodies(), (const int*)scene_axis_.p, (const int*)scene_off_.p,
                      val_[0].p, boxes, bp_nbig_.p);
@@ -99,7 +98,8 @@ template <class R> void World<R>::bp_count_enqueue() {
     if (n_ign_ > 0) { ign.off = ign_off_.p; ign.ids = ign_ids_.p; ign.order = order_; }
     const bool share = n >= kSweepSharedFrom;
     const int limit = big_window_limit(max_scene_);
-    launch(K_BP_SWEEP, grid_warps(share ? (n + kSweepShare - 1) / kSweepShare : n), share ? k_bp_count_shared<R> : k_bp_count<R>, n, limit, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, count_.p, bp_stage_.p,
+    launch(K_BP_SWEEP, grid_warps(share ? (n + kSweepShare - 1) / kSweepShare : n), share ? k_bp_count_shared<R> : k_bp_count<R>, n, limit,
+           (const int*)boxes.lost, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, count_.p, bp_stage_.p,
            bp_big_.p, bp_nbig_.p, ign);
     // crowded positions: windows in chunks of one block each (at most kMaxChunks per position); a
     // window holds at most the scene's other bodies, so scenes of at most `limit` bodies have none
@@ -163,7 +163,7 @@ template <class R> void World<R>::bp_tail() {
     if (n < 2) return;
     IgnoreLists ign;
     if (n_ign_ > 0) { ign.off = ign_off_.p; ign.ids = ign_ids_.p; ign.order = order_; }
-    launch(K_BP_SWEEP, grid_warps(n), k_bp_write<R>, n, limit, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, order_, count_.p, bp_stage_.p,
+    launch(K_BP_SWEEP, grid_warps(n), k_bp_write<R>, n, limit, (const int*)bp_nbig_.p + 1, scene_axis_.p, smn_.p, smx_.p, sflag_.p, ssc_.p, order_, count_.p, bp_stage_.p,
            pairs_.p, pair_cap_, status_.p, ign, NS_, (const int*)scene_off_.p, pair_scene_off_.p);
     if (max_scene_ > limit)
         launch(K_BP_SWEEP, 2 * kBigSweepBlocks, k_bp_write_chunks<R>, n, (const R*)smn_.p, (const R*)smx_.p, (const int*)sflag_.p,
@@ -177,7 +177,7 @@ template <class R> void World<R>::bp_tail() {
 // step runs it beside its narrowphase and solver, on a stream of its own.
 template <class R> void World<R>::bp_axis() {
     if (N_ < 2) return;
-    launch_block(K_BP_AXIS, NS_, 64, k_bp_axis<R>, (const R*)smn_.p, (const R*)smx_.p, N_, (const int*)scene_off_.p, scene_axis_.p);
+    launch_block(K_BP_AXIS, NS_, 64, k_bp_axis<R>, (const R*)smn_.p, (const R*)smx_.p, N_, (const int*)scene_off_.p, scene_axis_.p, bp_nbig_.p + 1);
 }
 template <class R> void World<R>::bp_axis_begin() {
     PE_CK(cudaEventRecord(axis_ev_[0], st_));   // the pair list has been written: its sweep reads the axes

@@ -108,3 +108,51 @@ def test_windows_of_blocks_in_a_large_scene():
         assert np.array_equal(g.pairs(), o.pairs())
         assert g.axis == o.axis
     g.close()
+
+
+def _swept(mn, mx, kinematic, axis):
+    """The pairs of one scene's sweep in chunks of 32 from each position on; a box that is not a number has
+    zero's place in the order."""
+    order = np.argsort(np.nan_to_num(mn[:, axis]), kind="stable")
+    mn, mx, kinematic = mn[order], mx[order], kinematic[order]
+    out = []
+    with np.errstate(invalid="ignore"):
+        for i in range(len(mn)):
+            for j0 in range(i + 1, len(mn), 32):
+                j = np.arange(j0, min(j0 + 32, len(mn)))
+                inside = ~(mn[j, axis] > mx[i, axis])
+                hit = inside & ~((mn[i] > mx[j]) | (mn[j] > mx[i])).any(1) & ~(kinematic[i] & kinematic[j])
+                out += [(order[i], order[k]) for k in j[hit]]
+                if len(j) < 32 or not inside.all():
+                    break
+    return np.array(out, np.int32).reshape(-1, 2)
+
+
+@pytest.mark.parametrize("n", [5000, 16389])   # a warp per position, and one for four
+@pytest.mark.parametrize("lost", [1, 2, 3, 30])
+@pytest.mark.parametrize("bits", [32, 64])
+def test_windows_beside_boxes_that_are_not_numbers(bits, lost, n):
+    """Windows that end shortly before such boxes, of single boxes and of slabs longer than the blocks' limit."""
+    sb = sc.SceneBuilder(dt=1.0 / 60.0, iterations=2, gravity=(0.0, 0.0, 0.0))
+    box = sb.shape(sc.BOX, (12.4, 0.9, 0.9))   # twelve partners each: more than are kept for the write
+    for i in range(n - 4):
+        sb.body(box, (float(i - n + 300), 0.0, 0.0), mass=1.0)
+    for k in range(4):
+        sb.body(sb.shape(sc.BOX, (4400.0, 1.0, 2.0)), (-2200.0 - 9.0 * k - 5.3, 0.0, 0.0), mass=0.0, kinematic=True)
+    g = pg.GpuWorld(sb.build(bits), bits)
+    st = g.state()
+    at = np.random.default_rng(lost).permutation(n - 4)[:lost]
+    st["origin"][at] = np.nan
+    kinematic = np.arange(n) >= n - 4
+    for again in range(2):
+        g.axis = 0
+        g.set_state({"origin": st["origin"]})
+        g.integrate()
+        g.broadphase()
+        s = g.state(fields=("aabb_min", "aabb_max"))
+        want = _swept(s["aabb_min"], s["aabb_max"], kinematic, 0)
+        got = g.pairs().reshape(-1, 2)
+        assert np.isnan(s["aabb_min"][at]).all() != bool(again) and len(want) > 11 * n
+        assert np.array_equal(got, want)
+        st["origin"][at] = 1e4 + 20.0 * np.arange(lost)[:, None]   # then no such box any more
+    g.close()
