@@ -12,6 +12,10 @@
 //
 // Islands of up to kWarpIsland items run inside one warp with the tokens in shared memory
 // (k_isl_warp); larger ones over the whole grid with the tokens in global memory (k_isl_flow).
+//
+// A caller's result may name one body on both sides (SELF; no sweep gives such a pair).  Its item holds
+// the body's token once, on side b; side a starts every iteration from the same velocities and is dropped
+// after it.
 #pragma once
 #include "pe_k_solver.cuh"
 
@@ -130,7 +134,7 @@ __host__ __device__ inline long long class_base(int c, long long bound) {
 // (One thread per island of up to 16 items, the larger ones a block each with a barrier per level:
 // 266 + 150 us of the 501-body pile's step, 1,448 + 718 us of the 4,096 piles'; together with the
 // item-sized islands in one kernel here the steps are 309 us and 1.24 ms shorter.)
-template <class R, bool JOINTS>
+template <class R, bool JOINTS, bool SELF>
 __global__ void __launch_bounds__(kWarpBlock, sizeof(R) == 4 ? 4 : 2)
 k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, const uint32_t* order, Results<R> res, Joints<R> J, Bodies<R> B,
            Rows<R> rows, int iterations, int color_min, int* n_colors, int* status) {
@@ -179,7 +183,8 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
         t.ia = -1; t.ib = -1;
         if (active) t.load(order[lo + idx], res, J, B, rows);
         // the island's items on this item's bodies (bit per item), and on which side they hold them
-        const int da = active && !t.a.kin ? t.ia : -2, db = active && !t.b.kin ? t.ib : -2;
+        const bool own_a = active && !t.a.kin && !(SELF && t.ia == t.ib);   // side a has a token of its own
+        const int da = own_a ? t.ia : -2, db = active && !t.b.kin ? t.ib : -2;
         unsigned ma = 0, mab = 0, mb = 0, mbb = 0;
         for (int j = 0; j < s; j++) {
             const int oa = __shfl_sync(full, t.ia, g0 + j), ob = __shfl_sync(full, t.ib, g0 + j);
@@ -191,13 +196,13 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
         }
         const unsigned before = (1u << idx) - 1u, after = ~(before | (1u << idx));
         const bool wrap_a = (ma & after) == 0, wrap_b = (mb & after) == 0;
-        const int na = active && !t.a.kin ? __ffs(wrap_a ? ma : ma & after) - 1 : 0, nb = active && !t.b.kin ? __ffs(wrap_b ? mb : mb & after) - 1 : 0;
+        const int na = own_a ? __ffs(wrap_a ? ma : ma & after) - 1 : 0, nb = active && !t.b.kin ? __ffs(wrap_b ? mb : mb & after) - 1 : 0;
         const int sa = (mab >> na) & 1, sb = (mbb >> nb) & 1;
         const bool keep_a = na == idx, keep_b = nb == idx;   // the body's only item: its token stays in registers
         tok_it[warp][0][lane] = tok_it[warp][1][lane] = -1;
         int lev_a = 0, lev_b = 0;
-        bool have_a = !active || t.a.kin, have_b = !active || t.b.kin;
-        if (active && !t.a.kin && (ma & before) == 0) { t.a.v = B.vec(VX, t.ia); t.a.w = B.vec(WX, t.ia); have_a = true; }
+        bool have_a = !own_a, have_b = !active || t.b.kin;
+        if (own_a && (ma & before) == 0) { t.a.v = B.vec(VX, t.ia); t.a.w = B.vec(WX, t.ia); have_a = true; }
         if (active && !t.b.kin && (mb & before) == 0) { t.b.v = B.vec(VX, t.ib); t.b.w = B.vec(WX, t.ib); have_b = true; }
         int it = active ? 0 : its;
         __syncwarp();
@@ -221,6 +226,7 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
             }
             // (the vote also puts every read of this round's tokens before its writes)
             if (run) {
+                if (SELF && t.ia == t.ib) { t.a.v = t.b.v; t.a.w = t.b.w; }
                 if (iterations > 0) t.iterate(J, rows);
                 const int lev = (lev_a > lev_b ? lev_a : lev_b) + 1;
                 if (it == 0 && m > color_min) deepest = deepest > lev ? deepest : lev;
@@ -239,7 +245,7 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
                     tok_it[warp][side][g0 + nl] = it + (wrap ? 1 : 0);
                     have = false;
                 };
-                give(t.a, t.ia, wrap_a, na, sa, keep_a, have_a);
+                if (!SELF || own_a) give(t.a, t.ia, wrap_a, na, sa, keep_a, have_a);
                 give(t.b, t.ib, wrap_b, nb, sb, keep_b, have_b);
                 it++;
             }
@@ -334,7 +340,7 @@ constexpr int kFlowStall = 1 << 21;   // polls in a row without progress after w
 // time is the latency of the longest chain, a hand-over through L2 plus one item's rows.  (A block
 // per island with a barrier per level, and one barrier over the whole grid per level for large
 // islands, took 3.4 and 11 us per level and iteration.)
-template <class R, bool JOINTS>
+template <class R, bool JOINTS, bool SELF>
 __global__ void __launch_bounds__(kFlowBlock, sizeof(R) == 4 ? 4 : 2)
 k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows) {
     constexpr int NW = token_words<R>();
@@ -347,6 +353,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
     const int its = f.iterations > 0 ? f.iterations : 1;
     const bool coloring = f.mode != 0 && *f.n_big > 0;
     auto dynamic = [&](int i) { return (B.flags[i] & BF_KINEMATIC) == 0; };
+    auto own_a = [&](int2 q) { return !(SELF && q.x == q.y) && dynamic(q.x); };   // side a has a token of its own
     auto island_size = [&](int s) { return f.isl_off[s + 1] - f.isl_off[s]; };
 
     // the flow items, in island order
@@ -368,7 +375,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
     // every body's entries
     for (int j = t; j < M; j += T) {
         const int2 q = item_bodies(f.item[j], res, J);
-        if (dynamic(q.x)) f.next[2 * j] = atomicExch(&f.head[q.x], 2 * j);
+        if (own_a(q)) f.next[2 * j] = atomicExch(&f.head[q.x], 2 * j);
         if (dynamic(q.y)) f.next[2 * j + 1] = atomicExch(&f.head[q.y], 2 * j + 1);
     }
     grid.sync();
@@ -399,7 +406,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
     for (int j = t; j < M; j += T) {
         const int2 q = item_bodies(f.item[j], res, J);
         const bool colors = coloring && island_size(f.isl[j]) > f.big_items;
-        if (dynamic(q.x)) link(2 * j, q.x, colors);
+        if (own_a(q)) link(2 * j, q.x, colors);
         if (dynamic(q.y)) link(2 * j + 1, q.y, colors);
     }
     grid.sync();
@@ -429,7 +436,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
             bool moved = false;
             if (j < M) {
                 const int2 q = item_bodies(f.item[j], res, J);
-                const bool da = dynamic(q.x), db = dynamic(q.y);
+                const bool da = own_a(q), db = dynamic(q.y);
                 uint4 wa = make_uint4(0, 0, 0, 1), wb = wa;
                 if (da) wa = ld_word(f.box + (size_t)(2 * j) * NW);
                 if (db) wb = ld_word(f.box + (size_t)(2 * j + 1) * NW);
@@ -484,7 +491,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
         for (int j = t; j < M; j += T) {
             if (island_size(f.isl[j]) <= f.big_items) continue;
             const int2 q = item_bodies(f.item[j], res, J);
-            if (dynamic(q.x)) link(2 * j, q.x, false);
+            if (own_a(q)) link(2 * j, q.x, false);
             if (dynamic(q.y)) link(2 * j + 1, q.y, false);
         }
         grid.sync();
@@ -500,9 +507,9 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
     bool have_a = false, have_b = false;
     auto take_item = [&](int j) {
         x.load(f.item[j], res, J, B, rows);
-        have_a = x.a.kin;
+        have_a = x.a.kin || (SELF && x.ia == x.ib);
         have_b = x.b.kin;
-        if (!x.a.kin) succ_a = f.succ[2 * j];
+        if (!have_a) succ_a = f.succ[2 * j];
         if (!x.b.kin) succ_b = f.succ[2 * j + 1];
         lev_a = 0;
         lev_b = 0;
@@ -534,6 +541,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
         if (j < M) {
             if (!have_a) have_a = token_get(f.box + (size_t)(2 * j) * NW, x.a, it, lev_a);
             if (!have_b) have_b = token_get(f.box + (size_t)(2 * j + 1) * NW, x.b, it, lev_b);
+            if (SELF && have_b && x.ia == x.ib) { x.a.v = x.b.v; x.a.w = x.b.w; }
         }
         if constexpr (kByWarp) {
             const bool ready = j < M && have_a && have_b && f.iterations > 0 && !(JOINTS && (x.id & kJointItem));
@@ -579,7 +587,7 @@ k_isl_flow(FlowArgs<R> f, Results<R> res, Joints<R> J, Bodies<R> B, Rows<R> rows
                     }
                     have = false;
                 };
-                give(x.a, x.ia, 2 * j, succ_a, have_a);
+                if (!SELF || x.ia != x.ib) give(x.a, x.ia, 2 * j, succ_a, have_a);
                 give(x.b, x.ib, 2 * j + 1, succ_b, have_b);
                 if (it == 0) {
                     if (m > f.big_items) { if (f.mode == 0) atomicMax(&f.isl_levels[f.isl[j]], lev); }

@@ -316,7 +316,7 @@ private:
     DBuf<uint32_t> flow_item_;
     DBuf<int> flow_isl_, flow_color_, flow_head_, flow_next_, flow_succ_, flow_ff_;
     DBuf<uint4> flow_box_;
-    template <bool JOINTS> void solve_islands(int mode, const uint32_t* order);
+    template <bool JOINTS, bool SELF> void solve_islands(int mode, const uint32_t* order);
     // the pair count and the step's counters, written by kernels to page-locked memory
     // (k_step_counters writes them in this order)
     enum HostStat { HS_STATUS = 0, HS_ROWS, HS_ACTIVE, HS_ISLANDS, HS_BIG, HS_COLORS, HS_P, HS_CLS, HS_COUNT = HS_CLS + PC_COUNT };
@@ -367,6 +367,7 @@ private:
         const void* order;
         int n, ns, pair_cap, nj, n_ign, s, bcap, max_scene;
         unsigned classes;
+        int self;
         int plan[PC_COUNT];
         StepParams prm;
         R margin;
@@ -455,6 +456,7 @@ private:
     int max_scene_ = 0;           // bodies of the largest scene (set with h_scene_off_; the crowded-window kernels run above big_window_limit)
     DBuf<int2> pairs_;
     int P_ = 0, pair_cap_ = 0;
+    bool self_pairs_ = false, self_ = false;   // pairs, results with a body on both sides (a caller's)
     // narrowphase
     DBuf<int> cls_, cls_count_, order_np_;
     DBuf<int> res_a_, res_b_, res_np_;

@@ -121,6 +121,8 @@ static std::vector<int> scene_offsets(int n, const int* a, const std::vector<int
 template <class R> void World<R>::set_pairs(int n, const int* p) {
     for (int i = 0; i < 2 * n; i++) if (p[i] < 0 || p[i] >= N_) throw std::runtime_error("pair body index out of range");
     ensure_pair_capacity(std::max(n, 1));
+    self_pairs_ = false;
+    for (int i = 0; i < n; i++) self_pairs_ = self_pairs_ || p[2 * i] == p[2 * i + 1];
     if (n) PE_CK(cudaMemcpyAsync(pairs_.p, p, (size_t)n * sizeof(int2), cudaMemcpyHostToDevice, st_));
     h_pair_scene_off_ = scene_offsets(n, p, h_scene_off_);
     PE_CK(cudaMemcpyAsync(pair_scene_off_.p, h_pair_scene_off_.data(), (NS_ + 1) * sizeof(int), cudaMemcpyHostToDevice, st_));
@@ -201,6 +203,8 @@ void World<R>::set_results(int n, const int* a, const int* b, const int* ps, con
     PE_CK(cudaMemcpyAsync(dcnt_.p + DC_R, &n, sizeof(int), cudaMemcpyHostToDevice, st_));
     PE_CK(cudaStreamSynchronize(st_));
     R_ = n;
+    self_ = false;
+    for (int i = 0; i < n; i++) self_ = self_ || a[i] == b[i];
 }
 
 } // namespace pe

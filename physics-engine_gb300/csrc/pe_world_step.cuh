@@ -198,6 +198,7 @@ template <class R> int World<R>::broadphase() {
     bp_axis();
     PE_CK(cudaGetLastError());
     P_ = P;
+    if (N_ >= 2) self_pairs_ = false;   // (below two bodies the pair list stays)
     return P;
 }
 
@@ -332,6 +333,7 @@ template <class R> void World<R>::narrowphase() {
     np_enqueue();
     PE_CK(cudaGetLastError());
     R_ = P_;
+    self_ = self_pairs_;
 }
 
 // Solver without host waits: rows (on a side stream), islands (pe_k_islands.cuh), the iterations
@@ -376,20 +378,21 @@ template <class R> void World<R>::solve_enqueue(int mode) {
     }
     PE_CK(cudaEventRecord(join_ev_[0], side_[0]));
     PE_CK(cudaStreamWaitEvent(st_, join_ev_[0], 0));
-    if (NJ > 0) solve_islands<true>(mode, order);
-    else solve_islands<false>(mode, order);
+    if (self_) solve_islands<true, true>(mode, order);
+    else if (NJ > 0) solve_islands<true, false>(mode, order);
+    else solve_islands<false, false>(mode, order);
     launch_block(K_MISC, 1, 32, k_step_counters, (const int*)status_.p, (const int*)rows_total_.p, Ad, (const int*)isl_n_.p,
                  (const int*)(dcnt_.p + DC_NBIG), (const int*)isl_big_.p, (const int*)isl_levels_.p,
                  mode == 0 ? (const int*)nullptr : (const int*)ncol_.p, (const int*)cls_count_.p + 2 * PC_COUNT, hstat_);
 }
 
 // The solver's iterations: the islands that fit a warp, then those that do not.
-template <class R> template <bool JOINTS> void World<R>::solve_islands(int mode, const uint32_t* order) {
+template <class R> template <bool JOINTS, bool SELF> void World<R>::solve_islands(int mode, const uint32_t* order) {
     const int bound = pair_cap_ + n_joints_, small = tun_.small_island_items, big = tun_.big_island_items;
     int* n_list = dcnt_.p + DC_NLIST;
     int* colors = mode == 0 ? nullptr : ncol_.p;
     // (a warp for every island, up to the resident ones: see the islands per warp)
-    launch_block(K_SI_SERIAL, pgrid(bound, kWarpBlock / 32, k_isl_warp<R, JOINTS>, kWarpBlock), kWarpBlock, k_isl_warp<R, JOINTS>,
+    launch_block(K_SI_SERIAL, pgrid(bound, kWarpBlock / 32, k_isl_warp<R, JOINTS, SELF>, kWarpBlock), kWarpBlock, k_isl_warp<R, JOINTS, SELF>,
                  (const int*)isl_list_.p, (const int*)n_list, bound, (const int*)isl_off_.p, order, results(), joints(), bodies(), rows(),
                  prm_.iterations, small, colors, status_.p);
     FlowArgs<R> f;
@@ -399,8 +402,8 @@ template <class R> template <bool JOINTS> void World<R>::solve_islands(int mode,
     f.item = flow_item_.p; f.isl = flow_isl_.p; f.color = flow_color_.p; f.head = flow_head_.p; f.next = flow_next_.p; f.succ = flow_succ_.p;
     f.box = flow_box_.p; f.isl_levels = isl_levels_.p; f.isl_colors = isl_colors_.p; f.isl_state = isl_state_.p;
     f.any_first_fit = flow_ff_.p; f.n_colors = ncol_.p; f.status = status_.p;
-    launch_coop(K_SI_COLOR, resident(k_isl_flow<R, JOINTS>, kFlowBlock, 0), kFlowBlock, k_isl_flow<R, JOINTS>, f, results(), joints(), bodies(),
-                rows());
+    launch_coop(K_SI_COLOR, resident(k_isl_flow<R, JOINTS, SELF>, kFlowBlock, 0), kFlowBlock, k_isl_flow<R, JOINTS, SELF>, f, results(),
+                joints(), bodies(), rows());
 }
 
 // The step's second host wait: its counters and status.
@@ -437,6 +440,7 @@ template <class R> void World<R>::graph_sig(GraphSig& g) const {
     g.order = order_;
     g.n = N_; g.ns = NS_; g.pair_cap = pair_cap_; g.nj = n_joints_; g.n_ign = n_ign_; g.s = S_;
     g.classes = possible_classes();
+    g.self = self_;
     g.bcap = bcap_;
     g.max_scene = max_scene_;   // which sort the scenes take, and whether windows are swept in chunks
     std::memcpy(g.plan, stream_of_, sizeof g.plan);
@@ -547,6 +551,8 @@ template <class R> void World<R>::step(int n, int mode) {
         const int P = N_ < 2 ? P_ : hstat_[HS_P];
         prepare_tail(P);
         P_ = P;
+        if (N_ >= 2) self_pairs_ = false;
+        self_ = self_pairs_;
         cur_dist_ ^= 1;
         run_tail(mode);
         R_ = P;
