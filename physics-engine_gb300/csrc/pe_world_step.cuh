@@ -361,7 +361,7 @@ template <class R> void World<R>::solve_enqueue(int mode) {
     a.n_colors = mode == 0 ? nullptr : ncol_.p;
     const uint32_t* order = val_[0].p;
     int label_passes = 0;
-    for (int m = NJ > 0 ? N_ : N_ - 1; m > 0; m >>= 8) label_passes++;   // joint labels reach n_bodies
+    for (int m = std::max(NJ > 0 ? N_ : N_ - 1, 1); m > 0; m >>= 8) label_passes++;   // joint labels reach n_bodies; one at least places the keys
     if (bound <= kIslandOne && N_ <= kIslandOneBodies) {
         const size_t smem = island_one_smem(N_);
         launch_smem(K_ISLAND, 1, kIslandBlock, smem, k_islands_one, a, label_passes);

@@ -65,3 +65,22 @@ def test_modes_agree_on_results_of_a_body_with_itself(iterations, bits):
             got, _ = _gpu(scene, both, bits, mode, dict(small_island_items=1, big_island_items=big))
             for k in ("lin_vel", "ang_vel"):
                 np.testing.assert_array_equal(got[k], ref[k], err_msg=f"{mode} {big}: {k}")
+
+
+@pytest.mark.parametrize("m", [1, 2, 40, 2500])
+def test_world_of_one_body(m):
+    """All results are one island there, however many: its items in order."""
+    scene, both, _, _ = _with_self_results([1], 32, seed=8)
+    keep = 1   # the only dynamic body
+    for f in BODY:
+        setattr(scene, f, getattr(scene, f)[keep:keep + 1])
+    r = np.random.default_rng(m)
+    at = r.integers(0, len(both["res_a"]), m)
+    res = {k: v[at] for k, v in both.items()}
+    res["res_a"] = res["res_b"] = np.zeros(m, np.int32)
+    for mode in (pg.SERIAL_ORDER, pg.COLORED):
+        got, n = _gpu(scene, res, 32, mode)
+        assert (n["islands"], n["active"]) == (1, m)
+        ref, _ = _gpu(scene, res, 32, pg.SERIAL_ORDER, dict(small_island_items=0, big_island_items=1))
+        for k in ("lin_vel", "ang_vel"):
+            np.testing.assert_array_equal(got[k], ref[k])
