@@ -332,7 +332,11 @@ template <class R> struct FlowArgs {
 constexpr int kFlowBlock = 128, kFlowFirstFit = 1, kFlowLeft = 2;
 constexpr int kByWarpMost = 4;   // ready results of a warp up to which each takes the whole warp: 4 x 40 instructions against 170 for all at once, so that
                                // five would take longer
-constexpr int kFlowStall = 1 << 21;   // polls in a row without progress after which a warp gives up (seconds)
+// Polls in a row without progress after which a warp gives up (some ten seconds).  A warp holds an item of
+// every stride (38,912 in FP64, 77,824 in FP32), so it waits for a chain of about that many others at most,
+// however long the island: 0.4 s at the 10 us an item that 1,000,000 hinges in a row take in FP64 and, at
+// eight points an item beside a busy FP64 pipe, a second, where 1 << 21 polls would end.
+constexpr int kFlowStall = 1 << 24;
 
 // Islands that one warp does not take, all of them in one cooperative launch (a waiting item needs
 // the items it waits for to be resident).  Flow item j belongs to lane j mod `per` of warp j / per, with
