@@ -45,6 +45,11 @@ struct SceneData {
     int n_bodies() const { return (int)body_shape.size(); }
 };
 
+// does the range of `size` bytes from `start` on hold `bytes` bytes from p on
+inline bool range_holds(unsigned long long start, unsigned long long size, unsigned long long p, unsigned long long bytes) {
+    return p >= start && p - start <= size && bytes <= size - (p - start);
+}
+
 // unit-mass local inertia of the analytic shapes (box_shape.cpp:16-23, sphere_shape.cpp:7-11,
 // cylinder_shape.cpp:25-31)
 template <class R> M3<R> box_inertia(const V3<R>& size);

@@ -1,6 +1,7 @@
 // World<R> member definitions, part 3: transfers between the caller's arrays and the device
 // (body state, sweep axes, pairs, contact results).
 #pragma once
+#include <cuda.h>
 #include "pe_world_step.cuh"
 
 namespace pe {
@@ -22,17 +23,37 @@ template <class R> R* World<R>::staging(size_t n) {
     return stage_;
 }
 
+// The allocation or registration that a device address lies in; false where there is none.
+static bool pinned_range(const void* p, unsigned long long& start, size_t& size) {
+    using Query = CUresult(CUDAAPI*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Query>(f);
+    }();
+    const CUdeviceptr d = reinterpret_cast<CUdeviceptr>(p);
+    return query && query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) == CUDA_SUCCESS &&
+           query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) == CUDA_SUCCESS;
+}
+
 // The device's address of a caller's array of `bytes` bytes that kernels may use in place: page-locked
-// memory from end to end, aligned for its values.  nullptr: it goes through the staging buffer.
+// memory from end to end (one allocation or registration holds it all: between two lies memory that no
+// kernel may touch), aligned for its values.  nullptr: it goes through the staging buffer.
 static void* direct_address(const void* p, size_t bytes, size_t align) {
     if (bytes == 0 || bytes > kDirectBytes || reinterpret_cast<uintptr_t>(p) % align != 0) return nullptr;
-    cudaPointerAttributes at, end;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess || cudaPointerGetAttributes(&end, static_cast<const char*>(p) + bytes - 1) != cudaSuccess) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         (void)cudaGetLastError();
         return nullptr;
     }
-    if (at.type != cudaMemoryTypeHost || end.type != cudaMemoryTypeHost || !at.devicePointer || !end.devicePointer ||
-        static_cast<char*>(end.devicePointer) - static_cast<char*>(at.devicePointer) != (ptrdiff_t)(bytes - 1))
+    unsigned long long start = 0;
+    size_t size = 0;
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer || !pinned_range(at.devicePointer, start, size) ||
+        !range_holds(start, size, reinterpret_cast<unsigned long long>(at.devicePointer), bytes))
         return nullptr;
     return at.devicePointer;
 }
