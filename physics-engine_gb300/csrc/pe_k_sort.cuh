@@ -59,8 +59,7 @@ template <int BLOCK, class T> __device__ __forceinline__ T tiles_before(const T*
 // histograms into offsets, else the scatter's blocks add up the tiles before theirs themselves.  The
 // digit is the key's, or, with `scene` set, that of scene[value] (the more significant key of
 // bodies of several scenes).  The item count is n, or *nd when nd is set (a count the device computed:
-// the grid covers the upper bound n, and the tiles past the count do nothing; nothing at all is done
-// when the count is at most `small`, which another kernel sorts).
+// the grid covers the upper bound n, and the tiles past the count do nothing).
 //
 // A tile's items are ranked warp by warp: each warp counts its own 32 x ITEMS items in order, and the
 // block meets three times per tile (4,096 items in 16 rounds of six barriers took 35 us alone on an SM).
@@ -79,11 +78,11 @@ template <class K> struct RadixArgs {
     const int* scene;
     int n;
     const int* nd;
-    int small, shift;
+    int shift;
     int* hist;
     int tiles;
 };
-__global__ void k_radix_offsets(int* hist, int tiles, int tile_items, int n, const int* nd, int small);
+__global__ void k_radix_offsets(int* hist, int tiles, int tile_items, int n, const int* nd);
 
 template <class K> __device__ __forceinline__ int digit_of(const RadixArgs<K>& a, K key, uint32_t val) {
     return a.scene ? (a.scene[val] >> a.shift) & 0xff : (int)(key >> a.shift) & 0xff;
@@ -93,7 +92,7 @@ template <class K, int ITEMS> __global__ void __launch_bounds__(kBlock) k_radix_
     __shared__ int cnt[256];
     const int n = a.nd ? *a.nd : a.n;
     const int base = blockIdx.x * (kBlock * ITEMS);
-    if (n <= a.small || base >= n) return;
+    if (base >= n) return;
     cnt[threadIdx.x] = 0;
     __syncthreads();
 #pragma unroll
@@ -109,7 +108,7 @@ template <class K, int ITEMS> __global__ void __launch_bounds__(kBlock) k_radix_
     constexpr int W = kBlock / 32, TILE = kBlock * ITEMS;
     __shared__ int cnt[W][256];   // per warp and digit: items so far, then the first one's place
     const int n = a.nd ? *a.nd : a.n;
-    if (n <= a.small || (int)blockIdx.x * TILE >= n) return;
+    if ((int)blockIdx.x * TILE >= n) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d0 = threadIdx.x;
     const int first = blockIdx.x * TILE + warp * 32 * ITEMS + lane;
     K key[ITEMS];

@@ -201,7 +201,7 @@ extern "C" int pe_gpu_sap_pairs_noalloc(int device, int n, const float* aabb_min
     k_sap_keys<<<g, kBlock, 0, st>>>(n, aabb_min, axis, key[0], val[0], scene_axis);
     int cur = 0;
     for (int shift = 0; shift < 32; shift += 8, cur ^= 1) {   // as World::radix_pass
-        const RadixArgs<uint32_t> a{key[cur], val[cur], key[cur ^ 1], val[cur ^ 1], nullptr, n, nullptr, -1, shift, hist, radix_tiles(n)};
+        const RadixArgs<uint32_t> a{key[cur], val[cur], key[cur ^ 1], val[cur ^ 1], nullptr, n, nullptr, shift, hist, radix_tiles(n)};
         k_radix_hist<uint32_t, kRadixItems><<<a.tiles, kBlock, 0, st>>>(a);
         k_radix_scatter<uint32_t, kRadixItems><<<a.tiles, kBlock, 0, st>>>(a);
     }

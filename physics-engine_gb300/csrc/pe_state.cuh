@@ -122,6 +122,6 @@ struct Tuning {
 };
 
 // device status word bits
-enum StatusBits { ST_PAIR_OVERFLOW = 1, ST_ROW_OVERFLOW = 2, ST_COLOR_OVERFLOW = 4, ST_FLOW_STALL = 8 };
+enum StatusBits { ST_PAIR_OVERFLOW = 1, ST_FLOW_STALL = 8 };
 
 } // namespace pe

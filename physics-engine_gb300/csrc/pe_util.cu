@@ -1,5 +1,5 @@
 // Precision-independent device utilities: exclusive scan, stable LSD radix sort passes, pair bucketing,
-// contact islands, and the constant-memory unit meshes.
+// and contact islands.
 #include "pe_kernels.cuh"
 
 namespace pe {
@@ -45,9 +45,8 @@ __global__ void k_scan_apply(int* data, int n, const int* aux, int* total, int* 
 
 // ---------------------------------------------------------------- radix sort
 // one block per digit: its counts in the tiles become the counts of the tiles before, its total goes to the last row
-__global__ void __launch_bounds__(kBlock) k_radix_offsets(int* hist, int tiles, int tile_items, int n0, const int* nd, int small) {
+__global__ void __launch_bounds__(kBlock) k_radix_offsets(int* hist, int tiles, int tile_items, int n0, const int* nd) {
     const int n = nd ? *nd : n0, d = blockIdx.x;
-    if (n <= small) return;
     const int live = (n + tile_items - 1) / tile_items;
     int carry = 0;
     for (int t0 = 0; t0 < live; t0 += kBlock) {

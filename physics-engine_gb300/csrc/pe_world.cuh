@@ -53,11 +53,11 @@ template <class T> struct DBuf {   // device array that grows on demand
 
 // kernel groups for per-kernel device time (profiling mode)
 enum KernelId { K_INTEGRATE = 0, K_BP_KEYS, K_RADIX, K_SCAN, K_BP_GATHER, K_BP_SWEEP, K_BP_AXIS, K_NP_BUCKET, K_NP, K_NP_SAT,
-                K_SI_SETUP, K_ISLAND, K_SI_SERIAL, K_SI_COLOR, K_GC_COLOR, K_GC_SOLVE, K_SI_MISC, K_MISC, K_COUNT };
+                K_SI_SETUP, K_ISLAND, K_SI_SERIAL, K_SI_COLOR, K_MISC, K_COUNT };
 inline const char* kernel_name(int k) {
     static const char* n[K_COUNT] = {"integrate", "bp_keys", "radix_sort", "scan", "bp_gather", "bp_sweep", "bp_axis",
                                      "np_bucket", "narrowphase", "np_sat", "si_setup", "islands", "si_serial", "si_colored",
-                                     "big_island_color", "big_island_solve", "si_misc", "misc"};
+                                     "misc"};
     return k >= 0 && k < K_COUNT ? n[k] : "";
 }
 

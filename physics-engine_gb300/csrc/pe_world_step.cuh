@@ -23,7 +23,7 @@ template <class R> template <class K> void World<R>::radix_pass(RadixArgs<K>& a)
     a.hist = hist_.p;
     const bool big = radix_big(a.n);
     launch(K_RADIX, a.tiles, big ? k_radix_hist<K, kRadixItemsBig> : k_radix_hist<K, kRadixItems>, a);
-    if (a.tiles > kRadixFused) launch(K_RADIX, 256, k_radix_offsets, a.hist, a.tiles, radix_tile(a.n), a.n, a.nd, a.small);
+    if (a.tiles > kRadixFused) launch(K_RADIX, 256, k_radix_offsets, a.hist, a.tiles, radix_tile(a.n), a.n, a.nd);
     launch(K_RADIX, a.tiles, big ? k_radix_scatter<K, kRadixItemsBig> : k_radix_scatter<K, kRadixItems>, a);
     K* key = a.key_out;
     uint32_t* val = a.val_out;
@@ -85,7 +85,7 @@ template <class R> void World<R>::bp_count_enqueue() {
         using K = typename KeyOf<R>::type;
         K* key[2] = {reinterpret_cast<K*>(key_[0].p), reinterpret_cast<K*>(key_[1].p)};
         launch(K_BP_KEYS, grid(n), k_bp_keys<R>, bodies(), scene_axis_.p, key[0], val_[0].p);
-        RadixArgs<K> a{key[0], val_[0].p, key[1], val_[1].p, nullptr, n, nullptr, -1, 0, nullptr, 0};
+        RadixArgs<K> a{key[0], val_[0].p, key[1], val_[1].p, nullptr, n, nullptr, 0, nullptr, 0};
         hist_.ensure(radix_hist_ints(n));
         for (a.shift = 0; a.shift < (int)sizeof(K) * 8; a.shift += 8) radix_pass(a);
         a.scene = bscene_.p;
@@ -369,7 +369,7 @@ template <class R> void World<R>::solve_enqueue(int mode) {
         launch(K_ISLAND, pgrid(std::max(cap, N_), kActTile, k_act_sums), k_act_sums, a);
         launch(K_ISLAND, act_tiles(cap), k_act_apply, a);
         launch(K_ISLAND, pgrid(bound, kBlock, k_isl_keys), k_isl_keys, a);
-        RadixArgs<uint32_t> r{a.key[0], a.val[0], a.key[1], a.val[1], nullptr, bound, Md, -1, 0, nullptr, 0};
+        RadixArgs<uint32_t> r{a.key[0], a.val[0], a.key[1], a.val[1], nullptr, bound, Md, 0, nullptr, 0};
         for (int k = 0; k < label_passes; k++, r.shift += 8) radix_pass(r);
         order = r.val;
         launch(K_ISLAND, scan_tiles(bound), k_head_sums, a, r.key);
