@@ -447,6 +447,7 @@ template <class R> void World<R>::graph_sig(GraphSig& g) const {
     std::memcpy(&g.prm, &prm_, sizeof prm_);
     std::memcpy(&g.margin, &margin_, sizeof margin_);
     std::memcpy(&g.tun, &tun_, sizeof tun_);
+    g.tun.color_block = g.tun.level_block = 0;   // no kernel reads them
 }
 
 // Replays `ex` if its signature `held` matches `sig`, else captures `enqueue` into it (updating the

@@ -1,12 +1,11 @@
 """Autotuner of the step's scheduling settings (pe_gpu_tuning in include/pe_gpu.h).
 
-The settings decide which kernel takes which work and with how many threads: the estimated SAT work
-from which a pair gets a block of warps, the island sizes that run on one thread or grid-wide, the
-threads per island block, the largest scene sorted inside one block, the streams the narrowphase's
-classes are spread over.  In serial-order mode no setting changes a result bit; in coloured mode
-neither do these, as long as no island needs more levels than `exact_levels_colored` (a setting the
-tuner leaves alone, because it trades the reference's order for fewer colours).  The reference's
-counterpart is the fixed work split of its thread pool, batch = count / threads / 2 + 1
+The settings decide which kernel takes which work: the estimated SAT work from which a pair gets a
+block of warps, the island size from which coloured mode may run an island by first-fit colour, the
+largest scene sorted inside one block, the streams the narrowphase's classes are spread over.  In
+coloured mode `exact_levels_colored` trades the reference's order for fewer colours: the tuner leaves
+it alone, and `small_island_items`, which only decides which islands count their colours, and the two
+block sizes, which no kernel reads any more.  The reference's counterpart is the fixed work split of its thread pool, batch = count / threads / 2 + 1
 (src/utils/thread_pool.h:85-102).
 
 tune() times the candidates of each setting in turn (coordinate descent, the others at their best
@@ -28,15 +27,10 @@ TABLE_DIR = Path(__file__).resolve().parent / "tuning"
 CANDIDATES = {
     "sat_heavy_cost": [50000, 100000, 200000, 400000, 1000000, 2000000, 4000000, 8000000, 16000000],
     "side_streams": [1, 2, 4],
-    "small_island_items": [2, 4, 8, 16, 32],
-    "color_block": [32, 64, 128, 256],
-    "level_block": [64, 128, 256],
     "big_island_items": [1024, 4096, 16384],
     "scene_sort_max": [0, 2048],
 }
-NOISE = 0.005                     # run-to-run spread of the per-candidate timings (0.5 %)
-SERIAL_ONLY = {"level_block"}     # used by the serial-order solver only
-COLORED_ONLY = {"color_block"}    # used by the coloured solver only
+NOISE = 0.005   # run-to-run spread of the per-candidate timings (0.5 %)
 
 
 def table_path(gpu_name):
@@ -92,8 +86,6 @@ def tune(device=0, real_bits=32, mode=None, scenes=4096, steps=8, preroll=120, r
     base = _time_steps(g, snapshot, steps, mode, repeats)
     log(f"defaults: {base:.3f} ms/step")
     for name, values in CANDIDATES.items():
-        if (name in SERIAL_ONLY and mode != pg.SERIAL_ORDER) or (name in COLORED_ONLY and mode != pg.COLORED):
-            continue
         res = {}
         for v in values:
             try:
