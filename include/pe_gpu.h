@@ -126,9 +126,10 @@ int pe_gpu_set_params(pe_gpu_world* w, double dt, double gx, double gy, double g
  * :426-429).  Default 0; a margin >= 0 reproduces the reference compiled with that PE_MARGIN. */
 int pe_gpu_set_contact_margin(pe_gpu_world* w, double margin);
 
-/* Scheduling settings of the step: which kernel takes which work, with how many threads.  They
+/* Scheduling settings of the step: which kernel takes which work.  They
  * replace the reference's fixed work split of its thread pool (batch = count / threads / 2 + 1,
- * src/utils/thread_pool.h:85-102).  In serial-order mode no valid setting changes a result bit; in
+ * src/utils/thread_pool.h:85-102).  In serial-order mode no valid setting changes a result bit, but
+ * for sat_heavy_cost on rare pairs of a convex mesh (projections that fall over its first vertices); in
  * coloured mode none does while every island needs at most exact_levels_colored levels (above, a
  * big island is coloured first-fit).  pe_gb300.autotune picks them by timing a small batched case;
  * the defaults are those below. */

@@ -168,8 +168,8 @@ __device__ __forceinline__ int sweep_warp(int i, int n, int lane, const int* sce
 }
 
 // A position whose window along the axis holds more than big_window_limit candidates (a floor or a wall
-// spanning the scene) is swept by blocks instead of a warp: 256 candidates per iteration, warp
-// ballots plus a block prefix of the warp counts keep the pairs in ascending j.
+// spanning the scene) is swept by blocks instead of a warp, in chunks (below): 256 candidates at a
+// time, warp ballots plus a block prefix of the warp counts keep the pairs in ascending j.
 // The limit: what a warp sweeps in some 32 steps of four chunks, and at least an eighth of the largest
 // scene, so that only bodies that span the scene exceed it.  Where bodies lie so close that ordinary
 // windows hold thousands, nearly every position would go to the blocks, two searches and a chunk each

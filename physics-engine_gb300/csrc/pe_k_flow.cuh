@@ -146,7 +146,8 @@ k_isl_warp(const int* list, const int* n_list, int bound, const int* isl_off, co
     const unsigned full = 0xffffffffu;
     // Islands per warp: as many as its lanes hold, and fewer while there are warps to spare.  A warp takes
     // as long as its slowest lanes in every round, and its lanes' joints and rows of different length run
-    // one after the other (200 FP64 chains, four islands a warp before and one now: 921 / 857 us).
+    // one after the other (200 FP64 chains, four islands a warp before and one now, in turn on one GPU:
+    // 921 / 857 us; 835 to 1,050 us from one GPU to another).
     int units[kWarpClasses], total = 0, spread = 0;
     for (int sp = 0; sp <= 5; sp++) {
         int sum = 0;

@@ -19,9 +19,9 @@
 namespace pe {
 namespace {
 
+// A warp sweeps every window here, of up to 16,383 candidates too (kNoBigWindow): the pairs are those that
+// the world's blocks give for its longest windows.
 constexpr int kSapMaxBodies = 16384;
-// no window of a scene this small can exceed the world's crowded-window threshold, so the warp
-// sweep alone gives the world's pairs (the block sweeps of crowded windows never have work here)
 constexpr size_t kAlign = 256;
 constexpr size_t al(size_t b) { return (b + kAlign - 1) / kAlign * kAlign; }
 constexpr int kSapTiles = kSapMaxBodies / (kBlock * kRadixItems);

@@ -30,9 +30,11 @@ public:
         r_ = real_bits / 8;
     }
 
-    // Device bytes a live scene is charged: body state (55 reals + ints), broadphase temporaries, and
-    // room for 6 pairs (result records with 8 contact slots of 18 reals and two distance pools) and
-    // 6 solver rows of 23 reals per body.
+    // Device bytes a live scene is charged, an estimate: body state (49 reals + ints), broadphase
+    // temporaries, 6 pairs (result records with 8 contact slots of 18 reals and two distance pools) and
+    // 6 solver rows of 24 reals per body.  The world allocates by pair slots, up to half as many again as
+    // it has pairs, with room for 8 rows and their hand-over in each (some 1.7 KB in FP32): about the charge
+    // at the 2 pairs a body that piles have, two to three times it at 6.
     double footprint(const SceneData& d) const {
         const double r = r_;
         const double per_body = NBF * r + 64 + 6 * (40 + kSlots * (NPF + 2) * r) + 6 * NRF * r;

@@ -106,10 +106,12 @@ struct StepParams {
     int iterations;
 };
 
-// Scheduling settings of the step: which kernel takes which work and with how many threads.  In
-// serial-order mode no setting changes a result bit.  In coloured mode none does either while every
-// island above big_island_items needs at most exact_levels_colored levels (one with more runs by
-// first-fit colour): the autotuner leaves that one setting alone.
+// Scheduling settings of the step: which kernel takes which work.  In serial-order mode no setting
+// changes a result bit, but for sat_heavy_cost on rare pairs of a hull that an axis with a falling run
+// decides (a warp keeps some of those axes out, a block of warps does not: see sat_staged's balls).  In
+// coloured mode none does either while every island above big_island_items needs at most
+// exact_levels_colored levels (one with more runs by first-fit colour): the autotuner leaves that one
+// setting alone.
 struct Tuning {
     int sat_heavy_cost = 200000;      // SAT pairs whose estimated work reaches this run on a block of warps
     int small_island_items = 8;       // islands up to this many items count no colours
